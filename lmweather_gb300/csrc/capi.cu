@@ -387,15 +387,7 @@ int lmw_plane_destroy(lmw_plane *p) {
   })
 
 int lmw_plane_set_params(lmw_plane *p, double gravity, double depth, double f0, double beta, double viscosity, double drag, int linear) {
-  return PLN({
-    p->e->p.gravity = gravity;
-    p->e->p.depth = depth;
-    p->e->p.f0 = f0;
-    p->e->p.beta = beta;
-    p->e->p.viscosity = viscosity;
-    p->e->p.drag = drag;
-    p->e->p.linear = linear != 0;
-  });
+  return PLN(p->e->set_params(gravity, depth, f0, beta, viscosity, drag, linear != 0));
 }
 int lmw_plane_reset(lmw_plane *p) { return PLN(p->e->reset()); }
 int lmw_plane_set_h(lmw_plane *p, const double *h, size_t n) {

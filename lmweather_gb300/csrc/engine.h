@@ -1,5 +1,6 @@
 // Engine objects behind the C ABI: device-resident state, one CUDA stream per object.
 #pragma once
+#include <limits>
 #include <memory>
 
 #include "lmw_internal.h"
@@ -15,6 +16,8 @@ struct PlaneConfig {
   bool linear = false;
 };
 
+struct PlaneDivisors;
+
 class PlaneEngine {
  public:
   explicit PlaneEngine(const PlaneConfig &c);
@@ -27,6 +30,7 @@ class PlaneEngine {
   double dx() const { return p.lx / p.nx; }
   double dy() const { return p.ly / p.ny; }
 
+  void set_params(double gravity, double depth, double f0, double beta, double viscosity, double drag, bool linear);
   void reset();
   void set_h(const double *g, size_t n);
   void set_u(const double *g, size_t n);
@@ -68,9 +72,13 @@ class PlaneEngine {
   HostBuf<Reduce> hred;
   HostBuf<double> stage;
   int nblk_red = 0;
-  cudaGraphExec_t graph = nullptr;
-  double graph_dt = 0;
-  int graph_steps = 0;
+  std::shared_ptr<const PlaneDivisors> div;  // the stencil's division parameters (fixed with the spacings)
+  static constexpr int GRAPH_STEPS = 16;
+  cudaGraphExec_t graph = nullptr;  // GRAPH_STEPS steps
+  DevBuf<double> coef;              // RK4 stage coefficients of step size coef_dt
+  double coef_dt = std::numeric_limits<double>::quiet_NaN();
+  void enqueue_stages(double dt, const double *cdev);
+  double stable_from(const Reduce &r, double safety) const;
   void reduce(Reduce &r);
   double read_scalars(int n, double *out);
   void row_harmonic(int kind, int m, int j, double shift, double *re, double *im);

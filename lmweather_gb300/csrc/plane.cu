@@ -1,15 +1,16 @@
 // Beta-plane C-grid shallow water on the GPU (FP64), the lmweather Plane model (cpp/plane.cpp).
 //
-// One fused kernel per RK4 stage: a CTA loads a (TY+2) x (TX+2) tile of h, u, v (periodic in x, rows
+// One fused kernel per RK4 stage: a CTA loads a (rows+2) x (TX+2) tile of h, u, v (periodic in x, rows
 // clamped at the walls) into shared memory, forms the Bernoulli function B and the absolute vorticity eta
 // for the tile plus its one-cell halo, evaluates du, dv, dh, and applies the RK4 stage update in the same
-// pass (stage input, accumulator and, at the last stage, the state). Every arithmetic expression follows
-// the reference's order of evaluation and this file is compiled with --fmad=false, so that the result is
-// bitwise identical to cpp/plane.cpp:59-158 built without FMA contraction.
+// pass (stage input, accumulator and, at the last stage, the state). Every value is the one the reference's
+// order of evaluation gives (plane_stage says where fewer operations give it) and this file is compiled with
+// --fmad=false, so that the result is bitwise identical to cpp/plane.cpp:59-158 built without FMA contraction.
 #include <cmath>
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "engine.h"
@@ -18,40 +19,93 @@
 namespace lmw {
 namespace {
 
-constexpr int TX = 32, TY = 8;
+constexpr int TX = 32;  // tile width: one warp per row of cells
 
 struct PlaneDev {
   int nx, ny, lin;
   double dxx, dyy, dxx2, dyy2, g, depth, f0, beta, visc, drag, ly, hly;  // hly = 0.5 ly (exact)
   double zh[4], zl[4];  // two-term reciprocals of dxx, dyy, dxx2, dyy2 (in that order), for div_fixed
-  int fastdiv;                      // every divisor and its reciprocal are normal numbers
+  FixedDiv2 fd[4];      // the same divisors for div_fixed2
+  int hasdrag, hasvisc; // drag, viscosity not zero (tested on the integer pipe)
+  int fastdiv;          // 2: all four divisors qualify for div_fixed2; 1: they and their reciprocals are normal numbers
 };
 
-// the stencil's divisions by the grid spacings: div_fixed when the host found the spacings normal, else IEEE
-__device__ __forceinline__ double div_by(const PlaneDev &p, double x, double y, int k) {
+// what div_fixed2 does not answer: div_fixed when the host found the spacings normal, else IEEE
+__device__ __noinline__ double div_general(double x, double y, double zh, double zl, int fastdiv) {
   int fast;
-  return p.fastdiv ? div_fixed(x, y, p.zh[k], p.zl[k], fast) : x / y;
+  return fastdiv ? div_fixed(x, y, zh, zl, fast) : x / y;
+}
+// the stencil's divisions by the grid spacings, K = 0..3: dxx, dyy, dxx2, dyy2
+template <int K> __device__ __forceinline__ double div_by(const PlaneDev &p, double x) {
+  int ok;
+  const double q = div_fixed2(x, p.fd[K], ok);
+  if (p.fastdiv == 2 && ok) return q;
+  return div_general(x, K == 0 ? p.dxx : K == 1 ? p.dyy : K == 2 ? p.dxx2 : p.dyy2, p.zh[K], p.zl[K], p.fastdiv);
 }
 
 __device__ __forceinline__ int wrapx(int i, int nx) { return ((i % nx) + nx) % nx; }
 
 // stage 0..3 with coefficients c = 0.5 dt, 0.5 dt, dt, dt/6 (cpp/plane.cpp:143-158)
-__global__ void __launch_bounds__(TX *TY) plane_stage(PlaneDev p, int stage, double c, const double *__restrict__ hi,
-                                                      const double *__restrict__ ui, const double *__restrict__ vi,
-                                                      double *h0, double *u0, double *v0, double *ah, double *au, double *av,
-                                                      double *ho, double *uo, double *vo) {
-  __shared__ double sh[TY + 2][TX + 2], su[TY + 2][TX + 2], sv[TY + 2][TX + 2];
-  __shared__ double sB[TY + 1][TX + 1], sE[TY + 1][TX + 1];
+//
+// Bound: the FP64 pipe (about 1.7 warp lanes per clock and SM; HBM and L2 are idle beside it), so what counts is the
+// number of FP64 instructions. The reference's values are kept bit for bit with fewer of them:
+//   - its factors 0.5, 0.25 and 2 are exact, so they are folded into the neighbouring operation (q vbar = 0.125 RN(s1 s2)
+//     inside the FMA that subtracts the pressure term; the Bernoulli function's 0.25; the flux's 0.5 in the continuity
+//     equation's step, whose accumulator holds k / -0.5; acc + 2 k as an FMA). Only where a product is subnormal
+//     (below 2^-1022) could the reference's extra rounding show;
+//   - squares, fluxes and B are formed once per point in shared memory, not once per neighbour;
+//   - divisions by the spacings take two operations (div_fixed2) where that is proven, not three;
+//   - drag U is left out for drag = 0.
+// That is 54 FP64 operations per cell and stage instead of 86 (nonlinear, inviscid).
+// A tile is TX x ty_n cells: the CTAs are dealt to the tile columns as evenly as they go, and a column's CTAs cut its
+// rows evenly. A tile's 3 TX ty_n updates (u, v, h: one role per warp) are dealt to the NT threads, so a tile of one row
+// still has three warps working at once. The base state and the accumulator of a thread's updates are loaded ahead of
+// the tile. plane_tiling picks the number of CTAs and the form.
+// EARLY: the next stage's CTAs launch while this one's wait for their predecessor (griddepcontrol), which takes the
+// launch out of the chain from stage to stage. They are placed where there is room, so every SM has to hold the same
+// number of CTAs: with some SMs idle they would pile up there (300 x 200 in 130 tiles: 36 us a stage, against 14 us
+// without the early launch). Otherwise the next stage's CTAs launch when the last wave has only its updates left.
+// Stage time before and now (us): 60 x 30 12.4 -> 3.8, 200 x 100 14.3 -> 5.3, 1024 x 512 118.9 -> 68.3 (its 54
+// operations a cell take 53 at 0.53e12 a second), 4000 x 2000 1678 -> 953.
+template <int TYMAX, int NT, bool EARLY>
+__global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int stage, double c, const double *coef, const double *hi,
+                                                             const double *ui, const double *vi, double *h0, double *u0, double *v0, double *ah,
+                                                             double *au, double *av, double *ho, double *uo, double *vo) {
+  constexpr int TY = TYMAX;
+  __shared__ double sh[TY + 2][TX + 2], su[TY + 2][TX + 2], sv[TY + 2][TX + 2], qu[TY + 2][TX + 2], qv[TY + 2][TX + 2];
+  __shared__ double sB[TY + 1][TX + 1], sE[TY + 1][TX + 1], sF[TY][TX + 1], sG[TY + 1][TX], sf[TY + 1];
+  constexpr int ITEMS = (3 * TY * TX + NT - 1) / NT;
   const int nx = p.nx, ny = p.ny;
-  const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
-  const int tid = threadIdx.y * TX + threadIdx.x;
-  // tile load: local (ly, lx) <-> global (j0 - 1 + ly, i0 - 1 + lx), periodic in x
-  for (int e = tid; e < (TY + 2) * (TX + 2); e += TX * TY) {
-    int ly = e / (TX + 2), lx = e % (TX + 2);
-    int jg = j0 - 1 + ly, ig = wrapx(i0 - 1 + lx, nx);
+  const int tiles_x = (nx + TX - 1) / TX, ctas = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
+  const int col = cta * tiles_x / ctas, first = (col * ctas + tiles_x - 1) / tiles_x, rows = ((col + 1) * ctas + tiles_x - 1) / tiles_x - first;
+  const int i0 = col * TX, j0 = (cta - first) * ny / rows, ty_n = (cta - first + 1) * ny / rows - j0, ncell = ty_n * TX;
+  const int tid = threadIdx.x;
+  if (coef != nullptr) c = coef[stage];  // written before the first of a chain of stages
+  if (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // the updates of this thread: role 0 u, 1 v, 2 h
+  double xv[ITEMS], kv[ITEMS];
+#pragma unroll
+  for (int k = 0; k < ITEMS; k++) {
+    const int e = tid + k * NT, role = e < ncell ? 0 : e < 2 * ncell ? 1 : e < 3 * ncell ? 2 : 3, w = e - role * ncell;
+    const int i = i0 + w % TX, j = j0 + w / TX;
+    xv[k] = kv[k] = 0;
+    if (role < 3 && i < nx && j < ny) {
+      const size_t o = static_cast<size_t>(j) * nx + i;
+      xv[k] = role == 0 ? u0[o] : role == 1 ? v0[o] : h0[o];
+      if (stage > 0) kv[k] = role == 0 ? au[o] : role == 1 ? av[o] : ah[o];
+    }
+  }
+  // tile load: local (ly, lx) <-> global (j0 - 1 + ly, i0 - 1 + lx), periodic in x; columns past nx are not used
+  for (int e = tid; e < (ty_n + 2) * (TX + 2); e += NT) {
+    const int ly = e / (TX + 2), lx = e % (TX + 2);
+    const int jg = j0 - 1 + ly;
+    int ig = i0 - 1 + lx;
+    ig = ig < 0 ? ig + nx : ig >= nx ? ig - nx : ig;
+    if (ig >= nx) ig = 0;
     double hv = 0, uv = 0, vv = 0;
     if (jg >= 0 && jg < ny) {
-      size_t o = static_cast<size_t>(jg) * nx + ig;
+      const size_t o = static_cast<size_t>(jg) * nx + ig;
       hv = hi[o];
       uv = ui[o];
     }
@@ -59,94 +113,154 @@ __global__ void __launch_bounds__(TX *TY) plane_stage(PlaneDev p, int stage, dou
     sh[ly][lx] = hv;
     su[ly][lx] = uv;
     sv[ly][lx] = vv;
+    if (!p.lin) {
+      qu[ly][lx] = uv * uv;
+      qv[ly][lx] = vv * vv;
+    }
+  }
+  // the Coriolis parameter of the corner rows
+  if (tid >= NT - ty_n - 1) {
+    const int ly = tid - (NT - ty_n - 1);
+    sf[ly] = p.f0 + p.beta * ((j0 + ly) * p.dyy - p.hly);
   }
   __syncthreads();
-  // Bernoulli B at cells (j0-1+ly, i0-1+lx) and absolute vorticity at corners (j0+ly, i0+lx), cpp/plane.cpp:70-92
-  for (int e = tid; e < (TY + 1) * (TX + 1); e += TX * TY) {
-    int ly = e / (TX + 1), lx = e % (TX + 1);
-    int jb = j0 - 1 + ly;
+  // Bernoulli B at cells (j0-1+ly, i0-1+lx), absolute vorticity at corners (j0+ly, i0+lx), cpp/plane.cpp:70-92, and twice
+  // the fluxes of the west faces (j0+ly, i0+lx) and south faces (j0+ly, i0+lx), cpp/plane.cpp:119-128 (the fluxes
+  // themselves in the linear model)
+  for (int e = tid; e < (ty_n + 1) * (TX + 1); e += NT) {
+    const int ly = e / (TX + 1), lx = e % (TX + 1);
+    if (i0 + lx > nx || j0 + ly > ny) continue;
+    const int jb = j0 - 1 + ly, je = j0 + ly;
     double b = 0;
-    if (jb >= 0 && jb < ny) {
-      double k = 0;
-      if (!p.lin) {
-        double ua = su[ly][lx], ub = su[ly][lx + 1], va = sv[ly][lx], vb = sv[ly + 1][lx];
-        k = 0.5 * (0.5 * (ua * ua + ub * ub) + 0.5 * (va * va + vb * vb));
-      }
-      b = p.g * sh[ly][lx] + k;
+    if (jb >= 0) {
+      b = p.g * sh[ly][lx];
+      if (!p.lin) b = __fma_rn(0.25, (qu[ly][lx] + qu[ly][lx + 1]) + (qv[ly][lx] + qv[ly + 1][lx]), b);
     }
     sB[ly][lx] = b;
-    int je = j0 + ly;
-    double eta = 0;
-    if (je <= ny) {
-      double f = p.f0 + p.beta * (je * p.dyy - p.hly);
-      double zeta = 0;
-      if (!p.lin) {
-        double dvdx = div_by(p, sv[ly + 1][lx + 1] - sv[ly + 1][lx], p.dxx, 0);
-        double uj = je < ny ? su[ly + 1][lx + 1] : su[ly][lx + 1];
-        double ujm = je > 0 ? su[ly][lx + 1] : su[ly + 1][lx + 1];
-        zeta = dvdx - div_by(p, uj - ujm, p.dyy, 1);
-      }
-      eta = f + zeta;
+    double zeta = 0;
+    if (!p.lin) {
+      const double dvdx = div_by<0>(p, sv[ly + 1][lx + 1] - sv[ly + 1][lx]);
+      const double uj = je < ny ? su[ly + 1][lx + 1] : su[ly][lx + 1];
+      const double ujm = je > 0 ? su[ly][lx + 1] : su[ly + 1][lx + 1];
+      zeta = dvdx - div_by<1>(p, uj - ujm);
     }
-    sE[ly][lx] = eta;
+    sE[ly][lx] = sf[ly] + zeta;
+    if (ly < ty_n) {
+      const double u = su[ly + 1][lx + 1];
+      sF[ly][lx] = p.lin ? p.depth * u : (sh[ly + 1][lx] + sh[ly + 1][lx + 1]) * u;
+    }
+    if (lx < TX) {
+      const double v = sv[ly + 1][lx + 1];
+      sG[ly][lx] = je == 0 || je == ny ? 0.0 : p.lin ? p.depth * v : (sh[ly][lx + 1] + sh[ly + 1][lx + 1]) * v;
+    }
   }
   __syncthreads();
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int i = i0 + tx, j = j0 + ty;
-  if (i >= nx || j >= ny) return;
-  const double U = su[ty + 1][tx + 1], V = sv[ty + 1][tx + 1], Hc = sh[ty + 1][tx + 1];
-  // du at the u point (i, j): cpp/plane.cpp:94-105
-  double du;
-  {
-    double q = 0.5 * (sE[ty][tx] + sE[ty + 1][tx]);
-    double vbar = 0.25 * (sv[ty + 1][tx] + sv[ty + 1][tx + 1] + sv[ty + 2][tx] + sv[ty + 2][tx + 1]);
-    double r = q * vbar - div_by(p, sB[ty + 1][tx + 1] - sB[ty + 1][tx], p.dxx, 0) - p.drag * U;
-    if (p.visc != 0) {
-      double uy1 = j + 1 < ny ? su[ty + 2][tx + 1] : U, uy0 = j > 0 ? su[ty][tx + 1] : U;
-      r += p.visc * (div_by(p, su[ty + 1][tx + 2] - 2 * U + su[ty + 1][tx], p.dxx2, 2) + div_by(p, uy1 - 2 * U + uy0, p.dyy2, 3));
-    }
-    du = r;
-  }
-  // dv at the v point (i, j), interior rows only: cpp/plane.cpp:106-117
-  double dv = 0;
-  if (j >= 1) {
-    double q = 0.5 * (sE[ty][tx] + sE[ty][tx + 1]);
-    double ubar = 0.25 * (su[ty][tx + 1] + su[ty][tx + 2] + su[ty + 1][tx + 1] + su[ty + 1][tx + 2]);
-    double r = -q * ubar - div_by(p, sB[ty + 1][tx + 1] - sB[ty][tx + 1], p.dyy, 1) - p.drag * V;
-    if (p.visc != 0) {
-      double vy1 = j + 1 < ny ? sv[ty + 2][tx + 1] : 0.0, vy0 = j - 1 > 0 ? sv[ty][tx + 1] : 0.0;
-      r += p.visc * (div_by(p, sv[ty + 1][tx + 2] - 2 * V + sv[ty + 1][tx], p.dxx2, 2) + div_by(p, vy1 - 2 * V + vy0, p.dyy2, 3));
-    }
-    dv = r;
-  }
-  // dh: continuity in flux form, cpp/plane.cpp:119-128
-  double dh;
-  {
-    double hw = p.lin ? p.depth : 0.5 * (sh[ty + 1][tx] + Hc);
-    double fe = (p.lin ? p.depth : 0.5 * (Hc + sh[ty + 1][tx + 2])) * su[ty + 1][tx + 2];
-    double fw = hw * U;
-    double fn = 0, fs = 0;
-    if (j + 1 < ny) fn = (p.lin ? p.depth : 0.5 * (Hc + sh[ty + 2][tx + 1])) * sv[ty + 2][tx + 1];
-    if (j > 0) fs = (p.lin ? p.depth : 0.5 * (sh[ty][tx + 1] + Hc)) * V;
-    dh = -(div_by(p, fe - fw, p.dxx, 0) + div_by(p, fn - fs, p.dyy, 1));
-  }
-  const size_t o = static_cast<size_t>(j) * nx + i;
-  // RK4 bookkeeping: cpp/plane.cpp:146-156 (acc = k1 + 2 k2 + 2 k3, state += dt/6 (acc + k4))
-  auto upd = [&](double k, double *x0, double *acc, double *out, size_t idx) {
-    if (stage == 0) {
-      out[idx] = x0[idx] + c * k;
-      acc[idx] = k;
-    } else if (stage < 3) {
-      out[idx] = x0[idx] + c * k;
-      acc[idx] = acc[idx] + 2 * k;
+  if (!EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const double ch = p.lin ? -c : -0.5 * c;  // dh = -0.5 (twice the flux divergence)
+#pragma unroll
+  for (int k = 0; k < ITEMS; k++) {
+    const int e = tid + k * NT, role = e < ncell ? 0 : e < 2 * ncell ? 1 : e < 3 * ncell ? 2 : 3, w = e - role * ncell;
+    const int tx = w % TX, ty = w / TX, i = i0 + tx, j = j0 + ty;
+    if (role >= 3 || i >= nx || j >= ny) continue;
+    double r;
+    if (role == 0) {
+      // du at the u point (i, j): cpp/plane.cpp:94-105
+      const double U = su[ty + 1][tx + 1];
+      const double s2 = sv[ty + 1][tx] + sv[ty + 1][tx + 1] + sv[ty + 2][tx] + sv[ty + 2][tx + 1];
+      r = __fma_rn(0.125, (sE[ty][tx] + sE[ty + 1][tx]) * s2, -div_by<0>(p, sB[ty + 1][tx + 1] - sB[ty + 1][tx]));
+      if (p.hasdrag) r = r - p.drag * U;
+      if (p.hasvisc) {
+        const double uy1 = j + 1 < ny ? su[ty + 2][tx + 1] : U, uy0 = j > 0 ? su[ty][tx + 1] : U;
+        r += p.visc * (div_by<2>(p, __fma_rn(-2.0, U, su[ty + 1][tx + 2]) + su[ty + 1][tx]) + div_by<3>(p, __fma_rn(-2.0, U, uy1) + uy0));
+      }
+    } else if (role == 1) {
+      // dv at the v point (i, j), interior rows only: cpp/plane.cpp:106-117
+      r = 0;
+      if (j >= 1) {
+        const double V = sv[ty + 1][tx + 1];
+        const double s2 = su[ty][tx + 1] + su[ty][tx + 2] + su[ty + 1][tx + 1] + su[ty + 1][tx + 2];
+        r = __fma_rn(-0.125, (sE[ty][tx] + sE[ty][tx + 1]) * s2, -div_by<1>(p, sB[ty + 1][tx + 1] - sB[ty][tx + 1]));
+        if (p.hasdrag) r = r - p.drag * V;
+        if (p.hasvisc) {
+          const double vy1 = j + 1 < ny ? sv[ty + 2][tx + 1] : 0.0, vy0 = j - 1 > 0 ? sv[ty][tx + 1] : 0.0;
+          r += p.visc * (div_by<2>(p, __fma_rn(-2.0, V, sv[ty + 1][tx + 2]) + sv[ty + 1][tx]) + div_by<3>(p, __fma_rn(-2.0, V, vy1) + vy0));
+        }
+      }
     } else {
-      x0[idx] = x0[idx] + c * (acc[idx] + k);
+      r = div_by<0>(p, sF[ty][tx + 1] - sF[ty][tx]) + div_by<1>(p, sG[ty + 1][tx] - sG[ty][tx]);
     }
+    // RK4 bookkeeping: cpp/plane.cpp:146-156 (acc = k1 + 2 k2 + 2 k3, state += dt/6 (acc + k4)); for h, r = k / -0.5
+    // (linear: -k), which its accumulator keeps and its coefficient takes up
+    const double cc = role == 2 ? ch : c;
+    const size_t o = static_cast<size_t>(j) * nx + i;
+    double *out = role == 0 ? uo : role == 1 ? vo : ho, *acc = role == 0 ? au : role == 1 ? av : ah;
+    if (stage < 3) {
+      out[o] = xv[k] + cc * r;
+      acc[o] = stage == 0 ? r : __fma_rn(2.0, r, kv[k]);
+      if (role == 1 && j == ny - 1) vo[o + nx] = v0[o + nx];  // the northern wall row ny does not move
+    } else {
+      (role == 0 ? u0 : role == 1 ? v0 : h0)[o] = xv[k] + cc * (kv[k] + r);
+    }
+  }
+}
+
+// How a grid is cut. FORM 0: at most one one-row tile per SM; 1, 2: one or two CTAs on every SM, tiles of up to sixteen
+// rows; 3: more. 0 to 2 launch early. In 3 the rows of a tile are the number up to sixteen that leaves the fullest SM
+// the least to do, counting the FP64 instructions per warp of a tile: 2 for each loaded point, 17 for each corner, 33
+// for each cell (sixteen rows lose 4 % to the halo, eight 7 %). Measured, us a stage: 200 x 100 in form 1 5.2, 2 7.0,
+// 3 8.5; 400 x 200 (too tall for form 1) in 2 13.8, 3 15.1.
+constexpr int PLANE_SMS = 152, PLANE_TY = 16;
+struct Tiling {
+  int form, ctas, ty;  // ty: rows of the tallest tile
+};
+Tiling plane_tiling(int nx, int ny) {
+  const int tx = (nx + TX - 1) / TX;
+  if (tx * ny <= PLANE_SMS) return {0, tx * ny, 1};
+  for (int per_sm = 1; per_sm <= 2; per_sm++) {
+    const int least = per_sm * PLANE_SMS / tx;  // CTAs of the column with the fewest
+    if (least > 0 && (ny + least - 1) / least <= PLANE_TY && (per_sm * PLANE_SMS + tx - 1) / tx <= ny)
+      return {per_sm, per_sm * PLANE_SMS, (ny + least - 1) / least};
+  }
+  Tiling best{3, 0, 0};
+  double bc = 1e300;
+  for (int rows = (ny + PLANE_TY - 1) / PLANE_TY; rows <= (ny + 7) / 8; rows++) {
+    const int ty = (ny + rows - 1) / rows, load = ((ty + 2) * (TX + 2) + 31) / 32, corner = ((ty + 1) * (TX + 1) + 31) / 32;
+    const double cost = static_cast<double>((tx * rows + PLANE_SMS - 1) / PLANE_SMS) * (2 * load + 17 * corner + 33 * ty);
+    if (cost < bc) {
+      bc = cost;
+      best = {3, tx * rows, ty};
+    }
+  }
+  return best;
+}
+
+template <int TY, int NT, bool EARLY, class... A> void plane_launch(const PlaneDev &p, int ctas, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(NT);
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  LMW_CUDA(cudaLaunchKernelEx(&cfg, plane_stage<TY, NT, EARLY>, p, args...));
+}
+// one RK4 stage with coefficient coef[stage] (device memory; null: c): state (h0, u0, v0), stage input (hi, ui, vi), accumulator, next stage input
+void stage_launch(const PlaneDev &p, cudaStream_t s, int stage, double c, const double *coef, const double *hi, const double *ui, const double *vi, double *h0,
+                  double *u0, double *v0, double *ah, double *au, double *av, double *ho, double *uo, double *vo) {
+  const Tiling t = plane_tiling(p.nx, p.ny);
+  auto run = [&](auto ty, auto nt, auto early) {
+    plane_launch<decltype(ty)::value, decltype(nt)::value, decltype(early)::value>(p, t.ctas, s, stage, c, coef, hi, ui, vi, h0, u0, v0, ah, au, av, ho, uo,
+                                                                                   vo);
   };
-  upd(dh, h0, ah, ho, o);
-  upd(du, u0, au, uo, o);
-  upd(dv, v0, av, vo, o);  // rows 0 (wall) .. ny-1; dv = 0 on the wall
-  if (j == ny - 1) upd(0.0, v0, av, vo, o + nx);  // the northern wall row ny
+  using std::integral_constant;
+  const integral_constant<int, PLANE_TY> tall;
+  if (t.form == 0) run(integral_constant<int, 1>(), integral_constant<int, 128>(), std::true_type());
+  // one CTA per SM: sixteen warps (97 x 160: 5.2 us a stage against 7.2 with eight; 100 x 64: 4.0 against 4.2)
+  else if (t.form == 1) run(tall, integral_constant<int, 512>(), std::true_type());
+  else if (t.form == 2) run(tall, integral_constant<int, 256>(), std::true_type());
+  else run(tall, integral_constant<int, 256>(), std::false_type());
 }
 
 // ---------------------------------------------------------------- reductions (guards and diagnostics)
@@ -291,7 +405,20 @@ __global__ void plane_harmonic_energy_sum(const double2 *__restrict__ c, int row
   out[0] = s / ny;
 }
 
-PlaneDev make_dev(const PlaneConfig &c) {
+// the divisors of the stencil: dx, dy and their squares
+struct Divisors {
+  FixedDiv2 fd[4];
+  bool proven = true;
+};
+Divisors make_divisors(const PlaneConfig &c) {
+  const double dx = c.lx / c.nx, dy = c.ly / c.ny, dv[4] = {dx, dy, dx * dx, dy * dy};
+  Divisors d;
+  for (int k = 0; k < 4; k++)
+    if (!fixed_div2_setup(dv[k], d.fd[k])) d.proven = false;
+  return d;
+}
+
+PlaneDev make_dev(const PlaneConfig &c, const Divisors &div) {
   PlaneDev d;
   d.nx = c.nx;
   d.ny = c.ny;
@@ -308,10 +435,15 @@ PlaneDev make_dev(const PlaneConfig &c) {
   d.drag = c.drag;
   d.ly = c.ly;
   d.hly = 0.5 * c.ly;
+  d.hasdrag = c.drag != 0 ? 1 : 0;
+  d.hasvisc = c.viscosity != 0 ? 1 : 0;
   const double dv[4] = {d.dxx, d.dyy, d.dxx2, d.dyy2};
   d.fastdiv = 1;
-  for (int k = 0; k < 4; k++)
+  for (int k = 0; k < 4; k++) {
     if (!fixed_div_reciprocal(dv[k], d.zh[k], d.zl[k])) d.fastdiv = 0;
+    d.fd[k] = div.fd[k];
+  }
+  if (d.fastdiv && div.proven) d.fastdiv = 2;
   return d;
 }
 
@@ -357,6 +489,8 @@ __global__ void division_selftest(const unsigned long long *__restrict__ xb, int
 }
 
 }  // namespace
+
+struct PlaneDivisors : Divisors {};
 
 void division_selftest_run(const uint64_t *x, int nx, const double *y, int ny, long long *counts) {
   if (nx < 0 || ny < 0 || nx > (1 << 26) || ny > 4096) throw InvalidArgument("counts out of range");
@@ -457,14 +591,13 @@ void plane_step_noalloc(const PlaneConfig &c, double *h, double *u, double *v, d
   double *ah = sc + 6 * kNoAllocFieldCap, *au = sc + 7 * kNoAllocFieldCap, *av = sc + 8 * kNoAllocFieldCap;
   // every stage-0 launch writes all of a and the accumulator before any later stage reads them: nothing in the
   // scratch has to start at zero
-  PlaneDev d = make_dev(c);
-  dim3 grid((c.nx + TX - 1) / TX, (c.ny + TY - 1) / TY), block(TX, TY);
+  PlaneDev d = make_dev(c, make_divisors(c));
   const double half = 0.5 * dt, c6 = dt / 6;
   for (int s = 0; s < steps; s++) {
-    plane_stage<<<grid, block, 0, stream>>>(d, 0, half, h, u, v, h, u, v, ah, au, av, ha, ua, va);
-    plane_stage<<<grid, block, 0, stream>>>(d, 1, half, ha, ua, va, h, u, v, ah, au, av, hb, ub, vb);
-    plane_stage<<<grid, block, 0, stream>>>(d, 2, dt, hb, ub, vb, h, u, v, ah, au, av, ha, ua, va);
-    plane_stage<<<grid, block, 0, stream>>>(d, 3, c6, ha, ua, va, h, u, v, ah, au, av, nullptr, nullptr, nullptr);
+    stage_launch(d, stream, 0, half, nullptr, h, u, v, h, u, v, ah, au, av, ha, ua, va);
+    stage_launch(d, stream, 1, half, nullptr, ha, ua, va, h, u, v, ah, au, av, hb, ub, vb);
+    stage_launch(d, stream, 2, dt, nullptr, hb, ub, vb, h, u, v, ah, au, av, ha, ua, va);
+    stage_launch(d, stream, 3, c6, nullptr, ha, ua, va, h, u, v, ah, au, av, nullptr, nullptr, nullptr);
     LMW_LAUNCH_CHECK();
     g_launches += 4;
   }
@@ -475,7 +608,9 @@ PlaneEngine::PlaneEngine(const PlaneConfig &c) : p(c) {
   if (c.nx < 4 || c.ny < 4 || c.nx > 4000 || c.ny > 4000 || static_cast<int64_t>(c.nx) * c.ny > 8000000)
     throw InvalidArgument("grid must be at least 4 x 4 and at most 8 million cells");
   if (!(c.lx > 0 && c.ly > 0)) throw InvalidArgument("domain sizes must be positive");
+  div = std::make_shared<const PlaneDivisors>(PlaneDivisors{make_divisors(c)});
   LMW_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  coef.alloc(4);
   for (DevBuf<double> *b : {&h0, &u0, &ha, &ua, &hb, &ub, &ah, &au}) b->alloc(ncell());
   for (DevBuf<double> *b : {&v0, &va, &vb, &av}) b->alloc(nvpt());
   nblk_red = 2 * 152;
@@ -621,51 +756,67 @@ void PlaneEngine::jet(double u0v, double width, double noise_rms, uint64_t seed)
   t = 0;
 }
 
-void PlaneEngine::enqueue_step(double dt) {
-  PlaneDev d = make_dev(p);
-  dim3 grid((p.nx + TX - 1) / TX, (p.ny + TY - 1) / TY), block(TX, TY);
+// One RK4 step. cdev: the stage coefficients in device memory (the captured graph, which serves every step size), or
+// null: those of dt by value
+void PlaneEngine::enqueue_stages(double dt, const double *cdev) {
+  const PlaneDev d = make_dev(p, *div);
   const double half = 0.5 * dt, c6 = dt / 6;
   // stage inputs: x0 -> a -> b -> a
-  plane_stage<<<grid, block, 0, stream>>>(d, 0, half, h0.p, u0.p, v0.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, ha.p, ua.p, va.p);
-  plane_stage<<<grid, block, 0, stream>>>(d, 1, half, ha.p, ua.p, va.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, hb.p, ub.p, vb.p);
-  plane_stage<<<grid, block, 0, stream>>>(d, 2, dt, hb.p, ub.p, vb.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, ha.p, ua.p, va.p);
-  plane_stage<<<grid, block, 0, stream>>>(d, 3, c6, ha.p, ua.p, va.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, nullptr, nullptr, nullptr);
-  LMW_LAUNCH_CHECK();
+  stage_launch(d, stream, 0, half, cdev, h0.p, u0.p, v0.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, ha.p, ua.p, va.p);
+  stage_launch(d, stream, 1, half, cdev, ha.p, ua.p, va.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, hb.p, ub.p, vb.p);
+  stage_launch(d, stream, 2, dt, cdev, hb.p, ub.p, vb.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, ha.p, ua.p, va.p);
+  stage_launch(d, stream, 3, c6, cdev, ha.p, ua.p, va.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, nullptr, nullptr, nullptr);
   g_launches += 4;
 }
 
-// a chunk of RK4 steps as one CUDA graph (captured once per step size and chunk length)
+void PlaneEngine::enqueue_step(double dt) { enqueue_stages(dt, nullptr); }
+
+void PlaneEngine::set_params(double gravity, double depth, double f0, double beta, double viscosity, double drag, bool linear) {
+  p.gravity = gravity;
+  p.depth = depth;
+  p.f0 = f0;
+  p.beta = beta;
+  p.viscosity = viscosity;
+  p.drag = drag;
+  p.linear = linear;
+  if (graph) cudaGraphExecDestroy(graph);  // it holds the parameters it was captured with
+  graph = nullptr;
+}
+
+// `steps` RK4 steps: graphs of GRAPH_STEPS steps (captured once per set of parameters), the rest launched singly
 void PlaneEngine::launch_chunk(double dt, int steps) {
-  if (steps <= 0) return;
-  if (!graph || graph_dt != dt || graph_steps != steps) {
-    if (graph) cudaGraphExecDestroy(graph);
-    graph = nullptr;
-    cudaGraph_t g;
-    uint64_t before = g_launches;
-    LMW_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    for (int s = 0; s < steps; s++) enqueue_step(dt);
-    LMW_CUDA(cudaStreamEndCapture(stream, &g));
-    g_launches = before;
-    LMW_CUDA(cudaGraphInstantiate(&graph, g, 0));
-    cudaGraphDestroy(g);
-    graph_dt = dt;
-    graph_steps = steps;
+  if (steps >= GRAPH_STEPS && coef_dt != dt) {
+    const double c[4] = {0.5 * dt, 0.5 * dt, dt, dt / 6};
+    LMW_CUDA(cudaMemcpyAsync(coef.p, c, sizeof c, cudaMemcpyHostToDevice, stream));  // pageable: staged before it returns
+    coef_dt = dt;
   }
-  LMW_CUDA(cudaGraphLaunch(graph, stream));
-  g_launches += 4ull * steps;
+  for (; steps >= GRAPH_STEPS; steps -= GRAPH_STEPS) {
+    if (!graph) {
+      cudaGraph_t g;
+      const uint64_t before = g_launches;
+      LMW_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+      for (int s = 0; s < GRAPH_STEPS; s++) enqueue_stages(0.0, coef.p);
+      LMW_CUDA(cudaStreamEndCapture(stream, &g));
+      g_launches = before;
+      LMW_CUDA(cudaGraphInstantiate(&graph, g, 0));
+      cudaGraphDestroy(g);
+    }
+    LMW_CUDA(cudaGraphLaunch(graph, stream));
+    g_launches += 4ull * GRAPH_STEPS;
+  }
+  for (int s = 0; s < steps; s++) enqueue_stages(dt, nullptr);
 }
 
 double PlaneEngine::kernel_time(double dt, int reps) {
-  PlaneDev d = make_dev(p);
-  dim3 grid((p.nx + TX - 1) / TX, (p.ny + TY - 1) / TY), block(TX, TY);
+  PlaneDev d = make_dev(p, *div);
   cudaEvent_t e0, e1;
   LMW_CUDA(cudaEventCreate(&e0));
   LMW_CUDA(cudaEventCreate(&e1));
   // stage 1 reads the base state and stage input a, writes stage input b and the accumulator: x0 is untouched
-  plane_stage<<<grid, block, 0, stream>>>(d, 1, 0.5 * dt, ha.p, ua.p, va.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, hb.p, ub.p, vb.p);
+  stage_launch(d, stream, 1, 0.5 * dt, nullptr, ha.p, ua.p, va.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, hb.p, ub.p, vb.p);
   LMW_CUDA(cudaEventRecord(e0, stream));
   for (int r = 0; r < reps; r++)
-    plane_stage<<<grid, block, 0, stream>>>(d, 1, 0.5 * dt, ha.p, ua.p, va.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, hb.p, ub.p, vb.p);
+    stage_launch(d, stream, 1, 0.5 * dt, nullptr, ha.p, ua.p, va.p, h0.p, u0.p, v0.p, ah.p, au.p, av.p, hb.p, ub.p, vb.p);
   LMW_CUDA(cudaEventRecord(e1, stream));
   LMW_LAUNCH_CHECK();
   LMW_CUDA(cudaEventSynchronize(e1));
@@ -684,7 +835,7 @@ void PlaneEngine::step(double dt) {
 }
 
 void PlaneEngine::reduce(Reduce &r) {
-  PlaneDev d = make_dev(p);
+  PlaneDev d = make_dev(p, *div);
   plane_reduce<<<nblk_red, RED_THREADS, 0, stream>>>(d, h0.p, u0.p, v0.p, part.p);
   plane_reduce_final<<<1, 32, 0, stream>>>(part.p, nblk_red, dred.p);
   LMW_LAUNCH_CHECK();
@@ -696,10 +847,15 @@ void PlaneEngine::reduce(Reduce &r) {
 
 // cpp/plane.cpp:131-141
 double PlaneEngine::stable_dt(double safety) {
+  Reduce r;
+  if (!p.linear) reduce(r);
+  return stable_from(r, safety);
+}
+
+// the same from a reduction of the present state (the linear model needs none)
+double PlaneEngine::stable_from(const Reduce &r, double safety) const {
   double hmax = p.linear ? p.depth : 0, umax = 0;
   if (!p.linear) {
-    Reduce r;
-    reduce(r);
     umax = r.max[0];
     hmax = std::max(hmax, r.max[1]);
   }
@@ -714,8 +870,11 @@ double PlaneEngine::stable_dt(double safety) {
 void PlaneEngine::run(double seconds, double dt) {
   if (!(seconds >= 0)) throw InvalidArgument("run: seconds must not be negative");
   if (seconds == 0) return;
-  if (!(dt > 0)) dt = stable_dt(0.5);
-  const double limit = stable_dt(std::sqrt(0.5));
+  // one reduction gives the automatic step and the limit
+  Reduce r;
+  if (!p.linear) reduce(r);
+  if (!(dt > 0)) dt = stable_from(r, 0.5);
+  const double limit = stable_from(r, std::sqrt(0.5));
   if (!(dt <= limit))
     throw InvalidArgument("run: dt = " + fmt_f(dt) + " s exceeds the RK4 stability limit of about " + fmt_f(limit) +
                           " s for the present state: use a smaller dt");
@@ -728,15 +887,13 @@ void PlaneEngine::run(double seconds, double dt) {
     // steps up to and including the next guard point ((i & 63) == 63 or the last step)
     int64_t next = std::min<int64_t>(n - 1, i | 63);
     int chunk = static_cast<int>(next - i + 1);
-    if (chunk == 64) launch_chunk(hstep, 64);
-    else for (int s = 0; s < chunk; s++) enqueue_step(hstep);
+    launch_chunk(hstep, chunk);
     for (int s = 0; s < chunk; s++) t += hstep;
     i = next + 1;
-    Reduce r;
     reduce(r);
     double s = r.sum[0] + r.sum[1] + r.sum[2];
     if (!std::isfinite(s)) throw RuntimeError("the integration blew up (not finite): use a smaller dt");
-    const double now = stable_dt(std::sqrt(0.5));
+    const double now = stable_from(r, std::sqrt(0.5));
     if (!(hstep <= now))
       throw RuntimeError("run: dt = " + fmt_f(hstep) + " s exceeds the RK4 stability limit of about " + fmt_f(now) + " s reached at t = " +
                          fmt_f(t) + " s (the flow accelerated): use a smaller dt");
@@ -756,7 +913,7 @@ double PlaneEngine::read_scalars(int n, double *out) {
 double PlaneEngine::probe(int kind, double x, double y) {
   if (kind < 0 || kind > 2) throw InvalidArgument("field must be 0 (h), 1 (u) or 2 (v)");
   if (!std::isfinite(x) || !std::isfinite(y)) throw InvalidArgument("point outside the domain");
-  plane_point<<<1, 1, 0, stream>>>(make_dev(p), h0.p, u0.p, v0.p, kind, x, y, 0, 0, diag.p);
+  plane_point<<<1, 1, 0, stream>>>(make_dev(p, *div), h0.p, u0.p, v0.p, kind, x, y, 0, 0, diag.p);
   g_launches += 1;
   double r;
   return read_scalars(1, &r);
@@ -765,7 +922,7 @@ double PlaneEngine::probe(int kind, double x, double y) {
 // cpp/plane.cpp:220-226; corners i in 0..nx, j in 0..ny
 double PlaneEngine::zeta_at_corner(int i, int j) {
   if (i < 0 || i > p.nx || j < 0 || j > p.ny) throw InvalidArgument("corner outside the grid");
-  plane_point<<<1, 1, 0, stream>>>(make_dev(p), h0.p, u0.p, v0.p, 3, 0.0, 0.0, i, j, diag.p);
+  plane_point<<<1, 1, 0, stream>>>(make_dev(p, *div), h0.p, u0.p, v0.p, 3, 0.0, 0.0, i, j, diag.p);
   g_launches += 1;
   double r;
   return read_scalars(1, &r);
