@@ -104,6 +104,7 @@ struct SphereConfig {
 
 struct SphereTables;
 struct SplitPlan;
+struct Tc64Plan;
 
 class SphereEngine {
  public:
@@ -204,6 +205,8 @@ class SphereEngine {
  private:
   SphereTables *tab = nullptr;
   SplitPlan *split = nullptr;
+  Tc64Plan *tc64 = nullptr;  // FP64 Legendre sums on the tensor cores (truncations up to 170)
+  void check_tc64_status();
   bool split_packed = false;
   void check_split_status();
   void ensure_packed();
@@ -222,6 +225,7 @@ class SphereEngine {
   DevBuf<double> tq0, tqs, tqacc, fourq, foldq, refq, tgrid;  // tracer state, stage input, accumulator; transforms
   void ensure_tracer();
   void tracer_stage(int stage, double dt, int part);
+  void trc_syn_launch(const double2 *x, const double2 *q, double2 *dst, int count);
   std::vector<int> gflag_h;
   void upload_member_flags(int member);
   DevBuf<double> gridin;

@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(SYN_THREADS) sph_synth(SphDev d, SphTab<R> t, 
   const double2 *xz = x + static_cast<size_t>(b) * 3 * d.ntri, *xd = xz + d.ntri, *xf = xd + d.ntri;
   C2 sp = mk2(R(0), R(0)), sc = sp, hp = sp, hc = sp, zs = sp, fs = sp;
   const int base = d.tri[m];
+  pdl_wait();
   if (live) {
 #pragma unroll 2
     for (int n = m + c; n <= d.N; n += NCH) {
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(SYN_THREADS) sph_synth(SphDev d, SphTab<R> t, 
 #pragma unroll
   for (int i = 0; i < SYN_Q; i++) part[c][i][lane] = v[i];
   __syncthreads();
+  pdl_trigger();
   // even (n - m) pieces are those of even c, odd pieces those of odd c, each summed in the order of c
   R e[SYN_Q], o[SYN_Q];
   if constexpr (NCH <= 8) {
@@ -450,6 +452,7 @@ __global__ void __launch_bounds__(GRID_THREADS) sph_grid(SphDev d, SphTab<R> t, 
   C2 *sm = reinterpret_cast<C2 *>(smraw);
   const int b = blockIdx.y, jh = blockIdx.x;
   const int js = jh, jn = d.nlat - 1 - jh, n = d.nlon, rl = fft_row<3>(n);  // padded rows
+  pdl_wait();
   const C2 *f_s = four + (static_cast<size_t>(b) * d.nlat + js) * 4 * d.M;
   const C2 *f_n = four + (static_cast<size_t>(b) * d.nlat + jn) * 4 * d.M;
   load_pair_spectra<C2, 3>(sm, 4, d, f_s, f_n, d.M);
@@ -483,6 +486,7 @@ __global__ void __launch_bounds__(GRID_THREADS) sph_grid(SphDev d, SphTab<R> t, 
   }
   __syncthreads();
   fft_forward_dif<C2, 3>(sm, NSLOT, n, d.logn, t.tw);
+  pdl_trigger();
   // separate the two latitudes, normalise by nlon (cpp/sphere.cpp:128), weight and fold
   const R inv = R(1) / n, wd = t.wd[js], wj = t.w[js];
   C2 *o = fold + (static_cast<size_t>(b) * d.nh + jh) * NSLOT * 2 * d.M;
@@ -501,6 +505,152 @@ __global__ void __launch_bounds__(GRID_THREADS) sph_grid(SphDev d, SphTab<R> t, 
     o[(r * 2 + 0) * d.M + m] = cadd(Xs, Xn);
     o[(r * 2 + 1) * d.M + m] = csub(Xs, Xn);
   }
+}
+
+// ------------------------------------------------------------------------------------------------ FP64 grid stage
+// The work of sph_grid (below the FP32 engines' form) in FP64, where the pipe is narrow (about 1.7 lanes per clock and
+// SM) and one CTA per latitude pair left most SMs idle at low resolution: a cluster of five CTAs takes a latitude
+// pair, each one inverse transform (U, V, zeta, Phi) and, after reading the other fields' grid rows through
+// distributed shared memory, one of the five products and its forward transform.
+//
+// FFT of one row of n = 2^logn complex values, decimation in time from bit-reversed to natural order, in place: one
+// thread per butterfly and component, so that n threads share the chain. x = u + w v takes two FMAs per component and
+// y = u - w v = 2 u - x one, six FP64 operations per butterfly instead of eight; the first two stages, whose twiddles
+// are 1 and +-i, take four. Both components of a butterfly sit in neighbouring lanes of one warp, which reads all
+// their inputs before it writes. Twiddles exp(-2 pi i k / n), k < n/2, in shared memory.
+constexpr int G64_CTAS = 5;
+__host__ __device__ constexpr int g64_threads(int n) { return n < 32 ? 32 : n < 256 ? n : 256; }
+
+template <bool INV> __device__ __forceinline__ void fft64(double2 *s, int logn, const double2 *tw) {
+  const int n = 1 << logn;
+  for (int st = 0; st < logn; st++) {
+    const int h = 1 << st, mask = h - 1;
+    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+      const int p = e >> 1, c = e & 1, lo = p & mask, i0 = ((p >> st) << (st + 1)) + lo;
+      double *us = reinterpret_cast<double *>(s + i0) + c, *ys = reinterpret_cast<double *>(s + i0 + h) + c;
+      const double u = *us;
+      const double2 v = s[i0 + h];
+      double x, y;
+      if (st < 2) {
+        // w = 1, or for the odd butterflies of stage 1 +i (inverse) or -i: i v = (-v.y, v.x)
+        const double t = lo == 0 ? (c ? v.y : v.x) : (c ? v.x : v.y);
+        const double ts = lo != 0 && (c == 0) == INV ? -t : t;
+        x = u + ts;
+        y = u - ts;
+      } else {
+        // component c of w v (w conjugated for the inverse): w.x v.x - w.y v.y or w.x v.y + w.y v.x
+        const double2 w = tw[lo << (logn - 1 - st)];
+        const double a = c ? v.y : v.x, b = c ? v.x : v.y, wi = (c != 0) == INV ? -w.y : w.y;
+        x = fma(w.x, a, fma(wi, b, u));
+        y = fma(2.0, u, -x);
+      }
+      __syncwarp(n < 32 ? (1u << n) - 1u : 0xffffffffu);
+      *us = x;
+      *ys = y;
+    }
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// the shared-memory address `a` of this CTA in CTA `rank` of the cluster, and a complex value there
+__device__ __forceinline__ uint32_t cluster_map(const void *a, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(a))), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ double2 cluster_load(uint32_t base, int i) {
+  double2 v;
+  asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(base + static_cast<uint32_t>(i) * 16u) : "memory");
+  return v;
+}
+// bit-reversed spectrum of one field at a latitude pair (Y[m] = X_s[m] + i X_n[m], Y[n-m] = conj(X_s[m]) + i conj(X_n[m]);
+// Im X[0] dropped as in cpp/sphere.cpp:132) in the zeroed row s
+__device__ __forceinline__ void g64_load(double2 *s, const SphDev &d, const double2 *__restrict__ fs, const double2 *__restrict__ fn) {
+  for (int m = threadIdx.x; m < d.M; m += blockDim.x) {
+    const double2 a = fs[m], c = fn[m];
+    if (m == 0) {
+      s[0] = make_double2(a.x, c.x);
+    } else {
+      s[bitrev(m, d.logn)] = make_double2(a.x - c.y, a.y + c.x);
+      s[bitrev(d.nlon - m, d.logn)] = make_double2(a.x + c.y, c.x - a.y);
+    }
+  }
+}
+// the row's forward transform separated into its two latitudes, normalised by nlon (cpp/sphere.cpp:128), weighted and
+// folded: o[m] south + north, o[M + m] south - north
+__device__ __forceinline__ void g64_fold(const double2 *s, const SphDev &d, double wt, double2 *__restrict__ o) {
+  const int n = d.nlon;
+  const double w = wt * (0.5 / n);
+  for (int m = threadIdx.x; m < d.M; m += blockDim.x) {
+    const double2 y = s[m], z = s[(n - m) & (n - 1)];  // X_s = (y + conj z) / 2, X_n = -i (y - conj z) / 2
+    const double sx = y.x + z.x, dx = y.x - z.x, sy = y.y - z.y, dy = y.y + z.y;
+    o[m] = make_double2(w * (sx + dy), w * (sy - dx));
+    o[d.M + m] = make_double2(w * (sx - dy), w * (sy + dx));
+  }
+}
+
+// grid: (5 nh, B), clusters of five along x. T42, one member: 22.5 -> 8.8 us; T170: 64.5 -> 61.9 us; T42 x 16:
+// 57.4 -> 51.4 us
+__global__ void __launch_bounds__(256) sph_grid64(SphDev d, SphTab<double> t, const double2 *__restrict__ four, const double *__restrict__ fgrid,
+                                                  const double *__restrict__ hsgrid, double2 *__restrict__ fold) {
+  extern __shared__ double2 g64_sm[];
+  const int n = d.nlon;
+  double2 *inv = g64_sm, *fwd = g64_sm + n, *tw = g64_sm + 2 * n;
+  const int r = static_cast<int>(cluster_rank()), jh = blockIdx.x / G64_CTAS, b = blockIdx.y;
+  const int js = jh, jn = d.nlat - 1 - jh;
+  for (int e = threadIdx.x; e < n / 2; e += blockDim.x) tw[e] = t.tw[e];
+  if (r < 4)
+    for (int e = threadIdx.x; e < n; e += blockDim.x) inv[e] = make_double2(0.0, 0.0);
+  const int gf = d.gflag[b];
+  const double f0 = d.om2[b] * d.mu[js], r2om = t.r2om[js];  // 1 / (2 (1 - mu^2)); f0 and -f0 at the mirror latitudes
+  const double wt = r < 4 ? t.wd[js] : t.w[js];
+  __syncthreads();
+  pdl_wait();
+  if (r < 4) {
+    const double2 *f = four + static_cast<size_t>(b) * d.nlat * 4 * d.M + r * d.M;
+    g64_load(inv, d, f + static_cast<size_t>(js) * 4 * d.M, f + static_cast<size_t>(jn) * 4 * d.M);
+    __syncthreads();
+    fft64<true>(inv, d.logn, tw);
+  }
+  cluster_arrive();
+  cluster_wait();
+  // nonlinear products, cpp/sphere.cpp:348-359 (real part: southern latitude, imaginary part: northern): U eta, V eta,
+  // U Phi, V Phi, Phi + E, into bit-reversed order
+  const double *fr_s = fgrid + (static_cast<size_t>(b) * d.nlat + js) * n, *fr_n = fgrid + (static_cast<size_t>(b) * d.nlat + jn) * n;
+  const double *hr_s = hsgrid + (static_cast<size_t>(b) * d.nlat + js) * n, *hr_n = hsgrid + (static_cast<size_t>(b) * d.nlat + jn) * n;
+  const uint32_t aU = cluster_map(inv, 0), aV = cluster_map(inv, 1), aY = cluster_map(inv, r < 2 ? 2 : 3);
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    double2 y = cluster_load(aY, k), o;
+    if (r < 4) {
+      const double2 x = cluster_load((r & 1) ? aV : aU, k);
+      if (r < 2) {
+        y.x += (gf & 1) ? fr_s[k] : f0;
+        y.y += (gf & 1) ? fr_n[k] : -f0;
+      }
+      o = make_double2(x.x * y.x, x.y * y.y);
+    } else {
+      const double2 U = cluster_load(aU, k), V = cluster_load(aV, k);
+      if (gf & 2) {
+        y.x = fma(d.g, hr_s[k], y.x);
+        y.y = fma(d.g, hr_n[k], y.y);
+      }
+      o = make_double2(fma(fma(U.x, U.x, V.x * V.x), r2om, y.x), fma(fma(U.y, U.y, V.y * V.y), r2om, y.y));
+    }
+    fwd[bitrev(k, d.logn)] = o;
+  }
+  cluster_arrive();  // the other CTAs' rows are read
+  __syncthreads();
+  fft64<false>(fwd, d.logn, tw);
+  pdl_trigger();
+  g64_fold(fwd, d, wt, fold + ((static_cast<size_t>(b) * d.nh + jh) * NSLOT + r) * 2 * d.M);
+  cluster_wait();
 }
 
 // ------------------------------------------------------------------------------------------------ analysis + RK4
@@ -531,6 +681,7 @@ __global__ void __launch_bounds__(ANA_THREADS) sph_analysis(SphDev d, SphTab<R> 
   const C2 *fb = fold + static_cast<size_t>(b) * d.nh * NSLOT * 2 * d.M;
   const int sP = par * d.M + m, sH = (1 - par) * d.M + m;  // parity slot for P and H terms
   C2 aP = mk2(R(0), R(0)), bH = aP, bP = aP, aH = aP, uP = aP, vH = aP, eP = aP;
+  pdl_wait();
   if (live) {
 #pragma unroll 2
     for (int jh = c; jh < d.nh; jh += NCH) {
@@ -549,6 +700,7 @@ __global__ void __launch_bounds__(ANA_THREADS) sph_analysis(SphDev d, SphTab<R> 
 #pragma unroll
   for (int i = 0; i < ANA_Q; i++) part[c][i][lane] = v[i];
   __syncthreads();
+  pdl_trigger();
   R tsum[ANA_Q];
   if constexpr (NCH <= 8) {
     if (c != 0 || !live) return;
@@ -942,6 +1094,7 @@ double irwin_hall(uint64_t &st) {
 }  // namespace lmw
 
 #include "sphere_split.cuh"
+#include "sphere_tc64.cuh"
 #include "sphere_tracer.cuh"
 
 namespace lmw {
@@ -1068,7 +1221,6 @@ static void allow_max_shared_memory() {
   if (done_for_device == dev) return;
   LMW_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const int dyn = optin - 2048;  // the kernels' static shared memory stays below 2 KB
-  LMW_CUDA(cudaFuncSetAttribute(sph_grid<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(sph_grid<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(sph_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(sph_grid_in, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
@@ -1080,6 +1232,10 @@ static void allow_max_shared_memory() {
     LMW_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(split_syn_ws<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(split_syn_ws<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_syn<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_syn<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   for (int logn : {0, 6, 7, 8, 9, 10})
     for (int fmax : {3, 4})
       for (int direct : {0, 1}) LMW_CUDA(cudaFuncSetAttribute(split_grid_kernel(direct, fmax, logn), cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
@@ -1091,6 +1247,31 @@ static SphTab<double> tab64(const SphereTables &t) {
 }
 static SphTab<float> tab32(const SphereTables &t) {
   return SphTab<float>{t.Ps32.p, t.Hs32.p, t.Pa32.p, t.Ha32.p, t.w32.p, t.wd32.p, t.r2om32.p, t.kfac32.p, t.lapl32.p, t.tw32.p};
+}
+
+// launch of a stage kernel (one that calls pdl_wait) that may start while its predecessor drains, in clusters of
+// `cluster` CTAs along x
+template <class... P, class... A>
+static void stage_launch(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  LMW_CUDA(cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...));
+}
+
+// the FP64 synthesis of `count` members
+static void syn64_launch(const SphDev &d, const Tc64Dev &z, size_t smem, int count, const double2 *x, double2 *four, cudaStream_t stream) {
+  stage_launch(tc64_syn<4>, dim3(z.nsl * ((count + z.nbt - 1) / z.nbt), d.M), T64_THREADS, smem, stream, 1, d, z, x, static_cast<const double2 *>(nullptr), four, count);
 }
 
 SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
@@ -1228,6 +1409,10 @@ SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
     }
 
   }
+  if (p.precision == kFP64 && N <= 170) {
+    tc64 = new Tc64Plan();
+    build_tc64(*tc64, h, make_sph(*this, *tab), p.radius, B, stream);
+  }
   x0.zero(stream);
   xs.zero(stream);
   xs2.zero(stream);
@@ -1245,11 +1430,17 @@ SphereEngine::~SphereEngine() {
     cudaStreamSynchronize(stream);
     cudaStreamDestroy(stream);
   }
+  delete tc64;
   delete split;
   delete tab;
 }
 
-// the tensor-core kernels record a nonzero code when a bounded wait ran out
+// the tensor-core kernels record a nonzero code when a bounded wait ran out. FP64: in pinned host memory, to be read
+// after the stream was waited for
+void SphereEngine::check_tc64_status() {
+  if (tc64 && *reinterpret_cast<volatile int *>(tc64->err.p) != 0)
+    throw DeviceError("a wait on the tensor cores timed out in the FP64 Legendre transforms");
+}
 void SphereEngine::check_split_status() {
   if (!split) return;
   int e = 0;
@@ -1307,6 +1498,11 @@ void SphereEngine::synth_grids(int member_first, int count) {
   SphDev d = make_sph(*this, *tab);
   const size_t st = static_cast<size_t>(member_first) * 3 * ntri;
   const size_t fo = static_cast<size_t>(member_first) * nlat * 4 * M;
+  if (tc64) {
+    syn64_launch(d, tc64_dev(*tc64, ntri + M), tc64->smem_syn, count, reinterpret_cast<const double2 *>(x0.p) + st, reinterpret_cast<double2 *>(four.p) + fo, stream);
+    g_launches += 1;
+    return;
+  }
   const int L = syn_lats(nh);
   dim3 g((nh + L - 1) / L, M, count);
   auto *k = L == 8 ? sph_synth<double, 8> : sph_synth<double, 32>;
@@ -1612,28 +1808,37 @@ void SphereEngine::upload_filter(double dt) {
 
 // One RK4 stage in the engine's precision: FP64 tables and buffers, or FP32 (tendencies in FP32, the state in FP64)
 template <class R>
-static void stage_kernels(const SphDev &d, const SphTab<R> &t, int B, int stage, double dt, const double *filt, const double2 *in,
+static void stage_kernels(const SphDev &d, const SphTab<R> &t, const Tc64Plan *tc64, int B, int stage, double dt, const double *filt, const double2 *in,
                           typename V2<R>::type *four, typename V2<R>::type *fold, double2 *x0, double2 *xs, double2 *acc,
                           const double *fgrid, const double *hsgrid, cudaStream_t stream, int which = -1, int zero = 0) {
-  const size_t smem = 5 * static_cast<size_t>(fft_row<3>(d.nlon)) * sizeof(typename V2<R>::type);  // padded FFT rows
   StageArgs sa;
   sa.stage = stage;
   sa.c = stage < 2 ? 0.5 * dt : (stage == 2 ? dt : dt / 6);
   sa.filt = filt;
   sa.zero = zero;
+  const bool tc = sizeof(R) == 8 && tc64 != nullptr;
+  const Tc64Dev z = tc ? tc64_dev(*tc64, d.ntri + d.M) : Tc64Dev{};
   if (which < 0 || which == 0) {
-    if (syn_lats(d.nh) == 8)
-      sph_synth<R, 8><<<dim3((d.nh + 7) / 8, d.M, B), SYN_THREADS, 0, stream>>>(d, t, in, four);
-    else
-      sph_synth<R, 32><<<dim3((d.nh + 31) / 32, d.M, B), SYN_THREADS, 0, stream>>>(d, t, in, four);
+    const int L = syn_lats(d.nh);
+    if constexpr (sizeof(R) == 8) {
+      if (tc) syn64_launch(d, z, tc64->smem_syn, B, in, four, stream);
+    }
+    if (!tc) stage_launch(L == 8 ? sph_synth<R, 8> : sph_synth<R, 32>, dim3((d.nh + L - 1) / L, d.M, B), SYN_THREADS, 0, stream, 1, d, t, in, four);
   }
-  if (which < 0 || which == 1) sph_grid<R><<<dim3(d.nh, B), GRID_THREADS, smem, stream>>>(d, t, four, fgrid, hsgrid, fold);
-  if (which < 0 || which == 2)
-  {
-    if (ana_coef(d.nh) == 8)
-      sph_analysis<R, 8><<<dim3((d.ntri + 7) / 8, B), ANA_THREADS, 0, stream>>>(d, t, fold, sa, x0, xs, acc);
+  if (which < 0 || which == 1) {
+    if constexpr (sizeof(R) == 8)
+      stage_launch(sph_grid64, dim3(G64_CTAS * d.nh, B), g64_threads(d.nlon), static_cast<size_t>(d.nlon) * 5 / 2 * sizeof(double2), stream, G64_CTAS, d, t,
+                   four, fgrid, hsgrid, fold);
     else
-      sph_analysis<R, 32><<<dim3((d.ntri + 31) / 32, B), ANA_THREADS, 0, stream>>>(d, t, fold, sa, x0, xs, acc);
+      stage_launch(sph_grid<R>, dim3(d.nh, B), GRID_THREADS, 5 * static_cast<size_t>(fft_row<3>(d.nlon)) * sizeof(typename V2<R>::type), stream, 1, d, t,
+                   four, fgrid, hsgrid, fold);
+  }
+  if (which < 0 || which == 2) {
+    const int C = ana_coef(d.nh);
+    if constexpr (sizeof(R) == 8) {
+      if (tc) stage_launch(tc64_ana<5>, dim3(B, d.M), T64_THREADS, tc64->smem_ana, stream, 1, d, z, fold, sa, x0, xs, acc);
+    }
+    if (!tc) stage_launch(C == 8 ? sph_analysis<R, 8> : sph_analysis<R, 32>, dim3((d.ntri + C - 1) / C, B), ANA_THREADS, 0, stream, 1, d, t, fold, sa, x0, xs, acc);
   }
 }
 
@@ -1706,21 +1911,22 @@ void SphereEngine::launch_stage(int stage, double dt) {
   SphDev d = make_sph(*this, *tab);
   const double2 *in = reinterpret_cast<const double2 *>(stage == 0 ? x0.p : xs.p);
   double2 *X0 = reinterpret_cast<double2 *>(x0.p), *XS = reinterpret_cast<double2 *>(xs.p), *AC = reinterpret_cast<double2 *>(acc.p);
+  const Tc64Plan *tc = tc64;
   if (p.precision == kFP64 && has_tracer) {
     // the tracer's kernels read the flow's stage input and its synthesised winds before the flow's analysis
     // overwrites the stage input
     for (int k = 0; k < 3; k++) {
-      stage_kernels<double>(d, tab64(*tab), B, stage, dt, filt.p, in, reinterpret_cast<double2 *>(four.p), reinterpret_cast<double2 *>(fold.p),
+      stage_kernels<double>(d, tab64(*tab), tc, B, stage, dt, filt.p, in, reinterpret_cast<double2 *>(four.p), reinterpret_cast<double2 *>(fold.p),
                             X0, XS, AC, fgrid.p, hsgrid.p, stream, k, advect_only ? 1 : 0);
       tracer_stage(stage, dt, k);
     }
     g_launches += 6;
   } else if (p.precision == kFP64) {
-    stage_kernels<double>(d, tab64(*tab), B, stage, dt, filt.p, in, reinterpret_cast<double2 *>(four.p), reinterpret_cast<double2 *>(fold.p),
+    stage_kernels<double>(d, tab64(*tab), tc, B, stage, dt, filt.p, in, reinterpret_cast<double2 *>(four.p), reinterpret_cast<double2 *>(fold.p),
                           X0, XS, AC, fgrid.p, hsgrid.p, stream);
     g_launches += 3;
   } else if (p.precision == kFP32) {
-    stage_kernels<float>(d, tab32(*tab), B, stage, dt, filt.p, in, reinterpret_cast<float2 *>(four32.p), reinterpret_cast<float2 *>(fold32.p),
+    stage_kernels<float>(d, tab32(*tab), nullptr, B, stage, dt, filt.p, in, reinterpret_cast<float2 *>(four32.p), reinterpret_cast<float2 *>(fold32.p),
                          X0, XS, AC, fgrid.p, hsgrid.p, stream);
     g_launches += 3;
   } else {
@@ -1748,25 +1954,38 @@ void SphereEngine::ensure_tracer() {
   graphs_clear();
 }
 
+// Fourier coefficients of q and delta of `count` members
+void SphereEngine::trc_syn_launch(const double2 *x, const double2 *q, double2 *dst, int count) {
+  const SphDev d = make_sph(*this, *tab);
+  if (tc64) {
+    const Tc64Dev z = tc64_dev(*tc64, ntri + M);
+    stage_launch(tc64_syn<2>, dim3(z.nsl * ((count + z.nbt - 1) / z.nbt), M), T64_THREADS, tc64->smem_syn, stream, 1, d, z, x, q, dst, count);
+  } else {
+    stage_launch(trc_synth, dim3((nh + 31) / 32, M, count), SYN_THREADS, 0, stream, 1, d, tab64(*tab), x, q, dst);
+  }
+}
+
 // part 0: q and delta synthesis, 1: grid products, 2: analysis and RK4 update of q
 void SphereEngine::tracer_stage(int stage, double dt, int part) {
   SphDev d = make_sph(*this, *tab);
   const double2 *in = reinterpret_cast<const double2 *>(stage == 0 ? x0.p : xs.p);
   const double2 *qin = reinterpret_cast<const double2 *>(stage == 0 ? tq0.p : tqs.p);
   if (part == 0) {
-    trc_synth<<<dim3((nh + 31) / 32, M, B), SYN_THREADS, 0, stream>>>(d, tab64(*tab), in, qin, reinterpret_cast<double2 *>(fourq.p));
+    trc_syn_launch(in, qin, reinterpret_cast<double2 *>(fourq.p), B);
   } else if (part == 1) {
-    const size_t smem = 4 * static_cast<size_t>(fft_row<3>(nlon)) * sizeof(double2);
-    trc_grid<<<dim3(nh, B), GRID_THREADS, smem, stream>>>(d, tab64(*tab), reinterpret_cast<const double2 *>(four.p),
-                                                          reinterpret_cast<const double2 *>(fourq.p), reinterpret_cast<double2 *>(foldq.p));
+    stage_launch(trc_grid, dim3(TRC_CTAS * nh, B), g64_threads(nlon), static_cast<size_t>(nlon) * 5 / 2 * sizeof(double2), stream, TRC_CTAS, d, tab64(*tab),
+                 reinterpret_cast<const double2 *>(four.p), reinterpret_cast<const double2 *>(fourq.p), reinterpret_cast<double2 *>(foldq.p));
   } else {
     StageArgs sa;
     sa.stage = stage;
     sa.c = stage < 2 ? 0.5 * dt : (stage == 2 ? dt : dt / 6);
     sa.filt = filt.p;
-    trc_analysis<<<dim3((ntri + 31) / 32, B), ANA_THREADS, 0, stream>>>(d, tab64(*tab), reinterpret_cast<const double2 *>(foldq.p), sa,
-                                                                        reinterpret_cast<double2 *>(tq0.p), reinterpret_cast<double2 *>(tqs.p),
-                                                                        reinterpret_cast<double2 *>(tqacc.p));
+    if (tc64)
+      stage_launch(tc64_ana<3>, dim3(B, M), T64_THREADS, tc64->smem_ana, stream, 1, d, tc64_dev(*tc64, ntri + M), reinterpret_cast<const double2 *>(foldq.p), sa,
+                   reinterpret_cast<double2 *>(tq0.p), reinterpret_cast<double2 *>(tqs.p), reinterpret_cast<double2 *>(tqacc.p));
+    else
+      stage_launch(trc_analysis, dim3((ntri + 31) / 32, B), ANA_THREADS, 0, stream, 1, d, tab64(*tab), reinterpret_cast<const double2 *>(foldq.p), sa,
+                 reinterpret_cast<double2 *>(tq0.p), reinterpret_cast<double2 *>(tqs.p), reinterpret_cast<double2 *>(tqacc.p));
   }
   LMW_LAUNCH_CHECK();
 }
@@ -1831,9 +2050,8 @@ void SphereEngine::tracer_state(double *qr, int member) {
 void SphereEngine::synth_tracer_grid(int member, double *dst) {
   SphDev d = make_sph(*this, *tab);
   const size_t fo = static_cast<size_t>(member) * nlat * 2 * M;
-  trc_synth<<<dim3((nh + 31) / 32, M, 1), SYN_THREADS, 0, stream>>>(d, tab64(*tab), reinterpret_cast<const double2 *>(x0.p) + static_cast<size_t>(member) * 3 * ntri,
-                                                                  reinterpret_cast<const double2 *>(tq0.p) + static_cast<size_t>(member) * ntri,
-                                                                  reinterpret_cast<double2 *>(fourq.p) + fo);
+  trc_syn_launch(reinterpret_cast<const double2 *>(x0.p) + static_cast<size_t>(member) * 3 * ntri,
+                 reinterpret_cast<const double2 *>(tq0.p) + static_cast<size_t>(member) * ntri, reinterpret_cast<double2 *>(fourq.p) + fo, 1);
   trc_to_grid<<<dim3(nh, 1), GRID_THREADS, static_cast<size_t>(nlon) * sizeof(double2), stream>>>(d, reinterpret_cast<const double2 *>(fourq.p) + fo, dst);
   LMW_LAUNCH_CHECK();
   g_launches += 2;
@@ -1897,10 +2115,10 @@ void SphereEngine::kernel_times(double dt, int reps, double *out) {
   // stage 1 reads x0 and writes the stage input and the accumulator: x0 is unchanged
   auto one = [&](int which) {
     if (p.precision == kFP64)
-      stage_kernels<double>(d, tab64(*tab), B, 1, dt, filt.p, X0, reinterpret_cast<double2 *>(four.p), reinterpret_cast<double2 *>(fold.p), X0,
+      stage_kernels<double>(d, tab64(*tab), tc64, B, 1, dt, filt.p, X0, reinterpret_cast<double2 *>(four.p), reinterpret_cast<double2 *>(fold.p), X0,
                             XS, AC, fgrid.p, hsgrid.p, stream, which);
     else if (p.precision == kFP32)
-      stage_kernels<float>(d, tab32(*tab), B, 1, dt, filt.p, X0, reinterpret_cast<float2 *>(four32.p), reinterpret_cast<float2 *>(fold32.p),
+      stage_kernels<float>(d, tab32(*tab), nullptr, B, 1, dt, filt.p, X0, reinterpret_cast<float2 *>(four32.p), reinterpret_cast<float2 *>(fold32.p),
                            X0, XS, AC, fgrid.p, hsgrid.p, stream, which);
     else
       split_stage(d, tab32(*tab), *split, B, 1, dt, filt.p, reinterpret_cast<float2 *>(fold32.p), X0, XS, XS2(), AC, fgrid.p,
@@ -2240,6 +2458,7 @@ void SphereEngine::step(double dt) {
   enqueue_step(dt);
   for (int b = 0; b < B; b++) t[b] += dt;
   LMW_CUDA(cudaStreamSynchronize(stream));
+  check_tc64_status();
   check_split_status();
 }
 
@@ -2256,6 +2475,7 @@ void SphereEngine::reduce_guard(Reduce &r, int member) {
   g_launches += 2;
   LMW_CUDA(cudaMemcpyAsync(hred.p, dred.p, sizeof(Reduce), cudaMemcpyDeviceToHost, stream));
   LMW_CUDA(cudaStreamSynchronize(stream));
+  check_tc64_status();
   r = hred.p[0];
 }
 
@@ -2283,6 +2503,7 @@ void SphereEngine::reduce_guard_all(bool exact) {
   g_launches += 2;
   LMW_CUDA(cudaMemcpyAsync(hred.p, dred.p, B * sizeof(Reduce), cudaMemcpyDeviceToHost, stream));
   LMW_CUDA(cudaStreamSynchronize(stream));
+  check_tc64_status();
 }
 
 // RK4 limit of member b from its guard reduction (cpp/sphere.cpp:438-447)

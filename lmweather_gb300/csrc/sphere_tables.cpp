@@ -87,10 +87,12 @@ void HostTables::build(int truncation) {
   }
   P.assign(static_cast<size_t>(ntri) * nh, 0.0);
   H.assign(static_cast<size_t>(ntri) * nh, 0.0);
+  P1.assign(static_cast<size_t>(M) * nh, 0.0);
   std::vector<double> col;
   for (int jh = 0; jh < nh; jh++)
     for (int m = 0; m <= N; m++) {
       legendre_column(m, N, mu[jh], col);
+      P1[static_cast<size_t>(m) * nh + jh] = col[N + 1 - m];
       for (int n = m; n <= N; n++) {
         size_t q = static_cast<size_t>(tri[m] + n - m);
         double plus = col[n + 1 - m], minus = (n > m) ? col[n - 1 - m] : 0.0;

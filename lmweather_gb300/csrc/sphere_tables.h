@@ -26,6 +26,7 @@ struct HostTables {
   std::vector<int> tri;
   // southern-half tables (latitudes jh = 0 .. nh-1), coefficient-major [tri][jh]
   std::vector<double> P, H;
+  std::vector<double> P1;  // P of n = T+1, [m][jh]
   void build(int truncation);
   double Pj(int j, int m, int n) const;  // any latitude, through the hemispheric symmetry
   double Hj(int j, int m, int n) const;

@@ -1,0 +1,587 @@
+// FP64 Legendre sums on the tensor cores by exact slicing (included by sphere.cu), truncations up to 170.
+//
+// GB300's FP64 pipe does about 0.5e12 multiply-adds a second, its BF16 tensor cores a thousand times that. The sums of a
+// wavenumber m are therefore formed from integers (the scheme of K. Ozaki, T. Ogita, S. Oishi and S. M. Rump, "Error-free
+// transformations of matrix multiplication by using fast routines of matrix multiplication and its applications",
+// Numerical Algorithms 59, 2012): every operand row is scaled by a power of two to integers of at most 2^56 and cut into
+// eight digits of seven bits (d_0 up to 128, the others -64..63), which BF16 holds exactly. The products of two digits
+// summed over a row of at most 172 coefficients or 128 latitudes, for all digit pairs (i, j) of one order s = i + j, stay
+// below 2^23, so the FP32 accumulators of tcgen05 hold them exactly. The eight orders s = 0..7 are then added as 64-bit
+// integers and rounded once. What is left out, the digits below 2^-57 of a row's largest element and the orders from 8
+// on (2^-55 of the largest product), is below FP64's own rounding of such a sum, and the result depends neither on
+// the order of summation nor on how members are batched. Rows whose largest element is below 2^-900 count as zero; a row
+// with an infinity or NaN gives NaN.
+//
+// All orders of one table digit j come from one MMA: A holds digit i of its rows in row block i, under seven blocks of
+// zeros, and for table digit j the MMA starts j blocks higher, which puts digit i into row block i + j of the accumulator.
+//
+// Sums use P_n^m alone, n = m..T+1. With (1 - mu^2) dP_n/dmu = -n eps_{n+1} P_{n+1} + (n+1) eps_n P_{n-1}
+// (cpp/sphere.cpp:91-94) the derivative terms of cpp/sphere.cpp:192-202 become spectral coefficients of U and V, and
+// those of cpp/sphere.cpp:364-371 combinations of the sums at n - 1 and n + 1: four sums instead of six, five instead of
+// seven, and one table.
+//
+// tc64_syn   one CTA per (m, up to 64 latitude pairs, one or two members): U, V, zeta, Phi coefficients -> digits in shared
+//            memory (rows: four complex values per member) -> even and odd n - m in two accumulators -> Fourier
+//            coefficients of both mirror latitudes.
+// tc64_ana   one CTA per (m, member): folded grid values -> digits (rows: five complex values) -> sums of both
+//            parities -> tendencies, RK4 update, filter.
+// The table digits are streamed by bulk copies, sixteen K columns of all eight digits a stage, and start before the
+// kernel waits for its predecessor.
+#pragma once
+#include "tc_common.cuh"
+
+namespace lmw {
+
+struct Tc64Plan {
+  int nh16 = 16, lrows = 16, nsl = 1, nhk = 16, ns = 3;  // padded latitude pairs, per slice, slices; K of the analysis; stages
+  int nbt = 1, ntiles = 1;                               // members per synthesis tile
+  int kc_max = 1, ra_max = 16;
+  size_t smem_syn = 0, smem_ana = 0;
+  DevBuf<__nv_bfloat16> tS, tA;
+  DevBuf<int> ke16, kc, ra16;    // synthesis: padded even columns, K chunks of 16; analysis: padded rows of (m, parity)
+  DevBuf<long> oS, oA;           // table offsets (elements)
+  DevBuf<int> eS, eA;            // row exponents: [m][nh16], [tri + m + n - m] (n to T+1)
+  DevBuf<double> cf;             // per (m, n), n to T+1, five coefficients (see Tc64Dev)
+  HostBuf<int> err;              // written by the device when a bounded wait ran out
+};
+
+struct Tc64Dev {
+  int nh16, lrows, nsl, nhk, ns, nbt, ntiles, ra_max, ext;  // ext: coefficients with n to T+1
+  const __nv_bfloat16 *tS, *tA;
+  const int *ke16, *kc, *ra16, *eS, *eA;
+  const long *oS, *oA;
+  const double *cf;  // [5][ext]: a m / (n (n+1)), a eps_n / n, a eps_{n+1} / (n+1), n eps_{n+1}, (n+1) eps_n
+  int *err;
+};
+
+namespace {
+
+constexpr int T64_DIG = 8, T64_THREADS = 256;
+constexpr int T64_NONE = -100000, T64_NAN = 100000;  // row exponents: no digits; not finite
+// A operand: core matrices 144 bytes apart along K and 288 between 8-row groups (the 16 spare bytes put the stores of
+// neighbouring columns on different banks)
+constexpr int T64_LBO = 144, T64_SBO = 288;
+
+// biased exponent of |v| (0 for subnormals and zero)
+__device__ __forceinline__ int t64_exp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+// row exponent e (every |v| < 2^e) from the largest biased exponent
+__host__ __device__ __forceinline__ int t64_row(int ex) { return ex == 2047 ? T64_NAN : ex < 123 ? T64_NONE : ex - 1022; }
+// v 2^(56 - e) rounded to an integer, by integer operations (|v| < 2^e)
+__device__ __forceinline__ long long t64_fixed(double v, int e) {
+  const long long bits = __double_as_longlong(v);
+  const int ex = static_cast<int>((bits >> 52) & 0x7ff), s = 1022 + e - ex;  // right shift of the significand times 8
+  if (ex == 0 || s > 58 || e == T64_NONE || e == T64_NAN) return 0;
+  const long long m8 = ((bits & 0xfffffffffffffll) | 0x10000000000000ll) << 3;
+  const long long x = s > 0 ? (m8 + (1ll << (s - 1))) >> s : m8;
+  return bits < 0 ? -x : x;
+}
+// the eight digits of x, most significant first, as BF16 bits
+__device__ __forceinline__ void t64_digits(long long x, unsigned short *out) {
+#pragma unroll
+  for (int i = T64_DIG - 1; i >= 0; i--) {
+    const int lo = static_cast<int>(x);
+    const int dgt = i == 0 ? lo : ((lo + 64) & 127) - 64;
+    x = (x - dgt) >> 7;
+    out[i] = static_cast<unsigned short>(__float_as_uint(__int_as_float(0x4B400000 + dgt) - 12582912.0f) >> 16);
+  }
+}
+// sum of the eight orders D[s] (exact integers) times 2^(7 (7 - s)), as high and low parts of value hi 2^28 + lo
+struct T64Sum {
+  long long hi, lo;
+};
+__device__ __forceinline__ T64Sum t64_sum(const int *D, int stride) {
+  T64Sum r;
+  r.hi = ((static_cast<long long>(D[0]) << 21) + (static_cast<long long>(D[stride]) << 14)) + ((static_cast<long long>(D[2 * stride]) << 7) + D[3 * stride]);
+  r.lo = ((static_cast<long long>(D[4 * stride]) << 21) + (static_cast<long long>(D[5 * stride]) << 14)) + ((static_cast<long long>(D[6 * stride]) << 7) + D[7 * stride]);
+  return r;
+}
+// |x| < 2^51 as a double, exactly
+__device__ __forceinline__ double t64_int(long long x) { return __longlong_as_double(0x4338000000000000ll + x) - 6755399441055744.0; }
+__device__ __forceinline__ double t64_value(long long hi, long long lo) { return fma(t64_int(hi), 268435456.0, t64_int(lo)); }
+// 2^(e - 63 + f) as two factors (e of an operand row, f of a table row); zero rows give zero, rows that are not finite NaN
+__device__ __forceinline__ double t64_pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+__device__ __forceinline__ double t64_scale_a(int e) { return e == T64_NAN ? __longlong_as_double(0x7ff8000000000000ll) : e == T64_NONE ? 0.0 : t64_pow2(e - 63); }
+__device__ __forceinline__ double t64_scale_b(int e) { return e == T64_NONE ? 0.0 : t64_pow2(e); }
+
+__device__ __forceinline__ uint64_t t64_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  return static_cast<uint64_t>((saddr >> 4) & 0x3FFFu) | (static_cast<uint64_t>(lbo >> 4) << 16) | (static_cast<uint64_t>(sbo >> 4) << 32) |
+         (static_cast<uint64_t>(1) << 46);
+}
+
+// ------------------------------------------------------------------------------------------------ tables
+// P_n^m at latitude pair jh, n to T+1 (P1: the row n = T+1)
+__device__ __forceinline__ double t64_p(const SphDev &d, const double *P1, int m, int n, int jh) {
+  return n <= d.N ? d.Ps[static_cast<size_t>(d.tri[m] + n - m) * d.nh + jh] : P1[static_cast<size_t>(m) * d.nh + jh];
+}
+// digits of the synthesis table: [slice][chunk][digit][lrows][16] in core matrices, rows latitudes, columns even n - m then
+// odd; grid M, thread: latitude
+__global__ void tc64_build_syn(SphDev d, Tc64Dev z, const double *__restrict__ P1, __nv_bfloat16 *__restrict__ tS, int *__restrict__ eS) {
+  const int m = blockIdx.x, kc = z.kc[m], ke16 = z.ke16[m];
+  for (int jh = threadIdx.x; jh < z.nh16; jh += blockDim.x) {
+    int ex = 0;
+    for (int n = m; n <= d.N + 1 && jh < d.nh; n++) ex = max(ex, t64_exp(t64_p(d, P1, m, n, jh)));
+    const int e = t64_row(ex), sl = jh / z.lrows, r = jh % z.lrows;
+    eS[m * z.nh16 + jh] = e;
+    for (int k = 0; k < kc * 16; k++) {
+      const int n = k < ke16 ? m + 2 * k : m + 1 + 2 * (k - ke16);
+      unsigned short dg[T64_DIG];
+      t64_digits(jh < d.nh && n <= d.N + 1 ? t64_fixed(t64_p(d, P1, m, n, jh), e) : 0, dg);
+      unsigned short *o = reinterpret_cast<unsigned short *>(tS) + z.oS[m] + (static_cast<long>(sl) * kc + k / 16) * T64_DIG * z.lrows * 16;
+      for (int i = 0; i < T64_DIG; i++) o[(i * z.lrows + (r & ~7)) * 16 + ((k & 15) >> 3) * 64 + (r & 7) * 8 + (k & 7)] = dg[i];
+    }
+  }
+}
+// digits of the analysis table of (m, parity): [chunk][digit][ra16][16], rows n = m + parity + 2 r, columns latitudes; grid
+// (M, 2), one warp per row
+__global__ void tc64_build_ana(SphDev d, Tc64Dev z, const double *__restrict__ P1, __nv_bfloat16 *__restrict__ tA, int *__restrict__ eA) {
+  const int m = blockIdx.x, p = blockIdx.y, ra = z.ra16[2 * m + p], lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < ra; r += blockDim.x >> 5) {
+    const int n = m + p + 2 * r;
+    int ex = 0;
+    if (n <= d.N + 1)
+      for (int jh = lane; jh < d.nh; jh += 32) ex = max(ex, t64_exp(t64_p(d, P1, m, n, jh)));
+    ex = __reduce_max_sync(0xffffffffu, ex);
+    const int e = t64_row(ex);
+    if (lane == 0 && n <= d.N + 1) eA[d.tri[m] + m + n - m] = e;
+    for (int k = lane; k < z.nhk; k += 32) {
+      unsigned short dg[T64_DIG];
+      t64_digits(k < d.nh && n <= d.N + 1 ? t64_fixed(t64_p(d, P1, m, n, k), e) : 0, dg);
+      unsigned short *o = reinterpret_cast<unsigned short *>(tA) + z.oA[2 * m + p] + static_cast<long>(k / 16) * T64_DIG * ra * 16;
+      for (int i = 0; i < T64_DIG; i++) o[(i * ra + (r & ~7)) * 16 + ((k & 15) >> 3) * 64 + (r & 7) * 8 + (k & 7)] = dg[i];
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------ shared pieces
+struct T64Bars {
+  uint64_t full[4], empty[4], done;
+  uint32_t tslot;
+  int fail, issued, consumed;
+};
+// tensor memory (warp 0) and barriers
+__device__ __forceinline__ void t64_setup(T64Bars &b, int ns, uint32_t ncols) {
+  if (threadIdx.x < 32) tc::tmem_alloc(tc::su32(&b.tslot), ncols);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ns; s++) {
+      tc::bar_init(tc::su32(&b.full[s]), 1);
+      tc::bar_init(tc::su32(&b.empty[s]), 1);
+    }
+    tc::bar_init(tc::su32(&b.done), 1);
+    tc::bar_init_fence();
+    b.fail = b.issued = b.consumed = 0;
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+}
+__device__ __forceinline__ void t64_failed(T64Bars &b, int *err, int code) {
+  b.fail = 1;
+  *reinterpret_cast<volatile int *>(err) = code;
+  __threadfence_system();
+}
+// producer step: chunk it (bytes from src) into stage it % ns
+__device__ __forceinline__ bool t64_copy(T64Bars &b, uint8_t *stages, int stage_bytes, int ns, int it, const void *src, uint32_t bytes, int *err) {
+  const int st = it % ns;
+  if (it >= ns && !tc::wait(tc::su32(&b.empty[st]), ((it / ns) - 1) & 1)) {
+    t64_failed(b, err, 11);
+    return false;
+  }
+  tc::expect_tx(tc::su32(&b.full[st]), bytes);
+  tc::bulk_g2s(tc::su32(stages + static_cast<size_t>(st) * stage_bytes), src, bytes, tc::su32(&b.full[st]));
+  b.issued = it + 1;
+  return true;
+}
+// MMA step: the eight table digits of stage it % ns (rows: N) against the A block at `a` (its first real row group zg
+// groups further down, gpo groups per digit), accumulated at `acc`
+__device__ __forceinline__ bool t64_mma(T64Bars &b, uint8_t *stages, int stage_bytes, int ns, int it, int N, uint32_t a, int gpo, uint32_t acc, bool first,
+                                        int *err) {
+  const int st = it % ns;
+  if (!tc::wait(tc::su32(&b.full[st]), (it / ns) & 1)) {
+    t64_failed(b, err, 12);
+    return false;
+  }
+  b.consumed = it + 1;
+  tc::fence_after();
+  const uint32_t bb = tc::su32(stages + static_cast<size_t>(st) * stage_bytes), idesc = tc::idesc_m128(N);
+#pragma unroll
+  for (int j = 0; j < T64_DIG; j++)
+    tc::mma(acc, t64_desc(a + (7 - j) * gpo * T64_SBO, T64_LBO, T64_SBO), t64_desc(bb + j * N * 32, 128, 256), idesc, first && j == 0 ? 0u : 1u);
+  tc::commit(tc::su32(&b.empty[st]));
+  return true;
+}
+// after the roles have met: wait for every MMA; after a failure a bounded wait for what is in flight. True when all is well
+__device__ __forceinline__ bool t64_finish(T64Bars &b, int ns, int *err) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (!b.fail) {
+      if (!tc::wait(tc::su32(&b.done), 0)) t64_failed(b, err, 13);
+    } else {
+      tc::wait_for(tc::su32(&b.done), 0, 200000000ull);
+      for (int it = b.consumed; it < b.issued; it++) tc::wait_for(tc::su32(&b.full[it % ns]), (it / ns) & 1, 200000000ull);
+    }
+  }
+  __syncthreads();
+  tc::fence_after();
+  return b.fail == 0;
+}
+__device__ __forceinline__ void t64_teardown(T64Bars &b, uint32_t ncols) {
+  tc::fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32) tc::tmem_free(b.tslot, ncols);
+}
+// 32 (or the first w = 16) accumulator columns of this thread's row as integers into dst
+__device__ __forceinline__ void t64_unload(uint32_t taddr, int w, int *dst, bool keep) {
+  float v[32];
+  if (w > 16) {
+    tc::ld32(taddr, v);
+  } else {
+    tc::ld8(taddr, v);
+    tc::ld8(taddr + 8, v + 8);
+  }
+  if (!keep) return;
+#pragma unroll
+  for (int i = 0; i < 32; i++)
+    if (i < w) dst[i] = __float2int_rn(v[i]);
+}
+
+// ------------------------------------------------------------------------------------------------ synthesis
+// grid: (slices x tiles, M). F = 4: U, V, zeta, Phi of x [B][3][ntri] into four [B][nlat][4][M]; F = 2 (tracer): q of qin
+// [B][ntri] and delta of x into [B][nlat][2][M].
+// T170, one member: 82.0 -> 18.5 us (FP64 pipe before); T42 x 16: 50.4 -> 13.7; T42, one member: 10.3 -> 7.3.
+template <int F>
+__global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, const double2 *__restrict__ x, const double2 *__restrict__ qin,
+                                                           double2 *__restrict__ four, int B) {
+  extern __shared__ __align__(1024) uint8_t t64_sm[];
+  __shared__ __align__(8) T64Bars bars;
+  __shared__ int rowexp[2][F];
+  const int tid = threadIdx.x, m = blockIdx.y, sl = blockIdx.x % z.nsl, tile = blockIdx.x / z.nsl;
+  const int L = z.lrows, kc = z.kc[m], ke16 = z.ke16[m], nbt = z.nbt, mt = min(nbt, B - tile * nbt), groups = 15 * nbt;
+  const int stage_bytes = T64_DIG * L * 32, ablk = groups * T64_SBO;
+  uint8_t *stages = t64_sm;
+  uint8_t *A = t64_sm + max(z.ns * stage_bytes, static_cast<int>(2 * 64 * nbt * (min(L, 32) + 1) * sizeof(int)));
+  const uint32_t ncols = max(32, 2 * L);
+  t64_setup(bars, z.ns, ncols);
+  const __nv_bfloat16 *src = z.tS + z.oS[m] + static_cast<long>(sl) * kc * T64_DIG * L * 16;
+  int copied = 0;
+  if (tid == 0)
+    for (; copied < min(kc, z.ns); copied++) t64_copy(bars, stages, stage_bytes, z.ns, copied, src + static_cast<long>(copied) * T64_DIG * L * 16, stage_bytes, z.err);
+  // the zero blocks above the digits
+  for (int e = tid; e < kc * 7 * nbt * (T64_SBO / 16); e += T64_THREADS) {
+    const int blk = e / (7 * nbt * (T64_SBO / 16)), o = e % (7 * nbt * (T64_SBO / 16));
+    *reinterpret_cast<uint4 *>(A + blk * ablk + o * 16) = make_uint4(0, 0, 0, 0);
+  }
+  if (tid < 2 * F) rowexp[tid / F][tid % F] = 0;
+  __syncthreads();
+  pdl_wait();
+  // thread k: column k, n = m + 2 k or m + 1 + 2 (k - ke16); the values of member ml in v[0..2F)
+  const int k = tid, n = k < ke16 ? m + 2 * k : m + 1 + 2 * (k - ke16), base = d.tri[m] - m;
+  const bool col = k < kc * 16, live = col && n <= d.N + 1;
+  const double *cf = z.cf + d.tri[m] + n;  // ext index of (m, n): tri[m] + m + n - m
+  for (int ml = 0; ml < nbt; ml++) {
+    double v[2 * F];
+#pragma unroll
+    for (int q = 0; q < 2 * F; q++) v[q] = 0;
+    if (live && ml < mt) {
+      const int b = tile * nbt + ml;
+      const double2 *xz = x + static_cast<size_t>(b) * 3 * d.ntri + base, *xd = xz + d.ntri, *xf = xd + d.ntri;
+      const double2 zero = make_double2(0.0, 0.0);
+      const double2 dn = n <= d.N ? xd[n] : zero;
+      if constexpr (F == 4) {
+        // U_n = -a [i m delta_n / (n (n+1)) + eps_n zeta_{n-1} / n - eps_{n+1} zeta_{n+1} / (n+1)], V_n the same with zeta_n,
+        // -delta_{n-1}, -delta_{n+1}; the (0, 0) coefficients have no wind
+        const double w0 = cf[0], w1 = cf[z.ext], w2 = cf[2 * z.ext];
+        const double2 zn = n <= d.N ? xz[n] : zero, fn = n <= d.N ? xf[n] : zero;
+        const double2 zl = n > m && n > 1 ? xz[n - 1] : zero, dl = n > m && n > 1 ? xd[n - 1] : zero;
+        const double2 zu = n < d.N ? xz[n + 1] : zero, du = n < d.N ? xd[n + 1] : zero;
+        v[0] = fma(w0, dn.y, fma(w2, zu.x, -(w1 * zl.x)));
+        v[1] = fma(-w0, dn.x, fma(w2, zu.y, -(w1 * zl.y)));
+        v[2] = fma(w0, zn.y, fma(w1, dl.x, -(w2 * du.x)));
+        v[3] = fma(-w0, zn.x, fma(w1, dl.y, -(w2 * du.y)));
+        v[4] = zn.x;
+        v[5] = zn.y;
+        v[6] = fn.x;
+        v[7] = fn.y;
+      } else {
+        const double2 qn = n <= d.N ? qin[static_cast<size_t>(b) * d.ntri + base + n] : zero;
+        v[0] = qn.x;
+        v[1] = qn.y;
+        v[2] = dn.x;
+        v[3] = dn.y;
+      }
+    }
+    if (tid < ((kc * 16 + 31) & ~31)) {
+#pragma unroll
+      for (int f = 0; f < F; f++) {
+        const int ex = __reduce_max_sync(0xffffffffu, max(t64_exp(v[2 * f]), t64_exp(v[2 * f + 1])));
+        if ((tid & 31) == 0) atomicMax(&rowexp[ml][f], ex);
+      }
+    }
+    __syncthreads();
+    if (col) {
+      uint8_t *o = A + (k >> 4) * ablk + (7 * nbt + ml) * T64_SBO + ((k & 15) >> 3) * T64_LBO + (k & 7) * 2;
+#pragma unroll
+      for (int q = 0; q < 2 * F; q++) {
+        unsigned short dg[T64_DIG];
+        t64_digits(t64_fixed(v[q], t64_row(rowexp[ml][q >> 1])), dg);
+#pragma unroll
+        for (int i = 0; i < T64_DIG; i++) *reinterpret_cast<unsigned short *>(o + i * nbt * T64_SBO + q * 16) = dg[i];
+      }
+    }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  const uint32_t tmem = bars.tslot;
+  if (tid == 0) {
+    for (; copied < kc; copied++)
+      if (!t64_copy(bars, stages, stage_bytes, z.ns, copied, src + static_cast<long>(copied) * T64_DIG * L * 16, stage_bytes, z.err)) break;
+  } else if (tid == 32) {
+    const int even = ke16 / 16;
+    for (int c = 0; c < kc; c++)
+      if (!t64_mma(bars, stages, stage_bytes, z.ns, c, L, tc::su32(A + c * ablk), nbt, tmem + (c < even ? 0 : L), c == 0 || c == even, z.err)) break;
+    tc::commit(tc::su32(&bars.done));
+  }
+  const bool ok = t64_finish(bars, z.ns, z.err);
+  pdl_trigger();
+  const int warp = tid >> 5, lane = tid & 31, quarter = warp & 3, row = quarter * 32 + lane, rows = 64 * nbt;
+  int *red = reinterpret_cast<int *>(t64_sm);  // [2][rows][w + 1]: even, odd
+  const int w = min(L, 32), ld = w + 1;
+  for (int cb = 0; ok && cb < L; cb += 32) {
+    if (quarter * 32 < rows)
+      t64_unload(tmem + (warp < 4 ? 0 : L) + cb + (static_cast<uint32_t>(quarter * 32) << 16), w, red + ((warp < 4 ? 0 : rows) + row) * ld, row < rows);
+    __syncthreads();
+    for (int e = tid; e < mt * F * w; e += T64_THREADS) {
+      const int i = e % w, f = (e / w) % F, ml = e / (w * F), jh = sl * L + cb + i;
+      if (jh >= d.nh) continue;
+      const double sa = t64_scale_a(t64_row(rowexp[ml][f])), sb = t64_scale_b(z.eS[m * z.nh16 + jh]);
+      double so[2], no[2];
+#pragma unroll
+      for (int ri = 0; ri < 2; ri++) {
+        const int r0 = ml * 8 + 2 * f + ri;
+        const T64Sum ev = t64_sum(red + r0 * ld + i, 8 * nbt * ld), od = t64_sum(red + (rows + r0) * ld + i, 8 * nbt * ld);
+        so[ri] = t64_value(ev.hi + od.hi, ev.lo + od.lo) * sb * sa;
+        no[ri] = t64_value(ev.hi - od.hi, ev.lo - od.lo) * sb * sa;
+      }
+      const size_t bo = static_cast<size_t>(tile * nbt + ml) * d.nlat;
+      four[((bo + jh) * F + f) * d.M + m] = make_double2(so[0], so[1]);
+      four[((bo + d.nlat - 1 - jh) * F + f) * d.M + m] = make_double2(no[0], no[1]);
+    }
+    __syncthreads();
+  }
+  t64_teardown(bars, ncols);
+}
+
+// ------------------------------------------------------------------------------------------------ analysis + RK4
+// grid: (B, M). SLOTS = 5: the flow (fold [B][nh][5][2][M]; x0, xs, acc [B][3][ntri]); SLOTS = 3: the tracer (U q, V q, q delta;
+// x0, xs, acc [B][ntri]).
+// T170, one member: 71.7 -> 34.5 us; T42 x 16: 45.1 -> 31.1; T42, one member: 8.2 -> 9.5.
+template <int SLOTS>
+__global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, const double2 *__restrict__ fold, StageArgs sa, double2 *__restrict__ x0,
+                                                           double2 *__restrict__ xs, double2 *__restrict__ acc) {
+  constexpr int Q = 2 * SLOTS, FIELDS = SLOTS == 5 ? 3 : 1, GPO = SLOTS == 5 ? 2 : 1;  // row groups per digit
+  extern __shared__ __align__(1024) uint8_t t64_sm[];
+  __shared__ __align__(8) T64Bars bars;
+  __shared__ int rowexp[2][Q];
+  const int tid = threadIdx.x, m = blockIdx.y, b = blockIdx.x;
+  const int kc = z.nhk / 16, ra0 = z.ra16[2 * m], ra1 = z.ra16[2 * m + 1], stage_bytes = T64_DIG * z.ra_max * 32, ablk = 15 * GPO * T64_SBO;
+  uint8_t *stages = t64_sm, *A = t64_sm + z.ns * stage_bytes;
+  uint32_t ncols = 32;
+  while (ncols < static_cast<uint32_t>(ra0 + ra1)) ncols <<= 1;
+  t64_setup(bars, z.ns, ncols);
+  // chunks: parity 0's kc, then parity 1's
+  auto chunk = [&](int it) { return z.tA + z.oA[2 * m + (it < kc ? 0 : 1)] + static_cast<long>(it < kc ? it : it - kc) * T64_DIG * (it < kc ? ra0 : ra1) * 16; };
+  auto bytes = [&](int it) { return static_cast<uint32_t>(T64_DIG * (it < kc ? ra0 : ra1) * 32); };
+  int copied = 0;
+  if (tid == 0)
+    for (; copied < min(2 * kc, z.ns); copied++) t64_copy(bars, stages, stage_bytes, z.ns, copied, chunk(copied), bytes(copied), z.err);
+  for (int e = tid; e < 2 * kc * 7 * GPO * (T64_SBO / 16); e += T64_THREADS) {
+    const int blk = e / (7 * GPO * (T64_SBO / 16)), o = e % (7 * GPO * (T64_SBO / 16));
+    *reinterpret_cast<uint4 *>(A + blk * ablk + o * 16) = make_uint4(0, 0, 0, 0);
+  }
+  if (tid < 2 * Q) rowexp[tid / Q][tid % Q] = 0;
+  __syncthreads();
+  pdl_wait();
+  // thread: latitude pair jh at parity p of the fold
+  const int p = tid / z.nhk, jh = tid % z.nhk;
+  const bool col = p < 2;
+  double v[Q];
+#pragma unroll
+  for (int s = 0; s < SLOTS; s++) {
+    const double2 g = col && jh < d.nh ? fold[((static_cast<size_t>(b) * d.nh + jh) * SLOTS + s) * 2 * d.M + p * d.M + m] : make_double2(0.0, 0.0);
+    v[2 * s] = g.x;
+    v[2 * s + 1] = g.y;
+  }
+  if (col) {
+    const bool whole = z.nhk >= 32;  // a warp has one parity
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      int ex = t64_exp(v[q]);
+      if (whole) ex = __reduce_max_sync(0xffffffffu, ex);
+      if (!whole || (tid & 31) == 0) atomicMax(&rowexp[p][q], ex);
+    }
+  }
+  __syncthreads();
+  if (col) {
+    uint8_t *o = A + (p * kc + (jh >> 4)) * ablk + 7 * GPO * T64_SBO + ((jh & 15) >> 3) * T64_LBO + (jh & 7) * 2;
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      unsigned short dg[T64_DIG];
+      t64_digits(t64_fixed(v[q], t64_row(rowexp[p][q])), dg);
+#pragma unroll
+      for (int i = 0; i < T64_DIG; i++) *reinterpret_cast<unsigned short *>(o + (i * GPO + (q >> 3)) * T64_SBO + (q & 7) * 16) = dg[i];
+    }
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  const uint32_t tmem = bars.tslot;
+  if (tid == 0) {
+    for (; copied < 2 * kc; copied++)
+      if (!t64_copy(bars, stages, stage_bytes, z.ns, copied, chunk(copied), bytes(copied), z.err)) break;
+  } else if (tid == 32) {
+    for (int it = 0; it < 2 * kc; it++)
+      if (!t64_mma(bars, stages, stage_bytes, z.ns, it, it < kc ? ra0 : ra1, tc::su32(A + it * ablk), GPO, tmem + (it < kc ? 0 : ra0), it == 0 || it == kc, z.err)) break;
+    tc::commit(tc::su32(&bars.done));
+  }
+  const bool ok = t64_finish(bars, z.ns, z.err);
+  pdl_trigger();
+  // sums S[q][n - m], n to T+1
+  const int warp = tid >> 5, lane = tid & 31, quarter = warp & 3, row = quarter * 32 + lane, next = d.N + 2 - m;
+  constexpr int ROWS = 64 * GPO, LD = 33;
+  int *red = reinterpret_cast<int *>(t64_sm);                                   // [2][ROWS][LD]: two blocks of 32 columns
+  double *S = reinterpret_cast<double *>(t64_sm + ((2 * ROWS * LD * sizeof(int) + 15) & ~15u));  // [Q][next + 1]
+  const int sld = next + 1, total = ra0 + ra1;
+  for (int cb = 0; ok && cb < total; cb += 64) {
+    const int c0 = cb + (warp < 4 ? 0 : 32), w = total - c0 >= 32 ? 32 : 16;
+    if (quarter * 32 < ROWS && c0 < total)
+      t64_unload(tmem + c0 + (static_cast<uint32_t>(quarter * 32) << 16), w, red + ((warp < 4 ? 0 : ROWS) + row) * LD, true);
+    __syncthreads();
+    for (int e = tid; e < Q * 64; e += T64_THREADS) {
+      const int i = e & 63, q = e >> 6, c = cb + i, pp = c < ra0 ? 0 : 1, r = pp ? c - ra0 : c, nn = m + pp + 2 * r;
+      if (c >= total || nn > d.N + 1) continue;
+      const T64Sum t = t64_sum(red + ((i >> 5) * ROWS + (q >> 3) * 8 + (q & 7)) * LD + (i & 31), 8 * GPO * LD);
+      S[q * sld + nn - m] = t64_value(t.hi, t.lo) * t64_scale_b(z.eA[d.tri[m] + nn]) * t64_scale_a(t64_row(rowexp[pp][q]));
+    }
+    __syncthreads();
+  }
+  if (ok) {
+    const double mm = static_cast<double>(m);
+    const size_t mb = static_cast<size_t>(b) * FIELDS * d.ntri;
+    for (int i = tid; i < d.N + 1 - m; i += T64_THREADS) {
+      const int n = m + i, q = d.tri[m] + i;
+      const double w3 = z.cf[3 * z.ext + d.tri[m] + n], w4 = z.cf[4 * z.ext + d.tri[m] + n];
+      auto at = [&](int s) { return make_double2(S[2 * s * sld + i], S[(2 * s + 1) * sld + i]); };
+      // the H sum: -n eps_{n+1} S(n+1) + (n+1) eps_n S(n-1)
+      auto deriv = [&](int s) {
+        const double2 u = make_double2(S[2 * s * sld + i + 1], S[(2 * s + 1) * sld + i + 1]);
+        const double2 l = i > 0 ? make_double2(S[2 * s * sld + i - 1], S[(2 * s + 1) * sld + i - 1]) : make_double2(0.0, 0.0);
+        return make_double2(fma(w4, l.x, -(w3 * u.x)), fma(w4, l.y, -(w3 * u.y)));
+      };
+      double2 kk[FIELDS];
+      if constexpr (SLOTS == 5) {
+        // cpp/sphere.cpp:380-383: dz = -D(A,B), dd = D(B,-A) + n(n+1)/a^2 (Phi + E), df = -D(U Phi, V Phi)
+        kk[0] = csub(deriv(1), imul(at(0), mm));
+        kk[1] = cadd(cadd(imul(at(1), mm), deriv(0)), cscale(at(4), d.lapl[n]));
+        kk[2] = csub(deriv(3), imul(at(2), mm));
+        if (q == 0 || sa.zero) kk[0] = kk[1] = kk[2] = make_double2(0.0, 0.0);  // cpp/sphere.cpp:387-389
+      } else {
+        kk[0] = cadd(at(2), csub(deriv(1), imul(at(0), mm)));  // cpp/sphere.cpp:250-263
+      }
+      double2 xv[FIELDS], av[FIELDS];
+#pragma unroll
+      for (int f = 0; f < FIELDS; f++) {
+        xv[f] = x0[mb + static_cast<size_t>(f) * d.ntri + q];
+        av[f] = sa.stage > 0 ? acc[mb + static_cast<size_t>(f) * d.ntri + q] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int f = 0; f < FIELDS; f++) {
+        const size_t o = mb + static_cast<size_t>(f) * d.ntri + q;
+        if (sa.stage < 3) {
+          acc[o] = sa.stage == 0 ? kk[f] : make_double2(fma(2.0, kk[f].x, av[f].x), fma(2.0, kk[f].y, av[f].y));
+          xs[o] = make_double2(fma(sa.c, kk[f].x, xv[f].x), fma(sa.c, kk[f].y, xv[f].y));
+        } else {
+          // cpp/sphere.cpp:428-434: x += dt/6 (k1 + 2k2 + 2k3 + k4), then the del^4 filter (the tracer: Phi's)
+          const double2 val = make_double2(fma(sa.c, av[f].x + kk[f].x, xv[f].x), fma(sa.c, av[f].y + kk[f].y, xv[f].y));
+          const double fac = sa.filt[(FIELDS == 1 || f == 2 ? 1 : 0) * d.M + n];
+          x0[o] = q == 0 ? val : cscale(val, fac);
+        }
+      }
+    }
+  }
+  t64_teardown(bars, ncols);
+}
+
+}  // namespace
+
+inline Tc64Dev tc64_dev(const Tc64Plan &p, int ext) {
+  return Tc64Dev{p.nh16, p.lrows, p.nsl, p.nhk, p.ns, p.nbt, p.ntiles, p.ra_max, ext, p.tS.p, p.tA.p, p.ke16.p, p.kc.p, p.ra16.p, p.eS.p, p.eA.p, p.oS.p, p.oA.p, p.cf.p, p.err.p};
+}
+
+// sizes, offsets and tables for members B (the digits are cut on the device from the FP64 tables)
+inline void build_tc64(Tc64Plan &p, const HostTables &h, const SphDev &d, double radius, int B, cudaStream_t stream) {
+  const int N = h.N, M = h.M, nh = h.nh, ext = h.ntri + M;
+  p.nh16 = pad16(nh);
+  p.lrows = std::min(p.nh16, 64);
+  p.nsl = p.nh16 / p.lrows;
+  p.nhk = pad16(nh);
+  p.nbt = B > 1 ? 2 : 1;
+  p.ntiles = (B + p.nbt - 1) / p.nbt;
+  std::vector<int> ke16(M), kc(M), ra16(2 * M);
+  std::vector<long> oS(M), oA(2 * M);
+  long ts = 0, ta = 0;
+  for (int m = 0; m <= N; m++) {
+    const int even = (N + 1 - m) / 2 + 1, odd = (N + 2 - m) / 2;  // n - m = 0..T+1-m
+    ke16[m] = pad16(even);
+    kc[m] = (ke16[m] + pad16(odd)) / 16;
+    p.kc_max = std::max(p.kc_max, kc[m]);
+    oS[m] = ts;
+    ts += static_cast<long>(p.nsl) * kc[m] * T64_DIG * p.lrows * 16;
+    for (int s = 0; s < 2; s++) {
+      ra16[2 * m + s] = pad16(s ? odd : even);
+      p.ra_max = std::max(p.ra_max, ra16[2 * m + s]);
+      oA[2 * m + s] = ta;
+      ta += static_cast<long>(p.nhk / 16) * T64_DIG * ra16[2 * m + s] * 16;
+    }
+  }
+  // the coefficients of U, V and of the derivative sums (legendre_eps: cpp/sphere.cpp:11)
+  std::vector<double> cf(5 * static_cast<size_t>(ext), 0.0);
+  for (int m = 0; m <= N; m++)
+    for (int n = m; n <= N + 1; n++) {
+      const size_t i = static_cast<size_t>(h.tri[m] + n);
+      const double el = n > m ? legendre_eps(n, m) : 0.0, eu = legendre_eps(n + 1, m);
+      cf[i] = n > 0 ? radius * m / (n * (n + 1.0)) : 0.0;
+      cf[ext + i] = n > 0 ? radius * el / n : 0.0;
+      cf[2 * static_cast<size_t>(ext) + i] = radius * eu / (n + 1.0);
+      cf[3 * static_cast<size_t>(ext) + i] = n * eu;
+      cf[4 * static_cast<size_t>(ext) + i] = (n + 1) * el;
+    }
+  auto up = [](auto &dst, const auto &src) {
+    dst.alloc(src.size());
+    LMW_CUDA(cudaMemcpy(dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice));
+  };
+  up(p.ke16, ke16);
+  up(p.kc, kc);
+  up(p.ra16, ra16);
+  up(p.oS, oS);
+  up(p.oA, oA);
+  up(p.cf, cf);
+  p.tS.alloc(ts);
+  p.tA.alloc(ta);
+  p.eS.alloc(static_cast<size_t>(M) * p.nh16);
+  p.eA.alloc(ext);
+  p.err.alloc(1);
+  p.err.p[0] = 0;
+  // an M = 128 MMA reads sixteen row groups from its A block: up to eight past the fifteen of one-group digits
+  const size_t margin = 8 * T64_SBO + 256;
+  const size_t red_syn = static_cast<size_t>(2 * 64 * p.nbt) * (std::min(p.lrows, 32) + 1) * sizeof(int);
+  p.smem_syn = std::max(static_cast<size_t>(p.ns) * T64_DIG * p.lrows * 32, red_syn) + static_cast<size_t>(p.kc_max) * 15 * p.nbt * T64_SBO + margin;
+  const size_t red_ana = static_cast<size_t>(2) * 128 * 33 * sizeof(int) + 16 + static_cast<size_t>(10) * (N + 3) * sizeof(double);
+  p.smem_ana = std::max(static_cast<size_t>(p.ns) * T64_DIG * p.ra_max * 32 + static_cast<size_t>(2) * (p.nhk / 16) * 30 * T64_SBO + margin, red_ana);
+  DevBuf<double> P1;
+  up(P1, h.P1);
+  const Tc64Dev z = tc64_dev(p, ext);
+  tc64_build_syn<<<M, 128, 0, stream>>>(d, z, P1.p, p.tS.p, p.eS.p);
+  tc64_build_ana<<<dim3(M, 2), 256, 0, stream>>>(d, z, P1.p, p.tA.p, p.eA.p);
+  LMW_LAUNCH_CHECK();
+  LMW_CUDA(cudaStreamSynchronize(stream));
+}
+
+}  // namespace lmw

@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(SYN_THREADS) trc_synth(SphDev d, SphTab<double
   const double2 *xd = x + static_cast<size_t>(b) * 3 * d.ntri + d.ntri, *xq = qin + static_cast<size_t>(b) * d.ntri;
   double2 qs = make_double2(0, 0), ds = qs;
   const int base = d.tri[m];
+  pdl_wait();
   if (live) {
 #pragma unroll 2
     for (int n = m + c; n <= d.N; n += SYN_CHUNKS) {
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(SYN_THREADS) trc_synth(SphDev d, SphTab<double
   part[c][2][lane] = ds.x;
   part[c][3][lane] = ds.y;
   __syncthreads();
+  pdl_trigger();
   if (threadIdx.x >= 64 || !live) return;
   const int side = threadIdx.x >> 5;
   double r[TRC_Q];
@@ -58,44 +60,44 @@ __global__ void __launch_bounds__(SYN_THREADS) trc_synth(SphDev d, SphTab<double
 }
 
 // four: the flow's [B][nlat][4][M] (U, V rows 0 and 1); fourq: [B][nlat][2][M]; foldq: [B][nh][TRC_SLOT][2][M]
-__global__ void __launch_bounds__(GRID_THREADS) trc_grid(SphDev d, SphTab<double> t, const double2 *__restrict__ four,
-                                                        const double2 *__restrict__ fourq, double2 *__restrict__ foldq) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  double2 *sm = reinterpret_cast<double2 *>(smraw);
-  const int b = blockIdx.y, jh = blockIdx.x;
-  const int js = jh, jn = d.nlat - 1 - jh, n = d.nlon, rl = fft_row<3>(n);
-  load_pair_spectra<double2, 3>(sm, 2, d, four + (static_cast<size_t>(b) * d.nlat + js) * 4 * d.M,
-                                   four + (static_cast<size_t>(b) * d.nlat + jn) * 4 * d.M, d.M);
-  load_pair_spectra<double2, 3>(sm + 2 * rl, 2, d, fourq + (static_cast<size_t>(b) * d.nlat + js) * 2 * d.M,
-                                   fourq + (static_cast<size_t>(b) * d.nlat + jn) * 2 * d.M, d.M);
-  fft_inverse_dit<double2, 3>(sm, 4, n, d.logn, t.tw);
-  // cpp/sphere.cpp:255-258: A = U q, B = V q, C = q delta (real part: southern latitude, imaginary: northern)
-  double2 *rU = sm, *rV = sm + rl, *rQ = sm + 2 * rl, *rD = sm + 3 * rl;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    const int kp = fft_at<3>(k);
-    const double2 U = rU[kp], V = rV[kp], Q = rQ[kp], D = rD[kp];
-    rU[kp] = make_double2(U.x * Q.x, U.y * Q.y);
-    rV[kp] = make_double2(V.x * Q.x, V.y * Q.y);
-    rQ[kp] = make_double2(Q.x * D.x, Q.y * D.y);
-  }
+// A cluster of four CTAs per latitude pair, as sph_grid64: one inverse transform each (U, V, q, delta), three products
+// and their forward transforms.
+constexpr int TRC_CTAS = 4;
+__global__ void __launch_bounds__(256) trc_grid(SphDev d, SphTab<double> t, const double2 *__restrict__ four, const double2 *__restrict__ fourq,
+                                                double2 *__restrict__ foldq) {
+  extern __shared__ double2 g64_sm[];
+  const int n = d.nlon;
+  double2 *inv = g64_sm, *fwd = g64_sm + n, *tw = g64_sm + 2 * n;
+  const int r = static_cast<int>(cluster_rank()), jh = blockIdx.x / TRC_CTAS, b = blockIdx.y;
+  const int js = jh, jn = d.nlat - 1 - jh;
+  for (int e = threadIdx.x; e < n / 2; e += blockDim.x) tw[e] = t.tw[e];
+  for (int e = threadIdx.x; e < n; e += blockDim.x) inv[e] = make_double2(0.0, 0.0);
+  const double wt = r < 2 ? t.wd[js] : t.w[js];
   __syncthreads();
-  fft_forward_dif<double2, 3>(sm, TRC_SLOT, n, d.logn, t.tw);
-  const double inv = 1.0 / n, wd = t.wd[js], wj = t.w[js];
-  double2 *o = foldq + (static_cast<size_t>(b) * d.nh + jh) * TRC_SLOT * 2 * d.M;
-  for (int e = threadIdx.x; e < TRC_SLOT * d.M; e += blockDim.x) {
-    const int r = e / d.M, m = e - r * d.M;
-    const double2 *row = sm + static_cast<size_t>(r) * rl;
-    const double2 Ym = row[fft_at<3>(bitrev(m, d.logn))], Yc = conjd(row[fft_at<3>(bitrev((n - m) & (n - 1), d.logn))]);
-    const double hinv = 0.5 * inv;
-    double2 Xs = cscale(cadd(Ym, Yc), hinv);
-    const double2 tt = csub(Ym, Yc);
-    double2 Xn = make_double2(hinv * tt.y, -hinv * tt.x);
-    const double wt = r < 2 ? wd : wj;
-    Xs = cscale(Xs, wt);
-    Xn = cscale(Xn, wt);
-    o[(r * 2 + 0) * d.M + m] = cadd(Xs, Xn);
-    o[(r * 2 + 1) * d.M + m] = csub(Xs, Xn);
+  pdl_wait();
+  const int rows = r < 2 ? 4 : 2;
+  const double2 *f = (r < 2 ? four : fourq) + static_cast<size_t>(b) * d.nlat * rows * d.M + (r & 1) * d.M;
+  g64_load(inv, d, f + static_cast<size_t>(js) * rows * d.M, f + static_cast<size_t>(jn) * rows * d.M);
+  __syncthreads();
+  fft64<true>(inv, d.logn, tw);
+  cluster_arrive();
+  cluster_wait();
+  // cpp/sphere.cpp:255-258: A = U q, B = V q, C = q delta (real part: southern latitude, imaginary: northern)
+  if (r < TRC_SLOT) {
+    const uint32_t ax = cluster_map(inv, r < 2 ? r : 3), aq = cluster_map(inv, 2);
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+      const double2 x = cluster_load(ax, k), q = cluster_load(aq, k);
+      fwd[bitrev(k, d.logn)] = make_double2(x.x * q.x, x.y * q.y);
+    }
   }
+  cluster_arrive();  // the other CTAs' rows are read
+  if (r < TRC_SLOT) {
+    __syncthreads();
+    fft64<false>(fwd, d.logn, tw);
+    pdl_trigger();
+    g64_fold(fwd, d, wt, foldq + ((static_cast<size_t>(b) * d.nh + jh) * TRC_SLOT + r) * 2 * d.M);
+  }
+  cluster_wait();
 }
 
 // q0: tracer state, qs: stage input, qacc: RK4 accumulator, all [B][ntri]
@@ -110,6 +112,7 @@ __global__ void __launch_bounds__(ANA_THREADS) trc_analysis(SphDev d, SphTab<dou
   const double2 *fb = foldq + static_cast<size_t>(b) * d.nh * TRC_SLOT * 2 * d.M;
   const int sP = par * d.M + m, sH = (1 - par) * d.M + m;
   double2 aP = make_double2(0, 0), bH = aP, cP = aP;
+  pdl_wait();
   if (live) {
 #pragma unroll 2
     for (int jh = c; jh < d.nh; jh += ANA_CHUNKS) {
