@@ -279,142 +279,6 @@ __device__ void fft_forward_dif(C2 *s, int rows, int n, int logn, const C2 *__re
     hi = st;
   }
 }
-// Compile-time forms of the same groups: the transform length 2^LOGN, the group's first stage ST and its size F
-// are template constants, so every element and twiddle address of a thread is its base plus an immediate (no
-// per-element index arithmetic). Where the padding lets a group's elements sit at a fixed step from their first
-// one (rows unpadded, ST >= PAD, or a first group no wider than the padding period) the step is a constant;
-// otherwise the element offsets are computed as in dit_group. Same butterflies, twiddles and order as
-// dit_group / dif_group, so the same bits.
-template <int PAD, int ST, int F> __host__ __device__ constexpr bool fft_fixed_step() { return PAD == 0 || ST >= PAD || (ST == 0 && F <= PAD); }
-template <int PAD, int ST> __host__ __device__ constexpr int fft_step() { return PAD == 0 ? (1 << ST) : (ST >= PAD ? (1 << ST) + (1 << (ST - PAD)) : 1); }
-
-template <class C2, int F, int PAD, int LOGN, int ST>
-__device__ __forceinline__ void dit_group_c(C2 *s, int rows, const C2 *__restrict__ tw) {
-  constexpr int E = 1 << F, N = 1 << LOGN, HALFN = N >> 1, LO = (1 << ST) - 1, QB = LOGN - F, RL = PAD ? N + (N >> PAD) : N;
-  constexpr bool FIXED = fft_fixed_step<PAD, ST, F>();
-  constexpr int STEP = fft_step<PAD, ST>();
-  for (int e = threadIdx.x; e < (rows << QB); e += blockDim.x) {
-    const int r = e >> QB, q = e & ((1 << QB) - 1);
-    const int i0 = ((q >> ST) << (ST + F)) + (q & LO);
-    C2 *row = s + r * RL, *p0 = row + fft_at<PAD>(i0);
-    C2 x[E];
-#pragma unroll
-    for (int j = 0; j < E; j++) x[j] = FIXED ? p0[j * STEP] : row[fft_at<PAD>(i0 + (j << ST))];
-#pragma unroll
-    for (int f = 0; f < F; f++) {
-      const int h = 1 << f, stride = HALFN >> (ST + f);
-      const C2 *twb = tw + (q & LO) * stride;
-      C2 wv[E / 2];
-#pragma unroll
-      for (int jj = 0; jj < h; jj++) {
-        if (TW_SYM<C2> && jj >= (h >> 1) && h >= 2) wv[jj] = mk2(-wv[jj - (h >> 1)].y, wv[jj - (h >> 1)].x);
-        else wv[jj] = conjd(twb[(jj << ST) * stride]);
-      }
-#pragma unroll
-      for (int j = 0; j < E; j++) {
-        if (j & h) continue;
-        const C2 w = wv[j & (h - 1)];
-        const C2 t = cmul_tw(w, x[j + h]), u = x[j];
-        x[j] = cadd(u, t);
-        x[j + h] = csub(u, t);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < E; j++) {
-      if (FIXED) p0[j * STEP] = x[j];
-      else row[fft_at<PAD>(i0 + (j << ST))] = x[j];
-    }
-  }
-}
-template <class C2, int F, int PAD, int LOGN, int ST>
-__device__ __forceinline__ void dif_group_c(C2 *s, int rows, const C2 *__restrict__ tw) {
-  constexpr int E = 1 << F, N = 1 << LOGN, HALFN = N >> 1, LO = (1 << ST) - 1, QB = LOGN - F, RL = PAD ? N + (N >> PAD) : N;
-  constexpr bool FIXED = fft_fixed_step<PAD, ST, F>();
-  constexpr int STEP = fft_step<PAD, ST>();
-  for (int e = threadIdx.x; e < (rows << QB); e += blockDim.x) {
-    const int r = e >> QB, q = e & ((1 << QB) - 1);
-    const int i0 = ((q >> ST) << (ST + F)) + (q & LO);
-    C2 *row = s + r * RL, *p0 = row + fft_at<PAD>(i0);
-    C2 x[E];
-#pragma unroll
-    for (int j = 0; j < E; j++) x[j] = FIXED ? p0[j * STEP] : row[fft_at<PAD>(i0 + (j << ST))];
-#pragma unroll
-    for (int f = F - 1; f >= 0; f--) {
-      const int h = 1 << f, stride = HALFN >> (ST + f);
-      const C2 *twb = tw + (q & LO) * stride;
-      C2 wv[E / 2];
-#pragma unroll
-      for (int jj = 0; jj < h; jj++) {
-        if (TW_SYM<C2> && jj >= (h >> 1) && h >= 2) wv[jj] = mk2(wv[jj - (h >> 1)].y, -wv[jj - (h >> 1)].x);
-        else wv[jj] = twb[(jj << ST) * stride];
-      }
-#pragma unroll
-      for (int j = 0; j < E; j++) {
-        if (j & h) continue;
-        const C2 u = x[j], v = x[j + h];
-        x[j] = cadd(u, v);
-        x[j + h] = cmul_tw(wv[j & (h - 1)], csub(u, v));
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < E; j++) {
-      if (FIXED) p0[j * STEP] = x[j];
-      else row[fft_at<PAD>(i0 + (j << ST))] = x[j];
-    }
-  }
-}
-// the group schedules of fft_inverse_dit / fft_forward_dif for a stage-group size FG, unrolled at compile time
-template <class C2, int PAD, int LOGN, int FG, int ST = 0>
-__device__ __forceinline__ void dit_sched(C2 *s, int rows, const C2 *__restrict__ tw) {
-  if constexpr (ST < LOGN) {
-    constexpr int F = LOGN - ST >= FG ? FG : LOGN - ST;
-    dit_group_c<C2, F, PAD, LOGN, ST>(s, rows, tw);
-    __syncthreads();
-    dit_sched<C2, PAD, LOGN, FG, ST + F>(s, rows, tw);
-  }
-}
-template <class C2, int PAD, int LOGN, int FG, int HI = LOGN>
-__device__ __forceinline__ void dif_sched(C2 *s, int rows, const C2 *__restrict__ tw) {
-  if constexpr (HI > 0) {
-    constexpr int F = HI >= FG ? FG : HI;
-    dif_group_c<C2, F, PAD, LOGN, HI - F>(s, rows, tw);
-    __syncthreads();
-    dif_sched<C2, PAD, LOGN, FG, HI - F>(s, rows, tw);
-  }
-}
-// fft_inverse_dit / fft_forward_dif for a length 2^LOGN fixed at compile time (fmax: stages per group, 2..FMAX)
-template <class C2, int PAD, int FMAX, int LOGN>
-__device__ void fft_inverse_dit_c(C2 *s, int rows, const C2 *__restrict__ tw, int fmax) {
-  if constexpr (FMAX >= 4) {
-    if (fmax >= 4) {
-      dit_sched<C2, PAD, LOGN, 4>(s, rows, tw);
-      return;
-    }
-  }
-  if constexpr (FMAX >= 3) {
-    if (fmax >= 3) {
-      dit_sched<C2, PAD, LOGN, 3>(s, rows, tw);
-      return;
-    }
-  }
-  dit_sched<C2, PAD, LOGN, 2>(s, rows, tw);
-}
-template <class C2, int PAD, int FMAX, int LOGN>
-__device__ void fft_forward_dif_c(C2 *s, int rows, const C2 *__restrict__ tw, int fmax) {
-  if constexpr (FMAX >= 4) {
-    if (fmax >= 4) {
-      dif_sched<C2, PAD, LOGN, 4>(s, rows, tw);
-      return;
-    }
-  }
-  if constexpr (FMAX >= 3) {
-    if (fmax >= 3) {
-      dif_sched<C2, PAD, LOGN, 3>(s, rows, tw);
-      return;
-    }
-  }
-  dif_sched<C2, PAD, LOGN, 2>(s, rows, tw);
-}
 __device__ __forceinline__ int bitrev(int k, int logn) { return static_cast<int>(__brev(static_cast<unsigned>(k)) >> (32 - logn)); }
 
 // Load the Fourier coefficients of `rows` fields at latitudes js (real part) and jn (imaginary part) into
@@ -517,10 +381,17 @@ __global__ void __launch_bounds__(GRID_THREADS) sph_grid(SphDev d, SphTab<R> t, 
 // thread per butterfly and component, so that n threads share the chain. x = u + w v takes two FMAs per component and
 // y = u - w v = 2 u - x one, six FP64 operations per butterfly instead of eight; the first two stages, whose twiddles
 // are 1 and +-i, take four. Both components of a butterfly sit in neighbouring lanes of one warp, which reads all
-// their inputs before it writes. Twiddles exp(-2 pi i k / n), k < n/2, in shared memory.
+// their inputs before it writes. Twiddles: those of stage st at tw[2^st + lo], lo < 2^st,
+// contiguous (from the table's stride they met on one bank).
 constexpr int G64_CTAS = 5;
 __host__ __device__ constexpr int g64_threads(int n) { return n < 32 ? 32 : n < 256 ? n : 256; }
 
+__device__ __forceinline__ void fft64_twiddles(double2 *tw, int logn, const double2 *__restrict__ table) {
+  for (int e = threadIdx.x; e < 1 << logn; e += blockDim.x) {
+    const int st = 31 - __clz(e | 1);
+    tw[e] = table[(e - (1 << st)) << (logn - 1 - st) & ((1 << (logn - 1)) - 1)];
+  }
+}
 template <bool INV> __device__ __forceinline__ void fft64(double2 *s, int logn, const double2 *tw) {
   const int n = 1 << logn;
   for (int st = 0; st < logn; st++) {
@@ -539,7 +410,7 @@ template <bool INV> __device__ __forceinline__ void fft64(double2 *s, int logn, 
         y = u - ts;
       } else {
         // component c of w v (w conjugated for the inverse): w.x v.x - w.y v.y or w.x v.y + w.y v.x
-        const double2 w = tw[lo << (logn - 1 - st)];
+        const double2 w = tw[h + lo];
         const double a = c ? v.y : v.x, b = c ? v.x : v.y, wi = (c != 0) == INV ? -w.y : w.y;
         x = fma(w.x, a, fma(wi, b, u));
         y = fma(2.0, u, -x);
@@ -548,7 +419,8 @@ template <bool INV> __device__ __forceinline__ void fft64(double2 *s, int logn, 
       *us = x;
       *ys = y;
     }
-    __syncthreads();
+    if (st < 4) __syncwarp();  // up to stage 4 a warp's sixteen butterflies stay within 32 elements of their own
+    else __syncthreads();
   }
 }
 
@@ -596,8 +468,8 @@ __device__ __forceinline__ void g64_fold(const double2 *s, const SphDev &d, doub
   }
 }
 
-// grid: (5 nh, B), clusters of five along x. T42, one member: 22.5 -> 8.8 us; T170: 64.5 -> 61.9 us; T42 x 16:
-// 57.4 -> 51.4 us
+// grid: (5 nh, B), clusters of five along x. T42, one member: 22.5 -> 8.5 us; T170: 64.5 -> 61.9 us; T42 x 16:
+// 57.4 -> 50.4 us
 __global__ void __launch_bounds__(256) sph_grid64(SphDev d, SphTab<double> t, const double2 *__restrict__ four, const double *__restrict__ fgrid,
                                                   const double *__restrict__ hsgrid, double2 *__restrict__ fold) {
   extern __shared__ double2 g64_sm[];
@@ -605,7 +477,7 @@ __global__ void __launch_bounds__(256) sph_grid64(SphDev d, SphTab<double> t, co
   double2 *inv = g64_sm, *fwd = g64_sm + n, *tw = g64_sm + 2 * n;
   const int r = static_cast<int>(cluster_rank()), jh = blockIdx.x / G64_CTAS, b = blockIdx.y;
   const int js = jh, jn = d.nlat - 1 - jh;
-  for (int e = threadIdx.x; e < n / 2; e += blockDim.x) tw[e] = t.tw[e];
+  fft64_twiddles(tw, d.logn, t.tw);
   if (r < 4)
     for (int e = threadIdx.x; e < n; e += blockDim.x) inv[e] = make_double2(0.0, 0.0);
   const int gf = d.gflag[b];
@@ -1827,7 +1699,7 @@ static void stage_kernels(const SphDev &d, const SphTab<R> &t, const Tc64Plan *t
   }
   if (which < 0 || which == 1) {
     if constexpr (sizeof(R) == 8)
-      stage_launch(sph_grid64, dim3(G64_CTAS * d.nh, B), g64_threads(d.nlon), static_cast<size_t>(d.nlon) * 5 / 2 * sizeof(double2), stream, G64_CTAS, d, t,
+      stage_launch(sph_grid64, dim3(G64_CTAS * d.nh, B), g64_threads(d.nlon), static_cast<size_t>(d.nlon) * 3 * sizeof(double2), stream, G64_CTAS, d, t,
                    four, fgrid, hsgrid, fold);
     else
       stage_launch(sph_grid<R>, dim3(d.nh, B), GRID_THREADS, 5 * static_cast<size_t>(fft_row<3>(d.nlon)) * sizeof(typename V2<R>::type), stream, 1, d, t,
@@ -1866,18 +1738,18 @@ static void split_stage(const SphDev &d, const SphTab<float> &t, const SplitPlan
         throw InvalidArgument("split precision: the warp-specialised synthesis does not fit");
       const int items = d.M * sp.ntiles * sp.syn_split;
       auto *k = sp.syn_ws == 2 ? split_syn_ws<2> : split_syn_ws<1>;
-      k<<<std::min(items, sp.nsm * sp.syn_ws), SPLIT_SYN_WS_THREADS, smem, stream>>>(d, sd, B, sp.ns_syn, buf_cols, slot);
+      stage_launch(k, dim3(std::min(items, sp.nsm * sp.syn_ws)), SPLIT_SYN_WS_THREADS, smem, stream, 1, d, sd, B, sp.ns_syn, buf_cols, slot);
     } else {
-      split_syn<<<dim3(sp.ntiles, sp.syn_split, d.M), SPLIT_THREADS, sp.smem_syn, stream>>>(d, sd, B, sp.ns_syn);
+      stage_launch(split_syn, dim3(sp.ntiles, sp.syn_split, d.M), SPLIT_THREADS, sp.smem_syn, stream, 1, d, sd, B, sp.ns_syn);
     }
   }
   if (which < 0 || which == 1) {
     const dim3 grid(d.nh / sp.jb, B);
-    const size_t bytes = 5 * static_cast<size_t>(sp.jb) * fft_row<3>(d.nlon) * sizeof(float2);
     // the FFT group bound sets the kernel's register budget: 4 (sixteen elements a thread) two CTAs per SM,
     // else three
-    auto *k = split_grid_kernel(sp.direct, sp.fgrp >= 4 ? 4 : 3, sp.grid_fixed ? d.logn : 0);
-    k<<<grid, GRID_THREADS, bytes, stream>>>(d, t, sd, fgrid, hsgrid);
+    const int logn = sp.grid_fixed ? d.logn : 0;
+    stage_launch(split_grid_kernel(sp.direct, sp.fgrp >= 4 ? 4 : 3, logn), grid, split_grid_threads(logn), split_grid_bytes(sp.jb, d.nlon), stream, 1, d, t, sd,
+                 fgrid, hsgrid);
   }
   if (which < 0 || which == 2) {
     if (sp.ana_both && 2 * sp.ra_pair > 512) throw InvalidArgument("split precision: both parities' accumulators exceed tensor memory");
@@ -1894,7 +1766,7 @@ static void split_stage(const SphDev &d, const SphTab<float> &t, const SplitPlan
       const int grid = std::min(items, sp.nsm * sp.ana_ws);
       auto *k = sp.ana_ws == 2 ? (sp.ana_both ? split_ana_ws<true, 2> : split_ana_ws<false, 2>)
                                : (sp.ana_both ? split_ana_ws<true, 1> : split_ana_ws<false, 1>);
-      k<<<grid, SPLIT_WS_THREADS, smem, stream>>>(d, sd, t, sa, B, sp.ns_ana, buf_cols, slot, x0, xf, xin, xout, ac);
+      stage_launch(k, dim3(grid), SPLIT_WS_THREADS, smem, stream, 1, d, sd, t, sa, B, sp.ns_ana, buf_cols, slot, x0, xf, xin, xout, ac);
       return;
     }
     const int grid = sp.ana_grid > 0 ? std::min(items, sp.ana_grid) : items;
@@ -1903,7 +1775,7 @@ static void split_stage(const SphDev &d, const SphTab<float> &t, const SplitPlan
                                  : (sp.direct ? split_ana<false, true, 3> : split_ana<false, false, 3>))
                   : (sp.ana_both ? (sp.direct ? split_ana<true, true, 2> : split_ana<true, false, 2>)
                                  : (sp.direct ? split_ana<false, true, 2> : split_ana<false, false, 2>));
-    k<<<grid, SPLIT_ANA_THREADS, sp.smem_ana, stream>>>(d, sd, t, sa, B, sp.ns_ana, x0, xf, xin, xout, ac);
+    stage_launch(k, dim3(grid), SPLIT_ANA_THREADS, sp.smem_ana, stream, 1, d, sd, t, sa, B, sp.ns_ana, x0, xf, xin, xout, ac);
   }
 }
 
@@ -1973,7 +1845,7 @@ void SphereEngine::tracer_stage(int stage, double dt, int part) {
   if (part == 0) {
     trc_syn_launch(in, qin, reinterpret_cast<double2 *>(fourq.p), B);
   } else if (part == 1) {
-    stage_launch(trc_grid, dim3(TRC_CTAS * nh, B), g64_threads(nlon), static_cast<size_t>(nlon) * 5 / 2 * sizeof(double2), stream, TRC_CTAS, d, tab64(*tab),
+    stage_launch(trc_grid, dim3(TRC_CTAS * nh, B), g64_threads(nlon), static_cast<size_t>(nlon) * 3 * sizeof(double2), stream, TRC_CTAS, d, tab64(*tab),
                  reinterpret_cast<const double2 *>(four.p), reinterpret_cast<const double2 *>(fourq.p), reinterpret_cast<double2 *>(foldq.p));
   } else {
     StageArgs sa;
@@ -2202,7 +2074,7 @@ void SphereEngine::autotune_split() {
   // analysis operands, which the analysis streams; dir 0: FP32 fold, gathered by the analysis)
   for (int dir = 1; dir >= 0; dir--)
     for (int jb = SPLIT_JB_MAX; jb >= 1; jb /= 2)
-      if (nh % jb == 0 && 5 * static_cast<size_t>(jb) * fft_row<3>(nlon) * sizeof(float2) <= static_cast<size_t>(optin - 2048))
+      if (nh % jb == 0 && split_grid_bytes(jb, nlon) <= static_cast<size_t>(optin - 2048))
         for (int fg = 4; fg >= 2; fg--) cands.push_back({1, jb, fg, 0, dir, 0, 1e30});
   // one stage (no double buffering inside a CTA) leaves room for a third CTA per SM, whose copies overlap the others'
   for (int ns = 1; ns <= SPLIT_MAX_STAGES; ns++) {
@@ -2355,7 +2227,7 @@ void SphereEngine::set_split_plan(const int *in) {
   LMW_CUDA(cudaGetDevice(&dev));
   LMW_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   if (!(jb == 1 || jb == 2 || jb == 4 || jb == 8) || jb > SPLIT_JB_MAX || nh % jb != 0 ||
-      5 * static_cast<size_t>(jb) * fft_row<3>(nlon) * sizeof(float2) > static_cast<size_t>(optin - 2048))
+      split_grid_bytes(jb, nlon) > static_cast<size_t>(optin - 2048))
     throw InvalidArgument("split plan: latitude pairs per grid CTA must be 1, 2, 4 or 8, divide the latitude pairs and fit in shared memory");
   if (fg < 2 || fg > 4) throw InvalidArgument("split plan: FFT stages per pass must be 2, 3 or 4");
   if (nss < 1 || nss > SPLIT_MAX_STAGES || nsa < 1 || nsa > SPLIT_MAX_STAGES)

@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_syn(SphDev d, SplitDev
   uint32_t ncols = 32;
   while (ncols < static_cast<uint32_t>(4 * nh16)) ncols <<= 1;
   split_setup(&tslot, ncols, full, empty, &done, ns);
+  pdl_wait();
   const uint32_t tmem = tslot;
   TwoGemm G;
   const long kp = sd.kps[m];
@@ -342,6 +343,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_syn(SphDev d, SplitDev
   G.acc[1][0] = tmem + 2 * nh16;
   G.acc[1][1] = tmem + 3 * nh16;
   const bool ok = run_two_gemm(G, sd.pieces, sd.terms, ns, smem, full, empty, &done, sd.err);
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = warp * 32 + lane;
   // accumulator columns in blocks of 32 (TMEM -> shared memory by the warps that own live rows, then coalesced
   // stores by every thread): block cb covers jh in [32 cb, 32 cb + 32) of the four accumulators H E, H O, P E, P O
@@ -452,6 +454,7 @@ __global__ void __launch_bounds__(SPLIT_SYN_WS_THREADS, CTAS) split_syn_ws(SphDe
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
+  pdl_wait();
   auto item_of = [&](int item, int &m, int &tile, int &jh0) {
     const int per_m = sd.ntiles * nsl;
     m = item / per_m;
@@ -627,6 +630,7 @@ __global__ void __launch_bounds__(SPLIT_SYN_WS_THREADS, CTAS) split_syn_ws(SphDe
       it++;
     }
   }
+  pdl_trigger();
   __syncthreads();
   if (tid == 0) {
     if (!s_fail) {
@@ -646,13 +650,11 @@ __global__ void __launch_bounds__(SPLIT_SYN_WS_THREADS, CTAS) split_syn_ws(SphDe
 // as the analysis operands (BF16 pieces in the chunk layout, jb consecutive latitudes per store), which the
 // analysis streams with bulk copies; otherwise written m-major as FP32 fold[m][slot][parity][member][jh] (jb
 // latitudes per store), which the analysis gathers (cheaper for a few members, where jb is small)
-// FMAX: the largest FFT stage group the instantiation takes (4: sixteen elements per thread, two CTAs per SM)
-// LOGN: log2 of the transform length when it is fixed at compile time (the FFT groups then address shared memory
-// with immediates), 0 for any length. Register budget: three CTAs per SM (77 registers) for the three-stage groups
-// and for the four-stage groups of transforms up to 256 points, where the rows of a CTA's latitude pairs leave room
-// for a third CTA or the fixed addressing frees the registers; two for the any-length and longer forms
-template <bool DIRECT, int FMAX, int LOGN>
-__global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 || (LOGN > 0 && LOGN <= 8) ? 3 : 2) split_grid(SphDev d, SphTab<float> t, SplitDev sd, const double *__restrict__ fgrid,
+// FMAX: the largest FFT stage group the instantiation takes (4: sixteen elements per thread, two CTAs per SM; 3: three).
+// This is the any-length form (transforms under 64 points, and plans that ask for it); split_grid2 is the one compiled for
+// lengths 2^6 .. 2^10.
+template <bool DIRECT, int FMAX>
+__global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 ? 3 : 2) split_grid(SphDev d, SphTab<float> t, SplitDev sd, const double *__restrict__ fgrid,
                                                            const double *__restrict__ hsgrid) {
   extern __shared__ __align__(16) unsigned char smraw[];
   float2 *sm = reinterpret_cast<float2 *>(smraw);  // rows f * jb + p: U, V, zeta, Phi and the fifth product of pair p
@@ -660,7 +662,7 @@ __global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 || (LOGN > 0 && LOGN <=
   const int b = blockIdx.y, jh0 = blockIdx.x * JB;
   const int tile = b / sd.nbt, ml = b - tile * sd.nbt;
   constexpr int PSG = FMAX >= 4 ? 4 : 3;  // row padding: one element per 16 for sixteen-element FFT groups, else per 8
-  const int logn = LOGN ? LOGN : d.logn;
+  const int logn = d.logn;
   const int n = 1 << logn, M = d.M, rl = fft_row<PSG>(n);  // padded rows: element i at fft_at<PSG>(i)
   // the untilted Coriolis parameter 2 Omega mu of the CTA's latitudes (south, north), rounded to FP32 once
   __shared__ float cor[2 * SPLIT_JB_MAX];
@@ -670,6 +672,7 @@ __global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 || (LOGN > 0 && LOGN <=
   }
   for (int e = threadIdx.x; e < 4 * JB * rl; e += blockDim.x) sm[e] = make_float2(0, 0);
   __syncthreads();
+  pdl_wait();
   for (int e = threadIdx.x; e < JB * M; e += blockDim.x) {
     const int pr = e / M, m = e - pr * M;
     const float4 *rec = reinterpret_cast<const float4 *>(sd.dsyn + ((static_cast<long>(b) * d.nh + jh0 + pr) * M + m) * SPLIT_NQ);
@@ -688,8 +691,7 @@ __global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 || (LOGN > 0 && LOGN <=
     }
   }
   __syncthreads();
-  if constexpr (LOGN > 0) fft_inverse_dit_c<float2, PSG, FMAX, LOGN>(sm, 4 * JB, t.tw, sd.fgrp);
-  else fft_inverse_dit<float2, PSG, FMAX>(sm, 4 * JB, n, logn, t.tw, sd.fgrp);
+  fft_inverse_dit<float2, PSG, FMAX>(sm, 4 * JB, n, logn, t.tw, sd.fgrp);
   const float g = static_cast<float>(d.g);
   for (int e = threadIdx.x; e < JB * n; e += blockDim.x) {
     const int pr = e >> logn, k = e & (n - 1);
@@ -724,8 +726,8 @@ __global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 || (LOGN > 0 && LOGN <=
     rU[kp] = A; rV[kp] = Bv; rZ[kp] = UP; rP[kp] = VP; rE[kp] = PE;
   }
   __syncthreads();
-  if constexpr (LOGN > 0) fft_forward_dif_c<float2, PSG, FMAX, LOGN>(sm, 5 * JB, t.tw, sd.fgrp);
-  else fft_forward_dif<float2, PSG, FMAX>(sm, 5 * JB, n, logn, t.tw, sd.fgrp);
+  fft_forward_dif<float2, PSG, FMAX>(sm, 5 * JB, n, logn, t.tw, sd.fgrp);
+  pdl_trigger();
   const float inv = 1.0f / n, hinv = 0.5f * inv;
   // one work item per (m, slot r): the folded values of this CTA's latitude pairs at both parities. Direct
   // operands: the five slots of one m are consecutive threads, so a warp's stores of one row pair land in the
@@ -828,23 +830,335 @@ __global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 || (LOGN > 0 && LOGN <=
   }
 }
 
+// ------------------------------------------------------------------------------------------- grid (FP32), packed pairs
+// The work of split_grid for the transform lengths 2^6 .. 2^10. Bound: instruction issue and latency (51 % of the issue slots
+// at 22 % of the warps in split_grid), so two rows go through every instruction: row r = f JB + p (field f, latitude pair
+// p) shares 16-byte elements with row r ^ 1, (re, re', im, im'), and the butterflies are Blackwell's packed FP32
+// operations on (re, re') and (im, im'): half the arithmetic and half the shared-memory instructions, each lane rounding
+// as the scalar operation does, so the values are split_grid's bit for bit. The BF16 pieces of two latitudes are
+// rounded by one conversion, and the third pieces only where a plan keeps them. JB = 1 pairs the fields U and V, zeta and
+// Phi. Rows are padded by one element per 16 (sixteen-element groups) or 8 against bank conflicts.
+// T85 x 128: 90.1 -> 78.8 us; T42 x 384: 59.4 -> 56.7; T21 x 512: 26.6 -> 16.6; T106 x 18 (three pieces): 65.6 -> 53.6.
+__device__ __forceinline__ uint64_t pk(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t padd(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t psub(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pmul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pfma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+struct C2x2 {
+  uint64_t re, im;
+};
+// w x as cmul_tw: (fma(w.x, x.re, -(w.y x.im)), fma(w.x, x.im, w.y x.re))
+__device__ __forceinline__ C2x2 pcmul(float2 w, C2x2 x) {
+  const uint64_t wx = pk(w.x, w.x), wy = pk(w.y, w.y), ny = pk(-w.y, -w.y);
+  return {pfma(wx, x.re, pmul(ny, x.im)), pfma(wx, x.im, pmul(wy, x.re))};
+}
+// F stages from stage ST of `pairs` row pairs: decimation in time with conjugated twiddles (INV) or in frequency; the
+// butterflies, their order and twiddles are those of dit_group / dif_group
+template <bool INV, int F, int PAD, int LOGN, int ST> __device__ __forceinline__ void fft_group2(float4 *s, int pairs, const float2 *__restrict__ tw) {
+  constexpr int E = 1 << F, N = 1 << LOGN, HALFN = N >> 1, LO = (1 << ST) - 1, QB = LOGN - F, RL = N + (N >> PAD);
+  // rows are padded so that a group's elements sit at a fixed step where ST >= PAD or the group starts a padding period
+  constexpr bool FIXED = ST >= PAD || (ST == 0 && F <= PAD);
+  constexpr int STEP = ST >= PAD ? (1 << ST) + (1 << (ST - PAD)) : 1;
+  for (int e = threadIdx.x; e < (pairs << QB); e += blockDim.x) {
+    const int r = e >> QB, q = e & ((1 << QB) - 1);
+    const int i0 = ((q >> ST) << (ST + F)) + (q & LO);
+    float4 *row = s + r * RL, *p0 = row + fft_at<PAD>(i0);
+    C2x2 x[E];
+#pragma unroll
+    for (int j = 0; j < E; j++) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(FIXED ? p0 + j * STEP : row + fft_at<PAD>(i0 + (j << ST)));
+      x[j] = {v.x, v.y};
+    }
+#pragma unroll
+    for (int ff = 0; ff < F; ff++) {
+      const int f = INV ? ff : F - 1 - ff;
+      const int h = 1 << f, stride = HALFN >> (ST + f);
+      const float2 *twb = tw + (q & LO) * stride;
+      // the upper half of a stage's twiddles is the lower half times +i (INV) or -i (see dit_group)
+      float2 wv[E / 2];
+#pragma unroll
+      for (int jj = 0; jj < h; jj++) {
+        if (jj >= (h >> 1) && h >= 2) wv[jj] = INV ? mk2(-wv[jj - (h >> 1)].y, wv[jj - (h >> 1)].x) : mk2(wv[jj - (h >> 1)].y, -wv[jj - (h >> 1)].x);
+        else wv[jj] = INV ? conjd(twb[(jj << ST) * stride]) : twb[(jj << ST) * stride];
+      }
+#pragma unroll
+      for (int j = 0; j < E; j++) {
+        if (j & h) continue;
+        const C2x2 u = x[j];
+        if (INV) {
+          const C2x2 t = pcmul(wv[j & (h - 1)], x[j + h]);
+          x[j] = {padd(u.re, t.re), padd(u.im, t.im)};
+          x[j + h] = {psub(u.re, t.re), psub(u.im, t.im)};
+        } else {
+          const C2x2 v = x[j + h];
+          x[j] = {padd(u.re, v.re), padd(u.im, v.im)};
+          x[j + h] = pcmul(wv[j & (h - 1)], {psub(u.re, v.re), psub(u.im, v.im)});
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < E; j++)
+      *reinterpret_cast<ulonglong2 *>(FIXED ? p0 + j * STEP : row + fft_at<PAD>(i0 + (j << ST))) = make_ulonglong2(x[j].re, x[j].im);
+  }
+}
+// the transform in groups of FG stages: inverse from stage 0 up, forward from the last stage down (the schedules of
+// fft_inverse_dit / fft_forward_dif)
+template <bool INV, int PAD, int LOGN, int FG, int AT> __device__ __forceinline__ void fft_sched2(float4 *s, int pairs, const float2 *__restrict__ tw) {
+  if constexpr (INV && AT < LOGN) {
+    constexpr int F = LOGN - AT >= FG ? FG : LOGN - AT;
+    fft_group2<true, F, PAD, LOGN, AT>(s, pairs, tw);
+    __syncthreads();
+    fft_sched2<true, PAD, LOGN, FG, AT + F>(s, pairs, tw);
+  } else if constexpr (!INV && AT > 0) {
+    constexpr int F = AT >= FG ? FG : AT;
+    fft_group2<false, F, PAD, LOGN, AT - F>(s, pairs, tw);
+    __syncthreads();
+    fft_sched2<false, PAD, LOGN, FG, AT - F>(s, pairs, tw);
+  }
+}
+template <bool INV, int PAD, int FMAX, int LOGN> __device__ __forceinline__ void fft2(float4 *s, int pairs, const float2 *__restrict__ tw, int fg) {
+  constexpr int AT = INV ? 0 : LOGN;
+  if constexpr (FMAX >= 4) fft_sched2<INV, PAD, LOGN, 4, AT>(s, pairs, tw);
+  else if (fg >= 3) fft_sched2<INV, PAD, LOGN, 3, AT>(s, pairs, tw);
+  else fft_sched2<INV, PAD, LOGN, 2, AT>(s, pairs, tw);
+}
+// the products of cpp/sphere.cpp:348-359 at one point of one hemisphere, as split_grid forms them
+struct GridPoint {
+  float A, B, UP, VP, PE;
+};
+__device__ __forceinline__ GridPoint grid_point(float U, float V, float Z, float P, float f, float hs, float g, float r2om, bool lx) {
+  GridPoint o;
+  const float eta = Z + f;
+  o.A = U * eta;
+  o.B = V * eta;
+  o.UP = U * P;
+  o.VP = V * P;
+  o.PE = (lx ? 0.0f : P) + g * hs + (U * U + V * V) * r2om;
+  return o;
+}
+// two FP32 values rounded to BF16 (the first in the low half), and what the rounding left
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+__host__ __device__ constexpr int grid2_threads(int logn) { return logn <= 6 ? 128 : 256; }
+
+template <bool DIRECT, int FMAX, int LOGN>
+__global__ void __launch_bounds__(grid2_threads(LOGN), (FMAX < 4 ? 3 : 2) * 256 / grid2_threads(LOGN))
+    split_grid2(SphDev d, SphTab<float> t, SplitDev sd, const double *__restrict__ fgrid, const double *__restrict__ hsgrid) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float4 *sm = reinterpret_cast<float4 *>(smraw);  // row pairs
+  const int JB = sd.jb, b = blockIdx.y, jh0 = blockIdx.x * JB;
+  const int tile = b / sd.nbt, ml = b - tile * sd.nbt;
+  constexpr int PSG = FMAX >= 4 ? 4 : 3, n = 1 << LOGN, RL = n + (n >> PSG);
+  const int M = d.M;
+  auto at = [&](int pair, int i) -> float4 & { return sm[pair * RL + fft_at<PSG>(i)]; };
+  // the untilted Coriolis parameter 2 Omega mu of the CTA's latitudes (south, north), rounded to FP32 once
+  __shared__ float cor[2 * SPLIT_JB_MAX];
+  if (threadIdx.x < 2 * JB) {
+    const int pr = threadIdx.x >> 1, js = jh0 + pr, j = (threadIdx.x & 1) ? d.nlat - 1 - js : js;
+    cor[threadIdx.x] = static_cast<float>(d.om2[b] * d.mu[j]);
+  }
+  for (int e = threadIdx.x; e < 2 * JB * RL; e += blockDim.x) sm[e] = make_float4(0, 0, 0, 0);
+  __syncthreads();
+  pdl_wait();
+  // Fourier records -> spectra of the pairs of rows: south + i north at m, and the conjugate at n - m
+  auto put = [&](int pair, int m, float2 a, float2 c, float2 a2, float2 c2) {
+    if (m == 0) {
+      at(pair, 0) = make_float4(a.x, a2.x, c.x, c2.x);
+    } else {
+      at(pair, bitrev(m, LOGN)) = make_float4(a.x - c.y, a2.x - c2.y, a.y + c.x, a2.y + c2.x);
+      at(pair, bitrev(n - m, LOGN)) = make_float4(a.x + c.y, a2.x + c2.y, c.x - a.y, c2.x - a2.y);
+    }
+  };
+  const int half = JB >> 1;
+  if (JB == 1) {
+    for (int m = threadIdx.x; m < M; m += blockDim.x) {
+      const float4 *rec = reinterpret_cast<const float4 *>(sd.dsyn + ((static_cast<long>(b) * d.nh + jh0) * M + m) * SPLIT_NQ);
+      const float4 s0 = rec[0], s1 = rec[1], n0 = rec[2], n1 = rec[3];
+      put(0, m, make_float2(s0.x, s0.y), make_float2(n0.x, n0.y), make_float2(s0.z, s0.w), make_float2(n0.z, n0.w));
+      put(1, m, make_float2(s1.x, s1.y), make_float2(n1.x, n1.y), make_float2(s1.z, s1.w), make_float2(n1.z, n1.w));
+    }
+  } else {
+    for (int e = threadIdx.x; e < half * M; e += blockDim.x) {
+      const int pp = e / M, m = e - pp * M;
+      const float4 *rec = reinterpret_cast<const float4 *>(sd.dsyn + ((static_cast<long>(b) * d.nh + jh0 + 2 * pp) * M + m) * SPLIT_NQ);
+      const float4 *rec2 = rec + M * (SPLIT_NQ / 4);
+      const float4 s0 = rec[0], s1 = rec[1], n0 = rec[2], n1 = rec[3], u0 = rec2[0], u1 = rec2[1], v0 = rec2[2], v1 = rec2[3];
+      put(pp, m, make_float2(s0.x, s0.y), make_float2(n0.x, n0.y), make_float2(u0.x, u0.y), make_float2(v0.x, v0.y));
+      put(half + pp, m, make_float2(s0.z, s0.w), make_float2(n0.z, n0.w), make_float2(u0.z, u0.w), make_float2(v0.z, v0.w));
+      put(2 * half + pp, m, make_float2(s1.x, s1.y), make_float2(n1.x, n1.y), make_float2(u1.x, u1.y), make_float2(v1.x, v1.y));
+      put(3 * half + pp, m, make_float2(s1.z, s1.w), make_float2(n1.z, n1.w), make_float2(u1.z, u1.w), make_float2(v1.z, v1.w));
+    }
+  }
+  __syncthreads();
+  fft2<true, PSG, FMAX, LOGN>(sm, 2 * JB, t.tw, sd.fgrp);
+  const float g = static_cast<float>(d.g);
+  const bool lx = sd.lin_exact != 0;  // the linear terms are added in spectral space (see split_grid)
+  const int gf = d.gflag[b];
+  // Coriolis and orography at (latitude pair pr, side, k): rows are read for tilted or mountain members only
+  auto cori = [&](int pr, int side, int k) -> float {
+    if (!(gf & 1)) return lx ? 0.0f : cor[2 * pr + side];
+    const int j = side ? d.nlat - 1 - (jh0 + pr) : jh0 + pr;
+    return d2f_int(fgrid[(static_cast<size_t>(b) * d.nlat + j) * n + k]);
+  };
+  auto oro = [&](int pr, int side, int k) -> float {
+    if (!(gf & 2)) return 0.0f;
+    const int j = side ? d.nlat - 1 - (jh0 + pr) : jh0 + pr;
+    return d2f_int(hsgrid[(static_cast<size_t>(b) * d.nlat + j) * n + k]);
+  };
+  if (JB == 1) {
+    const float r2om = t.r2om[jh0];
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+      const float4 UV = at(0, k), ZP = at(1, k);  // (U.s, V.s, U.n, V.n), (zeta.s, Phi.s, zeta.n, Phi.n)
+      const GridPoint s = grid_point(UV.x, UV.y, ZP.x, ZP.y, cori(0, 0, k), oro(0, 0, k), g, r2om, lx);
+      const GridPoint o = grid_point(UV.z, UV.w, ZP.z, ZP.w, cori(0, 1, k), oro(0, 1, k), g, r2om, lx);
+      at(0, k) = make_float4(s.A, s.B, o.A, o.B);
+      at(1, k) = make_float4(s.UP, s.VP, o.UP, o.VP);
+      at(2, k) = make_float4(s.PE, 0.0f, o.PE, 0.0f);
+    }
+  } else {
+    for (int e = threadIdx.x; e < half * n; e += blockDim.x) {
+      const int pp = e >> LOGN, k = e & (n - 1);
+      const float4 U = at(pp, k), V = at(half + pp, k), Z = at(2 * half + pp, k), P = at(3 * half + pp, k);
+      const float ra = t.r2om[jh0 + 2 * pp], rb = t.r2om[jh0 + 2 * pp + 1];
+      const GridPoint s0 = grid_point(U.x, V.x, Z.x, P.x, cori(2 * pp, 0, k), oro(2 * pp, 0, k), g, ra, lx);
+      const GridPoint s1 = grid_point(U.y, V.y, Z.y, P.y, cori(2 * pp + 1, 0, k), oro(2 * pp + 1, 0, k), g, rb, lx);
+      const GridPoint n0 = grid_point(U.z, V.z, Z.z, P.z, cori(2 * pp, 1, k), oro(2 * pp, 1, k), g, ra, lx);
+      const GridPoint n1 = grid_point(U.w, V.w, Z.w, P.w, cori(2 * pp + 1, 1, k), oro(2 * pp + 1, 1, k), g, rb, lx);
+      at(pp, k) = make_float4(s0.A, s1.A, n0.A, n1.A);
+      at(half + pp, k) = make_float4(s0.B, s1.B, n0.B, n1.B);
+      at(2 * half + pp, k) = make_float4(s0.UP, s1.UP, n0.UP, n1.UP);
+      at(3 * half + pp, k) = make_float4(s0.VP, s1.VP, n0.VP, n1.VP);
+      at(4 * half + pp, k) = make_float4(s0.PE, s1.PE, n0.PE, n1.PE);
+    }
+  }
+  __syncthreads();
+  fft2<false, PSG, FMAX, LOGN>(sm, (5 * JB + 1) / 2, t.tw, sd.fgrp);
+  pdl_trigger();
+  const float inv = 1.0f / n, hinv = 0.5f * inv;
+  // one work item per (m, slot r): the folded values of this CTA's latitude pairs at both parities (see split_grid)
+  for (int e = threadIdx.x; e < M * 5; e += blockDim.x) {
+    const int m = DIRECT ? e / 5 : e % M, r = DIRECT ? e - 5 * (e / 5) : e / M;
+    const int im = bitrev(m, LOGN), ic = bitrev((n - m) & (n - 1), LOGN);
+    float2 f0[SPLIT_JB_MAX], f1[SPLIT_JB_MAX];
+    auto fold = [&](int pr, float2 Ym, float2 Yc) {
+      const int js = jh0 + pr;
+      float2 Xs = cscale(cadd(Ym, Yc), hinv);
+      const float2 tt = csub(Ym, Yc);
+      float2 Xn = make_float2(hinv * tt.y, -hinv * tt.x);
+      const float wt = r < 4 ? t.wd[js] : t.w[js];
+      Xs = cscale(Xs, wt);
+      Xn = cscale(Xn, wt);
+      f0[pr] = cadd(Xs, Xn);
+      f1[pr] = csub(Xs, Xn);
+    };
+    if (JB == 1) {
+      const float4 a = at(r >> 1, im), c = at(r >> 1, ic);
+      fold(0, (r & 1) ? make_float2(a.y, a.w) : make_float2(a.x, a.z), conjd((r & 1) ? make_float2(c.y, c.w) : make_float2(c.x, c.z)));
+    } else {
+#pragma unroll
+      for (int pp = 0; pp < SPLIT_JB_MAX / 2; pp++) {
+        if (pp >= half) break;
+        const float4 a = at(r * half + pp, im), c = at(r * half + pp, ic);
+        fold(2 * pp, make_float2(a.x, a.z), conjd(make_float2(c.x, c.z)));
+        fold(2 * pp + 1, make_float2(a.y, a.w), conjd(make_float2(c.y, c.w)));
+      }
+    }
+#pragma unroll
+    for (int par = 0; par < 2; par++) {
+      const float2 *fv = par ? f1 : f0;
+      if constexpr (!DIRECT) {
+        float2 *o = sd.fold + ((static_cast<long>(m) * 10 + r * 2 + par) * gridDim.y + b) * d.nh + jh0;
+        if (JB >= 2) {
+#pragma unroll
+          for (int pr = 0; pr < SPLIT_JB_MAX; pr += 2) {
+            if (pr >= JB) break;
+            reinterpret_cast<float4 *>(o)[pr / 2] = make_float4(fv[pr].x, fv[pr].y, fv[pr + 1].x, fv[pr + 1].y);
+          }
+        } else {
+          o[0] = fv[0];
+        }
+      } else {
+        // slot r at parity p is a P row of (m, s = p) for r = 0, 1, 2, 4 and an H row of (m, s = 1 - p) for r = 0, 1, 3
+#pragma unroll
+        for (int ri = 0; ri < 2; ri++) {
+          uint32_t pc[3][SPLIT_JB_MAX / 2];
+#pragma unroll
+          for (int h = 0; h < SPLIT_JB_MAX / 2; h++) {
+            if (2 * h >= JB) break;
+            const float a = ri ? fv[2 * h].y : fv[2 * h].x, c = JB == 1 ? 0.0f : (ri ? fv[2 * h + 1].y : fv[2 * h + 1].x);
+            const uint32_t p0 = bf16_pair(a, c);
+            const float ra = a - __uint_as_float(p0 << 16), rc = c - __uint_as_float(p0 & 0xffff0000u);
+            const uint32_t p1 = bf16_pair(ra, rc);
+            pc[0][h] = p0;
+            pc[1][h] = p1;
+            if (sd.pieces > 2) pc[2][h] = bf16_pair(ra - __uint_as_float(p1 << 16), rc - __uint_as_float(p1 & 0xffff0000u));
+          }
+#pragma unroll
+          for (int isH = 0; isH < 2; isH++) {
+            if (isH ? (r == 2 || r == 4) : (r == 3)) continue;
+            const int s_op = isH ? 1 - par : par, R = isH ? sd.rAH : sd.rAP, q = isH ? (r == 3 ? 2 : r) : (r == 4 ? 3 : r);
+            const int row = (isH ? ml * 6 : ml * 8) + 2 * q + ri;
+            __nv_bfloat16 *dst = (isH ? sd.aA_H : sd.aA_P) + ((static_cast<long>(m) * 2 + s_op) * sd.ntiles + tile) * R * sd.nha + tile_off(row, jh0, R, sd.bka);
+            const long pstride = isH ? sd.aAH_size : sd.aAP_size;
+#pragma unroll
+            for (int pi = 0; pi < 3; pi++) {
+              if (pi >= sd.pieces) break;
+              __nv_bfloat16 *dp = dst + pi * pstride;
+              if (JB == 8) *reinterpret_cast<uint4 *>(dp) = make_uint4(pc[pi][0], pc[pi][1], pc[pi][2], pc[pi][3]);
+              else if (JB == 4) *reinterpret_cast<uint2 *>(dp) = make_uint2(pc[pi][0], pc[pi][1]);
+              else if (JB == 2) *reinterpret_cast<uint32_t *>(dp) = pc[pi][0];
+              else *reinterpret_cast<unsigned short *>(dp) = static_cast<unsigned short>(pc[pi][0]);
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
 // the grid kernel instantiation for a plan: operand form, FFT group bound and transform length (lengths 2^6 to
-// 2^10, T21 to T341, compiled for their length; others take the any-length form)
+// 2^10, T11 to T341, compiled for their length; 0: the any-length form), its threads and its shared memory
 using SplitGridFn = void (*)(SphDev, SphTab<float>, SplitDev, const double *, const double *);
+inline bool split_grid_fixed(int logn) { return logn >= 6 && logn <= 10; }
 template <bool DIRECT, int FMAX> inline SplitGridFn split_grid_for(int logn) {
   switch (logn) {
-    case 6: return split_grid<DIRECT, FMAX, 6>;
-    case 7: return split_grid<DIRECT, FMAX, 7>;
-    case 8: return split_grid<DIRECT, FMAX, 8>;
-    case 9: return split_grid<DIRECT, FMAX, 9>;
-    case 10: return split_grid<DIRECT, FMAX, 10>;
-    default: return split_grid<DIRECT, FMAX, 0>;
+    case 6: return split_grid2<DIRECT, FMAX, 6>;
+    case 7: return split_grid2<DIRECT, FMAX, 7>;
+    case 8: return split_grid2<DIRECT, FMAX, 8>;
+    case 9: return split_grid2<DIRECT, FMAX, 9>;
+    case 10: return split_grid2<DIRECT, FMAX, 10>;
+    default: return split_grid<DIRECT, FMAX>;
   }
 }
 inline SplitGridFn split_grid_kernel(int direct, int fmax, int logn) {
   if (fmax >= 4) return direct ? split_grid_for<true, 4>(logn) : split_grid_for<false, 4>(logn);
   return direct ? split_grid_for<true, 3>(logn) : split_grid_for<false, 3>(logn);
 }
+inline int split_grid_threads(int logn) { return split_grid_fixed(logn) ? grid2_threads(logn) : GRID_THREADS; }
+inline size_t split_grid_bytes(int jb, int nlon) { return static_cast<size_t>((5 * jb + 1) / 2) * fft_row<3>(nlon) * sizeof(float4); }
 
 // ------------------------------------------------------------------------------------------- synthesis operands
 // The next synthesis operands for coefficient (member b, m, n) from its value rounded to FP32: psi, chi, zeta, Phi
@@ -1021,6 +1335,7 @@ __global__ void __launch_bounds__(SPLIT_ANA_THREADS, MINB) split_ana(SphDev d, S
   uint8_t *aH = smem, *aP = smem + aH_bytes, *pipe = smem + aH_bytes + aP_bytes;
   bool ok = true, setup_done = false;
   int pipe_it = 0, calls = 0;
+  pdl_wait();
   for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
   const int m = m_slowest ? item / per_m : item % d.M, rest = m_slowest ? item % per_m : item / d.M;
   const int s_first = BOTH ? 0 : rest % 2, s_last = BOTH ? 1 : s_first;
@@ -1124,6 +1439,7 @@ __global__ void __launch_bounds__(SPLIT_ANA_THREADS, MINB) split_ana(SphDev d, S
   calls++;
   }
   const uint32_t tmem = tslot;
+  if (m_slowest) pdl_trigger();
   // accumulators -> shared memory [row][ld + 1] (the operand and pipeline buffers are free now); the odd row
   // stride puts the rows that one warp writes at once on different banks
   const int ldp = ld + 1;
@@ -1211,6 +1527,7 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
+  pdl_wait();
   // the item sequence every role walks (snake_item): (m, parity or both, tile), m the slowest index
   auto item_of = [&](int item, int &m, int &s_first, int &s_last, int &tile, int &R0, int &R1) {
     m = item / per_m;
@@ -1369,6 +1686,7 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
       it++;
     }
   }
+  pdl_trigger();
   __syncthreads();
   if (tid == 0) {
     // every MMA issued has finished (and its arrivals landed) before the CTA releases its memory; after a failure the

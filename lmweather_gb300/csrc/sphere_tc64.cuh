@@ -77,13 +77,16 @@ __device__ __forceinline__ long long t64_fixed(double v, int e) {
 }
 // the eight digits of x, most significant first, as BF16 bits
 __device__ __forceinline__ void t64_digits(long long x, unsigned short *out) {
+  // digit = ((y + 64) mod 128) - 64, y = (y + 64) / 128: the low four from 28 bits, the others from what they leave
+  int y = static_cast<int>(x) & 0xfffffff;
 #pragma unroll
-  for (int i = T64_DIG - 1; i >= 0; i--) {
-    const int lo = static_cast<int>(x);
-    const int dgt = i == 0 ? lo : ((lo + 64) & 127) - 64;
-    x = (x - dgt) >> 7;
-    out[i] = static_cast<unsigned short>(__float_as_uint(__int_as_float(0x4B400000 + dgt) - 12582912.0f) >> 16);
+  for (int i = T64_DIG - 1; i >= 1; i--) {
+    const int u = y + 64;
+    y = u >> 7;
+    if (i == 4) y += static_cast<int>(x >> 28);  // the carry of the low digits, and the high 29 bits
+    out[i] = static_cast<unsigned short>(__float_as_uint(__int_as_float(0x4B400000 | (u & 127)) - 12582976.0f) >> 16);
   }
+  out[0] = static_cast<unsigned short>(__float_as_uint(__int_as_float(0x4B400000 + y) - 12582912.0f) >> 16);
 }
 // sum of the eight orders D[s] (exact integers) times 2^(7 (7 - s)), as high and low parts of value hi 2^28 + lo
 struct T64Sum {
@@ -95,13 +98,37 @@ __device__ __forceinline__ T64Sum t64_sum(const int *D, int stride) {
   r.lo = ((static_cast<long long>(D[4 * stride]) << 21) + (static_cast<long long>(D[5 * stride]) << 14)) + ((static_cast<long long>(D[6 * stride]) << 7) + D[7 * stride]);
   return r;
 }
-// |x| < 2^51 as a double, exactly
-__device__ __forceinline__ double t64_int(long long x) { return __longlong_as_double(0x4338000000000000ll + x) - 6755399441055744.0; }
-__device__ __forceinline__ double t64_value(long long hi, long long lo) { return fma(t64_int(hi), 268435456.0, t64_int(lo)); }
-// 2^(e - 63 + f) as two factors (e of an operand row, f of a table row); zero rows give zero, rows that are not finite NaN
-__device__ __forceinline__ double t64_pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
-__device__ __forceinline__ double t64_scale_a(int e) { return e == T64_NAN ? __longlong_as_double(0x7ff8000000000000ll) : e == T64_NONE ? 0.0 : t64_pow2(e - 63); }
-__device__ __forceinline__ double t64_scale_b(int e) { return e == T64_NONE ? 0.0 : t64_pow2(e); }
+// (hi 2^28 + lo) 2^e rounded to nearest even, by integer operations (the FP64 pipe would take three times as long); |hi|,
+// |lo| < 2^47. e = ea + eb - 63 for the exponents ea of an operand row and eb of a table row
+__device__ __forceinline__ double t64_value(long long hi, long long lo, int ea, int eb) {
+  if (ea == T64_NAN) return __longlong_as_double(0x7ff8000000000000ll);
+  unsigned long long L = static_cast<unsigned long long>(hi) << 28;
+  long long H = hi >> 36;
+  L += static_cast<unsigned long long>(lo);
+  H += (lo >> 63) + (L < static_cast<unsigned long long>(lo) ? 1 : 0);
+  const unsigned long long sign = static_cast<unsigned long long>(H) & 0x8000000000000000ull;
+  if (sign) {
+    L = 0 - L;
+    H = ~H + (L == 0 ? 1 : 0);
+  }
+  if ((static_cast<unsigned long long>(H) | L) == 0 || ea == T64_NONE || eb == T64_NONE) return 0.0;
+  const int p = H ? 127 - __clzll(H) : 63 - __clzll(static_cast<long long>(L));  // the leading bit
+  unsigned long long m;
+  if (p <= 52) {
+    m = L << (52 - p);
+  } else {
+    const int sh = p - 52;  // at most 24: |hi 2^28 + lo| < 2^76
+    m = (static_cast<unsigned long long>(H) << (64 - sh)) | (L >> sh);
+    const unsigned long long rem = L & ((1ull << sh) - 1), half = 1ull << (sh - 1);
+    m += rem > half || (rem == half && (m & 1)) ? 1 : 0;
+  }
+  const int x = p + 1023 + ea + eb - 63;  // biased exponent
+  if (x >= 1 && x <= 2045) return __longlong_as_double(static_cast<long long>(sign | ((static_cast<unsigned long long>(x - 1) << 52) + m)));
+  // the ends of the range: scale in two steps
+  const double v = __longlong_as_double(static_cast<long long>(sign | ((static_cast<unsigned long long>(p + 1022) << 52) + m)));
+  const int e = ea + eb - 63, e1 = e / 2;
+  return v * __hiloint2double((e1 + 1023) << 20, 0) * __hiloint2double((e - e1 + 1023) << 20, 0);
+}
 
 __device__ __forceinline__ uint64_t t64_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   return static_cast<uint64_t>((saddr >> 4) & 0x3FFFu) | (static_cast<uint64_t>(lbo >> 4) << 16) | (static_cast<uint64_t>(sbo >> 4) << 32) |
@@ -247,7 +274,7 @@ __device__ __forceinline__ void t64_unload(uint32_t taddr, int w, int *dst, bool
 // ------------------------------------------------------------------------------------------------ synthesis
 // grid: (slices x tiles, M). F = 4: U, V, zeta, Phi of x [B][3][ntri] into four [B][nlat][4][M]; F = 2 (tracer): q of qin
 // [B][ntri] and delta of x into [B][nlat][2][M].
-// T170, one member: 82.0 -> 18.5 us (FP64 pipe before); T42 x 16: 50.4 -> 13.7; T42, one member: 10.3 -> 7.3.
+// T170, one member: 82.0 -> 19.0 us (FP64 pipe before); T42 x 16: 50.4 -> 11.7; T42, one member: 10.3 -> 7.5.
 template <int F>
 __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, const double2 *__restrict__ x, const double2 *__restrict__ qin,
                                                            double2 *__restrict__ four, int B) {
@@ -352,14 +379,14 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
     for (int e = tid; e < mt * F * w; e += T64_THREADS) {
       const int i = e % w, f = (e / w) % F, ml = e / (w * F), jh = sl * L + cb + i;
       if (jh >= d.nh) continue;
-      const double sa = t64_scale_a(t64_row(rowexp[ml][f])), sb = t64_scale_b(z.eS[m * z.nh16 + jh]);
+      const int ea = t64_row(rowexp[ml][f]), eb = z.eS[m * z.nh16 + jh];
       double so[2], no[2];
 #pragma unroll
       for (int ri = 0; ri < 2; ri++) {
         const int r0 = ml * 8 + 2 * f + ri;
         const T64Sum ev = t64_sum(red + r0 * ld + i, 8 * nbt * ld), od = t64_sum(red + (rows + r0) * ld + i, 8 * nbt * ld);
-        so[ri] = t64_value(ev.hi + od.hi, ev.lo + od.lo) * sb * sa;
-        no[ri] = t64_value(ev.hi - od.hi, ev.lo - od.lo) * sb * sa;
+        so[ri] = t64_value(ev.hi + od.hi, ev.lo + od.lo, ea, eb);
+        no[ri] = t64_value(ev.hi - od.hi, ev.lo - od.lo, ea, eb);
       }
       const size_t bo = static_cast<size_t>(tile * nbt + ml) * d.nlat;
       four[((bo + jh) * F + f) * d.M + m] = make_double2(so[0], so[1]);
@@ -373,7 +400,7 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
 // ------------------------------------------------------------------------------------------------ analysis + RK4
 // grid: (B, M). SLOTS = 5: the flow (fold [B][nh][5][2][M]; x0, xs, acc [B][3][ntri]); SLOTS = 3: the tracer (U q, V q, q delta;
 // x0, xs, acc [B][ntri]).
-// T170, one member: 71.7 -> 34.5 us; T42 x 16: 45.1 -> 31.1; T42, one member: 8.2 -> 9.5.
+// T170, one member: 71.7 -> 33.8 us; T42 x 16: 45.1 -> 29.8; T42, one member: 8.2 -> 9.4.
 template <int SLOTS>
 __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, const double2 *__restrict__ fold, StageArgs sa, double2 *__restrict__ x0,
                                                            double2 *__restrict__ xs, double2 *__restrict__ acc) {
@@ -458,7 +485,7 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
       const int i = e & 63, q = e >> 6, c = cb + i, pp = c < ra0 ? 0 : 1, r = pp ? c - ra0 : c, nn = m + pp + 2 * r;
       if (c >= total || nn > d.N + 1) continue;
       const T64Sum t = t64_sum(red + ((i >> 5) * ROWS + (q >> 3) * 8 + (q & 7)) * LD + (i & 31), 8 * GPO * LD);
-      S[q * sld + nn - m] = t64_value(t.hi, t.lo) * t64_scale_b(z.eA[d.tri[m] + nn]) * t64_scale_a(t64_row(rowexp[pp][q]));
+      S[q * sld + nn - m] = t64_value(t.hi, t.lo, t64_row(rowexp[pp][q]), z.eA[d.tri[m] + nn]);
     }
     __syncthreads();
   }

@@ -19,15 +19,22 @@ __device__ __forceinline__ uint64_t gtimer() {
 }
 
 // true when the phase completed, false when the wait ran out after `ns` nanoseconds
+__device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t phase) {
+  uint32_t done;
+  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done)
+               : "r"(bar), "r"(phase)
+               : "memory");
+  return done != 0;
+}
+// The timer is read only once a few tries (each of which the hardware suspends for a while) have failed: a wait that is
+// soon over costs no timer read and no sleep
 __device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t phase, unsigned long long ns) {
+  for (int k = 0; k < 32; k++)
+    if (try_wait(bar, phase)) return true;
   const uint64_t t0 = gtimer();
   while (true) {
-    uint32_t done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done)
-                 : "r"(bar), "r"(phase)
-                 : "memory");
-    if (done) return true;
+    if (try_wait(bar, phase)) return true;
     if (gtimer() - t0 > ns) return false;
     __nanosleep(20);
   }
