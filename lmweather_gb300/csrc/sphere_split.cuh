@@ -176,6 +176,7 @@ struct TwoGemm {
 __device__ bool run_two_gemm(const TwoGemm &G, int pieces, int terms, int ns, uint8_t *pipe, uint64_t *full, uint64_t *empty, uint64_t *done,
                              int *err, int it0 = 0, uint32_t done_phase = 0) {
   const int tid = threadIdx.x;
+  const int role = tc::uniform(tid >> 5);  // before any thread leaves its warp
   const bool astream = G.a[0] != nullptr;
   const int bk = G.bk;
   const uint32_t sbo = static_cast<uint32_t>(bk) * 16u;  // bytes between 8-row groups of a chunk
@@ -211,47 +212,43 @@ __device__ bool run_two_gemm(const TwoGemm &G, int pieces, int terms, int ns, ui
       }
       s_issued = it + 1;
     }
-  } else if (tid == 32) {
-    // MMA issuer
-    const uint32_t idesc = idesc_m128(G.bR);
-    const int tp[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
+  } else if (role == 1) {
+    // MMA issuer: the whole warp, one lane of which issues
+    const uint32_t idesc = idesc_m128(G.bR), pipe0 = su32(pipe), a16 = static_cast<uint32_t>(a_bytes) >> 4, b16 = static_cast<uint32_t>(b_bytes) >> 4;
     const int t0 = terms == 6 ? 0 : (terms == 3 ? 3 : 5);
-    bool started[2][2] = {{false, false}, {false, false}};
-    bool ok = true;
-    for (int it = 0; it < total && ok; it++) {
+    const bool leader = tc::elect_one();
+    uint32_t started = 0;  // bit 2 g + seg: that accumulator holds a product
+    for (int it = 0; it < total; it++) {
       const int git = it0 + it;
       const int st = git % ns, g = it < G.nchunk[0] ? 0 : 1, c = g == 0 ? it : it - G.nchunk[0];
-      if (!mbar_wait_bounded(su32(&full[st]), (git / ns) & 1)) {
+      if (!tc::wait_warp(su32(&full[st]), (git / ns) & 1)) {
         s_fail = 1;
         atomicExch(err, 3);
-        ok = false;
         break;
       }
       s_consumed = it + 1;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      uint8_t *base = pipe + st * stage_bytes;
+      const uint32_t base = pipe0 + st * stage_bytes;
+      // A piece pa at ad + pa * ap, B piece pb at bd + pb * b16; a K step of 16 columns is 256 bytes, so kk in descriptor units
+      const uint32_t ares = static_cast<uint32_t>(G.aR[g] * bk * 2);
+      const uint64_t ad = chunk_desc(astream ? base : G.a_res[g] + c * ares, sbo), bd = chunk_desc(base + pieces * a_bytes, sbo);
+      const uint32_t ap = astream ? a16 : (static_cast<uint32_t>(G.nchunk[g]) * ares) >> 4;
       for (int kk = 0; kk < bk; kk += 16) {
-        const int kg = c * bk + kk;
-        const int seg = kg >= G.kseg[g] ? 1 : 0;
-        for (int t = t0; t < 6; t++) {
-          const int pa = tp[t][0], pb = tp[t][1];
-          const uint32_t abase = astream ? su32(base + pa * a_bytes)
-                                         : G.a_res[g] + static_cast<uint32_t>((pa * G.nchunk[g] + c) * G.aR[g] * bk * 2);
-          const uint64_t ad = chunk_desc(abase + (kk / 8) * 128, sbo);
-          const uint64_t bd = chunk_desc(su32(base + pieces * a_bytes + pb * b_bytes + (kk / 8) * 128), sbo);
-          const uint32_t accum = started[g][seg] ? 1u : 0u;
-          asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-                           G.acc[g][seg]),
-                       "l"(ad), "l"(bd), "r"(idesc), "r"(accum)
-                       : "memory");
-          started[g][seg] = true;
+        const int seg = c * bk + kk >= G.kseg[g] ? 1 : 0;
+        const uint32_t acc = tc::uniform(G.acc[g][seg]), bit = 1u << (2 * g + seg);
+#pragma unroll
+        for (int t = 0; t < 6; t++) {
+          if (t < t0) continue;
+          const int pa = t == 0 ? 2 : (t == 1 || t == 3 ? 1 : 0), pb = t == 2 ? 2 : (t == 1 || t == 4 ? 1 : 0);
+          tc::mma(leader, acc, ad + pa * ap + kk, bd + pb * b16 + kk, idesc, started & bit ? 1u : 0u);
+          started |= bit;
         }
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(&empty[st])) : "memory");
+      tc::commit(leader, su32(&empty[st]));
     }
-    // completes `done` once every MMA this thread issued has finished (also after a failed wait, so that the
+    // completes `done` once every MMA this warp issued has finished (also after a failed wait, so that the
     // CTA can drain its own work before it frees tensor memory)
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(done)) : "memory");
+    tc::commit(leader, su32(done));
   }
   __syncthreads();
   if (tid == 0) {
@@ -421,6 +418,7 @@ __global__ void __launch_bounds__(SPLIT_SYN_WS_THREADS, CTAS) split_syn_ws(SphDe
   __shared__ uint32_t tslot;
   __shared__ int s_fail, s_issued, s_consumed, s_epi_ok;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int role = tc::uniform(warp);  // before any thread leaves its warp
   const int nh = sd.syn_nh, nsl = sd.nh16 / nh;  // latitudes per slice, slices
   const int nitems = d.M * sd.ntiles * nsl;
   const int bk = sd.bks;
@@ -498,30 +496,31 @@ __global__ void __launch_bounds__(SPLIT_SYN_WS_THREADS, CTAS) split_syn_ws(SphDe
         }
       }
     }
-  } else if (tid == 32) {
-    // MMA issuer: per operand g, K columns below ke16[m] (even n) into the E accumulator, the rest into O
-    const int tp[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
+  } else if (role == 1) {
+    // MMA issuer (the whole warp, one lane issues): per operand g, K columns below ke16[m] (even n) into the E accumulator,
+    // the rest into O
     const int t0 = sd.terms == 6 ? 0 : (sd.terms == 3 ? 3 : 5);
-    const uint32_t sbo = static_cast<uint32_t>(bk) * 16u;
-    const uint32_t idesc = idesc_m128(nh);
+    const uint32_t sbo = static_cast<uint32_t>(bk) * 16u, a16 = static_cast<uint32_t>(a_bytes) >> 4, b16 = static_cast<uint32_t>(b_bytes) >> 4;
+    const uint32_t idesc = idesc_m128(nh), pipe0 = su32(pipe), tm = tc::uniform(tmem);
+    const bool leader = tc::elect_one();
     int git = 0, it = 0;
     bool ok = true;
     for (int k = 0, item = snake_item(0); item < nitems && ok; item = snake_item(++k)) {
       int m, tile, jh0;
       item_of(item, m, tile, jh0);
-      const int nchunk = static_cast<int>(sd.kps[m] / bk), kseg = sd.ke16[m];
+      const int nchunk = tc::uniform(static_cast<int>(sd.kps[m] / bk)), kseg = tc::uniform(sd.ke16[m]);
       const int bb = it & 1;
-      if (it >= 2 && !mbar_wait_bounded(su32(&acce[bb]), ((it >> 1) - 1) & 1)) {
+      if (it >= 2 && !tc::wait_warp(su32(&acce[bb]), ((it >> 1) - 1) & 1)) {
         s_fail = 1;
         atomicExch(sd.err, 5);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       for (int g = 0; g < 2 && ok; g++) {
-        bool started[2] = {false, false};
+        uint32_t started = 0;
         for (int c = 0; c < nchunk; c++, git++) {
           const int st = git % ns;
-          if (!mbar_wait_bounded(su32(&full[st]), (git / ns) & 1)) {
+          if (!tc::wait_warp(su32(&full[st]), (git / ns) & 1)) {
             s_fail = 1;
             atomicExch(sd.err, 3);
             ok = false;
@@ -529,29 +528,27 @@ __global__ void __launch_bounds__(SPLIT_SYN_WS_THREADS, CTAS) split_syn_ws(SphDe
           }
           s_consumed = git + 1;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          uint8_t *base = pipe + static_cast<size_t>(st) * slot_bytes;
+          const uint32_t base = pipe0 + st * slot_bytes;
+          const uint64_t ad = chunk_desc(base, sbo), bd = chunk_desc(base + sd.pieces * a_bytes, sbo);
           for (int kk = 0; kk < bk; kk += 16) {
             const int seg = c * bk + kk >= kseg ? 1 : 0;
-            const uint32_t accc = tmem + static_cast<uint32_t>(bb * buf_cols + (2 * g + seg) * nh);
-            for (int tt = t0; tt < 6; tt++) {
-              const int pa = tp[tt][0], pb = tp[tt][1];
-              const uint64_t ad = chunk_desc(su32(base + pa * a_bytes + (kk / 8) * 128), sbo);
-              const uint64_t bd = chunk_desc(su32(base + sd.pieces * a_bytes + pb * b_bytes + (kk / 8) * 128), sbo);
-              const uint32_t accum = started[seg] ? 1u : 0u;
-              asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(accc),
-                           "l"(ad), "l"(bd), "r"(idesc), "r"(accum)
-                           : "memory");
-              started[seg] = true;
+            const uint32_t accc = tm + static_cast<uint32_t>(bb * buf_cols + (2 * g + seg) * nh), bit = 1u << seg;
+#pragma unroll
+            for (int t = 0; t < 6; t++) {
+              if (t < t0) continue;
+              const int pa = t == 0 ? 2 : (t == 1 || t == 3 ? 1 : 0), pb = t == 2 ? 2 : (t == 1 || t == 4 ? 1 : 0);
+              tc::mma(leader, accc, ad + pa * a16 + kk, bd + pb * b16 + kk, idesc, started & bit ? 1u : 0u);
+              started |= bit;
             }
           }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(&empty[st])) : "memory");
+          tc::commit(leader, su32(&empty[st]));
         }
       }
       if (!ok) break;
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(&accf[bb])) : "memory");
+      tc::commit(leader, su32(&accf[bb]));
       it++;
     }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(&done)) : "memory");
+    tc::commit(leader, su32(&done));
   } else if (warp >= 2) {
     // epilogue warps
     const int et = tid - 64;
@@ -1496,6 +1493,7 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
   __shared__ uint32_t tslot;
   __shared__ int s_fail, s_issued, s_consumed, s_epi_ok;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int role = tc::uniform(warp);  // before any thread leaves its warp
   const int per_m = (BOTH ? 1 : 2) * sd.ntiles;
   const int nitems = d.M * per_m;
   const int nchunk = sd.nha / sd.bka;
@@ -1575,11 +1573,11 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
         }
       }
     }
-  } else if (tid == 32) {
-    // MMA issuer
-    const int tp[6][2] = {{2, 0}, {1, 1}, {0, 2}, {1, 0}, {0, 1}, {0, 0}};
+  } else if (role == 1) {
+    // MMA issuer (the whole warp, one lane issues)
     const int t0 = sd.terms == 6 ? 0 : (sd.terms == 3 ? 3 : 5);
-    const uint32_t sbo = static_cast<uint32_t>(bk) * 16u;
+    const uint32_t sbo = static_cast<uint32_t>(bk) * 16u, a16 = static_cast<uint32_t>(a_bytes) >> 4, pipe0 = su32(pipe), tm = tc::uniform(tmem);
+    const bool leader = tc::elect_one();
     int git = 0, it = 0;
     bool ok = true;
     for (int k = 0, item = snake_item(0); item < nitems && ok; item = snake_item(++k)) {
@@ -1588,23 +1586,23 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
       if ((s_first ? R1 : R0) == 0) continue;
       const int bb = it & 1;
       // the epilogue has copied out what this buffer held two items ago
-      if (it >= 2 && !mbar_wait_bounded(su32(&acce[bb]), ((it >> 1) - 1) & 1)) {
+      if (it >= 2 && !tc::wait_warp(su32(&acce[bb]), ((it >> 1) - 1) & 1)) {
         s_fail = 1;
         atomicExch(sd.err, 5);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int ra0 = sd.ra16[2 * m];
+      const int ra0 = tc::uniform(sd.ra16[2 * m]);
       const int cb1 = BOTH ? 2 * ra0 : 0;
       for (int s = s_first; s <= s_last && ok; s++) {
-        const int ra = sd.ra16[2 * m + s];
+        const int ra = tc::uniform(sd.ra16[2 * m + s]);
         const uint32_t idesc = idesc_m128(ra);
-        const int bbytes = ra * bk * 2;
+        const uint32_t b16 = static_cast<uint32_t>(ra * bk * 2) >> 4;
         for (int g = 0; g < 2 && ok; g++) {
-          const uint32_t accc = tmem + static_cast<uint32_t>(bb * buf_cols + (s ? cb1 : 0) + (g ? ra : 0));
+          const uint32_t accc = tm + static_cast<uint32_t>(bb * buf_cols + (s ? cb1 : 0) + (g ? ra : 0));
           for (int c = 0; c < nchunk; c++, git++) {
             const int st = git % ns;
-            if (!mbar_wait_bounded(su32(&full[st]), (git / ns) & 1)) {
+            if (!tc::wait_warp(su32(&full[st]), (git / ns) & 1)) {
               s_fail = 1;
               atomicExch(sd.err, 3);
               ok = false;
@@ -1612,28 +1610,26 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
             }
             s_consumed = git + 1;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint8_t *base = pipe + static_cast<size_t>(st) * slot_bytes;
+            const uint32_t base = pipe0 + st * slot_bytes;
+            const uint64_t ad = chunk_desc(base, sbo), bd = chunk_desc(base + sd.pieces * a_bytes, sbo);
             for (int kk = 0; kk < bk; kk += 16) {
-              for (int tt = t0; tt < 6; tt++) {
-                const int pa = tp[tt][0], pb = tp[tt][1];
-                const uint64_t ad = chunk_desc(su32(base + pa * a_bytes + (kk / 8) * 128), sbo);
-                const uint64_t bd = chunk_desc(su32(base + sd.pieces * a_bytes + pb * bbytes + (kk / 8) * 128), sbo);
-                const uint32_t accum = (c > 0 || kk > 0 || tt > t0) ? 1u : 0u;
-                asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(accc),
-                             "l"(ad), "l"(bd), "r"(idesc), "r"(accum)
-                             : "memory");
+#pragma unroll
+              for (int t = 0; t < 6; t++) {
+                if (t < t0) continue;
+                const int pa = t == 0 ? 2 : (t == 1 || t == 3 ? 1 : 0), pb = t == 2 ? 2 : (t == 1 || t == 4 ? 1 : 0);
+                tc::mma(leader, accc, ad + pa * a16 + kk, bd + pb * b16 + kk, idesc, c > 0 || kk > 0 || t > t0 ? 1u : 0u);
               }
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(&empty[st])) : "memory");
+            tc::commit(leader, su32(&empty[st]));
           }
         }
       }
       if (!ok) break;
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(&accf[bb])) : "memory");
+      tc::commit(leader, su32(&accf[bb]));
       it++;
     }
     // completes `done` when every MMA issued has finished (the drain after a failure waits on it)
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(&done)) : "memory");
+    tc::commit(leader, su32(&done));
   } else if (warp >= 2) {
     // epilogue warps
     const int et = tid - 64;

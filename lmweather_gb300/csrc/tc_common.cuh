@@ -41,6 +41,9 @@ __device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t phase, unsigned 
 }
 __device__ __forceinline__ bool wait(uint32_t bar, uint32_t phase) { return wait_for(bar, phase, WAIT_NS); }
 
+// the same by a whole warp, with one outcome for all its lanes
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t phase) { return __all_sync(0xffffffffu, wait(bar, phase)) != 0; }
+
 __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
@@ -79,6 +82,26 @@ __device__ __forceinline__ void mma(uint32_t dtmem, uint64_t ad, uint64_t bd, ui
                : "memory");
 }
 
+// The MMA role is a whole warp whose control flow is uniform, with the instruction predicated on one elected lane:
+// descriptors and addresses then stay in uniform registers, where the instruction takes them from. Issued by a lone
+// thread of a divergent branch, each MMA took about 115 cycles whatever its size.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+
+__device__ __forceinline__ void mma(bool leader, uint32_t dtmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem),
+               "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(leader))
+               : "memory");
+}
+__device__ __forceinline__ void commit(bool leader, uint32_t bar) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar),
+               "r"(static_cast<uint32_t>(leader))
+               : "memory");
+}
 __device__ __forceinline__ void commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
