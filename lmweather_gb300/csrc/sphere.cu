@@ -47,6 +47,7 @@ namespace {
 // pairs (T <= 42), whose launches would otherwise occupy a fraction of the SMs. The choice depends on the grid
 // only, so every member of a truncation is summed in the same order whatever the batch.
 constexpr int SYN_THREADS = 256, SYN_Q = 12;
+constexpr int SYN_STAGE = 342;  // coefficients of one m up to T341
 constexpr int SYN_CHUNKS = 8;  // n-sum pieces of the 32-latitude blocks (the tracer's synthesis uses this form)
 __host__ __device__ constexpr int syn_lats(int nh) { return nh <= 32 ? 8 : 32; }
 
@@ -61,21 +62,48 @@ __global__ void __launch_bounds__(SYN_THREADS) sph_synth(SphDev d, SphTab<R> t, 
   const int lane = threadIdx.x % LATS, c = threadIdx.x / LATS;
   const int jh = blockIdx.x * LATS + lane;
   const bool live = jh < d.nh;
-  const double2 *xz = x + static_cast<size_t>(b) * 3 * d.ntri, *xd = xz + d.ntri, *xf = xd + d.ntri;
   C2 sp = mk2(R(0), R(0)), sc = sp, hp = sp, hc = sp, zs = sp, fs = sp;
   const int base = d.tri[m];
-  pdl_wait();
+  pdl_wait(x);
+  const double2 *xz = x + static_cast<size_t>(b) * 3 * d.ntri, *xd = xz + d.ntri, *xf = xd + d.ntri;
+  // psi, chi, zeta, Phi of coefficient n: psi = -a^2/(n(n+1)) zeta, cpp/sphere.cpp:185-190. FP32: the state is rounded on
+  // the integer pipe (the hardware conversion's values)
+  auto coef = [&](int n, C2 &psi, C2 &chi, C2 &z, C2 &f) {
+    const int q = base + n - m;
+    const double2 zd = xz[q], dd = xd[q], fd = xf[q];
+    z = mk2(to_arith<R>(zd.x), to_arith<R>(zd.y));
+    f = mk2(to_arith<R>(fd.x), to_arith<R>(fd.y));
+    const C2 dl = mk2(to_arith<R>(dd.x), to_arith<R>(dd.y));
+    const R k = t.kfac[n];
+    psi = cscale(z, k);
+    chi = cscale(dl, k);
+  };
+  // FP32: formed once per block (the conversions of a thread's own would cost five times its multiply-adds)
+  __shared__ float4 stage[sizeof(R) == 4 ? 2 * SYN_STAGE : 1];
+  if constexpr (sizeof(R) == 4) {
+    for (int i = threadIdx.x; i <= d.N - m; i += SYN_THREADS) {
+      C2 psi, chi, z, f;
+      coef(m + i, psi, chi, z, f);
+      stage[2 * i] = make_float4(psi.x, psi.y, chi.x, chi.y);
+      stage[2 * i + 1] = make_float4(z.x, z.y, f.x, f.y);
+    }
+    __syncthreads();
+  }
   if (live) {
 #pragma unroll 2
     for (int n = m + c; n <= d.N; n += NCH) {
       const int q = base + n - m;
       const R P = t.Ps[static_cast<size_t>(q) * d.nh + jh], H = t.Hs[static_cast<size_t>(q) * d.nh + jh];
-      const double2 zd = xz[q], dd = xd[q], fd = xf[q];
-      // FP32: the state is rounded on the integer pipe (the hardware conversion's values)
-      const C2 z = mk2(to_arith<R>(zd.x), to_arith<R>(zd.y)), dl = mk2(to_arith<R>(dd.x), to_arith<R>(dd.y)),
-               f = mk2(to_arith<R>(fd.x), to_arith<R>(fd.y));
-      const R k = t.kfac[n];  // psi = -a^2/(n(n+1)) zeta, cpp/sphere.cpp:185-190
-      const C2 psi = cscale(z, k), chi = cscale(dl, k);
+      C2 psi, chi, z, f;
+      if constexpr (sizeof(R) == 4) {
+        const float4 u = stage[2 * (n - m)], w = stage[2 * (n - m) + 1];
+        psi = mk2(u.x, u.y);
+        chi = mk2(u.z, u.w);
+        z = mk2(w.x, w.y);
+        f = mk2(w.z, w.w);
+      } else {
+        coef(n, psi, chi, z, f);
+      }
       sp = cfma(sp, psi, P);
       sc = cfma(sc, chi, P);
       hp = cfma(hp, psi, H);
@@ -316,7 +344,7 @@ __global__ void __launch_bounds__(GRID_THREADS) sph_grid(SphDev d, SphTab<R> t, 
   C2 *sm = reinterpret_cast<C2 *>(smraw);
   const int b = blockIdx.y, jh = blockIdx.x;
   const int js = jh, jn = d.nlat - 1 - jh, n = d.nlon, rl = fft_row<3>(n);  // padded rows
-  pdl_wait();
+  pdl_wait(four, fgrid, hsgrid);
   const C2 *f_s = four + (static_cast<size_t>(b) * d.nlat + js) * 4 * d.M;
   const C2 *f_n = four + (static_cast<size_t>(b) * d.nlat + jn) * 4 * d.M;
   load_pair_spectra<C2, 3>(sm, 4, d, f_s, f_n, d.M);
@@ -392,6 +420,10 @@ __device__ __forceinline__ void fft64_twiddles(double2 *tw, int logn, const doub
     tw[e] = table[(e - (1 << st)) << (logn - 1 - st) & ((1 << (logn - 1)) - 1)];
   }
 }
+// -x or x, on the integer pipe: the compiler's negation by a condition was an FP64 operation (T170 grid: 61.9 -> 48.3 us)
+__device__ __forceinline__ double flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? static_cast<int>(0x80000000u) : 0), __double2loint(x));
+}
 template <bool INV> __device__ __forceinline__ void fft64(double2 *s, int logn, const double2 *tw) {
   const int n = 1 << logn;
   for (int st = 0; st < logn; st++) {
@@ -404,14 +436,13 @@ template <bool INV> __device__ __forceinline__ void fft64(double2 *s, int logn, 
       double x, y;
       if (st < 2) {
         // w = 1, or for the odd butterflies of stage 1 +i (inverse) or -i: i v = (-v.y, v.x)
-        const double t = lo == 0 ? (c ? v.y : v.x) : (c ? v.x : v.y);
-        const double ts = lo != 0 && (c == 0) == INV ? -t : t;
+        const double ts = flip(lo == 0 ? (c ? v.y : v.x) : (c ? v.x : v.y), lo != 0 && (c == 0) == INV);
         x = u + ts;
         y = u - ts;
       } else {
         // component c of w v (w conjugated for the inverse): w.x v.x - w.y v.y or w.x v.y + w.y v.x
         const double2 w = tw[h + lo];
-        const double a = c ? v.y : v.x, b = c ? v.x : v.y, wi = (c != 0) == INV ? -w.y : w.y;
+        const double a = c ? v.y : v.x, b = c ? v.x : v.y, wi = flip(w.y, (c != 0) == INV);
         x = fma(w.x, a, fma(wi, b, u));
         y = fma(2.0, u, -x);
       }
@@ -468,40 +499,47 @@ __device__ __forceinline__ void g64_fold(const double2 *s, const SphDev &d, doub
   }
 }
 
-// grid: (5 nh, B), clusters of five along x. T42, one member: 22.5 -> 8.5 us; T170: 64.5 -> 61.9 us; T42 x 16:
-// 57.4 -> 50.4 us
-__global__ void __launch_bounds__(256) sph_grid64(SphDev d, SphTab<double> t, const double2 *__restrict__ four, const double *__restrict__ fgrid,
-                                                  const double *__restrict__ hsgrid, double2 *__restrict__ fold) {
+// grid: (CTAS nh, B), clusters of CTAS along x. T42, one member: 22.5 -> 7.2 us; T170: 64.5 -> 48.3 us; T42 x 16:
+// 57.4 -> 41.5 us
+// CTAS = 8: with the tracer, whose q and delta (fourq [B][nlat][2][M]) are two more inverse transforms and U q, V q and q delta
+// three more products (foldq [B][nh][3][2][M]).
+template <int CTAS>
+__global__ void __launch_bounds__(256) sph_grid64(SphDev d, SphTab<double> t, const double2 *__restrict__ four, const double2 *__restrict__ fourq,
+                                                  const double *__restrict__ fgrid, const double *__restrict__ hsgrid, double2 *__restrict__ fold,
+                                                  double2 *__restrict__ foldq) {
+  constexpr int FIELDS = CTAS == 8 ? 6 : 4;
   extern __shared__ double2 g64_sm[];
   const int n = d.nlon;
   double2 *inv = g64_sm, *fwd = g64_sm + n, *tw = g64_sm + 2 * n;
-  const int r = static_cast<int>(cluster_rank()), jh = blockIdx.x / G64_CTAS, b = blockIdx.y;
+  const int r = static_cast<int>(cluster_rank()), jh = blockIdx.x / CTAS, b = blockIdx.y;
   const int js = jh, jn = d.nlat - 1 - jh;
   fft64_twiddles(tw, d.logn, t.tw);
-  if (r < 4)
+  if (r < FIELDS)
     for (int e = threadIdx.x; e < n; e += blockDim.x) inv[e] = make_double2(0.0, 0.0);
   const int gf = d.gflag[b];
   const double f0 = d.om2[b] * d.mu[js], r2om = t.r2om[js];  // 1 / (2 (1 - mu^2)); f0 and -f0 at the mirror latitudes
-  const double wt = r < 4 ? t.wd[js] : t.w[js];
+  const double wt = r == 4 || r == 7 ? t.w[js] : t.wd[js];
   __syncthreads();
-  pdl_wait();
-  if (r < 4) {
-    const double2 *f = four + static_cast<size_t>(b) * d.nlat * 4 * d.M + r * d.M;
-    g64_load(inv, d, f + static_cast<size_t>(js) * 4 * d.M, f + static_cast<size_t>(jn) * 4 * d.M);
+  pdl_wait(four, fourq, fgrid, hsgrid);
+  if (r < FIELDS) {
+    const int W = r < 4 ? 4 : 2;
+    const double2 *f = (r < 4 ? four : fourq) + static_cast<size_t>(b) * d.nlat * W * d.M + (r < 4 ? r : r - 4) * d.M;
+    g64_load(inv, d, f + static_cast<size_t>(js) * W * d.M, f + static_cast<size_t>(jn) * W * d.M);
     __syncthreads();
     fft64<true>(inv, d.logn, tw);
   }
   cluster_arrive();
   cluster_wait();
   // nonlinear products, cpp/sphere.cpp:348-359 (real part: southern latitude, imaginary part: northern): U eta, V eta,
-  // U Phi, V Phi, Phi + E, into bit-reversed order
+  // U Phi, V Phi, Phi + E (and U q, V q, q delta, cpp/sphere.cpp:255-258), into bit-reversed order
   const double *fr_s = fgrid + (static_cast<size_t>(b) * d.nlat + js) * n, *fr_n = fgrid + (static_cast<size_t>(b) * d.nlat + jn) * n;
   const double *hr_s = hsgrid + (static_cast<size_t>(b) * d.nlat + js) * n, *hr_n = hsgrid + (static_cast<size_t>(b) * d.nlat + jn) * n;
-  const uint32_t aU = cluster_map(inv, 0), aV = cluster_map(inv, 1), aY = cluster_map(inv, r < 2 ? 2 : 3);
+  const uint32_t aU = cluster_map(inv, 0), aV = cluster_map(inv, 1), aY = cluster_map(inv, r < 2 ? 2 : r < 5 ? 3 : 4);
+  const uint32_t aX = cluster_map(inv, r == 0 || r == 2 || r == 5 ? 0 : r == 7 ? 5 : 1);
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
     double2 y = cluster_load(aY, k), o;
-    if (r < 4) {
-      const double2 x = cluster_load((r & 1) ? aV : aU, k);
+    if (r != 4) {
+      const double2 x = cluster_load(aX, k);
       if (r < 2) {
         y.x += (gf & 1) ? fr_s[k] : f0;
         y.y += (gf & 1) ? fr_n[k] : -f0;
@@ -521,7 +559,7 @@ __global__ void __launch_bounds__(256) sph_grid64(SphDev d, SphTab<double> t, co
   __syncthreads();
   fft64<false>(fwd, d.logn, tw);
   pdl_trigger();
-  g64_fold(fwd, d, wt, fold + ((static_cast<size_t>(b) * d.nh + jh) * NSLOT + r) * 2 * d.M);
+  g64_fold(fwd, d, wt, r < NSLOT ? fold + ((static_cast<size_t>(b) * d.nh + jh) * NSLOT + r) * 2 * d.M : foldq + ((static_cast<size_t>(b) * d.nh + jh) * 3 + r - NSLOT) * 2 * d.M);
   cluster_wait();
 }
 
@@ -550,10 +588,22 @@ __global__ void __launch_bounds__(ANA_THREADS) sph_analysis(SphDev d, SphTab<R> 
   const int q = blockIdx.x * COEF + lane;
   const bool live = q < d.ntri;
   const int m = live ? d.trim[q] : 0, n = live ? d.trin[q] : 0, par = (n - m) & 1;
-  const C2 *fb = fold + static_cast<size_t>(b) * d.nh * NSLOT * 2 * d.M;
   const int sP = par * d.M + m, sH = (1 - par) * d.M + m;  // parity slot for P and H terms
   C2 aP = mk2(R(0), R(0)), bH = aP, bP = aP, aH = aP, uP = aP, vH = aP, eP = aP;
-  pdl_wait();
+  pdl_wait(fold, x0, xs, acc);
+  const C2 *fb = fold + static_cast<size_t>(b) * d.nh * NSLOT * 2 * d.M;
+  // field c of the three is updated by the threads of piece c. They read what the update needs ahead of the sums (T170: 28.9
+  // -> 16.1 us), but not where 32 pieces share a block, whose occupancy that costs (T42 x 64: 38.1 -> 46.8)
+  const size_t ix = (static_cast<size_t>(b) * 3 + c) * d.ntri + q;
+  const bool upd = live && c < 3;
+  double2 xv = make_double2(0.0, 0.0), av = xv;
+  R lap = R(0);
+  auto ahead = [&]() {
+    xv = x0[ix];
+    if (sa.stage > 0) av = acc[ix];
+    lap = t.lapl[n];
+  };
+  if (COEF == 32 && upd) ahead();
   if (live) {
 #pragma unroll 2
     for (int jh = c; jh < d.nh; jh += NCH) {
@@ -573,64 +623,43 @@ __global__ void __launch_bounds__(ANA_THREADS) sph_analysis(SphDev d, SphTab<R> 
   for (int i = 0; i < ANA_Q; i++) part[c][i][lane] = v[i];
   __syncthreads();
   pdl_trigger();
-  R tsum[ANA_Q];
-  if constexpr (NCH <= 8) {
-    if (c != 0 || !live) return;
-#pragma unroll
-    for (int i = 0; i < ANA_Q; i++) {
-      R acc_i = 0;
-#pragma unroll
-      for (int k = 0; k < NCH; k++) acc_i += part[k][i][lane];
-      tsum[i] = acc_i;
-    }
-  } else {
-    // many pieces: every thread sums one (value, coefficient) first, in the order of the pieces
-    __shared__ R red[ANA_Q][COEF];
-    for (int w = threadIdx.x; w < ANA_Q * COEF; w += ANA_THREADS) {
-      const int i = w / COEF, l = w % COEF;
-      R acc_i = 0;
-      for (int k = 0; k < NCH; k++) acc_i += part[k][i][l];
-      red[i][l] = acc_i;
-    }
-    __syncthreads();
-    if (c != 0 || !live) return;
-#pragma unroll
-    for (int i = 0; i < ANA_Q; i++) tsum[i] = red[i][lane];
+  // every thread sums one (value, coefficient) first, in the order of the pieces; then one field per thread
+  __shared__ R red[ANA_Q][COEF];
+  for (int w = threadIdx.x; w < ANA_Q * COEF; w += ANA_THREADS) {
+    const int i = w / COEF, l = w % COEF;
+    R acc_i = 0;
+    for (int k = 0; k < NCH; k++) acc_i += part[k][i][l];
+    red[i][l] = acc_i;
   }
+  __syncthreads();
+  if (!upd) return;
+  if (COEF != 32) ahead();
+  R tsum[ANA_Q];
+#pragma unroll
+  for (int i = 0; i < ANA_Q; i++) tsum[i] = red[i][lane];
   aP = mk2(tsum[0], tsum[1]); aH = mk2(tsum[2], tsum[3]); bP = mk2(tsum[4], tsum[5]); bH = mk2(tsum[6], tsum[7]);
   uP = mk2(tsum[8], tsum[9]); vH = mk2(tsum[10], tsum[11]); eP = mk2(tsum[12], tsum[13]);
   const R mm = static_cast<R>(m);
   // cpp/sphere.cpp:380-383: dz = -D(A,B), dd = D(B,-A) + n(n+1)/a^2 (Phi + E), df = -D(U Phi, V Phi)
   C2 kz = csub(bH, imul(aP, mm));
-  C2 kd = cadd(cadd(imul(bP, mm), aH), cscale(eP, t.lapl[n]));
+  C2 kd = cadd(cadd(imul(bP, mm), aH), cscale(eP, lap));
   C2 kf = csub(vH, imul(uP, mm));
   if (q == 0 || sa.zero) kz = kd = kf = mk2(R(0), R(0));  // cpp/sphere.cpp:387-389
-  const size_t base = static_cast<size_t>(b) * 3 * d.ntri + q;
-  // the RK4 state accumulates in FP64 whatever the precision of the tendencies (FP32 widened on the integer pipe)
-  const double2 k[3] = {make_double2(from_arith(kz.x), from_arith(kz.y)), make_double2(from_arith(kd.x), from_arith(kd.y)),
-                        make_double2(from_arith(kf.x), from_arith(kf.y))};
-  // every load of the three fields is issued before any store (the buffers never alias)
-  double2 xv[3], av[3];
-#pragma unroll
-  for (int f = 0; f < 3; f++) {
-    xv[f] = x0[base + static_cast<size_t>(f) * d.ntri];
-    av[f] = sa.stage > 0 ? acc[base + static_cast<size_t>(f) * d.ntri] : make_double2(0.0, 0.0);
-  }
-#pragma unroll
-  for (int f = 0; f < 3; f++) {
-    const size_t i = base + static_cast<size_t>(f) * d.ntri;
-    if (sa.stage == 0) {
-      acc[i] = k[f];
-      xs[i] = cadd(xv[f], cscale(k[f], sa.c));
-    } else if (sa.stage < 3) {
-      acc[i] = cadd(av[f], cscale(k[f], 2.0));
-      xs[i] = cadd(xv[f], cscale(k[f], sa.c));
-    } else {
-      // cpp/sphere.cpp:428-434: x += dt/6 (k1 + 2k2 + 2k3 + k4), then the del^4 filter
-      double2 val = cadd(xv[f], cscale(cadd(av[f], k[f]), sa.c));
-      const double fac = sa.filt[(f == 2 ? 1 : 0) * d.M + n];
-      x0[i] = q == 0 ? val : cscale(val, fac);
-    }
+  // field c of the three. The RK4 state accumulates in FP64 whatever the precision of the tendencies (FP32 widened on
+  // the integer pipe)
+  const C2 kr = c == 0 ? kz : (c == 1 ? kd : kf);
+  const double2 k = make_double2(from_arith(kr.x), from_arith(kr.y));
+  if (sa.stage == 0) {
+    acc[ix] = k;
+    xs[ix] = cadd(xv, cscale(k, sa.c));
+  } else if (sa.stage < 3) {
+    acc[ix] = cadd(av, cscale(k, 2.0));
+    xs[ix] = cadd(xv, cscale(k, sa.c));
+  } else {
+    // cpp/sphere.cpp:428-434: x += dt/6 (k1 + 2k2 + 2k3 + k4), then the del^4 filter
+    const double2 val = cadd(xv, cscale(cadd(av, k), sa.c));
+    const double fac = sa.filt[(c == 2 ? 1 : 0) * d.M + n];
+    x0[ix] = q == 0 ? val : cscale(val, fac);
   }
 }
 
@@ -1093,6 +1122,9 @@ static void allow_max_shared_memory() {
   if (done_for_device == dev) return;
   LMW_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const int dyn = optin - 2048;  // the kernels' static shared memory stays below 2 KB
+  LMW_CUDA(cudaFuncSetAttribute(sph_grid64<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(sph_grid64<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(trc_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(sph_grid<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(sph_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(sph_grid_in, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
@@ -1107,7 +1139,8 @@ static void allow_max_shared_memory() {
   LMW_CUDA(cudaFuncSetAttribute(tc64_syn<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_syn<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_ana<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_syn<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   for (int logn : {0, 6, 7, 8, 9, 10})
     for (int fmax : {3, 4})
       for (int direct : {0, 1}) LMW_CUDA(cudaFuncSetAttribute(split_grid_kernel(direct, fmax, logn), cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
@@ -1121,29 +1154,10 @@ static SphTab<float> tab32(const SphereTables &t) {
   return SphTab<float>{t.Ps32.p, t.Hs32.p, t.Pa32.p, t.Ha32.p, t.w32.p, t.wd32.p, t.r2om32.p, t.kfac32.p, t.lapl32.p, t.tw32.p};
 }
 
-// launch of a stage kernel (one that calls pdl_wait) that may start while its predecessor drains, in clusters of
-// `cluster` CTAs along x
-template <class... P, class... A>
-static void stage_launch(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, int cluster, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = cluster;
-  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
-  LMW_CUDA(cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...));
-}
-
 // the FP64 synthesis of `count` members
 static void syn64_launch(const SphDev &d, const Tc64Dev &z, size_t smem, int count, const double2 *x, double2 *four, cudaStream_t stream) {
-  stage_launch(tc64_syn<4>, dim3(z.nsl * ((count + z.nbt - 1) / z.nbt), d.M), T64_THREADS, smem, stream, 1, d, z, x, static_cast<const double2 *>(nullptr), four, count);
+  stage_launch(tc64_syn<4>, dim3(z.nsl * ((count + z.nbt - 1) / z.nbt), d.M), T64_THREADS, smem, stream, 1, d, z, x, static_cast<const double2 *>(nullptr), four,
+               static_cast<double2 *>(nullptr), count);
 }
 
 SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
@@ -1371,7 +1385,7 @@ void SphereEngine::synth_grids(int member_first, int count) {
   const size_t st = static_cast<size_t>(member_first) * 3 * ntri;
   const size_t fo = static_cast<size_t>(member_first) * nlat * 4 * M;
   if (tc64) {
-    syn64_launch(d, tc64_dev(*tc64, ntri + M), tc64->smem_syn, count, reinterpret_cast<const double2 *>(x0.p) + st, reinterpret_cast<double2 *>(four.p) + fo, stream);
+    syn64_launch(d, tc64_dev(*tc64, ntri + M), tc64->smem_syn(tc64->nbt), count, reinterpret_cast<const double2 *>(x0.p) + st, reinterpret_cast<double2 *>(four.p) + fo, stream);
     g_launches += 1;
     return;
   }
@@ -1690,27 +1704,34 @@ static void stage_kernels(const SphDev &d, const SphTab<R> &t, const Tc64Plan *t
   sa.zero = zero;
   const bool tc = sizeof(R) == 8 && tc64 != nullptr;
   const Tc64Dev z = tc ? tc64_dev(*tc64, d.ntri + d.M) : Tc64Dev{};
+  const double2 *none = nullptr;
+  double2 *mut = nullptr;
   if (which < 0 || which == 0) {
     const int L = syn_lats(d.nh);
     if constexpr (sizeof(R) == 8) {
-      if (tc) syn64_launch(d, z, tc64->smem_syn, B, in, four, stream);
+      if (tc) syn64_launch(d, z, tc64->smem_syn(z.nbt), B, in, four, stream);
     }
     if (!tc) stage_launch(L == 8 ? sph_synth<R, 8> : sph_synth<R, 32>, dim3((d.nh + L - 1) / L, d.M, B), SYN_THREADS, 0, stream, 1, d, t, in, four);
   }
   if (which < 0 || which == 1) {
     if constexpr (sizeof(R) == 8)
-      stage_launch(sph_grid64, dim3(G64_CTAS * d.nh, B), g64_threads(d.nlon), static_cast<size_t>(d.nlon) * 3 * sizeof(double2), stream, G64_CTAS, d, t,
-                   four, fgrid, hsgrid, fold);
+      stage_launch(sph_grid64<5>, dim3(G64_CTAS * d.nh, B), g64_threads(d.nlon), static_cast<size_t>(d.nlon) * 3 * sizeof(double2), stream, G64_CTAS, d, t,
+                   four, none, fgrid, hsgrid, fold, mut);
     else
       stage_launch(sph_grid<R>, dim3(d.nh, B), GRID_THREADS, 5 * static_cast<size_t>(fft_row<3>(d.nlon)) * sizeof(typename V2<R>::type), stream, 1, d, t,
                    four, fgrid, hsgrid, fold);
   }
   if (which < 0 || which == 2) {
-    const int C = ana_coef(d.nh);
+    // FP64 comes here above T170 only, where the blocks have 32 coefficients
+    const int C = sizeof(R) == 8 ? 32 : ana_coef(d.nh);
     if constexpr (sizeof(R) == 8) {
-      if (tc) stage_launch(tc64_ana<5>, dim3(B, d.M), T64_THREADS, tc64->smem_ana, stream, 1, d, z, fold, sa, x0, xs, acc);
+      if (tc) stage_launch(tc64_ana<5>, dim3(B, d.M), T64_THREADS, tc64->smem_ana, stream, 1, d, z, fold, sa, x0, xs, acc, none, mut, mut, mut);
     }
-    if (!tc) stage_launch(C == 8 ? sph_analysis<R, 8> : sph_analysis<R, 32>, dim3((d.ntri + C - 1) / C, B), ANA_THREADS, 0, stream, 1, d, t, fold, sa, x0, xs, acc);
+    auto *k = sph_analysis<R, 32>;
+    if constexpr (sizeof(R) == 4) {
+      if (C == 8) k = sph_analysis<R, 8>;
+    }
+    if (!tc) stage_launch(k, dim3((d.ntri + C - 1) / C, B), ANA_THREADS, 0, stream, 1, d, t, fold, sa, x0, xs, acc);
   }
 }
 
@@ -1787,6 +1808,26 @@ void SphereEngine::launch_stage(int stage, double dt) {
   if (p.precision == kFP64 && has_tracer) {
     // the tracer's kernels read the flow's stage input and its synthesised winds before the flow's analysis
     // overwrites the stage input
+    if (tc) {
+      // one launch each for the flow and the tracer together
+      StageArgs sa;
+      sa.stage = stage;
+      sa.c = stage < 2 ? 0.5 * dt : (stage == 2 ? dt : dt / 6);
+      sa.filt = filt.p;
+      sa.zero = advect_only ? 1 : 0;
+      const Tc64Dev z = tc64_dev(*tc, ntri + M);
+      const double2 *qin = reinterpret_cast<const double2 *>(stage == 0 ? tq0.p : tqs.p);
+      double2 *F = reinterpret_cast<double2 *>(four.p), *FQ = reinterpret_cast<double2 *>(fourq.p), *G = reinterpret_cast<double2 *>(fold.p),
+              *GQ = reinterpret_cast<double2 *>(foldq.p);
+      stage_launch(tc64_syn<6>, dim3(z.nsl * B, M), T64_THREADS, tc->smem_syn(2), stream, 1, d, z, in, qin, F, FQ, B);
+      stage_launch(sph_grid64<8>, dim3(8 * nh, B), g64_threads(nlon), static_cast<size_t>(nlon) * 3 * sizeof(double2), stream, 8, d, tab64(*tab), F, FQ, fgrid.p, hsgrid.p,
+                   G, GQ);
+      stage_launch(tc64_ana<8>, dim3(B, M), T64_THREADS, tc->smem_ana, stream, 1, d, z, G, sa, X0, XS, AC, GQ, reinterpret_cast<double2 *>(tq0.p),
+                   reinterpret_cast<double2 *>(tqs.p), reinterpret_cast<double2 *>(tqacc.p));
+      g_launches += 3;
+      LMW_LAUNCH_CHECK();
+      return;
+    }
     for (int k = 0; k < 3; k++) {
       stage_kernels<double>(d, tab64(*tab), tc, B, stage, dt, filt.p, in, reinterpret_cast<double2 *>(four.p), reinterpret_cast<double2 *>(fold.p),
                             X0, XS, AC, fgrid.p, hsgrid.p, stream, k, advect_only ? 1 : 0);
@@ -1831,7 +1872,8 @@ void SphereEngine::trc_syn_launch(const double2 *x, const double2 *q, double2 *d
   const SphDev d = make_sph(*this, *tab);
   if (tc64) {
     const Tc64Dev z = tc64_dev(*tc64, ntri + M);
-    stage_launch(tc64_syn<2>, dim3(z.nsl * ((count + z.nbt - 1) / z.nbt), M), T64_THREADS, tc64->smem_syn, stream, 1, d, z, x, q, dst, count);
+    stage_launch(tc64_syn<2>, dim3(z.nsl * ((count + z.nbt - 1) / z.nbt), M), T64_THREADS, tc64->smem_syn(z.nbt), stream, 1, d, z, x, q,
+                 static_cast<double2 *>(nullptr), dst, count);
   } else {
     stage_launch(trc_synth, dim3((nh + 31) / 32, M, count), SYN_THREADS, 0, stream, 1, d, tab64(*tab), x, q, dst);
   }
@@ -1852,11 +1894,7 @@ void SphereEngine::tracer_stage(int stage, double dt, int part) {
     sa.stage = stage;
     sa.c = stage < 2 ? 0.5 * dt : (stage == 2 ? dt : dt / 6);
     sa.filt = filt.p;
-    if (tc64)
-      stage_launch(tc64_ana<3>, dim3(B, M), T64_THREADS, tc64->smem_ana, stream, 1, d, tc64_dev(*tc64, ntri + M), reinterpret_cast<const double2 *>(foldq.p), sa,
-                   reinterpret_cast<double2 *>(tq0.p), reinterpret_cast<double2 *>(tqs.p), reinterpret_cast<double2 *>(tqacc.p));
-    else
-      stage_launch(trc_analysis, dim3((ntri + 31) / 32, B), ANA_THREADS, 0, stream, 1, d, tab64(*tab), reinterpret_cast<const double2 *>(foldq.p), sa,
+    stage_launch(trc_analysis, dim3((ntri + 31) / 32, B), ANA_THREADS, 0, stream, 1, d, tab64(*tab), reinterpret_cast<const double2 *>(foldq.p), sa,
                  reinterpret_cast<double2 *>(tq0.p), reinterpret_cast<double2 *>(tqs.p), reinterpret_cast<double2 *>(tqacc.p));
   }
   LMW_LAUNCH_CHECK();

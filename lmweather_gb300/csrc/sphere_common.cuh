@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "pdl.cuh"
+
 namespace lmw {
 namespace {
 
@@ -81,12 +83,6 @@ template <> __device__ __forceinline__ float to_arith<float>(double x) { return 
 // a value of the kernel's arithmetic type widened to double: itself for FP64, f2d_int (exact) for FP32
 __device__ __forceinline__ double from_arith(double x) { return x; }
 __device__ __forceinline__ double from_arith(float x) { return f2d_int(x); }
-
-// Programmatic dependent launch: a stage kernel may start while its predecessor drains; it waits here (everything the
-// predecessor wrote is then visible) before it touches anything an earlier kernel writes, and lets its successor start
-// when only its outputs are left. Without the launch attribute both do nothing.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 constexpr int NSLOT = 5;  // A, B, U Phi, V Phi (times w/((1-mu^2)a)) and the Bernoulli function (times w)
 

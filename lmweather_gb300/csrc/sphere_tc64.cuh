@@ -36,7 +36,8 @@ struct Tc64Plan {
   int nh16 = 16, lrows = 16, nsl = 1, nhk = 16, ns = 3;  // padded latitude pairs, per slice, slices; K of the analysis; stages
   int nbt = 1, ntiles = 1;                               // members per synthesis tile
   int kc_max = 1, ra_max = 16;
-  size_t smem_syn = 0, smem_ana = 0;
+  size_t smem_ana = 0;
+  size_t smem_syn(int blocks) const;  // row blocks of eight rows (members; two with the tracer)
   DevBuf<__nv_bfloat16> tS, tA;
   DevBuf<int> ke16, kc, ra16;    // synthesis: padded even columns, K chunks of 16; analysis: padded rows of (m, parity)
   DevBuf<long> oS, oA;           // table offsets (elements)
@@ -58,9 +59,9 @@ namespace {
 
 constexpr int T64_DIG = 8, T64_THREADS = 256;
 constexpr int T64_NONE = -100000, T64_NAN = 100000;  // row exponents: no digits; not finite
-// A operand: core matrices 144 bytes apart along K and 288 between 8-row groups (the 16 spare bytes put the stores of
-// neighbouring columns on different banks)
-constexpr int T64_LBO = 144, T64_SBO = 288;
+// A operand: core matrices 128 bytes apart along K and 256 between 8-row groups. The digits' stores meet four to a bank;
+// with 16 spare bytes between core matrices they do not, which changed no time (T42 x 16, T170: within 2 %)
+constexpr int T64_LBO = 128, T64_SBO = 256;
 
 // biased exponent of |v| (0 for subnormals and zero)
 __device__ __forceinline__ int t64_exp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
@@ -218,22 +219,23 @@ __device__ __forceinline__ bool t64_copy(T64Bars &b, uint8_t *stages, int stage_
   b.issued = it + 1;
   return true;
 }
-// MMA step: the eight table digits of stage it % ns (rows: N) against the A block at `a` (its first real row group zg
-// groups further down, gpo groups per digit), accumulated at `acc`
-__device__ __forceinline__ bool t64_mma(T64Bars &b, uint8_t *stages, int stage_bytes, int ns, int it, int N, uint32_t a, int gpo, uint32_t acc, bool first,
-                                        int *err) {
+// MMA step, by a whole warp (`leader`: its issuing lane): the eight table digits of stage it % ns (rows: N) against the A
+// block at `a` (its first real row group 7 gpo groups further down, gpo groups per digit), accumulated at `acc`
+__device__ __forceinline__ bool t64_mma(T64Bars &b, uint32_t stages, int stage_bytes, int ns, int it, int N, uint32_t a, int gpo, uint32_t acc, bool first,
+                                        bool leader, int *err) {
   const int st = it % ns;
-  if (!tc::wait(tc::su32(&b.full[st]), (it / ns) & 1)) {
+  if (!tc::wait_warp(tc::su32(&b.full[st]), (it / ns) & 1)) {
     t64_failed(b, err, 12);
     return false;
   }
-  b.consumed = it + 1;
   tc::fence_after();
-  const uint32_t bb = tc::su32(stages + static_cast<size_t>(st) * stage_bytes), idesc = tc::idesc_m128(N);
+  const uint64_t ad = t64_desc(a + 7 * gpo * T64_SBO, T64_LBO, T64_SBO), bd = t64_desc(stages + st * stage_bytes, 128, 256);
+  const uint32_t idesc = tc::idesc_m128(N);
+  b.consumed = it + 1;
 #pragma unroll
   for (int j = 0; j < T64_DIG; j++)
-    tc::mma(acc, t64_desc(a + (7 - j) * gpo * T64_SBO, T64_LBO, T64_SBO), t64_desc(bb + j * N * 32, 128, 256), idesc, first && j == 0 ? 0u : 1u);
-  tc::commit(tc::su32(&b.empty[st]));
+    tc::mma(leader, acc, ad - static_cast<uint64_t>(j * gpo * (T64_SBO / 16)), bd + static_cast<uint64_t>(j * N * 2), idesc, first && j == 0 ? 0u : 1u);
+  tc::commit(leader, tc::su32(&b.empty[st]));
   return true;
 }
 // after the roles have met: wait for every MMA; after a failure a bounded wait for what is in flight. True when all is well
@@ -272,17 +274,20 @@ __device__ __forceinline__ void t64_unload(uint32_t taddr, int w, int *dst, bool
 }
 
 // ------------------------------------------------------------------------------------------------ synthesis
-// grid: (slices x tiles, M). F = 4: U, V, zeta, Phi of x [B][3][ntri] into four [B][nlat][4][M]; F = 2 (tracer): q of qin
-// [B][ntri] and delta of x into [B][nlat][2][M].
-// T170, one member: 82.0 -> 19.0 us (FP64 pipe before); T42 x 16: 50.4 -> 11.7; T42, one member: 10.3 -> 7.5.
+// grid: (slices x tiles, M). F = 4: U, V, zeta, Phi of x [B][3][ntri] into four [B][nlat][4][M], nbt members a tile; F = 2: the
+// tracer's q of qin [B][ntri] and delta of x into fourq [B][nlat][2][M]; F = 6: both in one launch, one member a tile, whose
+// second row block is q and delta.
+// T170, one member: 82.0 -> 18.7 us (FP64 pipe before); T42 x 16: 50.4 -> 11.6; T42, one member: 10.3 -> 6.9.
 template <int F>
 __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, const double2 *__restrict__ x, const double2 *__restrict__ qin,
-                                                           double2 *__restrict__ four, int B) {
+                                                           double2 *__restrict__ four, double2 *__restrict__ fourq, int B) {
   extern __shared__ __align__(1024) uint8_t t64_sm[];
   __shared__ __align__(8) T64Bars bars;
-  __shared__ int rowexp[2][F];
+  constexpr int RF = F == 2 ? 2 : 4;  // complex values of a row block
+  __shared__ int rowexp[2][RF];
   const int tid = threadIdx.x, m = blockIdx.y, sl = blockIdx.x % z.nsl, tile = blockIdx.x / z.nsl;
-  const int L = z.lrows, kc = z.kc[m], ke16 = z.ke16[m], nbt = z.nbt, mt = min(nbt, B - tile * nbt), groups = 15 * nbt;
+  // nbt row blocks: members, or the flow and the tracer of one
+  const int L = z.lrows, kc = z.kc[m], ke16 = z.ke16[m], nbt = F == 6 ? 2 : z.nbt, mt = F == 6 ? 2 : min(nbt, B - tile * nbt), groups = 15 * nbt;
   const int stage_bytes = T64_DIG * L * 32, ablk = groups * T64_SBO;
   uint8_t *stages = t64_sm;
   uint8_t *A = t64_sm + max(z.ns * stage_bytes, static_cast<int>(2 * 64 * nbt * (min(L, 32) + 1) * sizeof(int)));
@@ -297,23 +302,24 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
     const int blk = e / (7 * nbt * (T64_SBO / 16)), o = e % (7 * nbt * (T64_SBO / 16));
     *reinterpret_cast<uint4 *>(A + blk * ablk + o * 16) = make_uint4(0, 0, 0, 0);
   }
-  if (tid < 2 * F) rowexp[tid / F][tid % F] = 0;
+  if (tid < 2 * RF) rowexp[tid / RF][tid % RF] = 0;
   __syncthreads();
-  pdl_wait();
+  pdl_wait(x, qin);
   // thread k: column k, n = m + 2 k or m + 1 + 2 (k - ke16); the values of member ml in v[0..2F)
   const int k = tid, n = k < ke16 ? m + 2 * k : m + 1 + 2 * (k - ke16), base = d.tri[m] - m;
   const bool col = k < kc * 16, live = col && n <= d.N + 1;
   const double *cf = z.cf + d.tri[m] + n;  // ext index of (m, n): tri[m] + m + n - m
   for (int ml = 0; ml < nbt; ml++) {
-    double v[2 * F];
+    double v[2 * RF];
 #pragma unroll
-    for (int q = 0; q < 2 * F; q++) v[q] = 0;
+    for (int q = 0; q < 2 * RF; q++) v[q] = 0;
+    const bool flow = F == 4 || (F == 6 && ml == 0);
     if (live && ml < mt) {
-      const int b = tile * nbt + ml;
+      const int b = F == 6 ? tile : tile * nbt + ml;
       const double2 *xz = x + static_cast<size_t>(b) * 3 * d.ntri + base, *xd = xz + d.ntri, *xf = xd + d.ntri;
       const double2 zero = make_double2(0.0, 0.0);
       const double2 dn = n <= d.N ? xd[n] : zero;
-      if constexpr (F == 4) {
+      if (F >= 4 && flow) {
         // U_n = -a [i m delta_n / (n (n+1)) + eps_n zeta_{n-1} / n - eps_{n+1} zeta_{n+1} / (n+1)], V_n the same with zeta_n,
         // -delta_{n-1}, -delta_{n+1}; the (0, 0) coefficients have no wind
         const double w0 = cf[0], w1 = cf[z.ext], w2 = cf[2 * z.ext];
@@ -324,10 +330,12 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
         v[1] = fma(-w0, dn.x, fma(w2, zu.y, -(w1 * zl.y)));
         v[2] = fma(w0, zn.y, fma(w1, dl.x, -(w2 * du.x)));
         v[3] = fma(-w0, zn.x, fma(w1, dl.y, -(w2 * du.y)));
-        v[4] = zn.x;
-        v[5] = zn.y;
-        v[6] = fn.x;
-        v[7] = fn.y;
+        if constexpr (F >= 4) {
+          v[4] = zn.x;
+          v[5] = zn.y;
+          v[6] = fn.x;
+          v[7] = fn.y;
+        }
       } else {
         const double2 qn = n <= d.N ? qin[static_cast<size_t>(b) * d.ntri + base + n] : zero;
         v[0] = qn.x;
@@ -338,7 +346,7 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
     }
     if (tid < ((kc * 16 + 31) & ~31)) {
 #pragma unroll
-      for (int f = 0; f < F; f++) {
+      for (int f = 0; f < RF; f++) {
         const int ex = __reduce_max_sync(0xffffffffu, max(t64_exp(v[2 * f]), t64_exp(v[2 * f + 1])));
         if ((tid & 31) == 0) atomicMax(&rowexp[ml][f], ex);
       }
@@ -347,7 +355,8 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
     if (col) {
       uint8_t *o = A + (k >> 4) * ablk + (7 * nbt + ml) * T64_SBO + ((k & 15) >> 3) * T64_LBO + (k & 7) * 2;
 #pragma unroll
-      for (int q = 0; q < 2 * F; q++) {
+      for (int q = 0; q < 2 * RF; q++) {
+        if (F == 6 && !flow && q >= 4) break;
         unsigned short dg[T64_DIG];
         t64_digits(t64_fixed(v[q], t64_row(rowexp[ml][q >> 1])), dg);
 #pragma unroll
@@ -358,14 +367,17 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
   const uint32_t tmem = bars.tslot;
+  const int role = tc::uniform(tid >> 5);
   if (tid == 0) {
     for (; copied < kc; copied++)
       if (!t64_copy(bars, stages, stage_bytes, z.ns, copied, src + static_cast<long>(copied) * T64_DIG * L * 16, stage_bytes, z.err)) break;
-  } else if (tid == 32) {
+  } else if (role == 1) {
     const int even = ke16 / 16;
+    const uint32_t s0 = tc::su32(stages), a0 = tc::su32(A), t0 = tc::uniform(tmem);
+    const bool leader = tc::elect_one();
     for (int c = 0; c < kc; c++)
-      if (!t64_mma(bars, stages, stage_bytes, z.ns, c, L, tc::su32(A + c * ablk), nbt, tmem + (c < even ? 0 : L), c == 0 || c == even, z.err)) break;
-    tc::commit(tc::su32(&bars.done));
+      if (!t64_mma(bars, s0, stage_bytes, z.ns, c, L, a0 + c * ablk, nbt, t0 + (c < even ? 0 : L), c == 0 || c == even, leader, z.err)) break;
+    tc::commit(leader, tc::su32(&bars.done));
   }
   const bool ok = t64_finish(bars, z.ns, z.err);
   pdl_trigger();
@@ -376,8 +388,8 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
     if (quarter * 32 < rows)
       t64_unload(tmem + (warp < 4 ? 0 : L) + cb + (static_cast<uint32_t>(quarter * 32) << 16), w, red + ((warp < 4 ? 0 : rows) + row) * ld, row < rows);
     __syncthreads();
-    for (int e = tid; e < mt * F * w; e += T64_THREADS) {
-      const int i = e % w, f = (e / w) % F, ml = e / (w * F), jh = sl * L + cb + i;
+    for (int e = tid; e < (F == 6 ? 6 : mt * F) * w; e += T64_THREADS) {
+      const int i = e % w, v = e / w, f = F == 6 ? v & 3 : v % F, ml = F == 6 ? v >> 2 : v / F, jh = sl * L + cb + i;
       if (jh >= d.nh) continue;
       const int ea = t64_row(rowexp[ml][f]), eb = z.eS[m * z.nh16 + jh];
       double so[2], no[2];
@@ -388,9 +400,12 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
         so[ri] = t64_value(ev.hi + od.hi, ev.lo + od.lo, ea, eb);
         no[ri] = t64_value(ev.hi - od.hi, ev.lo - od.lo, ea, eb);
       }
-      const size_t bo = static_cast<size_t>(tile * nbt + ml) * d.nlat;
-      four[((bo + jh) * F + f) * d.M + m] = make_double2(so[0], so[1]);
-      four[((bo + d.nlat - 1 - jh) * F + f) * d.M + m] = make_double2(no[0], no[1]);
+      const bool trc = F == 2 || (F == 6 && ml == 1);
+      const size_t bo = static_cast<size_t>(F == 6 ? tile : tile * nbt + ml) * d.nlat;
+      const int W = trc ? 2 : 4;
+      double2 *o = (trc ? fourq : four) + f * d.M + m;
+      o[(bo + jh) * W * d.M] = make_double2(so[0], so[1]);
+      o[(bo + d.nlat - 1 - jh) * W * d.M] = make_double2(no[0], no[1]);
     }
     __syncthreads();
   }
@@ -398,13 +413,14 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
 }
 
 // ------------------------------------------------------------------------------------------------ analysis + RK4
-// grid: (B, M). SLOTS = 5: the flow (fold [B][nh][5][2][M]; x0, xs, acc [B][3][ntri]); SLOTS = 3: the tracer (U q, V q, q delta;
-// x0, xs, acc [B][ntri]).
-// T170, one member: 71.7 -> 33.8 us; T42 x 16: 45.1 -> 29.8; T42, one member: 8.2 -> 9.4.
+// grid: (B, M). SLOTS = 5: the flow (fold [B][nh][5][2][M]; x0, xs, acc [B][3][ntri]); SLOTS = 8: with the tracer (foldq
+// [B][nh][3][2][M]: U q, V q, q delta; q0, qs, qacc [B][ntri]).
+// T170, one member: 71.7 -> 29.6 us; T42 x 16: 45.1 -> 29.7; T42, one member: 8.2 -> 8.8.
 template <int SLOTS>
 __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, const double2 *__restrict__ fold, StageArgs sa, double2 *__restrict__ x0,
-                                                           double2 *__restrict__ xs, double2 *__restrict__ acc) {
-  constexpr int Q = 2 * SLOTS, FIELDS = SLOTS == 5 ? 3 : 1, GPO = SLOTS == 5 ? 2 : 1;  // row groups per digit
+                                                           double2 *__restrict__ xs, double2 *__restrict__ acc, const double2 *__restrict__ foldq,
+                                                           double2 *__restrict__ q0, double2 *__restrict__ qs, double2 *__restrict__ qacc) {
+  constexpr int Q = 2 * SLOTS, FIELDS = SLOTS == 8 ? 4 : 3, GPO = 2;  // GPO: row groups per digit
   extern __shared__ __align__(1024) uint8_t t64_sm[];
   __shared__ __align__(8) T64Bars bars;
   __shared__ int rowexp[2][Q];
@@ -426,24 +442,25 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
   }
   if (tid < 2 * Q) rowexp[tid / Q][tid % Q] = 0;
   __syncthreads();
-  pdl_wait();
+  pdl_wait(fold, foldq, x0, xs, acc, q0, qs, qacc);
   // thread: latitude pair jh at parity p of the fold
   const int p = tid / z.nhk, jh = tid % z.nhk;
   const bool col = p < 2;
   double v[Q];
 #pragma unroll
   for (int s = 0; s < SLOTS; s++) {
-    const double2 g = col && jh < d.nh ? fold[((static_cast<size_t>(b) * d.nh + jh) * SLOTS + s) * 2 * d.M + p * d.M + m] : make_double2(0.0, 0.0);
+    const double2 *src = s < 5 ? fold + ((static_cast<size_t>(b) * d.nh + jh) * 5 + s) * 2 * d.M : foldq + ((static_cast<size_t>(b) * d.nh + jh) * 3 + s - 5) * 2 * d.M;
+    const double2 g = col && jh < d.nh ? src[p * d.M + m] : make_double2(0.0, 0.0);
     v[2 * s] = g.x;
     v[2 * s + 1] = g.y;
   }
   if (col) {
-    const bool whole = z.nhk >= 32;  // a warp has one parity
+    // latitude pairs are padded to 16: a half warp has one parity
+    const unsigned half = 0xffffu << (tid & 16);
 #pragma unroll
     for (int q = 0; q < Q; q++) {
-      int ex = t64_exp(v[q]);
-      if (whole) ex = __reduce_max_sync(0xffffffffu, ex);
-      if (!whole || (tid & 31) == 0) atomicMax(&rowexp[p][q], ex);
+      const int ex = __reduce_max_sync(half, t64_exp(v[q]));
+      if ((tid & 15) == 0) atomicMax(&rowexp[p][q], ex);
     }
   }
   __syncthreads();
@@ -460,13 +477,38 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
   const uint32_t tmem = bars.tslot;
+  const int role = tc::uniform(tid >> 5);
   if (tid == 0) {
     for (; copied < 2 * kc; copied++)
       if (!t64_copy(bars, stages, stage_bytes, z.ns, copied, chunk(copied), bytes(copied), z.err)) break;
-  } else if (tid == 32) {
+  } else if (role == 1) {
+    const uint32_t s0 = tc::su32(stages), a0 = tc::su32(A), t0 = tc::uniform(tmem);
+    const bool leader = tc::elect_one();
     for (int it = 0; it < 2 * kc; it++)
-      if (!t64_mma(bars, stages, stage_bytes, z.ns, it, it < kc ? ra0 : ra1, tc::su32(A + it * ablk), GPO, tmem + (it < kc ? 0 : ra0), it == 0 || it == kc, z.err)) break;
-    tc::commit(tc::su32(&bars.done));
+      if (!t64_mma(bars, s0, stage_bytes, z.ns, it, it < kc ? ra0 : ra1, a0 + it * ablk, GPO, t0 + (it < kc ? 0 : ra0), it == 0 || it == kc, leader, z.err)) break;
+    tc::commit(leader, tc::su32(&bars.done));
+  }
+  // item e of the update: field e / cnt, n = m + e % cnt. What it reads is loaded while the MMAs run
+  const int cnt = d.N + 1 - m;
+  // field f of item i: the flow's three, then the tracer
+  auto place = [&](int f, int i) { return (f < 3 ? static_cast<size_t>(b) * 3 + f : static_cast<size_t>(b)) * d.ntri + d.tri[m] + i; };
+  constexpr int ITEMS = (FIELDS * 171 + T64_THREADS - 1) / T64_THREADS;
+  double2 xv[ITEMS], av[ITEMS];
+  double w3[ITEMS], w4[ITEMS], lap[ITEMS], fac[ITEMS];
+#pragma unroll
+  for (int r = 0; r < ITEMS; r++) {
+    const int e = tid + r * T64_THREADS, f = e / cnt, i = e - f * cnt;
+    xv[r] = av[r] = make_double2(0.0, 0.0);
+    w3[r] = w4[r] = lap[r] = fac[r] = 0;
+    if (f < FIELDS) {
+      const size_t o = place(f, i);
+      xv[r] = (f < 3 ? x0 : q0)[o];
+      if (sa.stage > 0) av[r] = (f < 3 ? acc : qacc)[o];
+      w3[r] = z.cf[3 * z.ext + d.tri[m] + m + i];
+      w4[r] = z.cf[4 * z.ext + d.tri[m] + m + i];
+      if (f == 1) lap[r] = d.lapl[m + i];
+      if (sa.stage == 3) fac[r] = sa.filt[(f >= 2 ? 1 : 0) * d.M + m + i];
+    }
   }
   const bool ok = t64_finish(bars, z.ns, z.err);
   pdl_trigger();
@@ -491,45 +533,35 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
   }
   if (ok) {
     const double mm = static_cast<double>(m);
-    const size_t mb = static_cast<size_t>(b) * FIELDS * d.ntri;
-    for (int i = tid; i < d.N + 1 - m; i += T64_THREADS) {
-      const int n = m + i, q = d.tri[m] + i;
-      const double w3 = z.cf[3 * z.ext + d.tri[m] + n], w4 = z.cf[4 * z.ext + d.tri[m] + n];
+#pragma unroll
+    for (int r = 0; r < ITEMS; r++) {
+      const int e = tid + r * T64_THREADS, f = e / cnt, i = e - f * cnt, q = d.tri[m] + i;
+      if (f >= FIELDS) continue;
       auto at = [&](int s) { return make_double2(S[2 * s * sld + i], S[(2 * s + 1) * sld + i]); };
       // the H sum: -n eps_{n+1} S(n+1) + (n+1) eps_n S(n-1)
       auto deriv = [&](int s) {
         const double2 u = make_double2(S[2 * s * sld + i + 1], S[(2 * s + 1) * sld + i + 1]);
         const double2 l = i > 0 ? make_double2(S[2 * s * sld + i - 1], S[(2 * s + 1) * sld + i - 1]) : make_double2(0.0, 0.0);
-        return make_double2(fma(w4, l.x, -(w3 * u.x)), fma(w4, l.y, -(w3 * u.y)));
+        return make_double2(fma(w4[r], l.x, -(w3[r] * u.x)), fma(w4[r], l.y, -(w3[r] * u.y)));
       };
-      double2 kk[FIELDS];
-      if constexpr (SLOTS == 5) {
+      double2 k;
+      if (f < 3) {
         // cpp/sphere.cpp:380-383: dz = -D(A,B), dd = D(B,-A) + n(n+1)/a^2 (Phi + E), df = -D(U Phi, V Phi)
-        kk[0] = csub(deriv(1), imul(at(0), mm));
-        kk[1] = cadd(cadd(imul(at(1), mm), deriv(0)), cscale(at(4), d.lapl[n]));
-        kk[2] = csub(deriv(3), imul(at(2), mm));
-        if (q == 0 || sa.zero) kk[0] = kk[1] = kk[2] = make_double2(0.0, 0.0);  // cpp/sphere.cpp:387-389
+        // slots: A, B, U Phi, V Phi, Phi + E; the zonal terms take A, B, U Phi, the others B, A, V Phi
+        const double2 dv = deriv(f == 0 ? 1 : f == 1 ? 0 : 3), iv = imul(at(f), mm);
+        k = f == 1 ? cadd(cadd(iv, dv), cscale(at(4), lap[r])) : csub(dv, iv);
+        if (q == 0 || sa.zero) k = make_double2(0.0, 0.0);  // cpp/sphere.cpp:387-389
       } else {
-        kk[0] = cadd(at(2), csub(deriv(1), imul(at(0), mm)));  // cpp/sphere.cpp:250-263
+        k = cadd(at(7), csub(deriv(6), imul(at(5), mm)));  // dq = A(q delta) - D(U q, V q), cpp/sphere.cpp:250-263
       }
-      double2 xv[FIELDS], av[FIELDS];
-#pragma unroll
-      for (int f = 0; f < FIELDS; f++) {
-        xv[f] = x0[mb + static_cast<size_t>(f) * d.ntri + q];
-        av[f] = sa.stage > 0 ? acc[mb + static_cast<size_t>(f) * d.ntri + q] : make_double2(0.0, 0.0);
-      }
-#pragma unroll
-      for (int f = 0; f < FIELDS; f++) {
-        const size_t o = mb + static_cast<size_t>(f) * d.ntri + q;
-        if (sa.stage < 3) {
-          acc[o] = sa.stage == 0 ? kk[f] : make_double2(fma(2.0, kk[f].x, av[f].x), fma(2.0, kk[f].y, av[f].y));
-          xs[o] = make_double2(fma(sa.c, kk[f].x, xv[f].x), fma(sa.c, kk[f].y, xv[f].y));
-        } else {
-          // cpp/sphere.cpp:428-434: x += dt/6 (k1 + 2k2 + 2k3 + k4), then the del^4 filter (the tracer: Phi's)
-          const double2 val = make_double2(fma(sa.c, av[f].x + kk[f].x, xv[f].x), fma(sa.c, av[f].y + kk[f].y, xv[f].y));
-          const double fac = sa.filt[(FIELDS == 1 || f == 2 ? 1 : 0) * d.M + n];
-          x0[o] = q == 0 ? val : cscale(val, fac);
-        }
+      const size_t o = place(f, i);
+      if (sa.stage < 3) {
+        (f < 3 ? acc : qacc)[o] = sa.stage == 0 ? k : make_double2(fma(2.0, k.x, av[r].x), fma(2.0, k.y, av[r].y));
+        (f < 3 ? xs : qs)[o] = make_double2(fma(sa.c, k.x, xv[r].x), fma(sa.c, k.y, xv[r].y));
+      } else {
+        // cpp/sphere.cpp:428-434: x += dt/6 (k1 + 2k2 + 2k3 + k4), then the del^4 filter (the tracer: Phi's)
+        const double2 val = make_double2(fma(sa.c, av[r].x + k.x, xv[r].x), fma(sa.c, av[r].y + k.y, xv[r].y));
+        (f < 3 ? x0 : q0)[o] = q == 0 ? val : cscale(val, fac[r]);
       }
     }
   }
@@ -542,6 +574,12 @@ inline Tc64Dev tc64_dev(const Tc64Plan &p, int ext) {
   return Tc64Dev{p.nh16, p.lrows, p.nsl, p.nhk, p.ns, p.nbt, p.ntiles, p.ra_max, ext, p.tS.p, p.tA.p, p.ke16.p, p.kc.p, p.ra16.p, p.eS.p, p.eA.p, p.oS.p, p.oA.p, p.cf.p, p.err.p};
 }
 
+// an M = 128 MMA reads sixteen row groups from its A block: with one row block of eight rows up to eight past the fifteen
+inline size_t Tc64Plan::smem_syn(int blocks) const {
+  const size_t red = static_cast<size_t>(2 * 64 * blocks) * (std::min(lrows, 32) + 1) * sizeof(int);
+  return std::max(static_cast<size_t>(ns) * T64_DIG * lrows * 32, red) + static_cast<size_t>(kc_max) * 15 * blocks * T64_SBO + 8 * T64_SBO + 256;
+}
+
 // sizes, offsets and tables for members B (the digits are cut on the device from the FP64 tables)
 inline void build_tc64(Tc64Plan &p, const HostTables &h, const SphDev &d, double radius, int B, cudaStream_t stream) {
   const int N = h.N, M = h.M, nh = h.nh, ext = h.ntri + M;
@@ -549,8 +587,6 @@ inline void build_tc64(Tc64Plan &p, const HostTables &h, const SphDev &d, double
   p.lrows = std::min(p.nh16, 64);
   p.nsl = p.nh16 / p.lrows;
   p.nhk = pad16(nh);
-  p.nbt = B > 1 ? 2 : 1;
-  p.ntiles = (B + p.nbt - 1) / p.nbt;
   std::vector<int> ke16(M), kc(M), ra16(2 * M);
   std::vector<long> oS(M), oA(2 * M);
   long ts = 0, ta = 0;
@@ -596,12 +632,11 @@ inline void build_tc64(Tc64Plan &p, const HostTables &h, const SphDev &d, double
   p.eA.alloc(ext);
   p.err.alloc(1);
   p.err.p[0] = 0;
-  // an M = 128 MMA reads sixteen row groups from its A block: up to eight past the fifteen of one-group digits
-  const size_t margin = 8 * T64_SBO + 256;
-  const size_t red_syn = static_cast<size_t>(2 * 64 * p.nbt) * (std::min(p.lrows, 32) + 1) * sizeof(int);
-  p.smem_syn = std::max(static_cast<size_t>(p.ns) * T64_DIG * p.lrows * 32, red_syn) + static_cast<size_t>(p.kc_max) * 15 * p.nbt * T64_SBO + margin;
-  const size_t red_ana = static_cast<size_t>(2) * 128 * 33 * sizeof(int) + 16 + static_cast<size_t>(10) * (N + 3) * sizeof(double);
-  p.smem_ana = std::max(static_cast<size_t>(p.ns) * T64_DIG * p.ra_max * 32 + static_cast<size_t>(2) * (p.nhk / 16) * 30 * T64_SBO + margin, red_ana);
+  // members per synthesis tile: two share an MMA (its 128 rows) where one each would not fit the SMs at once
+  p.nbt = B > 1 && static_cast<long>(M) * p.nsl * B > 2 * 152 ? 2 : 1;
+  p.ntiles = (B + p.nbt - 1) / p.nbt;
+  const size_t red_ana = static_cast<size_t>(2) * 128 * 33 * sizeof(int) + 16 + static_cast<size_t>(16) * (N + 3) * sizeof(double);
+  p.smem_ana = std::max(static_cast<size_t>(p.ns) * T64_DIG * p.ra_max * 32 + static_cast<size_t>(2) * (p.nhk / 16) * 30 * T64_SBO, red_ana);
   DevBuf<double> P1;
   up(P1, h.P1);
   const Tc64Dev z = tc64_dev(p, ext);

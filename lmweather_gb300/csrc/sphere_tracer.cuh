@@ -21,10 +21,10 @@ __global__ void __launch_bounds__(SYN_THREADS) trc_synth(SphDev d, SphTab<double
   const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
   const int jh = blockIdx.x * 32 + lane;
   const bool live = jh < d.nh;
-  const double2 *xd = x + static_cast<size_t>(b) * 3 * d.ntri + d.ntri, *xq = qin + static_cast<size_t>(b) * d.ntri;
   double2 qs = make_double2(0, 0), ds = qs;
   const int base = d.tri[m];
-  pdl_wait();
+  pdl_wait(x, qin);
+  const double2 *xd = x + static_cast<size_t>(b) * 3 * d.ntri + d.ntri, *xq = qin + static_cast<size_t>(b) * d.ntri;
   if (live) {
 #pragma unroll 2
     for (int n = m + c; n <= d.N; n += SYN_CHUNKS) {
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(256) trc_grid(SphDev d, SphTab<double> t, cons
   for (int e = threadIdx.x; e < n; e += blockDim.x) inv[e] = make_double2(0.0, 0.0);
   const double wt = r < 2 ? t.wd[js] : t.w[js];
   __syncthreads();
-  pdl_wait();
+  pdl_wait(four, fourq);
   const int rows = r < 2 ? 4 : 2;
   const double2 *f = (r < 2 ? four : fourq) + static_cast<size_t>(b) * d.nlat * rows * d.M + (r & 1) * d.M;
   g64_load(inv, d, f + static_cast<size_t>(js) * rows * d.M, f + static_cast<size_t>(jn) * rows * d.M);
@@ -109,10 +109,10 @@ __global__ void __launch_bounds__(ANA_THREADS) trc_analysis(SphDev d, SphTab<dou
   const int q = blockIdx.x * 32 + lane;
   const bool live = q < d.ntri;
   const int m = live ? d.trim[q] : 0, n = live ? d.trin[q] : 0, par = (n - m) & 1;
-  const double2 *fb = foldq + static_cast<size_t>(b) * d.nh * TRC_SLOT * 2 * d.M;
   const int sP = par * d.M + m, sH = (1 - par) * d.M + m;
   double2 aP = make_double2(0, 0), bH = aP, cP = aP;
-  pdl_wait();
+  pdl_wait(foldq);
+  const double2 *fb = foldq + static_cast<size_t>(b) * d.nh * TRC_SLOT * 2 * d.M;
   if (live) {
 #pragma unroll 2
     for (int jh = c; jh < d.nh; jh += ANA_CHUNKS) {
