@@ -130,6 +130,14 @@ inline void split3(double x, uint16_t *out, long stride) {
     r -= host_bf16_value(b);
   }
 }
+// Half a Fourier record (U, V, zeta, Phi of one latitude, m) as one 32-byte store: each thread's records lie M records apart, so
+// that the L1 pass per line, not the bytes, bounds these stores (T85 x 128, three products: 33.4 -> 25.1 us)
+__device__ __forceinline__ void st_half(float4 *dst, float2 U, float2 V, const float *zf) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(U.x), "f"(U.y), "f"(V.x), "f"(V.y), "f"(zf[0]), "f"(zf[1]),
+               "f"(zf[2]), "f"(zf[3])
+               : "memory");
+}
+
 // FP32 value -> BF16 pieces (the FP32 value carries every bit the products keep)
 __device__ __forceinline__ void fsplit(float x, __nv_bfloat16 *out, long stride, int pieces) {
   const __nv_bfloat16 h = __float2bfloat16_rn(x);
@@ -384,8 +392,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) split_syn(SphDev d, SplitDev
         for (int q = 0; q < 4; q++) hv[q] = side == 0 ? HE[q * 33] + HO[q * 33] : HO[q * 33] - HE[q * 33];
         const float2 U = cscale(csub(imul(make_float2(pv[2], pv[3]), mm), make_float2(hv[0], hv[1])), ia);
         const float2 V = cscale(cadd(imul(make_float2(pv[0], pv[1]), mm), make_float2(hv[2], hv[3])), ia);
-        dst[2 * side] = make_float4(U.x, U.y, V.x, V.y);
-        dst[2 * side + 1] = make_float4(pv[4], pv[5], pv[6], pv[7]);
+        st_half(dst + 2 * side, U, V, pv + 4);
       }
     }
   }
@@ -618,8 +625,7 @@ __global__ void __launch_bounds__(SPLIT_SYN_WS_THREADS, CTAS) split_syn_ws(SphDe
           for (int q = 0; q < 4; q++) hv[q] = side == 0 ? HE[q * ldp] + HO[q * ldp] : HO[q * ldp] - HE[q * ldp];
           const float2 U = cscale(csub(imul(make_float2(pv[2], pv[3]), mm), make_float2(hv[0], hv[1])), ia);
           const float2 V = cscale(cadd(imul(make_float2(pv[0], pv[1]), mm), make_float2(hv[2], hv[3])), ia);
-          dst[2 * side] = make_float4(U.x, U.y, V.x, V.y);
-          dst[2 * side + 1] = make_float4(pv[4], pv[5], pv[6], pv[7]);
+          st_half(dst + 2 * side, U, V, pv + 4);
         }
       }
       // the staging is free for the next item
@@ -669,7 +675,7 @@ __global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 ? 3 : 2) split_grid(Sph
   }
   for (int e = threadIdx.x; e < 4 * JB * rl; e += blockDim.x) sm[e] = make_float2(0, 0);
   __syncthreads();
-  pdl_wait();
+  pdl_wait(fgrid, hsgrid);
   for (int e = threadIdx.x; e < JB * M; e += blockDim.x) {
     const int pr = e / M, m = e - pr * M;
     const float4 *rec = reinterpret_cast<const float4 *>(sd.dsyn + ((static_cast<long>(b) * d.nh + jh0 + pr) * M + m) * SPLIT_NQ);
@@ -979,7 +985,7 @@ __global__ void __launch_bounds__(grid2_threads(LOGN), (FMAX < 4 ? 3 : 2) * 256 
   }
   for (int e = threadIdx.x; e < 2 * JB * RL; e += blockDim.x) sm[e] = make_float4(0, 0, 0, 0);
   __syncthreads();
-  pdl_wait();
+  pdl_wait(fgrid, hsgrid);
   // Fourier records -> spectra of the pairs of rows: south + i north at m, and the conjugate at n - m
   auto put = [&](int pair, int m, float2 a, float2 c, float2 a2, float2 c2) {
     if (m == 0) {
@@ -1158,22 +1164,27 @@ inline int split_grid_threads(int logn) { return split_grid_fixed(logn) ? grid2_
 inline size_t split_grid_bytes(int jb, int nlon) { return static_cast<size_t>((5 * jb + 1) / 2) * fft_row<3>(nlon) * sizeof(float4); }
 
 // ------------------------------------------------------------------------------------------- synthesis operands
-// The next synthesis operands for coefficient (member b, m, n) from its value rounded to FP32: psi, chi, zeta, Phi
+// What the operand addresses of wavenumber m need, read once per work item
+struct PackM {
+  int ke16;
+  long kp, oP, oH;
+};
+__device__ __forceinline__ PackM pack_m(const SplitDev &sd, int m) { return PackM{sd.ke16[m], sd.kps[m], sd.aS_off[m], sd.aSH_off[m]}; }
+// The next synthesis operands for coefficient (member ml of tile, m, n) from its value rounded to FP32: psi, chi, zeta, Phi
 // (P rows) and psi, chi (H rows) at column k(n) of wavenumber m; kf = -a^2 / (n (n + 1)) in FP32.
-__device__ __forceinline__ void pack_syn_coef(const SphDev &d, const SplitDev &sd, float kf, int b, int m, int n, float2 z, float2 dl, float2 f) {
-  const int tile = b / sd.nbt, ml = b - tile * sd.nbt;
-  const int ke16 = sd.ke16[m];
-  const int k = ((n - m) & 1) ? ke16 + ((n - m - 1) >> 1) : ((n - m) >> 1);
-  const long kp = sd.kps[m];
-  const long baseP = sd.aS_off[m] + static_cast<long>(tile) * sd.rSP * kp;
-  const long baseH = sd.aSH_off[m] + static_cast<long>(tile) * sd.rSH * kp;
+__device__ __forceinline__ void pack_syn_coef(const SplitDev &sd, const PackM &pm, float kf, int tile, int ml, int m, int n, float2 z, float2 dl, float2 f) {
+  const int k = ((n - m) & 1) ? pm.ke16 + ((n - m - 1) >> 1) : ((n - m) >> 1);
+  const long baseP = pm.oP + static_cast<long>(tile) * sd.rSP * pm.kp;
+  const long baseH = pm.oH + static_cast<long>(tile) * sd.rSH * pm.kp;
   // the linear-exact form synthesises Phi' = Phi - Phi_00 P_00: the mean enters the tendencies separately
   const bool mean = sd.lin_exact && n == 0;
   const float v[8] = {z.x * kf, z.y * kf, dl.x * kf, dl.y * kf, z.x, z.y, mean ? 0.0f : f.x, mean ? 0.0f : f.y};
+  // a member's eight P rows are one 8-row group, its four H rows half of one: rows 8 elements apart
+  __nv_bfloat16 *oP = sd.aS_P + baseP + tile_off(ml * 8, k, sd.rSP, sd.bks), *oH = sd.aS_H + baseH + tile_off(ml * 4, k, sd.rSH, sd.bks);
 #pragma unroll
-  for (int q = 0; q < 8; q++) fsplit(v[q], sd.aS_P + baseP + tile_off(ml * 8 + q, k, sd.rSP, sd.bks), sd.aSP_size, sd.pieces);
+  for (int q = 0; q < 8; q++) fsplit(v[q], oP + 8 * q, sd.aSP_size, sd.pieces);
 #pragma unroll
-  for (int q = 0; q < 4; q++) fsplit(v[q], sd.aS_H + baseH + tile_off(ml * 4 + q, k, sd.rSH, sd.bks), sd.aSH_size, sd.pieces);
+  for (int q = 0; q < 4; q++) fsplit(v[q], oH + 8 * q, sd.aSH_size, sd.pieces);
 }
 
 __device__ __forceinline__ float2 d2f2(double2 v) { return make_float2(d2f_int(v.x), d2f_int(v.y)); }
@@ -1198,7 +1209,7 @@ __global__ void split_pack_state(SphDev d, SplitDev sd, const float *__restrict_
   xf[ip] = z;
   xf[ip + d.ntri] = dl;
   xf[ip + 2 * d.ntri] = f;
-  pack_syn_coef(d, sd, kfac32[n], b, m, n, z, dl, f);
+  pack_syn_coef(sd, pack_m(sd, m), kfac32[n], b / sd.nbt, b % sd.nbt, m, n, z, dl, f);
 }
 
 // ------------------------------------------------------------------------------------------- analysis + RK4
@@ -1210,12 +1221,75 @@ __global__ void split_pack_state(SphDev d, SplitDev sd, const float *__restrict_
 // filter, in FP64); xf holds it rounded to FP32. The tendencies are FP32 (their nonlinear part carries the BF16
 // pieces' 2^-16 rounding), so the accumulator k1 + 2 k2 + 2 k3 (acc) and the stage inputs xf + c k of stages 0-2,
 // which the next stage only reads in FP32, are formed in FP32.
-__device__ __forceinline__ void ana_coef(const SphDev &d, const SplitDev &sd, const SphTab<float> &t, const StageArgs &sa,
-                                         double2 *__restrict__ x0, float2 *__restrict__ xf, const float2 *__restrict__ xin,
-                                         float2 *__restrict__ xout, float2 *__restrict__ acc, const float *dsm, int ldp, int m, int tile, int ml,
-                                         int s, int r, int cb1, int ra0, int ra1) {
-  const int b = tile * sd.nbt + ml, n = m + s + 2 * r;
-  const int cbs = s ? cb1 : 0, ras = s ? ra1 : ra0;
+// Every value it reads from memory is asked for by ana_load in one go, ahead of the sums (by a lone CTA per SM ahead of the
+// wait for them): read where they were used, four to five latencies in a row bound the analyses (T85 x 128, three
+// products: 48.8 -> 40.7 us).
+struct AnaMem {
+  double2 *__restrict__ x0;
+  float2 *__restrict__ xf;
+  const float2 *__restrict__ xin;
+  float2 *__restrict__ xout, *__restrict__ acc;
+};
+struct AnaItem {  // a work item's constants
+  int m, tile, tri, ne, cb1, ra0, ra1;
+  PackM pm;
+};
+struct AnaIn {
+  float2 y[3], up[2], dn[2], av[3];  // stage input at n, its zeta and delta at n + 1 and n - 1; RK4 accumulator
+  double2 xv[3];                     // the state: FP64 in the last stage, else its FP32 copy in the bits of x
+  float cA, cB, cC, lp, kf, om, phi;
+  bool coupled;
+};
+__device__ __forceinline__ AnaItem ana_item(const SphDev &d, const SplitDev &sd, int m, int tile, int cb1, int ra0, int ra1) {
+  return AnaItem{m, tile, d.tri[m], (d.N - m) / 2 + 1, cb1, ra0, ra1, pack_m(sd, m)};  // ne: coefficients of even n - m
+}
+__device__ __forceinline__ AnaIn ana_load(const SphDev &d, const SplitDev &sd, const SphTab<float> &t, const StageArgs &sa, const AnaMem &A,
+                                          const AnaItem &I, int ml, int s, int r) {
+  AnaIn v;
+  const int b = I.tile * sd.nbt + ml, m = I.m, n = m + s + 2 * r, q = I.tri + n - m;
+  // the FP64 state in triangle order (q); the FP32 buffers in parity order: this coefficient at qp, its
+  // neighbours n + 1 and n - 1 (the other parity) at qu and ql
+  const int qp = I.tri + (s ? I.ne + r : r), qu = I.tri + (s ? r + 1 : I.ne + r), ql = I.tri + (s ? r : I.ne + r - 1);
+  const size_t mb = static_cast<size_t>(b) * 3 * d.ntri;
+  const int nt = d.ntri;
+  // the stage input in FP32: the state's copy at stage 0, else the previous stage's output (a separate buffer:
+  // neighbouring n belong to other CTAs)
+  const float2 zero = make_float2(0.0f, 0.0f), *xf = A.xf + mb, *yin = sa.stage == 0 ? xf : A.xin + mb;
+  v.coupled = false;
+  v.lp = t.lapl[n];
+  v.kf = t.kfac[n];
+  if (sd.lin_exact) {
+    v.phi = xf[2 * nt].x * t.Ps[0];
+    v.coupled = !(d.gflag[b] & 1);
+    v.om = static_cast<float>(d.om2[b]);
+    v.cA = sd.lin32[q];
+    v.cB = sd.lin32[nt + q];
+    v.cC = sd.lin32[2 * nt + q];
+#pragma unroll
+    for (int f = 0; f < 3; f++) v.y[f] = yin[f * nt + qp];
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+      v.up[f] = n < d.N ? yin[f * nt + qu] : zero;
+      v.dn[f] = n > m ? yin[f * nt + ql] : zero;
+    }
+  }
+#pragma unroll
+  for (int f = 0; f < 3; f++) {
+    if (sa.stage < 3) {
+      const float2 x = xf[f * nt + qp];
+      v.xv[f].x = __hiloint2double(__float_as_int(x.y), __float_as_int(x.x));
+    } else {
+      v.xv[f] = (A.x0 + mb)[f * nt + q];
+    }
+    v.av[f] = sa.stage > 0 ? (A.acc + mb)[f * nt + qp] : zero;
+  }
+  return v;
+}
+// the coefficient's value after the stage, rounded to FP32, in nv; every buffer but the operands is stored
+__device__ __forceinline__ void ana_update(const SphDev &d, const SplitDev &sd, const StageArgs &sa, const AnaMem &A, const AnaItem &I, const AnaIn &v,
+                                           const float *dsm, int ldp, int ml, int s, int r, float2 *nv) {
+  const int m = I.m, n = m + s + 2 * r, q = I.tri + n - m;
+  const int cbs = s ? I.cb1 : 0, ras = s ? I.ra1 : I.ra0;
   const float *H = dsm + (ml * 6) * ldp + cbs + r, *P = dsm + (ml * 8) * ldp + cbs + ras + r;
   const float2 aH = make_float2(H[0 * ldp], H[1 * ldp]), bH = make_float2(H[2 * ldp], H[3 * ldp]), vH = make_float2(H[4 * ldp], H[5 * ldp]);
   const float2 aP = make_float2(P[0 * ldp], P[1 * ldp]), bP = make_float2(P[2 * ldp], P[3 * ldp]);
@@ -1223,35 +1297,21 @@ __device__ __forceinline__ void ana_coef(const SphDev &d, const SplitDev &sd, co
   const float mm = static_cast<float>(m);
   // cpp/sphere.cpp:380-389
   float2 kz = csub(bH, imul(aP, mm));
-  float2 kd = cadd(cadd(imul(bP, mm), aH), cscale(eP, t.lapl[n]));
+  float2 kd = cadd(cadd(imul(bP, mm), aH), cscale(eP, v.lp));
   float2 kf = csub(vH, imul(uP, mm));
-  const int q = d.tri[m] + n - m;
-  // the FP64 state in triangle order (q); the FP32 buffers in parity order: this coefficient at qp, its
-  // neighbours n + 1 and n - 1 (the other parity) at qu and ql
-  const int ne = (d.N - m) / 2 + 1;  // coefficients of even n - m
-  const int qp = d.tri[m] + (s ? ne + r : r), qu = d.tri[m] + (s ? r + 1 : ne + r), ql = d.tri[m] + (s ? r : ne + r - 1);
-  const size_t mb = static_cast<size_t>(b) * 3 * d.ntri, base = mb + q, basep = mb + qp;
-  // the stage input in FP32: the state's copy at stage 0, else the previous stage's output (a separate buffer:
-  // neighbouring n belong to other CTAs)
-  const float2 *yin = sa.stage == 0 ? xf : xin;
-  if (sd.lin_exact && q != 0) {
+  if (sd.lin_exact) {
     // the terms linear in the stage input y, in FP32 like the rest of the tendencies but outside the BF16 products:
     // n(n+1)/a^2 Phi_n in d delta; -Phi_mean delta_n in d Phi (D(U, V) = delta exactly for n <= T); for an untilted
     // axis the Coriolis terms -D(f U, f V) and D(f V, -f U) with f = 2 Omega mu, which couple n - 1, n, n + 1 of
     // the same m
-    auto yat = [&](int field, int qq) -> float2 { return yin[mb + static_cast<size_t>(field) * d.ntri + qq]; };
-    const float2 yz = yat(0, qp), yd = yat(1, qp), yf = yat(2, qp);
-    const float phibar = xf[mb + 2 * d.ntri].x * t.Ps[0];
-    const float lp = t.lapl[n];
-    kd.x += lp * yf.x;
-    kd.y += lp * yf.y;
-    kf.x -= phibar * yd.x;
-    kf.y -= phibar * yd.y;
-    if (!(d.gflag[b] & 1)) {
-      const float om = static_cast<float>(d.om2[b]);
-      const float cA = sd.lin32[q], cB = sd.lin32[d.ntri + q], cC = sd.lin32[2 * d.ntri + q];
-      const float2 zu = n < d.N ? yat(0, qu) : make_float2(0, 0), du = n < d.N ? yat(1, qu) : make_float2(0, 0);
-      const float2 zl = n > m ? yat(0, ql) : make_float2(0, 0), dd = n > m ? yat(1, ql) : make_float2(0, 0);
+    const float2 yz = v.y[0], yd = v.y[1], yf = v.y[2];
+    kd.x += v.lp * yf.x;
+    kd.y += v.lp * yf.y;
+    kf.x -= v.phi * yd.x;
+    kf.y -= v.phi * yd.y;
+    if (v.coupled) {
+      const float om = v.om, cA = v.cA, cB = v.cB, cC = v.cC;
+      const float2 zu = v.up[0], du = v.up[1], zl = v.dn[0], dd = v.dn[1];
       // -D(fU, fV)_n = -2 Omega (cA delta_{n+1} + cB delta_{n-1} - i cC zeta_n)
       kz.x -= om * (cA * du.x + cB * dd.x + cC * yz.y);
       kz.y -= om * (cA * du.y + cB * dd.y - cC * yz.x);
@@ -1262,46 +1322,60 @@ __device__ __forceinline__ void ana_coef(const SphDev &d, const SplitDev &sd, co
   }
   if (q == 0) kz = kd = kf = make_float2(0, 0);
   const float2 k[3] = {kz, kd, kf};
-  float2 nv[3];
-  if (sa.stage < 3) {
-    // every load of the three fields is issued before any store (the buffers never alias)
-    float2 yv[3], av[3];
+  const size_t mb = static_cast<size_t>(I.tile * sd.nbt + ml) * 3 * d.ntri;
+  const int qp = I.tri + (s ? I.ne + r : r);
 #pragma unroll
-    for (int f = 0; f < 3; f++) {
-      yv[f] = xf[basep + static_cast<size_t>(f) * d.ntri];
-      av[f] = sa.stage > 0 ? acc[basep + static_cast<size_t>(f) * d.ntri] : make_float2(0.0f, 0.0f);
-    }
-#pragma unroll
-    for (int f = 0; f < 3; f++) {
-      const size_t i = basep + static_cast<size_t>(f) * d.ntri;
-      acc[i] = sa.stage == 0 ? k[f] : make_float2(fmaf(2.0f, k[f].x, av[f].x), fmaf(2.0f, k[f].y, av[f].y));
-      nv[f] = make_float2(fmaf(sa.c32, k[f].x, yv[f].x), fmaf(sa.c32, k[f].y, yv[f].y));
+  for (int f = 0; f < 3; f++) {
+    const int i = f * d.ntri + qp;
+    const float2 av = v.av[f];
+    if (sa.stage < 3) {
+      (A.acc + mb)[i] = sa.stage == 0 ? k[f] : make_float2(fmaf(2.0f, k[f].x, av.x), fmaf(2.0f, k[f].y, av.y));
+      const float2 x = make_float2(__int_as_float(__double2loint(v.xv[f].x)), __int_as_float(__double2hiint(v.xv[f].x)));
+      nv[f] = make_float2(fmaf(sa.c32, k[f].x, x.x), fmaf(sa.c32, k[f].y, x.y));
       // the next stage input is kept when the linear-exact form reads it (the split synthesis reads the packed
-      // operands written below)
-      if (xout != nullptr) xout[i] = nv[f];
-    }
-  } else {
-    double2 xv[3];
-    float2 av[3];
-#pragma unroll
-    for (int f = 0; f < 3; f++) {
-      xv[f] = x0[base + static_cast<size_t>(f) * d.ntri];
-      av[f] = acc[basep + static_cast<size_t>(f) * d.ntri];
-    }
-#pragma unroll
-    for (int f = 0; f < 3; f++) {
-      const double2 sum = make_double2(f2d_int(av[f].x + k[f].x), f2d_int(av[f].y + k[f].y));
-      const double2 val = make_double2(fma(sa.c, sum.x, xv[f].x), fma(sa.c, sum.y, xv[f].y));
+      // operands)
+      if (A.xout != nullptr) (A.xout + mb)[i] = nv[f];
+    } else {
+      const double2 xv = v.xv[f];
+      const double2 sum = make_double2(f2d_int(av.x + k[f].x), f2d_int(av.y + k[f].y));
+      const double2 val = make_double2(fma(sa.c, sum.x, xv.x), fma(sa.c, sum.y, xv.y));
       const double fac = sa.filt[(f == 2 ? 1 : 0) * d.M + n];
       const double2 x1 = q == 0 ? val : cscale(val, fac);
-      x0[base + static_cast<size_t>(f) * d.ntri] = x1;
+      (A.x0 + mb)[f * d.ntri + q] = x1;
       nv[f] = d2f2(x1);
-      xf[basep + static_cast<size_t>(f) * d.ntri] = nv[f];
+      (A.xf + mb)[i] = nv[f];
     }
   }
-  pack_syn_coef(d, sd, t.kfac[n], b, m, n, nv[0], nv[1], nv[2]);
 }
-
+// Coefficients e0, e0 + step, ... of a work item's mt members (cnt each, BOTH: of both parities in turn, else of parity
+// s_first). `in` holds what ana_load gave for e0.
+template <bool BOTH> struct AnaLoop {
+  int cnt, s_first, total;
+  __device__ __forceinline__ void split(int e, int &ml, int &s, int &r) const {
+    ml = e / cnt;
+    const int j = e - ml * cnt;
+    s = BOTH ? (j & 1) : s_first;
+    r = BOTH ? (j >> 1) : j;
+  }
+  __device__ __forceinline__ AnaIn load(int e, const SphDev &d, const SplitDev &sd, const SphTab<float> &t, const StageArgs &sa, const AnaMem &A,
+                                        const AnaItem &I) const {
+    int ml, s, r;
+    split(e, ml, s, r);
+    return ana_load(d, sd, t, sa, A, I, ml, s, r);
+  }
+  template <bool PRE>
+  __device__ __forceinline__ void run(AnaIn &in, int e0, int step, const SphDev &d, const SplitDev &sd, const SphTab<float> &t, const StageArgs &sa,
+                                      const AnaMem &A, const AnaItem &I, const float *dsm, int ldp) const {
+    for (int e = e0; e < total; e += step) {
+      int ml, s, r;
+      split(e, ml, s, r);
+      if (!PRE || e != e0) in = ana_load(d, sd, t, sa, A, I, ml, s, r);
+      float2 nv[3];
+      ana_update(d, sd, sa, A, I, in, dsm, ldp, ml, s, r, nv);
+      pack_syn_coef(sd, I.pm, in.kf, I.tile, ml, I.m, I.m + s + 2 * r, nv[0], nv[1], nv[2]);
+    }
+  }
+};
 
 // BOTH = false: grid (M, 2, ntiles), one parity s = blockIdx.y per CTA. BOTH = true: grid (M, 1, ntiles), both
 // parities in one CTA one after the other (the GEMM pipeline's barriers continue their phases), so the epilogue
@@ -1332,7 +1406,8 @@ __global__ void __launch_bounds__(SPLIT_ANA_THREADS, MINB) split_ana(SphDev d, S
   uint8_t *aH = smem, *aP = smem + aH_bytes, *pipe = smem + aH_bytes + aP_bytes;
   bool ok = true, setup_done = false;
   int pipe_it = 0, calls = 0;
-  pdl_wait();
+  pdl_wait(x0, xf, xin, xout, acc);
+  const AnaMem A{x0, xf, xin, xout, acc};
   for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
   const int m = m_slowest ? item / per_m : item % d.M, rest = m_slowest ? item % per_m : item / d.M;
   const int s_first = BOTH ? 0 : rest % 2, s_last = BOTH ? 1 : s_first;
@@ -1343,6 +1418,9 @@ __global__ void __launch_bounds__(SPLIT_ANA_THREADS, MINB) split_ana(SphDev d, S
   const int ra0 = sd.ra16[2 * m], ra1 = sd.ra16[2 * m + 1];
   const int cb1 = BOTH ? 2 * ra0 : 0;                               // cb_0 = 0
   const int ld = BOTH ? 2 * (ra0 + ra1) : 2 * (s_first ? ra1 : ra0);  // accumulator columns (and dsm row length)
+  const AnaItem I = ana_item(d, sd, m, tile, cb1, ra0, ra1);
+  const int cnt = BOTH ? d.N - m + 1 : (s_first ? R1 : R0);
+  const AnaLoop<BOTH> loop{cnt, s_first, mt * cnt};
   // the previous item's epilogue has finished reading shared memory and tensor memory
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1463,14 +1541,8 @@ __global__ void __launch_bounds__(SPLIT_ANA_THREADS, MINB) split_ana(SphDev d, S
     }
   }
   __syncthreads();
-  if (ok) {
-    const int cnt = BOTH ? d.N - m + 1 : (s_first ? R1 : R0);
-    for (int e = threadIdx.x; e < mt * cnt; e += blockDim.x) {
-      const int ml = e / cnt, j = e - ml * cnt;
-      const int s = BOTH ? (j & 1) : s_first, r = BOTH ? (j >> 1) : j;
-      ana_coef(d, sd, t, sa, x0, xf, xin, xout, acc, dsm, ldp, m, tile, ml, s, r, cb1, ra0, ra1);
-    }
-  }
+  AnaIn in;
+  if (ok) loop.template run<false>(in, threadIdx.x, blockDim.x, d, sd, t, sa, A, I, dsm, ldp);
   }
   if (setup_done) split_teardown(tslot, ncols);
 }
@@ -1525,7 +1597,7 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tslot;
-  pdl_wait();
+  pdl_wait(x0, xf, xin, xout, acc);
   // the item sequence every role walks (snake_item): (m, parity or both, tile), m the slowest index
   auto item_of = [&](int item, int &m, int &s_first, int &s_last, int &tile, int &R0, int &R1) {
     m = item / per_m;
@@ -1632,12 +1704,21 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
     tc::commit(leader, su32(&done));
   } else if (warp >= 2) {
     // epilogue warps
+    const AnaMem A{x0, xf, xin, xout, acc};
     const int et = tid - 64;
     int it = 0;
     for (int k = 0, item = snake_item(0); item < nitems; item = snake_item(++k)) {
       int m, s_first, s_last, tile, R0, R1;
       item_of(item, m, s_first, s_last, tile, R0, R1);
       if ((s_first ? R1 : R0) == 0) continue;
+      const int mt = min(sd.nbt, B - tile * sd.nbt);
+      const int ra0 = sd.ra16[2 * m], ra1 = sd.ra16[2 * m + 1];
+      const int cb1 = BOTH ? 2 * ra0 : 0;
+      const int cnt = BOTH ? d.N - m + 1 : (s_first ? R1 : R0);
+      const AnaItem I = ana_item(d, sd, m, tile, cb1, ra0, ra1);
+      const AnaLoop<BOTH> loop{cnt, s_first, mt * cnt};
+      AnaIn in;
+      if (CTAS == 1 && et < loop.total) in = loop.load(et, d, sd, t, sa, A, I);
       const int bb = it & 1;
       if (et == 0) s_epi_ok = mbar_wait_bounded(su32(&accf[bb]), (it >> 1) & 1) ? 1 : 0;
       asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -1649,9 +1730,6 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int mt = min(sd.nbt, B - tile * sd.nbt);
-      const int ra0 = sd.ra16[2 * m], ra1 = sd.ra16[2 * m + 1];
-      const int cb1 = BOTH ? 2 * ra0 : 0;
       const int ld = BOTH ? 2 * (ra0 + (s_last ? ra1 : 0)) : 2 * (s_first ? ra1 : ra0);
       const int ldp = ld + 1;
       // accumulators -> shared memory: warp w reads tensor-memory lanes 32 (w % 4) .. + 31; warps 2..5 take the even
@@ -1671,12 +1749,7 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       asm volatile("bar.sync 1, 256;" ::: "memory");
       if (et == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(&acce[bb])) : "memory");
-      const int cnt = BOTH ? d.N - m + 1 : (s_first ? R1 : R0);
-      for (int e = et; e < mt * cnt; e += SPLIT_WS_EPI) {
-        const int ml = e / cnt, j = e - ml * cnt;
-        const int s = BOTH ? (j & 1) : s_first, r = BOTH ? (j >> 1) : j;
-        ana_coef(d, sd, t, sa, x0, xf, xin, xout, acc, dsm, ldp, m, tile, ml, s, r, cb1, ra0, ra1);
-      }
+      loop.template run<CTAS == 1>(in, et, SPLIT_WS_EPI, d, sd, t, sa, A, I, dsm, ldp);
       // the shared accumulator copy is free for the next item
       asm volatile("bar.sync 1, 256;" ::: "memory");
       it++;
