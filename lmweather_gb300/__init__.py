@@ -408,7 +408,7 @@ class Sphere:
         _check(self._lib.lmw_sphere_set_split_form(self._h, 1 if linear_exact else 0))
 
     def get_state(self, member: int = 0):
-        z, d, f = (np.zeros(self.nspec, np.complex128) for _ in range(3))
+        z, d, f = (np.empty(self.nspec, np.complex128) for _ in range(3))
         _check(self._lib.lmw_sphere_get_state(self._h, member, _dp(z.view(np.float64)), _dp(d.view(np.float64)),
                                               _dp(f.view(np.float64))))
         return z, d, f
@@ -468,7 +468,7 @@ class Sphere:
         return self.diagnostics(member)["error_linf"]
 
     def _grid(self, which: int, member: int) -> np.ndarray:
-        g = np.zeros((self.nlat, self.nlon))
+        g = np.empty((self.nlat, self.nlon))
         _check(self._lib.lmw_sphere_grid(self._h, member, which, _dp(g), g.size))
         return g
 
@@ -557,7 +557,7 @@ class Plane:
         return self
 
     def get(self):
-        h, u, v = np.zeros((self.ny, self.nx)), np.zeros((self.ny, self.nx)), np.zeros((self.ny + 1, self.nx))
+        h, u, v = np.empty((self.ny, self.nx)), np.empty((self.ny, self.nx)), np.empty((self.ny + 1, self.nx))
         _check(self._lib.lmw_plane_get(self._h, _dp(h), _dp(u), _dp(v)))
         return h, u, v
 
@@ -771,7 +771,7 @@ def gemm_bf16(a, b) -> np.ndarray:
     a, b = _f32(a), _f32(b)
     M, K = a.shape
     N = b.shape[0]
-    c = np.zeros((M, N), np.float32)
+    c = np.empty((M, N), np.float32)
     _check(load_library().lmw_gemm_bf16(_fp(a), _fp(b), M, N, K, _fp(c)))
     return c
 
@@ -809,13 +809,13 @@ class Mlp:
 
     def get_layer(self, layer: int):
         no, ni = self._shape(layer)
-        w, b = np.zeros((no, ni), np.float32), np.zeros(no, np.float32)
+        w, b = np.empty((no, ni), np.float32), np.empty(no, np.float32)
         _check(self._lib.lmw_mlp_get_layer(self._h, layer, _fp(w), _fp(b)))
         return w, b
 
     def forward(self, x) -> np.ndarray:
         x = _f32(x)
-        y = np.zeros((x.shape[0], self.dims[2]), np.float32)
+        y = np.empty((x.shape[0], self.dims[2]), np.float32)
         _check(self._lib.lmw_mlp_forward(self._h, _fp(x), x.shape[0], _fp(y)))
         return y
 
@@ -828,7 +828,7 @@ class Mlp:
 
     def grad(self, layer: int):
         no, ni = self._shape(layer)
-        gw, gb = np.zeros((no, ni), np.float32), np.zeros(no, np.float32)
+        gw, gb = np.empty((no, ni), np.float32), np.empty(no, np.float32)
         _check(self._lib.lmw_mlp_get_grad(self._h, layer, _fp(gw), _fp(gb)))
         return gw, gb
 

@@ -1,4 +1,12 @@
 // The C ABI (include/lmweather_gb300.h): exceptions become status codes, the message is kept per thread.
+#include <algorithm>
+#include <system_error>
+#include <thread>
+#include <vector>
+#ifdef __linux__
+#include <sys/mman.h>
+#include <unistd.h>
+#endif
 #include <cuda_profiler_api.h>
 
 #include <cstdio>
@@ -27,6 +35,41 @@ struct lmw_mlp {
 struct lmw_surrogate {
   lmw::Surrogate *s;
 };
+
+namespace lmw {
+
+void prefault(void *p, size_t bytes) {
+#ifdef __linux__
+  constexpr size_t kLeast = 1 << 20;
+  if (bytes < kLeast) return;
+  const size_t page = static_cast<size_t>(sysconf(_SC_PAGESIZE));
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p) / page * page, e = reinterpret_cast<uintptr_t>(p) + bytes;
+  unsigned char first = 1, last = 1;
+  if (mincore(reinterpret_cast<void *>(a), 1, &first) != 0 || mincore(reinterpret_cast<void *>((e - 1) / page * page), 1, &last) != 0) return;
+  const uintptr_t mid = (a + (e - a) / 2) / page * page;
+  unsigned char half = 1;
+  if (mincore(reinterpret_cast<void *>(mid), 1, &half) != 0 || ((first & last & half) & 1)) return;
+  constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE (Linux 5.14); where it is unknown the copy faults the pages
+  auto fill = [=](uintptr_t from, uintptr_t to) {
+    if (to > from) madvise(reinterpret_cast<void *>(from), to - from, kPopulateWrite);
+  };
+  const int parts = bytes >= 8 * kLeast ? 4 : 1;
+  const uintptr_t len = ((e - a) / parts + page - 1) / page * page;
+  std::vector<std::thread> others;
+  others.reserve(parts);
+  try {
+    for (int k = 1; k < parts; k++) others.emplace_back(fill, std::min(a + k * len, e), std::min(a + (k + 1) * len, e));
+  } catch (const std::system_error &) {  // no thread to be had: the copy faults what is left
+  }
+  fill(a, std::min(a + len, e));
+  for (auto &t : others) t.join();
+#else
+  (void)p;
+  (void)bytes;
+#endif
+}
+
+}  // namespace lmw
 
 namespace lmw {
 thread_local uint64_t g_launches = 0;
@@ -611,12 +654,12 @@ int lmw_mlp_get_layer(lmw_mlp *m, int layer, float *w, float *b) {
   return MLP(m, need(w != nullptr, "null weights"); m->m->get_layer(layer, w, b));
 }
 int lmw_mlp_forward(lmw_mlp *m, const float *x, int batch, float *y) {
-  return MLP(m, need(x != nullptr && y != nullptr, "null buffer"); m->m->upload_input(x, batch); m->m->forward(batch); m->m->check_status();
+  return MLP(m, need(x != nullptr && y != nullptr, "null buffer"); m->m->upload_input(x, batch); m->m->forward(batch);
              m->m->download_output(y, batch));
 }
 int lmw_mlp_backward(lmw_mlp *m, const float *x, const float *target, const float *mask, int batch, double *loss) {
   return MLP(m, need(x != nullptr && target != nullptr, "null buffer"); m->m->upload_input(x, batch); m->m->upload_target(target, mask, batch);
-             m->m->take_loss(); m->m->forward(batch); m->m->backward(batch); const double l = m->m->take_loss(); if (loss) *loss = l);
+             m->m->loss_acc.zero(m->m->stream); m->m->forward(batch); m->m->backward(batch); const double l = m->m->take_loss(); if (loss) *loss = l);
 }
 int lmw_mlp_get_grad(lmw_mlp *m, int layer, float *gw, float *gb) {
   return MLP(m, need(gw != nullptr, "null gradient buffer"); m->m->get_grad(layer, gw, gb));

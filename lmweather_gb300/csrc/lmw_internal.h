@@ -95,6 +95,11 @@ template <class T> struct HostBuf {
   }
 };
 
+// Faults the pages of a host buffer of `bytes` about to be filled by a device copy, if its ends are not resident: the copy
+// engine faults fresh pages one by one (1 GB/s), the kernel a range at once, and several ranges in parallel. The contents
+// are left alone.
+void prefault(void *p, size_t bytes);
+
 // Counts this library's kernel launches (for the benchmark's launch accounting).
 extern thread_local uint64_t g_launches;
 

@@ -204,6 +204,14 @@ __global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int sta
   }
 }
 
+// the stage coefficients into device memory (by value: a copy from the host's stack could still be under way when the
+// caller has returned)
+__global__ void plane_coef(double *c, double half, double full, double sixth) {
+  c[0] = c[1] = half;
+  c[2] = full;
+  c[3] = sixth;
+}
+
 // How a grid is cut. FORM 0: at most one one-row tile per SM; 1, 2: one or two CTAs on every SM, tiles of up to sixteen
 // rows; 3: more. 0 to 2 launch early. In 3 the rows of a tile are the number up to sixteen that leaves the fullest SM
 // the least to do, counting the FP64 instructions per warp of a tile: 2 for each loaded point, 17 for each corner, 33
@@ -670,6 +678,9 @@ void PlaneEngine::set_v(const double *g, size_t n) {
 }
 
 void PlaneEngine::get(double *h, double *u, double *v) {
+  if (h) prefault(h, ncell() * sizeof(double));
+  if (u) prefault(u, ncell() * sizeof(double));
+  if (v) prefault(v, nvpt() * sizeof(double));
   LMW_CUDA(cudaStreamSynchronize(stream));
   if (h) LMW_CUDA(cudaMemcpy(h, h0.p, ncell() * sizeof(double), cudaMemcpyDeviceToHost));
   if (u) LMW_CUDA(cudaMemcpy(u, u0.p, ncell() * sizeof(double), cudaMemcpyDeviceToHost));
@@ -786,8 +797,9 @@ void PlaneEngine::set_params(double gravity, double depth, double f0, double bet
 // `steps` RK4 steps: graphs of GRAPH_STEPS steps (captured once per set of parameters), the rest launched singly
 void PlaneEngine::launch_chunk(double dt, int steps) {
   if (steps >= GRAPH_STEPS && coef_dt != dt) {
-    const double c[4] = {0.5 * dt, 0.5 * dt, dt, dt / 6};
-    LMW_CUDA(cudaMemcpyAsync(coef.p, c, sizeof c, cudaMemcpyHostToDevice, stream));  // pageable: staged before it returns
+    plane_coef<<<1, 1, 0, stream>>>(coef.p, 0.5 * dt, dt, dt / 6);
+    LMW_LAUNCH_CHECK();
+    g_launches += 1;
     coef_dt = dt;
   }
   for (; steps >= GRAPH_STEPS; steps -= GRAPH_STEPS) {

@@ -17,6 +17,7 @@
 #include <numeric>
 #include <random>
 
+#include "pdl.cuh"
 #include "surrogate.h"
 #include "tc_common.cuh"
 
@@ -66,6 +67,7 @@ __global__ void __launch_bounds__(128, 1) mlp_gemm(GemmArgs g) {
   __shared__ int fail, issued, consumed;
   constexpr int STAGE = (128 + BN) * BK * 2;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int role = tc::uniform(warp);  // before any thread leaves its warp
   const int n0 = blockIdx.x * BN, m0 = blockIdx.y * 128;
   const int nk = g.K / BK;
   if (warp == 0) tc::tmem_alloc(tc::su32(&tslot), BN);
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(128, 1) mlp_gemm(GemmArgs g) {
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tslot;
+  pdl_wait();
   if (tid == 0) {
     const bf16 *a_src = g.A + static_cast<long>(m0 >> 7) * nk * TILE;
     for (int it = 0; it < nk; it++) {
@@ -102,28 +105,26 @@ __global__ void __launch_bounds__(128, 1) mlp_gemm(GemmArgs g) {
         tc::bulk_g2s(tc::su32(base + (j + 1) * TILE * 2), g.B + (static_cast<long>((n0 >> 7) + j) * nk + it) * TILE, TILE * 2, bar);
       issued = it + 1;
     }
-  } else if (tid == 32) {
-    const uint32_t idesc = tc::idesc_m128(BN);
-    bool ok = true;
+  } else if (role == 1) {
+    const uint32_t idesc = tc::idesc_m128(BN), acc = tc::uniform(tmem), base0 = tc::su32(smem);
+    const bool leader = tc::elect_one();
     for (int it = 0; it < nk; it++) {
       const int st = it % S;
-      if (!tc::wait(tc::su32(&full[st]), (it / S) & 1)) {
+      if (!tc::wait_warp(tc::su32(&full[st]), (it / S) & 1)) {
         fail = 1;
         atomicExch(g.err, 2);
-        ok = false;
         break;
       }
-      consumed = it + 1;
       tc::fence_after();
-      const uint32_t base = tc::su32(smem + st * STAGE);
+      const uint64_t ad = tc::chunk_desc(base0 + st * STAGE), bd = tc::chunk_desc(base0 + st * STAGE + TILE * 2);
+      consumed = it + 1;
 #pragma unroll
-      for (int kk = 0; kk < 4; kk++)
-        tc::mma(tmem, tc::chunk_desc(base + kk * 256), tc::chunk_desc(base + TILE * 2 + kk * 256), idesc, (it | kk) != 0 ? 1u : 0u);
-      tc::commit(tc::su32(&empty[st]));
+      for (int kk = 0; kk < 4; kk++) tc::mma(leader, acc, ad + kk * 16, bd + kk * 16, idesc, (it | kk) != 0 ? 1u : 0u);
+      tc::commit(leader, tc::su32(&empty[st]));
     }
     // completes `done` when every MMA issued so far has finished (after a failed wait too: the CTA drains its
     // own work before it frees tensor memory)
-    tc::commit(tc::su32(&done));
+    tc::commit(leader, tc::su32(&done));
   }
   __syncthreads();
   if (tid == 0) {
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(128, 1) mlp_gemm(GemmArgs g) {
   }
   __syncthreads();
   tc::fence_after();
+  pdl_trigger();
   if (!fail) {
     const int row = m0 + warp * 32 + lane;
     const uint32_t lanebase = tmem + (static_cast<uint32_t>(warp * 32) << 16);
@@ -191,7 +193,7 @@ __global__ void __launch_bounds__(128, 1) mlp_gemm(GemmArgs g) {
   if (warp == 0) tc::tmem_free(tmem, BN);
 }
 
-constexpr int S256 = 4, S128 = 3;
+constexpr int S256 = 4, S128 = 3, S128_ONE = 6;
 constexpr size_t smem_bytes(int bn, int s) { return static_cast<size_t>(s) * (128 + bn) * BK * 2; }
 
 void gemm_attrs() {
@@ -200,6 +202,7 @@ void gemm_attrs() {
   static bool done[64] = {false};
   if (dev < 0 || dev >= 64 || done[dev]) return;
   LMW_CUDA(cudaFuncSetAttribute(mlp_gemm<256, S256>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes(256, S256))));
+  LMW_CUDA(cudaFuncSetAttribute(mlp_gemm<128, S128_ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes(128, S128_ONE))));
   LMW_CUDA(cudaFuncSetAttribute(mlp_gemm<128, S128>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes(128, S128))));
   done[dev] = true;
 }
@@ -208,9 +211,12 @@ void gemm(const GemmArgs &g, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.M % 128 || g.N % 128 || g.K % BK) throw InvalidArgument("GEMM sizes must be multiples of 128 (M, N) and 64 (K)");
   gemm_attrs();
   const bool wide = g.N % 256 == 0 && (g.M / 128) * (g.N / 256) >= 148;
-  if (wide) mlp_gemm<256, S256><<<dim3(g.N / 256, g.M / 128), 128, smem_bytes(256, S256), s>>>(g);
-  else mlp_gemm<128, S128><<<dim3(g.N / 128, g.M / 128), 128, smem_bytes(128, S128), s>>>(g);
-  LMW_LAUNCH_CHECK();
+  // a tile's K loop is bound by its loads in flight: where every tile has an SM to itself it takes six stages, else three,
+  // so that two tiles share an SM
+  const int tiles = (g.M / 128) * (g.N / 128);
+  if (wide) stage_launch(mlp_gemm<256, S256>, dim3(g.N / 256, g.M / 128), 128, smem_bytes(256, S256), s, 1, g);
+  else if (tiles <= 152) stage_launch(mlp_gemm<128, S128_ONE>, dim3(g.N / 128, g.M / 128), 128, smem_bytes(128, S128_ONE), s, 1, g);
+  else stage_launch(mlp_gemm<128, S128>, dim3(g.N / 128, g.M / 128), 128, smem_bytes(128, S128), s, 1, g);
   g_launches += 1;
 }
 
@@ -218,6 +224,7 @@ void gemm(const GemmArgs &g, cudaStream_t s) {
 __global__ void transpose_blocked(const bf16 *__restrict__ in, bf16 *__restrict__ out, int R, int C) {
   __shared__ bf16 s[64][72];
   const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
+  pdl_wait(in);
   for (int e = threadIdx.x; e < 512; e += blockDim.x) {
     const int rr = e >> 3, cg = e & 7;
     const uint4 val = *reinterpret_cast<const uint4 *>(in + boff(r0 + rr, c0 + cg * 8, C));
@@ -237,8 +244,7 @@ __global__ void transpose_blocked(const bf16 *__restrict__ in, bf16 *__restrict_
 }
 
 void transpose(const bf16 *in, bf16 *out, int R, int C, cudaStream_t s) {
-  transpose_blocked<<<dim3(C / 64, R / 64), 256, 0, s>>>(in, out, R, C);
-  LMW_LAUNCH_CHECK();
+  stage_launch(transpose_blocked, dim3(C / 64, R / 64), 256, 0, s, 1, in, out, R, C);
   g_launches += 1;
 }
 
@@ -247,6 +253,7 @@ void transpose(const bf16 *in, bf16 *out, int R, int C, cudaStream_t s) {
 __global__ void rowsum_blocked(const bf16 *__restrict__ gt, float *__restrict__ out, int N, int batch) {
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= N) return;
+  pdl_wait(gt);
   float s = 0.0f;
   for (int k8 = lane * 8; k8 < batch; k8 += 256) {
     const uint4 v = *reinterpret_cast<const uint4 *>(gt + boff(row, k8, batch));
@@ -264,6 +271,7 @@ __global__ void loss_grad(const float *__restrict__ y, const float *__restrict__
                           float inv_b, double *loss) {
   const int b = blockIdx.x;
   float acc = 0.0f;
+  pdl_wait(y, t, mask);
   for (int f8 = threadIdx.x * 8; f8 < ld; f8 += blockDim.x * 8) {
     uint4 out;
     bf16 *p = reinterpret_cast<bf16 *>(&out);
@@ -304,6 +312,7 @@ struct AdamArgs {
 __global__ void adam_tile(AdamArgs a) {
   __shared__ bf16 s[64][72];
   const int k0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
+  pdl_wait();
   for (int e = threadIdx.x; e < 4096; e += blockDim.x) {
     const int rr = e >> 6, cc = e & 63;
     const long i = static_cast<long>(n0 + rr) * a.nin + k0 + cc;
@@ -338,6 +347,7 @@ __global__ void adam_vec(float *w, float *m, float *v, const float *g, int n, fl
                          const float *scale, float *ema, float ema_decay) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
+  pdl_wait();
   const float gi = g[i] * (scale ? *scale : 1.0f);
   const float mi = b1 * m[i] + (1.0f - b1) * gi;
   const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
@@ -403,6 +413,7 @@ __global__ void init_normal(float *w, int nout, int nin, int nout_l, int nin_l, 
 // row-major FP32 [rows][cols] (leading dimension ld) -> blocked BF16 [rows_p][cols_p], zero outside
 __global__ void pack_blocked(const float *__restrict__ src, int rows, int cols, int ld, bf16 *__restrict__ dst, int rows_p, int cols_p) {
   const long chunks = static_cast<long>(rows_p) * (cols_p / 8);
+  pdl_wait(src);
   for (long e = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; e < chunks; e += static_cast<long>(gridDim.x) * blockDim.x) {
     const int r = static_cast<int>(e / (cols_p / 8)), c8 = static_cast<int>(e % (cols_p / 8)) * 8;
     uint4 val;
@@ -492,6 +503,7 @@ Mlp::Mlp(int in_dim, int hidden_, int out_dim, int max_batch_, uint64_t seed, do
   clip.zero(stream);
   err.alloc(1);
   err.zero(stream);
+  hstat.alloc(2);
   LMW_CUDA(cudaStreamSynchronize(stream));
 }
 
@@ -527,6 +539,7 @@ void Mlp::get_layer(int l, float *w, float *b) {
   if (l < 0 || l >= NL) throw InvalidArgument("layer index out of range");
   Layer &Ly = L[l];
   const int nin_l = l == 0 ? din : hidden, nout_l = l == NL - 1 ? dout : hidden;
+  prefault(w, static_cast<size_t>(nin_l) * nout_l * sizeof(float));
   LMW_CUDA(cudaMemcpy2DAsync(w, nin_l * sizeof(float), Ly.w.p, Ly.nin * sizeof(float), nin_l * sizeof(float), nout_l, cudaMemcpyDeviceToHost, stream));
   if (b) LMW_CUDA(cudaMemcpyAsync(b, Ly.b.p, nout_l * sizeof(float), cudaMemcpyDeviceToHost, stream));
   LMW_CUDA(cudaStreamSynchronize(stream));
@@ -536,6 +549,7 @@ void Mlp::get_grad(int l, float *gw, float *gb) {
   if (l < 0 || l >= NL) throw InvalidArgument("layer index out of range");
   Layer &Ly = L[l];
   const int nin_l = l == 0 ? din : hidden, nout_l = l == NL - 1 ? dout : hidden;
+  prefault(gw, static_cast<size_t>(nin_l) * nout_l * sizeof(float));
   LMW_CUDA(cudaMemcpy2DAsync(gw, nin_l * sizeof(float), Ly.gw.p, Ly.nin * sizeof(float), nin_l * sizeof(float), nout_l, cudaMemcpyDeviceToHost, stream));
   if (gb) LMW_CUDA(cudaMemcpyAsync(gb, Ly.gb.p, nout_l * sizeof(float), cudaMemcpyDeviceToHost, stream));
   LMW_CUDA(cudaStreamSynchronize(stream));
@@ -547,29 +561,28 @@ static void check_batch(int batch, int max_batch) {
 
 void Mlp::upload_input(const float *x, int batch) {
   check_batch(batch, max_batch);
-  DevBuf<float> tmp;
-  tmp.alloc(static_cast<size_t>(batch) * din);
-  LMW_CUDA(cudaMemcpyAsync(tmp.p, x, tmp.bytes(), cudaMemcpyHostToDevice, stream));
-  pack_blocked<<<grid_for(static_cast<long>(batch) * dim[0] / 8, 256), 256, 0, stream>>>(tmp.p, batch, din, din, x0.p, batch, dim[0]);
-  LMW_LAUNCH_CHECK();
-  LMW_CUDA(cudaStreamSynchronize(stream));
+  if (!xin.p) xin.alloc(static_cast<size_t>(max_batch) * din);
+  LMW_CUDA(cudaMemcpyAsync(xin.p, x, static_cast<size_t>(batch) * din * sizeof(float), cudaMemcpyHostToDevice, stream));
+  stage_launch(pack_blocked, dim3(grid_for(static_cast<long>(batch) * dim[0] / 8, 256)), 256, 0, stream, 1, xin.p, batch, din, din, x0.p, batch, dim[0]);
 }
 
 void Mlp::upload_target(const float *t, const float *m, int batch) {
   check_batch(batch, max_batch);
-  target.zero(stream);
+  // (the padding columns stay zero from the construction on)
   LMW_CUDA(cudaMemcpy2DAsync(target.p, dim[4] * sizeof(float), t, dout * sizeof(float), dout * sizeof(float), batch, cudaMemcpyHostToDevice, stream));
   if (m) {
     mask.zero(stream);
     LMW_CUDA(cudaMemcpyAsync(mask.p, m, dout * sizeof(float), cudaMemcpyHostToDevice, stream));
   }
-  LMW_CUDA(cudaStreamSynchronize(stream));
 }
 
 void Mlp::download_output(float *yh, int batch) {
   check_batch(batch, max_batch);
+  prefault(yh, static_cast<size_t>(batch) * dout * sizeof(float));  // while the network runs
   LMW_CUDA(cudaMemcpy2DAsync(yh, dout * sizeof(float), y.p, dim[4] * sizeof(float), dout * sizeof(float), batch, cudaMemcpyDeviceToHost, stream));
+  read_status();
   LMW_CUDA(cudaStreamSynchronize(stream));
+  raise_status();
 }
 
 void Mlp::forward(int batch) {
@@ -610,8 +623,7 @@ void Mlp::forward(int batch) {
 void Mlp::backward(int batch) {
   check_batch(batch, max_batch);
   const int h = hidden;
-  loss_grad<<<batch, 256, 0, stream>>>(y.p, target.p, mask.p, dy.p, dim[4], 1.0f / batch, loss_acc.p);
-  LMW_LAUNCH_CHECK();
+  stage_launch(loss_grad, dim3(batch), 256, 0, stream, 1, y.p, target.p, mask.p, dy.p, dim[4], 1.0f / batch, loss_acc.p);
   g_launches += 1;
   // gradient of the current layer's output (pre-activation for hidden layers), blocked [batch][width]
   const bf16 *gcur = dy.p;
@@ -633,8 +645,7 @@ void Mlp::backward(int batch) {
     gw.ldc = win;
     gw.err = err.p;
     gemm(gw, stream);
-    rowsum_blocked<<<(wcur + 7) / 8, 256, 0, stream>>>(tgrad.p, L[l].gb.p, wcur, batch);
-    LMW_LAUNCH_CHECK();
+    stage_launch(rowsum_blocked, dim3((wcur + 7) / 8), 256, 0, stream, 1, tgrad.p, L[l].gb.p, wcur, batch);
     g_launches += 1;
     if (l == 0) break;
     GemmArgs gd{};
@@ -677,12 +688,10 @@ void Mlp::adam(double lr, double beta1, double beta2, double eps, double clip_ra
     const bool avg = ema_decay > 0 && Ly.we.p != nullptr;
     AdamArgs a{Ly.w.p, Ly.m.p, Ly.v.p, Ly.gw.p, Ly.wb.p, Ly.wt.p, Ly.nout, Ly.nin, static_cast<float>(lr), static_cast<float>(beta1), static_cast<float>(beta2),
                static_cast<float>(eps), c1, c2, 1, scale, avg ? Ly.we.p : nullptr, static_cast<float>(ema_decay)};
-    adam_tile<<<dim3(Ly.nin / 64, Ly.nout / 64), 256, 0, stream>>>(a);
-    LMW_LAUNCH_CHECK();
-    adam_vec<<<(Ly.nout + 255) / 256, 256, 0, stream>>>(Ly.b.p, Ly.mb.p, Ly.vb.p, Ly.gb.p, Ly.nout, static_cast<float>(lr), static_cast<float>(beta1),
+    stage_launch(adam_tile, dim3(Ly.nin / 64, Ly.nout / 64), 256, 0, stream, 1, a);
+    stage_launch(adam_vec, dim3((Ly.nout + 255) / 256), 256, 0, stream, 1, Ly.b.p, Ly.mb.p, Ly.vb.p, Ly.gb.p, Ly.nout, static_cast<float>(lr), static_cast<float>(beta1),
                                                        static_cast<float>(beta2), static_cast<float>(eps), c1, c2, scale, avg ? Ly.be.p : nullptr,
                                                        static_cast<float>(ema_decay));
-    LMW_LAUNCH_CHECK();
     g_launches += 2;
   }
 }
@@ -725,9 +734,13 @@ double Mlp::take_grad_norm_sum() {
 }
 
 void Mlp::check_status() {
-  int e = 0;
-  LMW_CUDA(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  read_status();
   LMW_CUDA(cudaStreamSynchronize(stream));
+  raise_status();
+}
+void Mlp::read_status() { LMW_CUDA(cudaMemcpyAsync(hstat.p + 1, err.p, sizeof(int), cudaMemcpyDeviceToHost, stream)); }
+void Mlp::raise_status() {
+  const int e = *reinterpret_cast<int *>(hstat.p + 1);
   if (e) {
     err.zero(stream);
     throw RuntimeError("a tensor-core GEMM of the network timed out waiting on its pipeline (code " + std::to_string(e) + ")");
@@ -735,12 +748,12 @@ void Mlp::check_status() {
 }
 
 double Mlp::take_loss() {
-  double v = 0;
-  LMW_CUDA(cudaMemcpyAsync(&v, loss_acc.p, sizeof(double), cudaMemcpyDeviceToHost, stream));
-  LMW_CUDA(cudaStreamSynchronize(stream));
+  LMW_CUDA(cudaMemcpyAsync(hstat.p, loss_acc.p, sizeof(double), cudaMemcpyDeviceToHost, stream));
   loss_acc.zero(stream);
-  check_status();
-  return v;
+  read_status();
+  LMW_CUDA(cudaStreamSynchronize(stream));
+  raise_status();
+  return hstat.p[0];
 }
 
 double Mlp::time_train_step(int batch, int reps) {

@@ -44,6 +44,8 @@ class Mlp {
   DevBuf<double> loss_acc, gnorm2, clip;
   DevBuf<float> gscale;
   DevBuf<int> err;
+  DevBuf<float> xin;                     // a host batch as it comes, row-major [batch][din] (allocated on first use)
+  HostBuf<double> hstat;                 // loss and error word read back (pinned)
 
   // host row-major weights of the logical size [nout][nin] and biases [nout]
   void set_layer(int l, const float *w, const float *b);
@@ -52,7 +54,7 @@ class Mlp {
   // host batch -> device (x [batch][din], target [batch][dout], mask [dout])
   void upload_input(const float *x, int batch);
   void upload_target(const float *t, const float *m, int batch);
-  void download_output(float *y_host, int batch);
+  void download_output(float *y_host, int batch);  // synchronises; raises if a GEMM timed out
 
   void forward(int batch);                 // x0 -> y
   void backward(int batch);                // y, target, mask -> gradients; loss accumulated into loss_acc
@@ -66,6 +68,8 @@ class Mlp {
   double take_grad_norm_sum();             // synchronises; the summed gradient norms since the last call
   double take_loss();                      // synchronises; returns and clears the accumulated loss
   void check_status();
+  void read_status();                      // queues the error word for raise_status
+  void raise_status();                     // after a synchronisation
   // average duration (ms) of one forward + backward + Adam step at this batch (CUDA events on the stream)
   double time_train_step(int batch, int reps);
   double time_forward(int batch, int reps);
