@@ -1138,9 +1138,11 @@ static void allow_max_shared_memory() {
   LMW_CUDA(cudaFuncSetAttribute(split_syn_ws<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_syn<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_syn<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<5, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<5, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_syn<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<8, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+  LMW_CUDA(cudaFuncSetAttribute(tc64_ana<8, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   for (int logn : {0, 6, 7, 8, 9, 10})
     for (int fmax : {3, 4})
       for (int direct : {0, 1}) LMW_CUDA(cudaFuncSetAttribute(split_grid_kernel(direct, fmax, logn), cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
@@ -1725,7 +1727,7 @@ static void stage_kernels(const SphDev &d, const SphTab<R> &t, const Tc64Plan *t
     // FP64 comes here above T170 only, where the blocks have 32 coefficients
     const int C = sizeof(R) == 8 ? 32 : ana_coef(d.nh);
     if constexpr (sizeof(R) == 8) {
-      if (tc) stage_launch(tc64_ana<5>, dim3(B, d.M), T64_THREADS, tc64->smem_ana, stream, 1, d, z, fold, sa, x0, xs, acc, none, mut, mut, mut);
+      if (tc) stage_launch(tc64->wide ? tc64_ana<5, 512> : tc64_ana<5, 256>, dim3(B, d.M), tc64->wide ? 512 : 256, tc64->smem_ana, stream, 1, d, z, fold, sa, x0, xs, acc, none, mut, mut, mut);
     }
     auto *k = sph_analysis<R, 32>;
     if constexpr (sizeof(R) == 4) {
@@ -1822,7 +1824,7 @@ void SphereEngine::launch_stage(int stage, double dt) {
       stage_launch(tc64_syn<6>, dim3(z.nsl * B, M), T64_THREADS, tc->smem_syn(2), stream, 1, d, z, in, qin, F, FQ, B);
       stage_launch(sph_grid64<8>, dim3(8 * nh, B), g64_threads(nlon), static_cast<size_t>(nlon) * 3 * sizeof(double2), stream, 8, d, tab64(*tab), F, FQ, fgrid.p, hsgrid.p,
                    G, GQ);
-      stage_launch(tc64_ana<8>, dim3(B, M), T64_THREADS, tc->smem_ana, stream, 1, d, z, G, sa, X0, XS, AC, GQ, reinterpret_cast<double2 *>(tq0.p),
+      stage_launch(tc->wide ? tc64_ana<8, 512> : tc64_ana<8, 256>, dim3(B, M), tc->wide ? 512 : 256, tc->smem_ana, stream, 1, d, z, G, sa, X0, XS, AC, GQ, reinterpret_cast<double2 *>(tq0.p),
                    reinterpret_cast<double2 *>(tqs.p), reinterpret_cast<double2 *>(tqacc.p));
       g_launches += 3;
       LMW_LAUNCH_CHECK();

@@ -33,9 +33,11 @@
 namespace lmw {
 
 struct Tc64Plan {
-  int nh16 = 16, lrows = 16, nsl = 1, nhk = 16, ns = 3;  // padded latitude pairs, per slice, slices; K of the analysis; stages
+  int nh16 = 16, lrows = 16, nsl = 1, nhk = 16;  // padded latitude pairs, per slice, slices; K of the analysis
+  int ns = 3, nsa = 3;                           // table chunks in flight: synthesis, analysis
   int nbt = 1, ntiles = 1;                               // members per synthesis tile
   int kc_max = 1, ra_max = 16;
+  bool wide = false;  // analysis CTAs of 512 threads
   size_t smem_ana = 0;
   size_t smem_syn(int blocks) const;  // row blocks of eight rows (members; two with the tracer)
   DevBuf<__nv_bfloat16> tS, tA;
@@ -47,7 +49,7 @@ struct Tc64Plan {
 };
 
 struct Tc64Dev {
-  int nh16, lrows, nsl, nhk, ns, nbt, ntiles, ra_max, ext;  // ext: coefficients with n to T+1
+  int nh16, lrows, nsl, nhk, ns, nsa, nbt, ntiles, ra_max, ext;  // ext: coefficients with n to T+1
   const __nv_bfloat16 *tS, *tA;
   const int *ke16, *kc, *ra16, *eS, *eA;
   const long *oS, *oA;
@@ -57,7 +59,7 @@ struct Tc64Dev {
 
 namespace {
 
-constexpr int T64_DIG = 8, T64_THREADS = 256;
+constexpr int T64_DIG = 8, T64_THREADS = 256, T64_STAGES = 8;  // T64_STAGES: most chunks in flight
 constexpr int T64_NONE = -100000, T64_NAN = 100000;  // row exponents: no digits; not finite
 // A operand: core matrices 128 bytes apart along K and 256 between 8-row groups. The digits' stores meet four to a bank;
 // with 16 spare bytes between core matrices they do not, which changed no time (T42 x 16, T170: within 2 %)
@@ -182,7 +184,7 @@ __global__ void tc64_build_ana(SphDev d, Tc64Dev z, const double *__restrict__ P
 
 // ------------------------------------------------------------------------------------------------ shared pieces
 struct T64Bars {
-  uint64_t full[4], empty[4], done;
+  uint64_t full[T64_STAGES], empty[T64_STAGES], done;
   uint32_t tslot;
   int fail, issued, consumed;
 };
@@ -277,7 +279,7 @@ __device__ __forceinline__ void t64_unload(uint32_t taddr, int w, int *dst, bool
 // grid: (slices x tiles, M). F = 4: U, V, zeta, Phi of x [B][3][ntri] into four [B][nlat][4][M], nbt members a tile; F = 2: the
 // tracer's q of qin [B][ntri] and delta of x into fourq [B][nlat][2][M]; F = 6: both in one launch, one member a tile, whose
 // second row block is q and delta.
-// T170, one member: 82.0 -> 18.7 us (FP64 pipe before); T42 x 16: 50.4 -> 11.6; T42, one member: 10.3 -> 6.9.
+// T170, one member: 82.0 -> 18.2 us (FP64 pipe before); T42 x 16: 50.4 -> 10.3; T42, one member: 10.3 -> 6.5.
 template <int F>
 __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, const double2 *__restrict__ x, const double2 *__restrict__ qin,
                                                            double2 *__restrict__ four, double2 *__restrict__ fourq, int B) {
@@ -305,63 +307,66 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
   if (tid < 2 * RF) rowexp[tid / RF][tid % RF] = 0;
   __syncthreads();
   pdl_wait(x, qin);
-  // thread k: column k, n = m + 2 k or m + 1 + 2 (k - ke16); the values of member ml in v[0..2F)
-  const int k = tid, n = k < ke16 ? m + 2 * k : m + 1 + 2 * (k - ke16), base = d.tri[m] - m;
-  const bool col = k < kc * 16, live = col && n <= d.N + 1;
-  const double *cf = z.cf + d.tri[m] + n;  // ext index of (m, n): tri[m] + m + n - m
-  for (int ml = 0; ml < nbt; ml++) {
-    double v[2 * RF];
+  // items: a complex value f of row block ml at column k, n = m + 2 k or m + 1 + 2 (k - ke16). Columns are padded to 16, so
+  // that a half warp has one (ml, f)
+  const int cols = kc * 16, total = (F == 6 ? 6 : mt * F) * cols, base = d.tri[m] - m;
+  constexpr int IT = ((F == 6 ? 6 : 2 * F) * 192 + T64_THREADS - 1) / T64_THREADS;
+  auto where = [&](int e, int &ml, int &f, int &k) {
+    const int v = e / cols;
+    k = e - v * cols;
+    ml = F == 6 ? v >> 2 : v / F;
+    f = F == 6 ? v & 3 : v % F;
+  };
+  double v[IT][2];
 #pragma unroll
-    for (int q = 0; q < 2 * RF; q++) v[q] = 0;
+  for (int r = 0; r < IT; r++) {
+    const int e = tid + r * T64_THREADS;
+    if (e >= total) break;
+    int ml, f, k;
+    where(e, ml, f, k);
+    const int n = k < ke16 ? m + 2 * k : m + 1 + 2 * (k - ke16);
+    const int b = F == 6 ? tile : tile * nbt + ml;
+    const double2 *xz = x + static_cast<size_t>(b) * 3 * d.ntri + base, *xd = xz + d.ntri, *xf = xd + d.ntri;
+    const double2 zero = make_double2(0.0, 0.0);
     const bool flow = F == 4 || (F == 6 && ml == 0);
-    if (live && ml < mt) {
-      const int b = F == 6 ? tile : tile * nbt + ml;
-      const double2 *xz = x + static_cast<size_t>(b) * 3 * d.ntri + base, *xd = xz + d.ntri, *xf = xd + d.ntri;
-      const double2 zero = make_double2(0.0, 0.0);
-      const double2 dn = n <= d.N ? xd[n] : zero;
-      if (F >= 4 && flow) {
-        // U_n = -a [i m delta_n / (n (n+1)) + eps_n zeta_{n-1} / n - eps_{n+1} zeta_{n+1} / (n+1)], V_n the same with zeta_n,
-        // -delta_{n-1}, -delta_{n+1}; the (0, 0) coefficients have no wind
-        const double w0 = cf[0], w1 = cf[z.ext], w2 = cf[2 * z.ext];
-        const double2 zn = n <= d.N ? xz[n] : zero, fn = n <= d.N ? xf[n] : zero;
-        const double2 zl = n > m && n > 1 ? xz[n - 1] : zero, dl = n > m && n > 1 ? xd[n - 1] : zero;
-        const double2 zu = n < d.N ? xz[n + 1] : zero, du = n < d.N ? xd[n + 1] : zero;
-        v[0] = fma(w0, dn.y, fma(w2, zu.x, -(w1 * zl.x)));
-        v[1] = fma(-w0, dn.x, fma(w2, zu.y, -(w1 * zl.y)));
-        v[2] = fma(w0, zn.y, fma(w1, dl.x, -(w2 * du.x)));
-        v[3] = fma(-w0, zn.x, fma(w1, dl.y, -(w2 * du.y)));
-        if constexpr (F >= 4) {
-          v[4] = zn.x;
-          v[5] = zn.y;
-          v[6] = fn.x;
-          v[7] = fn.y;
-        }
+    const double2 *ce = flow ? (f == 0 ? xd : f == 3 ? xf : xz) : f == 0 ? qin + static_cast<size_t>(b) * d.ntri + base : xd;
+    const double2 c = n <= d.N ? ce[n] : zero;
+    v[r][0] = c.x;
+    v[r][1] = c.y;
+    if (flow && f < 2) {
+      // U_n = -a [i m delta_n / (n (n+1)) + eps_n zeta_{n-1} / n - eps_{n+1} zeta_{n+1} / (n+1)], V_n the same with zeta_n,
+      // -delta_{n-1}, -delta_{n+1}; the (0, 0) coefficients have no wind
+      const double2 *nb = f == 0 ? xz : xd;
+      const bool live = n <= d.N + 1;
+      const double *cf = z.cf + d.tri[m] + (live ? n : m);  // ext index of (m, n): tri[m] + m + n - m
+      const double w0 = live ? cf[0] : 0.0, w1 = live ? cf[z.ext] : 0.0, w2 = live ? cf[2 * z.ext] : 0.0;
+      const double2 l = n > m && n > 1 && n <= d.N + 1 ? nb[n - 1] : zero, u = n < d.N ? nb[n + 1] : zero;
+      if (f == 0) {
+        v[r][0] = fma(w0, c.y, fma(w2, u.x, -(w1 * l.x)));
+        v[r][1] = fma(-w0, c.x, fma(w2, u.y, -(w1 * l.y)));
       } else {
-        const double2 qn = n <= d.N ? qin[static_cast<size_t>(b) * d.ntri + base + n] : zero;
-        v[0] = qn.x;
-        v[1] = qn.y;
-        v[2] = dn.x;
-        v[3] = dn.y;
+        v[r][0] = fma(w0, c.y, fma(w1, l.x, -(w2 * u.x)));
+        v[r][1] = fma(-w0, c.x, fma(w1, l.y, -(w2 * u.y)));
       }
     }
-    if (tid < ((kc * 16 + 31) & ~31)) {
+    const int ex = __reduce_max_sync(0xffffu << (tid & 16), max(t64_exp(v[r][0]), t64_exp(v[r][1])));
+    if ((tid & 15) == 0) atomicMax(&rowexp[ml][f], ex);
+  }
+  __syncthreads();
 #pragma unroll
-      for (int f = 0; f < RF; f++) {
-        const int ex = __reduce_max_sync(0xffffffffu, max(t64_exp(v[2 * f]), t64_exp(v[2 * f + 1])));
-        if ((tid & 31) == 0) atomicMax(&rowexp[ml][f], ex);
-      }
-    }
-    __syncthreads();
-    if (col) {
-      uint8_t *o = A + (k >> 4) * ablk + (7 * nbt + ml) * T64_SBO + ((k & 15) >> 3) * T64_LBO + (k & 7) * 2;
+  for (int r = 0; r < IT; r++) {
+    const int e = tid + r * T64_THREADS;
+    if (e >= total) break;
+    int ml, f, k;
+    where(e, ml, f, k);
+    uint8_t *o = A + (k >> 4) * ablk + (7 * nbt + ml) * T64_SBO + ((k & 15) >> 3) * T64_LBO + (k & 7) * 2 + f * 32;
+    const int er = t64_row(rowexp[ml][f]);
 #pragma unroll
-      for (int q = 0; q < 2 * RF; q++) {
-        if (F == 6 && !flow && q >= 4) break;
-        unsigned short dg[T64_DIG];
-        t64_digits(t64_fixed(v[q], t64_row(rowexp[ml][q >> 1])), dg);
+    for (int q = 0; q < 2; q++) {
+      unsigned short dg[T64_DIG];
+      t64_digits(t64_fixed(v[r][q], er), dg);
 #pragma unroll
-        for (int i = 0; i < T64_DIG; i++) *reinterpret_cast<unsigned short *>(o + i * nbt * T64_SBO + q * 16) = dg[i];
-      }
+      for (int i = 0; i < T64_DIG; i++) *reinterpret_cast<unsigned short *>(o + i * nbt * T64_SBO + q * 16) = dg[i];
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -415,9 +420,9 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
 // ------------------------------------------------------------------------------------------------ analysis + RK4
 // grid: (B, M). SLOTS = 5: the flow (fold [B][nh][5][2][M]; x0, xs, acc [B][3][ntri]); SLOTS = 8: with the tracer (foldq
 // [B][nh][3][2][M]: U q, V q, q delta; q0, qs, qacc [B][ntri]).
-// T170, one member: 71.7 -> 29.6 us; T42 x 16: 45.1 -> 29.7; T42, one member: 8.2 -> 8.8.
-template <int SLOTS>
-__global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, const double2 *__restrict__ fold, StageArgs sa, double2 *__restrict__ x0,
+// T170, one member: 71.7 -> 29.8 us; T42 x 16: 45.1 -> 26.2; T42, one member: 8.2 -> 7.5.
+template <int SLOTS, int NT>
+__global__ void __launch_bounds__(NT, 1) tc64_ana(SphDev d, Tc64Dev z, const double2 *__restrict__ fold, StageArgs sa, double2 *__restrict__ x0,
                                                            double2 *__restrict__ xs, double2 *__restrict__ acc, const double2 *__restrict__ foldq,
                                                            double2 *__restrict__ q0, double2 *__restrict__ qs, double2 *__restrict__ qacc) {
   constexpr int Q = 2 * SLOTS, FIELDS = SLOTS == 8 ? 4 : 3, GPO = 2;  // GPO: row groups per digit
@@ -426,52 +431,71 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
   __shared__ int rowexp[2][Q];
   const int tid = threadIdx.x, m = blockIdx.y, b = blockIdx.x;
   const int kc = z.nhk / 16, ra0 = z.ra16[2 * m], ra1 = z.ra16[2 * m + 1], stage_bytes = T64_DIG * z.ra_max * 32, ablk = 15 * GPO * T64_SBO;
-  uint8_t *stages = t64_sm, *A = t64_sm + z.ns * stage_bytes;
+  uint8_t *stages = t64_sm, *A = t64_sm + z.nsa * stage_bytes;
   uint32_t ncols = 32;
   while (ncols < static_cast<uint32_t>(ra0 + ra1)) ncols <<= 1;
-  t64_setup(bars, z.ns, ncols);
+  t64_setup(bars, z.nsa, ncols);
   // chunks: parity 0's kc, then parity 1's
   auto chunk = [&](int it) { return z.tA + z.oA[2 * m + (it < kc ? 0 : 1)] + static_cast<long>(it < kc ? it : it - kc) * T64_DIG * (it < kc ? ra0 : ra1) * 16; };
   auto bytes = [&](int it) { return static_cast<uint32_t>(T64_DIG * (it < kc ? ra0 : ra1) * 32); };
   int copied = 0;
   if (tid == 0)
-    for (; copied < min(2 * kc, z.ns); copied++) t64_copy(bars, stages, stage_bytes, z.ns, copied, chunk(copied), bytes(copied), z.err);
-  for (int e = tid; e < 2 * kc * 7 * GPO * (T64_SBO / 16); e += T64_THREADS) {
+    for (; copied < min(2 * kc, z.nsa); copied++) t64_copy(bars, stages, stage_bytes, z.nsa, copied, chunk(copied), bytes(copied), z.err);
+  for (int e = tid; e < 2 * kc * 7 * GPO * (T64_SBO / 16); e += NT) {
     const int blk = e / (7 * GPO * (T64_SBO / 16)), o = e % (7 * GPO * (T64_SBO / 16));
     *reinterpret_cast<uint4 *>(A + blk * ablk + o * 16) = make_uint4(0, 0, 0, 0);
   }
   if (tid < 2 * Q) rowexp[tid / Q][tid % Q] = 0;
   __syncthreads();
   pdl_wait(fold, foldq, x0, xs, acc, q0, qs, qacc);
-  // thread: latitude pair jh at parity p of the fold
-  const int p = tid / z.nhk, jh = tid % z.nhk;
-  const bool col = p < 2;
-  double v[Q];
+  // items: slot s of latitude pair jh at parity p of the fold; pairs are padded to 16, so that a half warp has one (s, p)
+  const int items = SLOTS * 2 * z.nhk;
+  constexpr int IT = (SLOTS * 256 + NT - 1) / NT;
+  auto where = [&](int e, int &s, int &p, int &jh) {
+    jh = e & (z.nhk - 1);  // a power of two
+    p = e / z.nhk & 1;
+    s = e / z.nhk >> 1;
+  };
+  double v[IT][2];
 #pragma unroll
-  for (int s = 0; s < SLOTS; s++) {
-    const double2 *src = s < 5 ? fold + ((static_cast<size_t>(b) * d.nh + jh) * 5 + s) * 2 * d.M : foldq + ((static_cast<size_t>(b) * d.nh + jh) * 3 + s - 5) * 2 * d.M;
-    const double2 g = col && jh < d.nh ? src[p * d.M + m] : make_double2(0.0, 0.0);
-    v[2 * s] = g.x;
-    v[2 * s + 1] = g.y;
+  for (int r = 0; r < IT; r++) {
+    const int e = tid + r * NT;
+    int s, p, jh;
+    where(e, s, p, jh);
+    v[r][0] = v[r][1] = 0;
+    if (e < items && jh < d.nh) {
+      const double2 *src = s < 5 ? fold + ((static_cast<size_t>(b) * d.nh + jh) * 5 + s) * 2 * d.M : foldq + ((static_cast<size_t>(b) * d.nh + jh) * 3 + s - 5) * 2 * d.M;
+      const double2 g = src[p * d.M + m];
+      v[r][0] = g.x;
+      v[r][1] = g.y;
+    }
   }
-  if (col) {
-    // latitude pairs are padded to 16: a half warp has one parity
-    const unsigned half = 0xffffu << (tid & 16);
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const int ex = __reduce_max_sync(half, t64_exp(v[q]));
-      if ((tid & 15) == 0) atomicMax(&rowexp[p][q], ex);
+  for (int r = 0; r < IT; r++) {
+    const int e = tid + r * NT;
+    if (e >= items) break;
+    int s, p, jh;
+    where(e, s, p, jh);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int ex = __reduce_max_sync(0xffffu << (tid & 16), t64_exp(v[r][q]));
+      if ((tid & 15) == 0) atomicMax(&rowexp[p][2 * s + q], ex);
     }
   }
   __syncthreads();
-  if (col) {
-    uint8_t *o = A + (p * kc + (jh >> 4)) * ablk + 7 * GPO * T64_SBO + ((jh & 15) >> 3) * T64_LBO + (jh & 7) * 2;
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
+  for (int r = 0; r < IT; r++) {
+    const int e = tid + r * NT;
+    if (e >= items) break;
+    int s, p, jh;
+    where(e, s, p, jh);
+    uint8_t *o = A + (p * kc + (jh >> 4)) * ablk + 7 * GPO * T64_SBO + ((jh & 15) >> 3) * T64_LBO + (jh & 7) * 2 + (s >> 2) * T64_SBO + (s & 3) * 32;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
       unsigned short dg[T64_DIG];
-      t64_digits(t64_fixed(v[q], t64_row(rowexp[p][q])), dg);
+      t64_digits(t64_fixed(v[r][q], t64_row(rowexp[p][2 * s + q])), dg);
 #pragma unroll
-      for (int i = 0; i < T64_DIG; i++) *reinterpret_cast<unsigned short *>(o + (i * GPO + (q >> 3)) * T64_SBO + (q & 7) * 16) = dg[i];
+      for (int i = 0; i < T64_DIG; i++) *reinterpret_cast<unsigned short *>(o + i * GPO * T64_SBO + q * 16) = dg[i];
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -480,24 +504,24 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
   const int role = tc::uniform(tid >> 5);
   if (tid == 0) {
     for (; copied < 2 * kc; copied++)
-      if (!t64_copy(bars, stages, stage_bytes, z.ns, copied, chunk(copied), bytes(copied), z.err)) break;
+      if (!t64_copy(bars, stages, stage_bytes, z.nsa, copied, chunk(copied), bytes(copied), z.err)) break;
   } else if (role == 1) {
     const uint32_t s0 = tc::su32(stages), a0 = tc::su32(A), t0 = tc::uniform(tmem);
     const bool leader = tc::elect_one();
     for (int it = 0; it < 2 * kc; it++)
-      if (!t64_mma(bars, s0, stage_bytes, z.ns, it, it < kc ? ra0 : ra1, a0 + it * ablk, GPO, t0 + (it < kc ? 0 : ra0), it == 0 || it == kc, leader, z.err)) break;
+      if (!t64_mma(bars, s0, stage_bytes, z.nsa, it, it < kc ? ra0 : ra1, a0 + it * ablk, GPO, t0 + (it < kc ? 0 : ra0), it == 0 || it == kc, leader, z.err)) break;
     tc::commit(leader, tc::su32(&bars.done));
   }
   // item e of the update: field e / cnt, n = m + e % cnt. What it reads is loaded while the MMAs run
   const int cnt = d.N + 1 - m;
   // field f of item i: the flow's three, then the tracer
   auto place = [&](int f, int i) { return (f < 3 ? static_cast<size_t>(b) * 3 + f : static_cast<size_t>(b)) * d.ntri + d.tri[m] + i; };
-  constexpr int ITEMS = (FIELDS * 171 + T64_THREADS - 1) / T64_THREADS;
+  constexpr int ITEMS = (FIELDS * 171 + NT - 1) / NT;
   double2 xv[ITEMS], av[ITEMS];
   double w3[ITEMS], w4[ITEMS], lap[ITEMS], fac[ITEMS];
 #pragma unroll
   for (int r = 0; r < ITEMS; r++) {
-    const int e = tid + r * T64_THREADS, f = e / cnt, i = e - f * cnt;
+    const int e = tid + r * NT, f = e / cnt, i = e - f * cnt;
     xv[r] = av[r] = make_double2(0.0, 0.0);
     w3[r] = w4[r] = lap[r] = fac[r] = 0;
     if (f < FIELDS) {
@@ -510,21 +534,21 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
       if (sa.stage == 3) fac[r] = sa.filt[(f >= 2 ? 1 : 0) * d.M + m + i];
     }
   }
-  const bool ok = t64_finish(bars, z.ns, z.err);
+  const bool ok = t64_finish(bars, z.nsa, z.err);
   pdl_trigger();
   // sums S[q][n - m], n to T+1
   const int warp = tid >> 5, lane = tid & 31, quarter = warp & 3, row = quarter * 32 + lane, next = d.N + 2 - m;
-  constexpr int ROWS = 64 * GPO, LD = 33;
-  int *red = reinterpret_cast<int *>(t64_sm);                                   // [2][ROWS][LD]: two blocks of 32 columns
-  double *S = reinterpret_cast<double *>(t64_sm + ((2 * ROWS * LD * sizeof(int) + 15) & ~15u));  // [Q][next + 1]
+  constexpr int ROWS = 64 * GPO, LD = 33, NB = NT / 128;  // NB column blocks of 32 at once
+  int *red = reinterpret_cast<int *>(t64_sm);                                   // [NB][ROWS][LD]
+  double *S = reinterpret_cast<double *>(t64_sm + ((NB * ROWS * LD * sizeof(int) + 15) & ~15u));  // [Q][next + 1]
   const int sld = next + 1, total = ra0 + ra1;
-  for (int cb = 0; ok && cb < total; cb += 64) {
-    const int c0 = cb + (warp < 4 ? 0 : 32), w = total - c0 >= 32 ? 32 : 16;
+  for (int cb = 0; ok && cb < total; cb += 32 * NB) {
+    const int c0 = cb + (warp >> 2) * 32, w = total - c0 >= 32 ? 32 : 16;
     if (quarter * 32 < ROWS && c0 < total)
-      t64_unload(tmem + c0 + (static_cast<uint32_t>(quarter * 32) << 16), w, red + ((warp < 4 ? 0 : ROWS) + row) * LD, true);
+      t64_unload(tmem + c0 + (static_cast<uint32_t>(quarter * 32) << 16), w, red + ((warp >> 2) * ROWS + row) * LD, true);
     __syncthreads();
-    for (int e = tid; e < Q * 64; e += T64_THREADS) {
-      const int i = e & 63, q = e >> 6, c = cb + i, pp = c < ra0 ? 0 : 1, r = pp ? c - ra0 : c, nn = m + pp + 2 * r;
+    for (int e = tid; e < Q * 32 * NB; e += NT) {
+      const int i = e & (32 * NB - 1), q = e / (32 * NB), c = cb + i, pp = c < ra0 ? 0 : 1, r = pp ? c - ra0 : c, nn = m + pp + 2 * r;
       if (c >= total || nn > d.N + 1) continue;
       const T64Sum t = t64_sum(red + ((i >> 5) * ROWS + (q >> 3) * 8 + (q & 7)) * LD + (i & 31), 8 * GPO * LD);
       S[q * sld + nn - m] = t64_value(t.hi, t.lo, t64_row(rowexp[pp][q]), z.eA[d.tri[m] + nn]);
@@ -535,7 +559,7 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
     const double mm = static_cast<double>(m);
 #pragma unroll
     for (int r = 0; r < ITEMS; r++) {
-      const int e = tid + r * T64_THREADS, f = e / cnt, i = e - f * cnt, q = d.tri[m] + i;
+      const int e = tid + r * NT, f = e / cnt, i = e - f * cnt, q = d.tri[m] + i;
       if (f >= FIELDS) continue;
       auto at = [&](int s) { return make_double2(S[2 * s * sld + i], S[(2 * s + 1) * sld + i]); };
       // the H sum: -n eps_{n+1} S(n+1) + (n+1) eps_n S(n-1)
@@ -571,7 +595,7 @@ __global__ void __launch_bounds__(T64_THREADS, 1) tc64_ana(SphDev d, Tc64Dev z, 
 }  // namespace
 
 inline Tc64Dev tc64_dev(const Tc64Plan &p, int ext) {
-  return Tc64Dev{p.nh16, p.lrows, p.nsl, p.nhk, p.ns, p.nbt, p.ntiles, p.ra_max, ext, p.tS.p, p.tA.p, p.ke16.p, p.kc.p, p.ra16.p, p.eS.p, p.eA.p, p.oS.p, p.oA.p, p.cf.p, p.err.p};
+  return Tc64Dev{p.nh16, p.lrows, p.nsl, p.nhk, p.ns, p.nsa, p.nbt, p.ntiles, p.ra_max, ext, p.tS.p, p.tA.p, p.ke16.p, p.kc.p, p.ra16.p, p.eS.p, p.eA.p, p.oS.p, p.oA.p, p.cf.p, p.err.p};
 }
 
 // an M = 128 MMA reads sixteen row groups from its A block: with one row block of eight rows up to eight past the fifteen
@@ -635,8 +659,24 @@ inline void build_tc64(Tc64Plan &p, const HostTables &h, const SphDev &d, double
   // members per synthesis tile: two share an MMA (its 128 rows) where one each would not fit the SMs at once
   p.nbt = B > 1 && static_cast<long>(M) * p.nsl * B > 2 * 152 ? 2 : 1;
   p.ntiles = (B + p.nbt - 1) / p.nbt;
-  const size_t red_ana = static_cast<size_t>(2) * 128 * 33 * sizeof(int) + 16 + static_cast<size_t>(16) * (N + 3) * sizeof(double);
-  p.smem_ana = std::max(static_cast<size_t>(p.ns) * T64_DIG * p.ra_max * 32 + static_cast<size_t>(2) * (p.nhk / 16) * 30 * T64_SBO, red_ana);
+  // Table chunks in flight: three where several CTAs share an SM and hide one another's waits, else as many as there are
+  // and fit, so that all of them have arrived when the predecessor ends
+  const auto stages = [](long ctas, size_t a, size_t stage, int chunks) {
+    const size_t room = 225 * 1024 / static_cast<size_t>(std::max(1l, std::min(2l, (ctas + 151) / 152))) - 1024;
+    const int fit = room > a ? static_cast<int>((room - a) / stage) : 0;
+    return ctas > 2 * 152 ? 3 : std::max(3, std::min({fit, chunks, T64_STAGES}));
+  };
+  const size_t a_syn = static_cast<size_t>(p.kc_max) * 30 * T64_SBO + 8 * T64_SBO + 256, a_ana = static_cast<size_t>(2) * (p.nhk / 16) * 30 * T64_SBO;
+  p.ns = stages(static_cast<long>(M) * p.nsl * p.ntiles, a_syn, static_cast<size_t>(T64_DIG) * p.lrows * 32, p.kc_max);
+  const size_t ana_stage = static_cast<size_t>(T64_DIG) * p.ra_max * 32;
+  // an analysis CTA that cannot share its SM (T170's operand) has it alone
+  const bool alone = a_ana + 3 * ana_stage > 112 * 1024;
+  p.nsa = stages(alone ? 1 : static_cast<long>(M) * B, a_ana, ana_stage, 2 * (p.nhk / 16));
+  // 512 threads shorten the digits, the sums and the update of a CTA that shares its SM with at most one other; more CTAs of
+  // 256 overlap their phases better (T170 x 4, one CTA per SM: 88.2 us with 256 threads, 82.1 with 512)
+  p.wide = alone || static_cast<long>(M) * B <= 2 * 152;
+  const size_t red_ana = static_cast<size_t>(p.wide ? 4 : 2) * 128 * 33 * sizeof(int) + 16 + static_cast<size_t>(16) * (N + 3) * sizeof(double);
+  p.smem_ana = std::max(static_cast<size_t>(p.nsa) * ana_stage + a_ana, red_ana);
   DevBuf<double> P1;
   up(P1, h.P1);
   const Tc64Dev z = tc64_dev(p, ext);

@@ -78,3 +78,21 @@ def test_fp32_sums_from_staged_coefficients(engine, T):
             assert np.array_equal(x, y)
         f, g = one.get_state()[2], ref.get_state()[2]
         assert np.linalg.norm(f - g) <= 1e-6 * np.linalg.norm(g)
+
+
+@pytest.mark.parametrize("T", [5, 15, 31, 33, 42, 62, 86])
+def test_batches_that_fill_the_gpu_keep_the_bits(engine, T):
+    """Past 304 (wavenumber, member) pairs the FP64 analysis takes narrower CTAs and the synthesis pairs its members."""
+    B, dt, states = 304 // (T + 1) + 2, 20000.0 / T, [initial(T, 100 * T + k) for k in range(2)]
+    many = engine.Sphere(T, diffusion=1e15, members=B)
+    for b in range(B):
+        many.set_state(*states[b % 2], member=b)
+    for _ in range(3):
+        many.step(dt)
+    for k in range(2):
+        one = engine.Sphere(T, diffusion=1e15)
+        one.set_state(*states[k])
+        one.run(3 * dt, dt)
+        for b in range(k, B, 2):
+            for x, y in zip(one.get_state(), many.get_state(member=b)):
+                assert np.array_equal(x, y)
