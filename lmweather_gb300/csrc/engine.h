@@ -186,6 +186,7 @@ class SphereEngine {
   DevBuf<int> gflag;   // per member: bit 0 tilted Coriolis grid, bit 1 orography
   DevBuf<double> om2;  // per member: 2 Omega
   uint64_t launches_per_step() const { return launches_step; }
+  double last_step_dt = 0;  // dt of the last step() (zero: none)
   // average duration (ms) per launch of each stage kernel class over `reps` launches (CUDA events on the
   // engine stream): out[0] synthesis, out[1] grid (FFTs + products), out[2] analysis + RK4 update. x0 unchanged.
   void kernel_times(double dt, int reps, double *out);
