@@ -1,17 +1,17 @@
-// Spectral-transform shallow water on the sphere (the lmweather Sphere model, cpp/sphere.cpp), FP64 path.
+// Spectral-transform shallow water on the sphere (the lmweather Sphere model, cpp/sphere.cpp), FP64 and FP32 paths.
 //
 // Per RK4 stage three kernels run on the engine stream:
-//   sph_synth     per zonal wavenumber m (paired with T-m for load balance) and southern latitude jh: the
-//                 six Legendre synthesis sums (psi P, chi P, psi H, chi H, zeta P, Phi P) split by the parity of
-//                 n-m, which gives both mirror latitudes at once (hemispheric fold); writes the Fourier
-//                 coefficients of U, V, zeta, Phi for both latitudes.
-//   sph_grid      per latitude pair: the two latitudes ride in the real and imaginary parts of one complex
-//                 FFT; inverse FFTs of U, V, zeta, Phi, the nonlinear products of cpp/sphere.cpp:348-359 in
-//                 place, forward FFTs of the five products, then the quadrature weights and the fold
-//                 (sum/difference of the mirror latitudes). The grid never leaves shared memory.
-//   sph_analysis  per spectral coefficient (m, n): the seven folded Legendre analysis sums, the tendencies
-//                 of cpp/sphere.cpp:372-389 and the RK4 stage update (cpp/sphere.cpp:416-434) with the del^4
-//                 filter fused into the last stage.
+//   synthesis     Fourier coefficients of U, V, zeta, Phi at both mirror latitudes of a pair from the Legendre sums of
+//                 either parity of n - m (hemispheric fold). FP64 up to T170: tc64_syn (sphere_tc64.cuh, four sums on the
+//                 tensor cores); FP32 and FP64 above: sph_synth (six sums: psi P, chi P, psi H, chi H, zeta P, Phi P).
+//   grid          per latitude pair: the two latitudes ride in the real and imaginary parts of one complex
+//                 FFT; inverse FFTs of U, V, zeta, Phi, the nonlinear products of cpp/sphere.cpp:348-359,
+//                 forward FFTs of the five products, then the quadrature weights and the fold
+//                 (sum/difference of the mirror latitudes). The grid never leaves shared memory. FP64: sph_grid64 (a
+//                 cluster per pair); FP32: sph_grid.
+//   analysis      the folded Legendre analysis sums, the tendencies of cpp/sphere.cpp:372-389 and the RK4 stage
+//                 update (cpp/sphere.cpp:416-434) with the del^4 filter fused into the last stage. tc64_ana (five sums) or
+//                 sph_analysis (seven), as for the synthesis.
 // Layouts: state x[member][field][tri] complex128, tri(m, n) = packed triangle offset; Fourier
 // coefficients four[member][lat][field][m]; folded analysis inputs fold[member][jh][slot][parity][m].
 #include <algorithm>
@@ -1717,11 +1717,12 @@ static void stage_kernels(const SphDev &d, const SphTab<R> &t, const Tc64Plan *t
   }
   if (which < 0 || which == 1) {
     if constexpr (sizeof(R) == 8)
-      stage_launch(sph_grid64<5>, dim3(G64_CTAS * d.nh, B), g64_threads(d.nlon), static_cast<size_t>(d.nlon) * 3 * sizeof(double2), stream, G64_CTAS, d, t,
+      stage_launch(sph_grid64<5>, dim3(G64_CTAS * d.nh, B), g64_threads(d.nlon), even_share(static_cast<size_t>(d.nlon) * 3 * sizeof(double2), static_cast<long>(G64_CTAS) * d.nh * B), stream, G64_CTAS, d, t,
                    four, none, fgrid, hsgrid, fold, mut);
     else
-      stage_launch(sph_grid<R>, dim3(d.nh, B), GRID_THREADS, 5 * static_cast<size_t>(fft_row<3>(d.nlon)) * sizeof(typename V2<R>::type), stream, 1, d, t,
-                   four, fgrid, hsgrid, fold);
+      stage_launch(sph_grid<R>, dim3(d.nh, B), GRID_THREADS,
+                   even_share(5 * static_cast<size_t>(fft_row<3>(d.nlon)) * sizeof(typename V2<R>::type), static_cast<long>(d.nh) * B), stream, 1, d, t, four, fgrid,
+                   hsgrid, fold);
   }
   if (which < 0 || which == 2) {
     // FP64 comes here above T170 only, where the blocks have 32 coefficients
@@ -1771,8 +1772,8 @@ static void split_stage(const SphDev &d, const SphTab<float> &t, const SplitPlan
     // the FFT group bound sets the kernel's register budget: 4 (sixteen elements a thread) two CTAs per SM,
     // else three
     const int logn = sp.grid_fixed ? d.logn : 0;
-    stage_launch(split_grid_kernel(sp.direct, sp.fgrp >= 4 ? 4 : 3, logn), grid, split_grid_threads(logn), split_grid_bytes(sp.jb, d.nlon), stream, 1, d, t, sd,
-                 fgrid, hsgrid);
+    stage_launch(split_grid_kernel(sp.direct, sp.fgrp >= 4 ? 4 : 3, logn), grid, split_grid_threads(logn),
+                 even_share(split_grid_bytes(sp.jb, d.nlon), static_cast<long>(grid.x) * B), stream, 1, d, t, sd, fgrid, hsgrid);
   }
   if (which < 0 || which == 2) {
     if (sp.ana_both && 2 * sp.ra_pair > 512) throw InvalidArgument("split precision: both parities' accumulators exceed tensor memory");
@@ -1822,7 +1823,7 @@ void SphereEngine::launch_stage(int stage, double dt) {
       double2 *F = reinterpret_cast<double2 *>(four.p), *FQ = reinterpret_cast<double2 *>(fourq.p), *G = reinterpret_cast<double2 *>(fold.p),
               *GQ = reinterpret_cast<double2 *>(foldq.p);
       stage_launch(tc64_syn<6>, dim3(z.nsl * B, M), T64_THREADS, tc->smem_syn(2), stream, 1, d, z, in, qin, F, FQ, B);
-      stage_launch(sph_grid64<8>, dim3(8 * nh, B), g64_threads(nlon), static_cast<size_t>(nlon) * 3 * sizeof(double2), stream, 8, d, tab64(*tab), F, FQ, fgrid.p, hsgrid.p,
+      stage_launch(sph_grid64<8>, dim3(8 * nh, B), g64_threads(nlon), even_share(static_cast<size_t>(nlon) * 3 * sizeof(double2), 8l * nh * B), stream, 8, d, tab64(*tab), F, FQ, fgrid.p, hsgrid.p,
                    G, GQ);
       stage_launch(tc->wide ? tc64_ana<8, 512> : tc64_ana<8, 256>, dim3(B, M), tc->wide ? 512 : 256, tc->smem_ana, stream, 1, d, z, G, sa, X0, XS, AC, GQ, reinterpret_cast<double2 *>(tq0.p),
                    reinterpret_cast<double2 *>(tqs.p), reinterpret_cast<double2 *>(tqacc.p));

@@ -412,7 +412,7 @@ __device__ __forceinline__ int snake_item(int k) {
 // ------------------------------------------------------------------------------------------- synthesis, warp-specialised
 // The same work as split_syn, by persistent CTAs whose warps take roles (as split_ana_ws): thread 0 streams the H
 // and P operand and table chunks of the CTA's items (m, member tile, latitude slice; dealt by snake_item) through
-// a ring of ns fixed-size stages; thread 32 issues the MMAs of item i into tensor-memory buffer i % 2 (four
+// a ring of ns fixed-size stages; warp 1 issues the MMAs of item i into tensor-memory buffer i % 2 (four
 // accumulators H E/O, P E/O of nh columns each) and commits it to accf[i % 2]; warps 2..9 copy a finished buffer
 // to shared memory, release it (acce) and write the item's Fourier records while the next item loads and
 // multiplies. Same products in the same order as split_syn, same epilogue arithmetic: the same bits. Every wait is
@@ -1550,7 +1550,7 @@ __global__ void __launch_bounds__(SPLIT_ANA_THREADS, MINB) split_ana(SphDev d, S
 // ------------------------------------------------------------------------------------------- analysis, warp-specialised
 // The same work as split_ana (direct operands), by persistent CTAs whose warps take roles, so that one item's
 // epilogue runs while the next item's operands load and multiply: thread 0 streams the H and P chunks of the CTA's
-// items (m, parity or both, member tile) through a ring of ns fixed-size stages; thread 32 issues the MMAs of item i
+// items (m, parity or both, member tile) through a ring of ns fixed-size stages; warp 1 issues the MMAs of item i
 // into tensor-memory accumulator buffer i % 2 and commits it to accf[i % 2]; warps 2..9 (256 threads) wait for it,
 // copy it to shared memory, release the buffer (acce[i % 2]) and run the epilogue (ana_coef, the same arithmetic as
 // split_ana). Items are dealt by snake_item. Every wait is bounded; after a failure each role stops,

@@ -57,7 +57,7 @@ struct GemmArgs {
 };
 
 // One 128 x BN output tile per CTA. Thread 0 streams (A, B) K chunks through S shared-memory stages with bulk
-// copies; thread 32 issues the MMAs (4 per chunk, K = 16 each) into a 128 x BN FP32 accumulator in TMEM and frees
+// copies; warp 1 issues the MMAs (4 per chunk, K = 16 each) into a 128 x BN FP32 accumulator in TMEM and frees
 // each stage with tcgen05.commit; then all four warps read their 32 TMEM lanes back and apply the epilogue.
 template <int BN, int S>
 __global__ void __launch_bounds__(128, 1) mlp_gemm(GemmArgs g) {
