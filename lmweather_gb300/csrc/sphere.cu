@@ -2215,21 +2215,76 @@ void SphereEngine::autotune_split() {
       dir = v;
     }
   }
-  const Cand *bg = pick(1, dir), *bs = pick(0, 0), *ba = pick(2, dir);
-  sp.direct = dir;
-  sp.jb = bg ? bg->jb : jb0;
-  sp.fgrp = bg ? bg->fg : fg0;
-  sp.ns_syn = bs ? bs->ns : nss0;
-  sp.smem_syn = bs ? bs->bytes : sms0;
-  sp.syn_split = bs ? bs->jb : sl0;
-  sp.syn_nh = sp.nh16 / sp.syn_split;
-  sp.syn_ws = bs ? bs->ws : sws0;
-  sp.ns_ana = ba ? ba->ns : nsa0;
-  sp.smem_ana = ba ? ba->bytes : sma0;
-  sp.ana_both = ba ? ba->jb : ab0;
-  sp.ana_grid = ba ? ba->fg : ag0;
-  sp.ana_minb = ba ? ba->mb : mb0;
-  sp.ana_ws = ba ? ba->ws : ws0;
+  auto choose = [&](int v, const Cand *bg, const Cand *bs, const Cand *ba) {
+    sp.direct = v;
+    sp.jb = bg ? bg->jb : jb0;
+    sp.fgrp = bg ? bg->fg : fg0;
+    sp.ns_syn = bs ? bs->ns : nss0;
+    sp.smem_syn = bs ? bs->bytes : sms0;
+    sp.syn_split = bs ? bs->jb : sl0;
+    sp.syn_nh = sp.nh16 / sp.syn_split;
+    sp.syn_ws = bs ? bs->ws : sws0;
+    sp.ns_ana = ba ? ba->ns : nsa0;
+    sp.smem_ana = ba ? ba->bytes : sma0;
+    sp.ana_both = ba ? ba->jb : ab0;
+    sp.ana_grid = ba ? ba->fg : ag0;
+    sp.ana_minb = ba ? ba->mb : mb0;
+    sp.ana_ws = ba ? ba->ws : ws0;
+  };
+  // In a run the kernels start while their predecessors drain, and what one leaves free for the next counts beside its own
+  // time: one member at T170 ran in 40 to 49 us a stage with plans whose kernels take 38 us one by one. So the candidates
+  // closest to the best of their kernel are compared again in whole stages, one kernel after another, for each interface
+  // (T170: 38.5 us every time; T42 x 384 119 -> 112, T85 x 128 155 -> 148).
+  auto chain = [&]() {
+    float best = 1e30f;
+    for (int round = 0; round < 2; round++) {
+      for (int k = 0; k < 3; k++) launch(k);
+      LMW_CUDA(cudaEventRecord(e0, stream));
+      for (int r = 0; r < 4; r++)
+        for (int k = 0; k < 3; k++) launch(k);
+      LMW_CUDA(cudaEventRecord(e1, stream));
+      LMW_LAUNCH_CHECK();
+      LMW_CUDA(cudaEventSynchronize(e1));
+      float ms = 0;
+      LMW_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+      best = std::min(best, ms);
+    }
+    return best;
+  };
+  auto close = [&](int which, int v) {
+    std::vector<const Cand *> r;
+    const Cand *b = pick(which, v);
+    for (const Cand &c : cands)
+      if (b && c.which == which && (which == 0 || c.dir == v) && c.best <= 1.3 * b->best) r.push_back(&c);
+    std::sort(r.begin(), r.end(), [](const Cand *x, const Cand *y) { return x->best < y->best; });
+    if (r.size() > 3) r.resize(3);
+    return r;
+  };
+  const Cand *win[3] = {pick(0, 0), pick(1, dir), pick(2, dir)};
+  int windir = dir;
+  float wintime = 1e30f;
+  for (int v = 0; v <= 1; v++) {
+    const Cand *cur[3] = {pick(0, 0), pick(1, v), pick(2, v)};
+    if (!cur[1] || !cur[2] || cur[1]->best + cur[2]->best > 1.3 * tbest) continue;
+    choose(v, cur[1], cur[0], cur[2]);
+    float now = chain();
+    for (int which : {2, 0, 1})
+      for (const Cand *c : close(which, v)) {
+        if (c == cur[which]) continue;
+        const Cand *was = cur[which];
+        cur[which] = c;
+        choose(v, cur[1], cur[0], cur[2]);
+        const float t = chain();
+        if (t < 0.99f * now) now = t;
+        else cur[which] = was;
+      }
+    if (now < wintime) {
+      wintime = now;
+      windir = v;
+      std::copy(cur, cur + 3, win);
+    }
+  }
+  choose(windir, win[1], win[0], win[2]);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   check_split_status();
