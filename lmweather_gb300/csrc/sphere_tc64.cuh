@@ -9,8 +9,7 @@
 // below 2^23, so the FP32 accumulators of tcgen05 hold them exactly. The eight orders s = 0..7 are then added as 64-bit
 // integers and rounded once. What is left out, the digits below 2^-57 of a row's largest element and the orders from 8
 // on (2^-55 of the largest product), is below FP64's own rounding of such a sum, and the result depends neither on
-// the order of summation nor on how members are batched. Rows whose largest element is below 2^-900 count as zero; a row
-// with an infinity or NaN gives NaN.
+// the order of summation nor on how members are batched. A row with an infinity or NaN gives NaN.
 //
 // All orders of one table digit j come from one MMA: A holds digit i of its rows in row block i, under seven blocks of
 // zeros, and for table digit j the MMA starts j blocks higher, which puts digit i into row block i + j of the accumulator.
@@ -28,6 +27,7 @@
 // The table digits are streamed by bulk copies, sixteen K columns of all eight digits a stage, and start before the
 // kernel waits for its predecessor.
 #pragma once
+#include "exact_slices.cuh"
 #include "tc_common.cuh"
 
 namespace lmw {
@@ -59,79 +59,10 @@ struct Tc64Dev {
 
 namespace {
 
-constexpr int T64_DIG = 8, T64_THREADS = 256, T64_STAGES = 8;  // T64_STAGES: most chunks in flight
-constexpr int T64_NONE = -100000, T64_NAN = 100000;  // row exponents: no digits; not finite
+constexpr int T64_THREADS = 256, T64_STAGES = 8;  // T64_STAGES: most chunks in flight
 // A operand: core matrices 128 bytes apart along K and 256 between 8-row groups. The digits' stores meet four to a bank;
 // with 16 spare bytes between core matrices they do not, which changed no time (T42 x 16, T170: within 2 %)
 constexpr int T64_LBO = 128, T64_SBO = 256;
-
-// biased exponent of |v| (0 for subnormals and zero)
-__device__ __forceinline__ int t64_exp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
-// row exponent e (every |v| < 2^e) from the largest biased exponent
-__host__ __device__ __forceinline__ int t64_row(int ex) { return ex == 2047 ? T64_NAN : ex < 123 ? T64_NONE : ex - 1022; }
-// v 2^(56 - e) rounded to an integer, by integer operations (|v| < 2^e)
-__device__ __forceinline__ long long t64_fixed(double v, int e) {
-  const long long bits = __double_as_longlong(v);
-  const int ex = static_cast<int>((bits >> 52) & 0x7ff), s = 1022 + e - ex;  // right shift of the significand times 8
-  if (ex == 0 || s > 58 || e == T64_NONE || e == T64_NAN) return 0;
-  const long long m8 = ((bits & 0xfffffffffffffll) | 0x10000000000000ll) << 3;
-  const long long x = s > 0 ? (m8 + (1ll << (s - 1))) >> s : m8;
-  return bits < 0 ? -x : x;
-}
-// the eight digits of x, most significant first, as BF16 bits
-__device__ __forceinline__ void t64_digits(long long x, unsigned short *out) {
-  // digit = ((y + 64) mod 128) - 64, y = (y + 64) / 128: the low four from 28 bits, the others from what they leave
-  int y = static_cast<int>(x) & 0xfffffff;
-#pragma unroll
-  for (int i = T64_DIG - 1; i >= 1; i--) {
-    const int u = y + 64;
-    y = u >> 7;
-    if (i == 4) y += static_cast<int>(x >> 28);  // the carry of the low digits, and the high 29 bits
-    out[i] = static_cast<unsigned short>(__float_as_uint(__int_as_float(0x4B400000 | (u & 127)) - 12582976.0f) >> 16);
-  }
-  out[0] = static_cast<unsigned short>(__float_as_uint(__int_as_float(0x4B400000 + y) - 12582912.0f) >> 16);
-}
-// sum of the eight orders D[s] (exact integers) times 2^(7 (7 - s)), as high and low parts of value hi 2^28 + lo
-struct T64Sum {
-  long long hi, lo;
-};
-__device__ __forceinline__ T64Sum t64_sum(const int *D, int stride) {
-  T64Sum r;
-  r.hi = ((static_cast<long long>(D[0]) << 21) + (static_cast<long long>(D[stride]) << 14)) + ((static_cast<long long>(D[2 * stride]) << 7) + D[3 * stride]);
-  r.lo = ((static_cast<long long>(D[4 * stride]) << 21) + (static_cast<long long>(D[5 * stride]) << 14)) + ((static_cast<long long>(D[6 * stride]) << 7) + D[7 * stride]);
-  return r;
-}
-// (hi 2^28 + lo) 2^e rounded to nearest even, by integer operations (the FP64 pipe would take three times as long); |hi|,
-// |lo| < 2^47. e = ea + eb - 63 for the exponents ea of an operand row and eb of a table row
-__device__ __forceinline__ double t64_value(long long hi, long long lo, int ea, int eb) {
-  if (ea == T64_NAN) return __longlong_as_double(0x7ff8000000000000ll);
-  unsigned long long L = static_cast<unsigned long long>(hi) << 28;
-  long long H = hi >> 36;
-  L += static_cast<unsigned long long>(lo);
-  H += (lo >> 63) + (L < static_cast<unsigned long long>(lo) ? 1 : 0);
-  const unsigned long long sign = static_cast<unsigned long long>(H) & 0x8000000000000000ull;
-  if (sign) {
-    L = 0 - L;
-    H = ~H + (L == 0 ? 1 : 0);
-  }
-  if ((static_cast<unsigned long long>(H) | L) == 0 || ea == T64_NONE || eb == T64_NONE) return 0.0;
-  const int p = H ? 127 - __clzll(H) : 63 - __clzll(static_cast<long long>(L));  // the leading bit
-  unsigned long long m;
-  if (p <= 52) {
-    m = L << (52 - p);
-  } else {
-    const int sh = p - 52;  // at most 24: |hi 2^28 + lo| < 2^76
-    m = (static_cast<unsigned long long>(H) << (64 - sh)) | (L >> sh);
-    const unsigned long long rem = L & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-    m += rem > half || (rem == half && (m & 1)) ? 1 : 0;
-  }
-  const int x = p + 1023 + ea + eb - 63;  // biased exponent
-  if (x >= 1 && x <= 2045) return __longlong_as_double(static_cast<long long>(sign | ((static_cast<unsigned long long>(x - 1) << 52) + m)));
-  // the ends of the range: scale in two steps
-  const double v = __longlong_as_double(static_cast<long long>(sign | ((static_cast<unsigned long long>(p + 1022) << 52) + m)));
-  const int e = ea + eb - 63, e1 = e / 2;
-  return v * __hiloint2double((e1 + 1023) << 20, 0) * __hiloint2double((e - e1 + 1023) << 20, 0);
-}
 
 __device__ __forceinline__ uint64_t t64_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   return static_cast<uint64_t>((saddr >> 4) & 0x3FFFu) | (static_cast<uint64_t>(lbo >> 4) << 16) | (static_cast<uint64_t>(sbo >> 4) << 32) |
