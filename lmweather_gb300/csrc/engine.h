@@ -248,8 +248,8 @@ class SphereEngine {
   void upload_filter(double dt);
   void launch_stage(int stage, double dt);
   void launch_chunk(double dt, int steps);
-  void synth_grids(int member_first, int count);  // state x0 -> Fourier coefficients of U, V, zeta, phi
-  void reduce_guard(Reduce &r, int member);
+  void synth_grids(int member_first, int count, bool limit);  // state x0 -> Fourier coefficients of U, V, zeta, phi
+  void reduce_guard(Reduce &r, int member, bool limit);  // limit: for the stability limit
   void reduce_guard_all(bool exact = true);
   double limit_from(const Reduce &r, int b, double safety) const;
   void analyze_grids_to_state(int member);

@@ -1137,7 +1137,6 @@ static void allow_max_shared_memory() {
   LMW_CUDA(cudaFuncSetAttribute(split_syn_ws<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(split_syn_ws<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_syn<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-  LMW_CUDA(cudaFuncSetAttribute(tc64_syn<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_ana<5, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_ana<5, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
   LMW_CUDA(cudaFuncSetAttribute(tc64_syn<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
@@ -1382,11 +1381,15 @@ void SphereEngine::set_orography(const double *hs, size_t n, int member) {
   upload_member_flags(member);
 }
 
-void SphereEngine::synth_grids(int member_first, int count) {
+// Grids that are handed out, diagnosed or kept as a reference come from plain FP64 sums, which keep the relative accuracy of
+// each wavenumber at each latitude (the sliced sums keep it to the largest coefficient and table value of the row: a T170
+// flow of m = 80 alone had no digit right at the poles). T170, one member: 82 us against 18. The stability limit (`limit`,
+// which needs the maxima alone) takes the synthesis of the stages
+void SphereEngine::synth_grids(int member_first, int count, bool limit) {
   SphDev d = make_sph(*this, *tab);
   const size_t st = static_cast<size_t>(member_first) * 3 * ntri;
   const size_t fo = static_cast<size_t>(member_first) * nlat * 4 * M;
-  if (tc64) {
+  if (limit && tc64) {
     syn64_launch(d, tc64_dev(*tc64, ntri + M), tc64->smem_syn(tc64->nbt), count, reinterpret_cast<const double2 *>(x0.p) + st, reinterpret_cast<double2 *>(four.p) + fo, stream);
     g_launches += 1;
     return;
@@ -1403,7 +1406,7 @@ void SphereEngine::synth_grids(int member_first, int count) {
 void SphereEngine::mark_reference(int member) {
   check_member(*this, member);
   SphDev d = make_sph(*this, *tab);
-  synth_grids(member, 1);
+  synth_grids(member, 1, false);
   const size_t smem = static_cast<size_t>(nlon) * sizeof(double2);
   sph_phi_grid<<<dim3(nh, 1), GRID_THREADS, smem, stream>>>(d, reinterpret_cast<const double2 *>(four.p) + static_cast<size_t>(member) * nlat * 4 * M,
                                                         refgrid.p + static_cast<size_t>(member) * ngrid());
@@ -1870,16 +1873,10 @@ void SphereEngine::ensure_tracer() {
   graphs_clear();
 }
 
-// Fourier coefficients of q and delta of `count` members
+// Fourier coefficients of q and delta of `count` members: plain sums, for the tracer's grids (as synth_grids) and the stages
+// above T170
 void SphereEngine::trc_syn_launch(const double2 *x, const double2 *q, double2 *dst, int count) {
-  const SphDev d = make_sph(*this, *tab);
-  if (tc64) {
-    const Tc64Dev z = tc64_dev(*tc64, ntri + M);
-    stage_launch(tc64_syn<2>, dim3(z.nsl * ((count + z.nbt - 1) / z.nbt), M), T64_THREADS, tc64->smem_syn(z.nbt), stream, 1, d, z, x, q,
-                 static_cast<double2 *>(nullptr), dst, count);
-  } else {
-    stage_launch(trc_synth, dim3((nh + 31) / 32, M, count), SYN_THREADS, 0, stream, 1, d, tab64(*tab), x, q, dst);
-  }
+  stage_launch(trc_synth, dim3((nh + 31) / 32, M, count), SYN_THREADS, 0, stream, 1, make_sph(*this, *tab), tab64(*tab), x, q, dst);
 }
 
 // part 0: q and delta synthesis, 1: grid products, 2: analysis and RK4 update of q
@@ -2437,9 +2434,9 @@ void SphereEngine::step(double dt) {
   check_split_status();
 }
 
-void SphereEngine::reduce_guard(Reduce &r, int member) {
+void SphereEngine::reduce_guard(Reduce &r, int member, bool limit) {
   SphDev d = make_sph(*this, *tab);
-  synth_grids(member, 1);
+  synth_grids(member, 1, limit);
   const size_t smem = 4 * static_cast<size_t>(nlon) * sizeof(double2);
   const size_t go = static_cast<size_t>(member) * ngrid();
   sph_diag<<<dim3(nh, 1), GRID_THREADS, smem, stream>>>(d, reinterpret_cast<const double2 *>(four.p) + static_cast<size_t>(member) * nlat * 4 * M,
@@ -2467,7 +2464,7 @@ void SphereEngine::reduce_guard_all(bool exact) {
         d, tab32(*tab), reinterpret_cast<const float2 *>(four32.p), diagrows.p);
     g_launches += 2;
   } else {
-    synth_grids(0, B);
+    synth_grids(0, B, true);
     const size_t smem = 4 * static_cast<size_t>(nlon) * sizeof(double2);
     sph_diag<<<dim3(nh, B), GRID_THREADS, smem, stream>>>(d, reinterpret_cast<const double2 *>(four.p), fgrid.p, hsgrid.p, refgrid.p, diagrows.p,
                                                           nullptr);
@@ -2502,7 +2499,7 @@ double SphereEngine::stable_dt_all(double safety) {
 // cpp/sphere.cpp:438-447
 double SphereEngine::stable_dt(double safety, int member) {
   Reduce r;
-  reduce_guard(r, member);
+  reduce_guard(r, member, true);
   double hmax = std::max(0.0, r.max[1]), wmax = r.max[0];
   if (!(hmax > 0)) throw RuntimeError("the height field must be positive to step the model");
   double omega = (N / p.radius) * (std::sqrt(p.gravity * hmax) + wmax) + 2 * omega_m[member];
@@ -2580,7 +2577,7 @@ void SphereEngine::run(double seconds, double dt) {
 void SphereEngine::diagnostics(double *out, int member) {
   check_member(*this, member);
   Reduce r;
-  reduce_guard(r, member);
+  reduce_guard(r, member, false);
   const size_t pk = static_cast<size_t>(ntri) * 2;
   double phi00[2];
   LMW_CUDA(cudaMemcpy(phi00, x0.p + static_cast<size_t>(member) * 3 * pk + 2 * pk, sizeof(phi00), cudaMemcpyDeviceToHost));
@@ -2598,7 +2595,7 @@ void SphereEngine::grid(int which, double *out, int member) {
   check_member(*this, member);
   if (which < 0 || which > 3) throw InvalidArgument("grid field must be 0 (height), 1 (u), 2 (v) or 3 (vorticity)");
   SphDev d = make_sph(*this, *tab);
-  synth_grids(member, 1);
+  synth_grids(member, 1, false);
   const size_t smem = 4 * static_cast<size_t>(nlon) * sizeof(double2);
   const size_t go = static_cast<size_t>(member) * ngrid();
   sph_diag<<<dim3(nh, 1), GRID_THREADS, smem, stream>>>(d, reinterpret_cast<const double2 *>(four.p) + static_cast<size_t>(member) * nlat * 4 * M,

@@ -207,16 +207,16 @@ __device__ __forceinline__ void t64_unload(uint32_t taddr, int w, int *dst, bool
 }
 
 // ------------------------------------------------------------------------------------------------ synthesis
-// grid: (slices x tiles, M). F = 4: U, V, zeta, Phi of x [B][3][ntri] into four [B][nlat][4][M], nbt members a tile; F = 2: the
-// tracer's q of qin [B][ntri] and delta of x into fourq [B][nlat][2][M]; F = 6: both in one launch, one member a tile, whose
-// second row block is q and delta.
+// grid: (slices x tiles, M). F = 4: U, V, zeta, Phi of x [B][3][ntri] into four [B][nlat][4][M], nbt members a tile; F = 6: with
+// the tracer's q of qin [B][ntri] and delta of x into fourq [B][nlat][2][M], one member a tile, whose second row block is q
+// and delta.
 // T170, one member: 82.0 -> 18.2 us (FP64 pipe before); T42 x 16: 50.4 -> 10.3; T42, one member: 10.3 -> 6.5.
 template <int F>
 __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, const double2 *__restrict__ x, const double2 *__restrict__ qin,
                                                            double2 *__restrict__ four, double2 *__restrict__ fourq, int B) {
   extern __shared__ __align__(1024) uint8_t t64_sm[];
   __shared__ __align__(8) T64Bars bars;
-  constexpr int RF = F == 2 ? 2 : 4;  // complex values of a row block
+  constexpr int RF = 4;  // complex values of a row block
   __shared__ int rowexp[2][RF];
   const int tid = threadIdx.x, m = blockIdx.y, sl = blockIdx.x % z.nsl, tile = blockIdx.x / z.nsl;
   // nbt row blocks: members, or the flow and the tracer of one
@@ -240,13 +240,13 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
   pdl_wait(x, qin);
   // items: a complex value f of row block ml at column k, n = m + 2 k or m + 1 + 2 (k - ke16). Columns are padded to 16, so
   // that a half warp has one (ml, f)
-  const int cols = kc * 16, total = (F == 6 ? 6 : mt * F) * cols, base = d.tri[m] - m;
-  constexpr int IT = ((F == 6 ? 6 : 2 * F) * 192 + T64_THREADS - 1) / T64_THREADS;
+  const int cols = kc * 16, total = (F == 6 ? 6 : 4 * mt) * cols, base = d.tri[m] - m;
+  constexpr int IT = ((F == 6 ? 6 : 8) * 192 + T64_THREADS - 1) / T64_THREADS;
   auto where = [&](int e, int &ml, int &f, int &k) {
     const int v = e / cols;
     k = e - v * cols;
-    ml = F == 6 ? v >> 2 : v / F;
-    f = F == 6 ? v & 3 : v % F;
+    ml = v >> 2;
+    f = v & 3;
   };
   double v[IT][2];
 #pragma unroll
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
     const int b = F == 6 ? tile : tile * nbt + ml;
     const double2 *xz = x + static_cast<size_t>(b) * 3 * d.ntri + base, *xd = xz + d.ntri, *xf = xd + d.ntri;
     const double2 zero = make_double2(0.0, 0.0);
-    const bool flow = F == 4 || (F == 6 && ml == 0);
+    const bool flow = F == 4 || ml == 0;
     const double2 *ce = flow ? (f == 0 ? xd : f == 3 ? xf : xz) : f == 0 ? qin + static_cast<size_t>(b) * d.ntri + base : xd;
     const double2 c = n <= d.N ? ce[n] : zero;
     v[r][0] = c.x;
@@ -324,8 +324,8 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
     if (quarter * 32 < rows)
       t64_unload(tmem + (warp < 4 ? 0 : L) + cb + (static_cast<uint32_t>(quarter * 32) << 16), w, red + ((warp < 4 ? 0 : rows) + row) * ld, row < rows);
     __syncthreads();
-    for (int e = tid; e < (F == 6 ? 6 : mt * F) * w; e += T64_THREADS) {
-      const int i = e % w, v = e / w, f = F == 6 ? v & 3 : v % F, ml = F == 6 ? v >> 2 : v / F, jh = sl * L + cb + i;
+    for (int e = tid; e < (F == 6 ? 6 : 4 * mt) * w; e += T64_THREADS) {
+      const int i = e % w, v = e / w, f = v & 3, ml = v >> 2, jh = sl * L + cb + i;
       if (jh >= d.nh) continue;
       const int ea = t64_row(rowexp[ml][f]), eb = z.eS[m * z.nh16 + jh];
       double so[2], no[2];
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(T64_THREADS, 2) tc64_syn(SphDev d, Tc64Dev z, 
         so[ri] = t64_value(ev.hi + od.hi, ev.lo + od.lo, ea, eb);
         no[ri] = t64_value(ev.hi - od.hi, ev.lo - od.lo, ea, eb);
       }
-      const bool trc = F == 2 || (F == 6 && ml == 1);
+      const bool trc = F == 6 && ml == 1;
       const size_t bo = static_cast<size_t>(F == 6 ? tile : tile * nbt + ml) * d.nlat;
       const int W = trc ? 2 : 4;
       double2 *o = (trc ? fourq : four) + f * d.M + m;
