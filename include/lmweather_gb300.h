@@ -317,6 +317,9 @@ int lmw_ensemble_set_split_form(lmw_ensemble *e, int linear_exact);
  * or guard check fails with LMW_DEVICE_ERROR ("a wait on the tensor cores timed out ..."). Failure-detection
  * hook (the failure is made on the host); no reference counterpart. */
 int lmw_sphere_inject_split_error(lmw_sphere *s, int code);
+/* the same for an FP64 engine up to T170, whose sums run on the tensor cores; its word is cleared when the error is
+ * raised, so that the engine goes on with the next state it is given. */
+int lmw_sphere_inject_fp64_error(lmw_sphere *s, int code);
 int lmw_ensemble_split_plan(lmw_ensemble *e, int group, int *out);
 int lmw_ensemble_kernel_times(lmw_ensemble *e, int group, int reps, double *ms);
 

@@ -42,6 +42,7 @@ _SIGS = {
     "lmw_division_selftest": (_I, [C.POINTER(C.c_uint64), _I, C.POINTER(C.c_double), _I, C.POINTER(C.c_longlong)]),
     "lmw_wait_selftest": (_I, [_I, _IP, _IP]),
     "lmw_sphere_inject_split_error": (_I, [_P, _I]),
+    "lmw_sphere_inject_fp64_error": (_I, [_P, _I]),
     "lmw_sphere_set_split_form": (_I, [_P, _I]),
     "lmw_ensemble_set_split_form": (_I, [_P, _I]),
     "lmw_launch_count": (C.c_uint64, []),

@@ -795,6 +795,12 @@ int lmw_sphere_inject_split_error(lmw_sphere *s, int code) {
     s->e->inject_split_error(code);
   });
 }
+int lmw_sphere_inject_fp64_error(lmw_sphere *s, int code) {
+  return guard([&] {
+    need(s != nullptr && s->e != nullptr, "null sphere handle");
+    s->e->inject_fp64_error(code);
+  });
+}
 int lmw_sphere_set_split_plan(lmw_sphere *s, const int *plan) {
   return guard([&] {
     need(s != nullptr && s->e != nullptr, "null sphere handle");

@@ -202,6 +202,7 @@ class SphereEngine {
   void set_split_form(int linear_exact);
   // writes `code` into the split path's error word, as a tensor-core wait that ran out does (failure tests)
   void inject_split_error(int code);
+  void inject_fp64_error(int code);  // the same for the FP64 sums
 
  private:
   SphereTables *tab = nullptr;

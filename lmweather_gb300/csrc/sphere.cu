@@ -1060,6 +1060,12 @@ void SphereEngine::inject_split_error(int code) {
   LMW_CUDA(cudaMemcpy(split->err.p, &code, sizeof(int), cudaMemcpyHostToDevice));
 }
 
+void SphereEngine::inject_fp64_error(int code) {
+  if (!tc64) throw InvalidArgument("the engine does not use the FP64 sums on the tensor cores");
+  LMW_CUDA(cudaStreamSynchronize(stream));
+  tc64->err.p[0] = code;
+}
+
 int conversion_selftest_run(const uint32_t *f, int nf, const uint64_t *x, int nx, int *mismatches) {
   if (nf < 0 || nx < 0) throw InvalidArgument("counts must not be negative");
   DevBuf<unsigned> fd;
@@ -1323,10 +1329,13 @@ SphereEngine::~SphereEngine() {
 }
 
 // the tensor-core kernels record a nonzero code when a bounded wait ran out. FP64: in pinned host memory, to be read
-// after the stream was waited for
+// after the stream was waited for, and cleared when it is raised: the engine serves the next state that it is given
 void SphereEngine::check_tc64_status() {
-  if (tc64 && *reinterpret_cast<volatile int *>(tc64->err.p) != 0)
-    throw DeviceError("a wait on the tensor cores timed out in the FP64 Legendre transforms");
+  if (!tc64) return;
+  volatile int *e = tc64->err.p;
+  if (*e == 0) return;
+  *e = 0;
+  throw DeviceError("a wait on the tensor cores timed out in the FP64 Legendre transforms");
 }
 void SphereEngine::check_split_status() {
   if (!split) return;
@@ -2052,6 +2061,7 @@ void SphereEngine::kernel_times(double dt, int reps, double *out) {
   cudaEventDestroy(e1);
   g_launches += 3ull * (reps + 1);
   split_packed = false;
+  check_tc64_status();
 }
 
 // Measured choice of the split path's launch plan (each candidate timed after its producer kernel): latitude pairs per grid CTA (8, 4, 2, 1), FFT stages fused per
