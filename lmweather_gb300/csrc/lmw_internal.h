@@ -95,6 +95,14 @@ template <class T> struct HostBuf {
   }
 };
 
+// Host data into device memory in the order of stream `s`, which must be the one whose kernels read it: cudaMemcpy of pageable
+// memory may return before its transfer has reached the device, and a non-blocking stream does not wait for it. The host
+// buffer is free on return.
+inline void copy_in(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+  LMW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
+  LMW_CUDA(cudaStreamSynchronize(s));
+}
+
 // Faults the pages of a host buffer of `bytes` about to be filled by a device copy, if its ends are not resident: the copy
 // engine faults fresh pages one by one (1 GB/s), the kernel a range at once, and several ranges in parallel. The contents
 // are left alone.

@@ -1056,8 +1056,7 @@ int wait_selftest_run(int timeout_us, int *completed, int *ran_out) {
 
 void SphereEngine::inject_split_error(int code) {
   if (!split) throw InvalidArgument("the engine is not in split precision");
-  LMW_CUDA(cudaStreamSynchronize(stream));
-  LMW_CUDA(cudaMemcpy(split->err.p, &code, sizeof(int), cudaMemcpyHostToDevice));
+  copy_in(split->err.p, &code, sizeof(int), stream);
 }
 
 void SphereEngine::inject_fp64_error(int code) {
@@ -1199,7 +1198,7 @@ SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
     }
   auto up = [&](DevBuf<double> &dst, const std::vector<double> &src) {
     dst.alloc(src.size());
-    LMW_CUDA(cudaMemcpy(dst.p, src.data(), src.size() * sizeof(double), cudaMemcpyHostToDevice));
+    copy_in(dst.p, src.data(), src.size() * sizeof(double), stream);
   };
   up(tab->Ps, h.P);
   up(tab->Hs, h.H);
@@ -1229,12 +1228,12 @@ SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
     tw[k] = make_double2(std::cos(ang), std::sin(ang));
   }
   tab->tw.alloc(tw.size());
-  LMW_CUDA(cudaMemcpy(tab->tw.p, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice));
+  copy_in(tab->tw.p, tw.data(), tw.size() * sizeof(double2), stream);
   if (p.precision != kFP64) {
     auto up32 = [&](DevBuf<float> &dst, const std::vector<double> &src) {
       std::vector<float> f(src.begin(), src.end());
       dst.alloc(f.size());
-      LMW_CUDA(cudaMemcpy(dst.p, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
+      copy_in(dst.p, f.data(), f.size() * sizeof(float), stream);
     };
     up32(tab->Ps32, h.P);
     up32(tab->Hs32, h.H);
@@ -1252,7 +1251,7 @@ SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
     for (size_t k = 0; k < tw.size(); k++)
       t32[k] = k < q4 || q4 == 0 ? make_float2(static_cast<float>(tw[k].x), static_cast<float>(tw[k].y)) : make_float2(t32[k - q4].y, -t32[k - q4].x);
     tab->tw32.alloc(t32.size());
-    LMW_CUDA(cudaMemcpy(tab->tw32.p, t32.data(), t32.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    copy_in(tab->tw32.p, t32.data(), t32.size() * sizeof(float2), stream);
   }
   std::vector<int> tm(ntri), tn(ntri);
   for (int m = 0; m <= N; m++)
@@ -1262,7 +1261,7 @@ SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
     }
   auto upi = [&](DevBuf<int> &dst, const std::vector<int> &src) {
     dst.alloc(src.size());
-    LMW_CUDA(cudaMemcpy(dst.p, src.data(), src.size() * sizeof(int), cudaMemcpyHostToDevice));
+    copy_in(dst.p, src.data(), src.size() * sizeof(int), stream);
   };
   upi(tab->trim, tm);
   upi(tab->trin, tn);
@@ -1294,7 +1293,7 @@ SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
   hstage.alloc(std::max<size_t>(4 * ngrid(), static_cast<size_t>(3) * 2 * nspec_ref()));
   if (p.precision == kSplitBF16) {
     split = new SplitPlan();
-    build_split_plan(*split, h, B, p.split_terms);
+    build_split_plan(*split, h, B, p.split_terms, stream);
     {
       int dev = 0;
       LMW_CUDA(cudaGetDevice(&dev));
@@ -1352,9 +1351,8 @@ static void check_member(const SphereEngine &e, int member) {
 // cpp/sphere.cpp:111-118 (with the member's own rotation rate)
 void SphereEngine::upload_member_flags(int member) {
   const double o2 = 2 * omega_m[member];
-  LMW_CUDA(cudaStreamSynchronize(stream));
-  LMW_CUDA(cudaMemcpy(gflag.p + member, &gflag_h[member], sizeof(int), cudaMemcpyHostToDevice));
-  LMW_CUDA(cudaMemcpy(om2.p + member, &o2, sizeof(double), cudaMemcpyHostToDevice));
+  copy_in(gflag.p + member, &gflag_h[member], sizeof(int), stream);
+  copy_in(om2.p + member, &o2, sizeof(double), stream);
 }
 
 void SphereEngine::set_axis_tilt(double alpha, int member) {
@@ -1369,8 +1367,7 @@ void SphereEngine::set_axis_tilt(double alpha, int member) {
       double lam = 2 * kPi * k / nlon, c = std::sqrt(1 - h.mu[j] * h.mu[j]);
       f[static_cast<size_t>(j) * nlon + k] = 2 * omega_m[member] * (-std::cos(lam) * c * std::sin(alpha) + h.mu[j] * std::cos(alpha));
     }
-  LMW_CUDA(cudaStreamSynchronize(stream));
-  LMW_CUDA(cudaMemcpy(fgrid.p + static_cast<size_t>(member) * ngrid(), f.data(), ngrid() * sizeof(double), cudaMemcpyHostToDevice));
+  copy_in(fgrid.p + static_cast<size_t>(member) * ngrid(), f.data(), ngrid() * sizeof(double), stream);
 }
 
 void SphereEngine::set_omega(double omega, int member) {
@@ -1383,8 +1380,7 @@ void SphereEngine::set_omega(double omega, int member) {
 void SphereEngine::set_orography(const double *hs, size_t n, int member) {
   check_member(*this, member);
   if (n != ngrid()) throw InvalidArgument("grid size mismatch");
-  LMW_CUDA(cudaStreamSynchronize(stream));
-  LMW_CUDA(cudaMemcpy(hsgrid.p + static_cast<size_t>(member) * ngrid(), hs, n * sizeof(double), cudaMemcpyHostToDevice));
+  copy_in(hsgrid.p + static_cast<size_t>(member) * ngrid(), hs, n * sizeof(double), stream);
   has_orog[member] = 1;
   gflag_h[member] |= 2;
   upload_member_flags(member);
@@ -1701,8 +1697,7 @@ void SphereEngine::upload_filter(double dt) {
       f[M + n] = std::exp(-p.diffusion * kp * kp * dt);
     }
   }
-  LMW_CUDA(cudaStreamSynchronize(stream));
-  LMW_CUDA(cudaMemcpy(filt.p, f.data(), 2 * M * sizeof(double), cudaMemcpyHostToDevice));
+  copy_in(filt.p, f.data(), 2 * M * sizeof(double), stream);
   filt_dt = dt;
 }
 
@@ -1939,8 +1934,7 @@ void SphereEngine::set_tracer_state(const double *qr, int member) {
   ensure_tracer();
   LMW_CUDA(cudaStreamSynchronize(stream));
   to_packed(qr, hstage.p);
-  LMW_CUDA(cudaMemcpy(tq0.p + static_cast<size_t>(member) * ntri * 2, hstage.p, static_cast<size_t>(ntri) * 2 * sizeof(double),
-                      cudaMemcpyHostToDevice));
+  copy_in(tq0.p + static_cast<size_t>(member) * ntri * 2, hstage.p, static_cast<size_t>(ntri) * 2 * sizeof(double), stream);
   if (!has_tracer) {
     has_tracer = true;
     graphs_clear();

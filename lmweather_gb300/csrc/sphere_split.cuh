@@ -1775,7 +1775,7 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
 }  // namespace
 
 // Pack the tables, size the operand buffers (once per engine).
-inline void build_split_plan(SplitPlan &sp, const HostTables &h, int B, int terms) {
+inline void build_split_plan(SplitPlan &sp, const HostTables &h, int B, int terms, cudaStream_t stream) {
   const int N = h.N, M = h.M, nh = h.nh;
   // the synthesis keeps four accumulators of its latitudes in the 512 tensor-memory columns: slices of at most 128
   if (pad16(nh) > 256) throw InvalidArgument("split precision supports truncations up to 341");
@@ -1855,9 +1855,9 @@ inline void build_split_plan(SplitPlan &sp, const HostTables &h, int B, int term
       }
     }
   }
-  auto up = [](DevBuf<__nv_bfloat16> &dst, const std::vector<uint16_t> &src) {
+  auto up = [&](DevBuf<__nv_bfloat16> &dst, const std::vector<uint16_t> &src) {
     dst.alloc(src.size());
-    LMW_CUDA(cudaMemcpy(dst.p, src.data(), src.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
+    copy_in(dst.p, src.data(), src.size() * sizeof(uint16_t), stream);
   };
   up(sp.tS_P, tSP);
   up(sp.tS_H, tSH);
@@ -1868,18 +1868,18 @@ inline void build_split_plan(SplitPlan &sp, const HostTables &h, int B, int term
   sp.aS_H.alloc(3 * sp.aSH_size);
   sp.aA_P.alloc(3 * sp.aAP_size);
   sp.aA_H.alloc(3 * sp.aAH_size);
-  for (auto *b : {&sp.aS_P, &sp.aS_H, &sp.aA_P, &sp.aA_H}) LMW_CUDA(cudaMemset(b->p, 0, b->bytes()));
+  for (auto *b : {&sp.aS_P, &sp.aS_H, &sp.aA_P, &sp.aA_H}) b->zero(stream);
   sp.dsyn.alloc(static_cast<size_t>(B) * nh * M * SPLIT_NQ);
-  LMW_CUDA(cudaMemset(sp.dsyn.p, 0, sp.dsyn.bytes()));
+  sp.dsyn.zero(stream);
   sp.err.alloc(1);
-  LMW_CUDA(cudaMemset(sp.err.p, 0, sizeof(int)));
-  auto upi = [](DevBuf<int> &dst, const std::vector<int> &src) {
+  sp.err.zero(stream);
+  auto upi = [&](DevBuf<int> &dst, const std::vector<int> &src) {
     dst.alloc(src.size());
-    LMW_CUDA(cudaMemcpy(dst.p, src.data(), src.size() * sizeof(int), cudaMemcpyHostToDevice));
+    copy_in(dst.p, src.data(), src.size() * sizeof(int), stream);
   };
-  auto upl = [](DevBuf<long> &dst, const std::vector<long> &src) {
+  auto upl = [&](DevBuf<long> &dst, const std::vector<long> &src) {
     dst.alloc(src.size());
-    LMW_CUDA(cudaMemcpy(dst.p, src.data(), src.size() * sizeof(long), cudaMemcpyHostToDevice));
+    copy_in(dst.p, src.data(), src.size() * sizeof(long), stream);
   };
   upi(sp.ke16_d, sp.ke16);
   upi(sp.kps_d, sp.kps);
@@ -1944,7 +1944,7 @@ inline void build_split_plan(SplitPlan &sp, const HostTables &h, int B, int term
     }
   std::vector<float> lin32(lin.begin(), lin.end());
   sp.lin32.alloc(lin32.size());
-  LMW_CUDA(cudaMemcpy(sp.lin32.p, lin32.data(), lin32.size() * sizeof(float), cudaMemcpyHostToDevice));
+  copy_in(sp.lin32.p, lin32.data(), lin32.size() * sizeof(float), stream);
 }
 
 // bytes past the end of a warp-specialised kernel's layout (ns stage slots of `slot` bytes, then `tail` bytes of

@@ -571,9 +571,9 @@ inline void build_tc64(Tc64Plan &p, const HostTables &h, const SphDev &d, double
       cf[3 * static_cast<size_t>(ext) + i] = n * eu;
       cf[4 * static_cast<size_t>(ext) + i] = (n + 1) * el;
     }
-  auto up = [](auto &dst, const auto &src) {
+  auto up = [&](auto &dst, const auto &src) {
     dst.alloc(src.size());
-    LMW_CUDA(cudaMemcpy(dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice));
+    copy_in(dst.p, src.data(), src.size() * sizeof(src[0]), stream);
   };
   up(p.ke16, ke16);
   up(p.kc, kc);
