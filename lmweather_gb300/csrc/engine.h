@@ -3,6 +3,7 @@
 #include <limits>
 #include <memory>
 
+#include "graph_slots.h"
 #include "lmw_internal.h"
 
 namespace lmw {
@@ -186,7 +187,6 @@ class SphereEngine {
   DevBuf<int> gflag;   // per member: bit 0 tilted Coriolis grid, bit 1 orography
   DevBuf<double> om2;  // per member: 2 Omega
   uint64_t launches_per_step() const { return launches_step; }
-  double last_step_dt = 0;  // dt of the last step() (zero: none)
   // average duration (ms) per launch of each stage kernel class over `reps` launches (CUDA events on the
   // engine stream): out[0] synthesis, out[1] grid (FFTs + products), out[2] analysis + RK4 update. x0 unchanged.
   void kernel_times(double dt, int reps, double *out);
@@ -238,14 +238,9 @@ class SphereEngine {
   std::vector<char> has_orog;
   double filt_dt = -1;
   uint64_t launches_step = 0;
-  // captured step chunks, keyed by (dt, steps); the guard-sized chunk and a run's remainder chunk both stay
-  struct ChunkGraph {
-    double dt;
-    int steps;
-    cudaGraphExec_t exec;
-  };
-  std::vector<ChunkGraph> graphs;
+  GraphSlots<cudaGraphExec_t> graphs;
   void graphs_clear();
+  cudaGraphExec_t capture(double dt, int steps);
   void upload_filter(double dt);
   void launch_stage(int stage, double dt);
   void launch_chunk(double dt, int steps);

@@ -1317,7 +1317,7 @@ SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
 }
 
 SphereEngine::~SphereEngine() {
-  for (const ChunkGraph &cg : graphs) cudaGraphExecDestroy(cg.exec);
+  graphs_clear();
   if (stream) {
     cudaStreamSynchronize(stream);
     cudaStreamDestroy(stream);
@@ -2391,47 +2391,47 @@ void SphereEngine::enqueue_step(double dt) {
   launches_step = 12;
 }
 
-void SphereEngine::graphs_clear() {
-  for (const ChunkGraph &cg : graphs) cudaGraphExecDestroy(cg.exec);
-  graphs.clear();
+void SphereEngine::graphs_clear() { graphs.clear(cudaGraphExecDestroy); }
+
+cudaGraphExec_t SphereEngine::capture(double dt, int steps) {
+  cudaGraphExec_t exec = nullptr;
+  cudaGraph_t g;
+  uint64_t before = g_launches;
+  LMW_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+  for (int s = 0; s < steps; s++)
+    for (int k = 0; k < 4; k++) launch_stage(k, dt);
+  LMW_CUDA(cudaStreamEndCapture(stream, &g));
+  g_launches = before;
+  LMW_CUDA(cudaGraphInstantiate(&exec, g, 0));
+  cudaGraphDestroy(g);
+  return exec;
 }
 
 void SphereEngine::launch_chunk(double dt, int steps) {
   if (steps <= 0) return;
   upload_filter(dt);
   ensure_packed();
-  cudaGraphExec_t exec = nullptr;
-  for (const ChunkGraph &cg : graphs)
-    if (cg.dt == dt && cg.steps == steps) exec = cg.exec;
+  cudaGraphExec_t exec = graphs.chunk(dt, steps);
   if (!exec) {
-    if (graphs.size() >= 4) {
-      cudaGraphExecDestroy(graphs.front().exec);
-      graphs.erase(graphs.begin());
-    }
-    cudaGraph_t g;
-    uint64_t before = g_launches;
-    LMW_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    for (int s = 0; s < steps; s++)
-      for (int k = 0; k < 4; k++) launch_stage(k, dt);
-    LMW_CUDA(cudaStreamEndCapture(stream, &g));
-    g_launches = before;
-    LMW_CUDA(cudaGraphInstantiate(&exec, g, 0));
-    cudaGraphDestroy(g);
-    graphs.push_back({dt, steps, exec});
+    exec = capture(dt, steps);
+    graphs.keep_chunk(dt, steps, exec, cudaGraphExecDestroy);
   }
   LMW_CUDA(cudaGraphLaunch(exec, stream));
   g_launches += 12ull * steps;
 }
 
 void SphereEngine::step(double dt) {
-  // from the second step of a row with one dt as a graph: one launch instead of twelve
-  if (dt == last_step_dt) {
-    launch_chunk(dt, 1);
+  // as a graph where one dt goes on: one launch instead of twelve
+  if (graphs.step(dt)) {
+    upload_filter(dt);
+    ensure_packed();
+    if (!graphs.step_graph()) graphs.keep_step(capture(dt, 1), cudaGraphExecDestroy);
+    LMW_CUDA(cudaGraphLaunch(graphs.step_graph(), stream));
+    g_launches += 12;
     launches_step = 12;
   } else {
     enqueue_step(dt);
   }
-  last_step_dt = dt;
   for (int b = 0; b < B; b++) t[b] += dt;
   LMW_CUDA(cudaStreamSynchronize(stream));
   check_tc64_status();
