@@ -30,6 +30,7 @@ UNITS = [
     ("tc_gemm.cu", []),
     ("surrogate.cu", []),
     ("sphere_tables.cpp", []),
+    ("prefault.cpp", []),
     ("wx_capi.cpp", []),
 ]
 

@@ -1,12 +1,4 @@
 // The C ABI (include/lmweather_gb300.h): exceptions become status codes, the message is kept per thread.
-#include <algorithm>
-#include <system_error>
-#include <thread>
-#include <vector>
-#ifdef __linux__
-#include <sys/mman.h>
-#include <unistd.h>
-#endif
 #include <cuda_profiler_api.h>
 
 #include <cstdio>
@@ -35,41 +27,6 @@ struct lmw_mlp {
 struct lmw_surrogate {
   lmw::Surrogate *s;
 };
-
-namespace lmw {
-
-void prefault(void *p, size_t bytes) {
-#ifdef __linux__
-  constexpr size_t kLeast = 1 << 20;
-  if (bytes < kLeast) return;
-  const size_t page = static_cast<size_t>(sysconf(_SC_PAGESIZE));
-  const uintptr_t a = reinterpret_cast<uintptr_t>(p) / page * page, e = reinterpret_cast<uintptr_t>(p) + bytes;
-  unsigned char first = 1, last = 1;
-  if (mincore(reinterpret_cast<void *>(a), 1, &first) != 0 || mincore(reinterpret_cast<void *>((e - 1) / page * page), 1, &last) != 0) return;
-  const uintptr_t mid = (a + (e - a) / 2) / page * page;
-  unsigned char half = 1;
-  if (mincore(reinterpret_cast<void *>(mid), 1, &half) != 0 || ((first & last & half) & 1)) return;
-  constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE (Linux 5.14); where it is unknown the copy faults the pages
-  auto fill = [=](uintptr_t from, uintptr_t to) {
-    if (to > from) madvise(reinterpret_cast<void *>(from), to - from, kPopulateWrite);
-  };
-  const int parts = bytes >= 8 * kLeast ? 4 : 1;
-  const uintptr_t len = ((e - a) / parts + page - 1) / page * page;
-  std::vector<std::thread> others;
-  others.reserve(parts);
-  try {
-    for (int k = 1; k < parts; k++) others.emplace_back(fill, std::min(a + k * len, e), std::min(a + (k + 1) * len, e));
-  } catch (const std::system_error &) {  // no thread to be had: the copy faults what is left
-  }
-  fill(a, std::min(a + len, e));
-  for (auto &t : others) t.join();
-#else
-  (void)p;
-  (void)bytes;
-#endif
-}
-
-}  // namespace lmw
 
 namespace lmw {
 thread_local uint64_t g_launches = 0;

@@ -10,6 +10,8 @@
 #include <string>
 #include <vector>
 
+#include "prefault.h"
+
 namespace lmw {
 
 // The reference's two exception kinds (std::invalid_argument / std::runtime_error) plus device failures.
@@ -102,11 +104,6 @@ inline void copy_in(void *dst, const void *src, size_t bytes, cudaStream_t s) {
   LMW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
   LMW_CUDA(cudaStreamSynchronize(s));
 }
-
-// Faults the pages of a host buffer of `bytes` about to be filled by a device copy, if its ends are not resident: the copy
-// engine faults fresh pages one by one (1 GB/s), the kernel a range at once, and several ranges in parallel. The contents
-// are left alone.
-void prefault(void *p, size_t bytes);
 
 // Counts this library's kernel launches (for the benchmark's launch accounting).
 extern thread_local uint64_t g_launches;
