@@ -43,6 +43,12 @@ template <int K> __device__ __forceinline__ double div_by(const PlaneDev &p, dou
   return div_general(x, K == 0 ? p.dxx : K == 1 ? p.dyy : K == 2 ? p.dxx2 : p.dyy2, p.zh[K], p.zl[K], p.fastdiv);
 }
 
+// r - drag U. With no drag that is r, but for a U that is not finite (NaN) and the sign of a zero
+__device__ __forceinline__ double drag_term(const PlaneDev &p, double r, double U) {
+  const bool special = (__double2hiint(U) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(r) == static_cast<int>(0x80000000u) && __double2loint(r) == 0);
+  return p.hasdrag || special ? r - p.drag * U : r;
+}
+
 __device__ __forceinline__ int wrapx(int i, int nx) { return ((i % nx) + nx) % nx; }
 
 // stage 0..3 with coefficients c = 0.5 dt, 0.5 dt, dt, dt/6 (cpp/plane.cpp:143-158)
@@ -55,7 +61,7 @@ __device__ __forceinline__ int wrapx(int i, int nx) { return ((i % nx) + nx) % n
 //     (below 2^-1022) could the reference's extra rounding show;
 //   - squares, fluxes and B are formed once per point in shared memory, not once per neighbour;
 //   - divisions by the spacings take two operations (div_fixed2) where that is proven, not three;
-//   - drag U is left out for drag = 0.
+//   - drag U is left out for drag = 0 (drag_term).
 // That is 54 FP64 operations per cell and stage instead of 86 (nonlinear, inviscid).
 // A tile is TX x ty_n cells: the CTAs are dealt to the tile columns as evenly as they go, and a column's CTAs cut its
 // rows evenly. A tile's 3 TX ty_n updates (u, v, h: one role per warp) are dealt to the NT threads, so a tile of one row
@@ -168,7 +174,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int sta
       const double U = su[ty + 1][tx + 1];
       const double s2 = sv[ty + 1][tx] + sv[ty + 1][tx + 1] + sv[ty + 2][tx] + sv[ty + 2][tx + 1];
       r = __fma_rn(0.125, (sE[ty][tx] + sE[ty + 1][tx]) * s2, -div_by<0>(p, sB[ty + 1][tx + 1] - sB[ty + 1][tx]));
-      if (p.hasdrag) r = r - p.drag * U;
+      r = drag_term(p, r, U);
       if (p.hasvisc) {
         const double uy1 = j + 1 < ny ? su[ty + 2][tx + 1] : U, uy0 = j > 0 ? su[ty][tx + 1] : U;
         r += p.visc * (div_by<2>(p, __fma_rn(-2.0, U, su[ty + 1][tx + 2]) + su[ty + 1][tx]) + div_by<3>(p, __fma_rn(-2.0, U, uy1) + uy0));
@@ -180,7 +186,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int sta
         const double V = sv[ty + 1][tx + 1];
         const double s2 = su[ty][tx + 1] + su[ty][tx + 2] + su[ty + 1][tx + 1] + su[ty + 1][tx + 2];
         r = __fma_rn(-0.125, (sE[ty][tx] + sE[ty][tx + 1]) * s2, -div_by<1>(p, sB[ty + 1][tx + 1] - sB[ty][tx + 1]));
-        if (p.hasdrag) r = r - p.drag * V;
+        r = drag_term(p, r, V);
         if (p.hasvisc) {
           const double vy1 = j + 1 < ny ? sv[ty + 2][tx + 1] : 0.0, vy0 = j - 1 > 0 ? sv[ty][tx + 1] : 0.0;
           r += p.visc * (div_by<2>(p, __fma_rn(-2.0, V, sv[ty + 1][tx + 2]) + sv[ty + 1][tx]) + div_by<3>(p, __fma_rn(-2.0, V, vy1) + vy0));
