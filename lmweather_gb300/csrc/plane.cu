@@ -43,9 +43,31 @@ template <int K> __device__ __forceinline__ double div_by(const PlaneDev &p, dou
   return div_general(x, K == 0 ? p.dxx : K == 1 ? p.dyy : K == 2 ? p.dxx2 : p.dyy2, p.zh[K], p.zl[K], p.fastdiv);
 }
 
+// 2^-E <= |x| < 2^E, by integer operations
+__device__ __forceinline__ unsigned magnitude(double x) { return static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu; }
+template <int E> __device__ __forceinline__ bool within(double x) {
+  return magnitude(x) - (static_cast<unsigned>(1023 - E) << 20) < static_cast<unsigned>(2 * E) << 20;
+}
+__device__ __forceinline__ bool is_zero(double x) { return (magnitude(x) | static_cast<unsigned>(__double2loint(x))) == 0u; }
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
+// What plane_stage leaves to the reference's own operations (see there): q vbar from the sums of two eta and four v, B from g h
+// and the sums of squares, and dh at cell (tx, ty) of a tile from its points
+__device__ __noinline__ double edge_product(double e2, double s2) { return 0.5 * e2 * (0.25 * s2); }
+__device__ __noinline__ double edge_bernoulli(double b, double qx, double qy) { return b + 0.5 * (0.5 * qx + 0.5 * qy); }
+__device__ __noinline__ double edge_dh(const PlaneDev &p, const double (*sh)[TX + 2], const double (*su)[TX + 2], const double (*sv)[TX + 2], int tx,
+                                       int ty, int j) {
+  const double hc = sh[ty + 1][tx + 1];
+  const double hw = p.lin ? p.depth : 0.5 * (sh[ty + 1][tx] + hc), he = p.lin ? p.depth : 0.5 * (hc + sh[ty + 1][tx + 2]);
+  const double fe = he * su[ty + 1][tx + 2], fw = hw * su[ty + 1][tx + 1];
+  double fn = 0, fs = 0;
+  if (j + 1 < p.ny) fn = (p.lin ? p.depth : 0.5 * (hc + sh[ty + 2][tx + 1])) * sv[ty + 2][tx + 1];
+  if (j > 0) fs = (p.lin ? p.depth : 0.5 * (sh[ty][tx + 1] + hc)) * sv[ty + 1][tx + 1];
+  return -(div_general(fe - fw, p.dxx, p.zh[0], p.zl[0], p.fastdiv) + div_general(fn - fs, p.dyy, p.zh[1], p.zl[1], p.fastdiv));
+}
+
 // r - drag U. With no drag that is r, but for a U that is not finite (NaN) and the sign of a zero
 __device__ __forceinline__ double drag_term(const PlaneDev &p, double r, double U) {
-  const bool special = (__double2hiint(U) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(r) == static_cast<int>(0x80000000u) && __double2loint(r) == 0);
+  const bool special = not_finite(U) || (__double2hiint(r) == static_cast<int>(0x80000000u) && __double2loint(r) == 0);
   return p.hasdrag || special ? r - p.drag * U : r;
 }
 
@@ -57,8 +79,12 @@ __device__ __forceinline__ int wrapx(int i, int nx) { return ((i % nx) + nx) % n
 // number of FP64 instructions. The reference's values are kept bit for bit with fewer of them:
 //   - its factors 0.5, 0.25 and 2 are exact, so they are folded into the neighbouring operation (q vbar = 0.125 RN(s1 s2)
 //     inside the FMA that subtracts the pressure term; the Bernoulli function's 0.25; the flux's 0.5 in the continuity
-//     equation's step, whose accumulator holds k / -0.5; acc + 2 k as an FMA). Only where a product is subnormal
-//     (below 2^-1022) could the reference's extra rounding show;
+//     equation's step, whose accumulator holds k / -0.5; acc + 2 k as an FMA). Where such a product could be subnormal or
+//     overflow, and round differently, the reference's own operations are called (edge_*), by tests on the integer pipe:
+//     for a sum of squares outside 2^-900 .. 2^900; for a sum of four v outside 2^-330 .. 2^330 or its product with eta's
+//     outside 2^-660 .. 2^660, zero apart (then neither factor is subnormal); and for a dh that is not finite or belongs to
+//     an h below 2^-600 (the error of a subnormal flux, 2^-1074 / 2^-50 at most, is lost in any other h). The tests cost
+//     60 x 30 two per cent (3.53 -> 3.62 us a stage of a run), 200 x 100 and 1024 x 512 nothing;
 //   - squares, fluxes and B are formed once per point in shared memory, not once per neighbour;
 //   - divisions by the spacings take two operations (div_fixed2) where that is proven, not three;
 //   - drag U is left out for drag = 0 (drag_term).
@@ -74,7 +100,7 @@ __device__ __forceinline__ int wrapx(int i, int nx) { return ((i % nx) + nx) % n
 // Stage time before and now (us): 60 x 30 12.4 -> 3.8, 200 x 100 14.3 -> 5.3, 1024 x 512 118.9 -> 68.3 (its 54
 // operations a cell take 53 at 0.53e12 a second), 4000 x 2000 1678 -> 953.
 template <int TYMAX, int NT, bool EARLY>
-__global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int stage, double c, const double *coef, const double *hi,
+__global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(const __grid_constant__ PlaneDev p, int stage, double c, const double *coef, const double *hi,
                                                              const double *ui, const double *vi, double *h0, double *u0, double *v0, double *ah,
                                                              double *au, double *av, double *ho, double *uo, double *vo) {
   constexpr int TY = TYMAX;
@@ -140,7 +166,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int sta
     double b = 0;
     if (jb >= 0) {
       b = p.g * sh[ly][lx];
-      if (!p.lin) b = __fma_rn(0.25, (qu[ly][lx] + qu[ly][lx + 1]) + (qv[ly][lx] + qv[ly + 1][lx]), b);
+      if (!p.lin) {
+        const double qx = qu[ly][lx] + qu[ly][lx + 1], qy = qv[ly][lx] + qv[ly + 1][lx], q = qx + qy;
+        if (within<900>(q)) b = __fma_rn(0.25, q, b);
+        else b = edge_bernoulli(b, qx, qy);
+      }
     }
     sB[ly][lx] = b;
     double zeta = 0;
@@ -173,7 +203,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int sta
       // du at the u point (i, j): cpp/plane.cpp:94-105
       const double U = su[ty + 1][tx + 1];
       const double s2 = sv[ty + 1][tx] + sv[ty + 1][tx + 1] + sv[ty + 2][tx] + sv[ty + 2][tx + 1];
-      r = __fma_rn(0.125, (sE[ty][tx] + sE[ty + 1][tx]) * s2, -div_by<0>(p, sB[ty + 1][tx + 1] - sB[ty + 1][tx]));
+      const double e2 = sE[ty][tx] + sE[ty + 1][tx], es = e2 * s2, pr = div_by<0>(p, sB[ty + 1][tx + 1] - sB[ty + 1][tx]);
+      if (is_zero(es) || (within<330>(s2) && within<660>(es))) r = __fma_rn(0.125, es, -pr);
+      else r = edge_product(e2, s2) - pr;
       r = drag_term(p, r, U);
       if (p.hasvisc) {
         const double uy1 = j + 1 < ny ? su[ty + 2][tx + 1] : U, uy0 = j > 0 ? su[ty][tx + 1] : U;
@@ -185,7 +217,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int sta
       if (j >= 1) {
         const double V = sv[ty + 1][tx + 1];
         const double s2 = su[ty][tx + 1] + su[ty][tx + 2] + su[ty + 1][tx + 1] + su[ty + 1][tx + 2];
-        r = __fma_rn(-0.125, (sE[ty][tx] + sE[ty][tx + 1]) * s2, -div_by<1>(p, sB[ty + 1][tx + 1] - sB[ty][tx + 1]));
+        const double e2 = sE[ty][tx] + sE[ty][tx + 1], es = e2 * s2, pr = div_by<1>(p, sB[ty + 1][tx + 1] - sB[ty][tx + 1]);
+        if (is_zero(es) || (within<330>(s2) && within<660>(es))) r = __fma_rn(-0.125, es, -pr);
+        else r = edge_product(-e2, s2) - pr;
         r = drag_term(p, r, V);
         if (p.hasvisc) {
           const double vy1 = j + 1 < ny ? sv[ty + 2][tx + 1] : 0.0, vy0 = j - 1 > 0 ? sv[ty][tx + 1] : 0.0;
@@ -194,6 +228,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) plane_stage(PlaneDev p, int sta
       }
     } else {
       r = div_by<0>(p, sF[ty][tx + 1] - sF[ty][tx]) + div_by<1>(p, sG[ty + 1][tx] - sG[ty][tx]);
+      if (!p.lin && (not_finite(r) || magnitude(xv[k]) < (423u << 20) || p.fastdiv != 2)) r = -2.0 * edge_dh(p, sh, su, sv, tx, ty, j);
     }
     // RK4 bookkeeping: cpp/plane.cpp:146-156 (acc = k1 + 2 k2 + 2 k3, state += dt/6 (acc + k4)); for h, r = k / -0.5
     // (linear: -k), which its accumulator keeps and its coefficient takes up
