@@ -516,13 +516,20 @@ constexpr size_t kNoAllocMaxCells = 262144;
 constexpr size_t kNoAllocFieldCap = kNoAllocMaxCells + 4096;
 static __device__ __align__(256) double g_noalloc_scratch[9 * kNoAllocFieldCap];
 
-// div_fixed against the IEEE division on every pair (x[i], y[k]): counts[0] = results that differ in any bit,
-// counts[1] = pairs the fast path answered (the rest took the IEEE division)
+// div_fixed and the stencil's division against the IEEE division on every pair (x[i], y[k]): counts[0] = results that differ in any bit,
+// counts[1] = pairs div_fixed's fast path answered (the rest took the IEEE division)
 __global__ void division_selftest(const unsigned long long *__restrict__ xb, int nx, const double *__restrict__ y,
-                                  const double *__restrict__ zh, const double *__restrict__ zl, int ny,
+                                  const double *__restrict__ zh, const double *__restrict__ zl, const FixedDiv2 *__restrict__ fd, int ny,
                                   unsigned long long *counts) {
   const long long total = static_cast<long long>(nx) * ny;
   unsigned long long bad = 0, fastn = 0;
+  // the stencil's division: two operations where they are proven, else div_general (zh = 0: not proven for this divisor)
+  auto differs = [&](double x, int k) {
+    int ok = 0;
+    double q = fd[k].zh != 0 ? div_fixed2(x, fd[k], ok) : 0.0;
+    if (!ok) q = div_general(x, y[k], zh[k], zl[k], 1);
+    return __double_as_longlong(q) != __double_as_longlong(x / y[k]);
+  };
   for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<long long>(gridDim.x) * blockDim.x) {
     const double x = __longlong_as_double(static_cast<long long>(xb[e % nx]));
@@ -530,9 +537,15 @@ __global__ void division_selftest(const unsigned long long *__restrict__ xb, int
     int fast = 0;
     const double a = div_fixed(x, y[k], zh[k], zl[k], fast);
     const double b = x / y[k];
-    bad += __double_as_longlong(a) != __double_as_longlong(b) ? 1 : 0;
+    bad += __double_as_longlong(a) != __double_as_longlong(b) || differs(x, k) ? 1 : 0;
     fastn += fast;
   }
+  // each divisor's own exceptional dividend
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ny; k += gridDim.x * blockDim.x)
+    for (int e = 1023 - 3; fd[k].zh != 0 && fd[k].bad_hi < 1u << 20 && e < 1023 + 4; e++) {
+      const double x = __hiloint2double(static_cast<int>(static_cast<unsigned>(e) << 20 | fd[k].bad_hi), static_cast<int>(fd[k].bad_lo));
+      bad += differs(x, k) || differs(-x, k) ? 1 : 0;
+    }
   if (bad) atomicAdd(&counts[0], bad);
   if (fastn) atomicAdd(&counts[1], fastn);
 }
@@ -547,8 +560,13 @@ void division_selftest_run(const uint64_t *x, int nx, const double *y, int ny, l
   for (int k = 0; k < ny; k++)
     if (!fixed_div_reciprocal(y[k], zh[k], zl[k]))
       throw InvalidArgument("divisor " + std::to_string(k) + " or its reciprocal is not a normal number");
+  std::vector<FixedDiv2> fd(std::max(ny, 1));
+  for (int k = 0; k < ny; k++)
+    if (!fixed_div2_setup(y[k], fd[k])) fd[k].zh = 0;
   DevBuf<unsigned long long> xd, cd;
   DevBuf<double> yd, hd, ld;
+  DevBuf<FixedDiv2> fdd;
+  fdd.alloc(fd.size());
   xd.alloc(std::max(nx, 1));
   yd.alloc(std::max(ny, 1));
   hd.alloc(std::max(ny, 1));
@@ -559,10 +577,11 @@ void division_selftest_run(const uint64_t *x, int nx, const double *y, int ny, l
     LMW_CUDA(cudaMemcpy(yd.p, y, ny * sizeof(double), cudaMemcpyHostToDevice));
     LMW_CUDA(cudaMemcpy(hd.p, zh.data(), ny * sizeof(double), cudaMemcpyHostToDevice));
     LMW_CUDA(cudaMemcpy(ld.p, zl.data(), ny * sizeof(double), cudaMemcpyHostToDevice));
+    LMW_CUDA(cudaMemcpy(fdd.p, fd.data(), ny * sizeof(FixedDiv2), cudaMemcpyHostToDevice));
   }
   LMW_CUDA(cudaMemset(cd.p, 0, 2 * sizeof(unsigned long long)));
   if (nx > 0 && ny > 0) {
-    division_selftest<<<1024, 256>>>(xd.p, nx, yd.p, hd.p, ld.p, ny, cd.p);
+    division_selftest<<<1024, 256>>>(xd.p, nx, yd.p, hd.p, ld.p, fdd.p, ny, cd.p);
     LMW_LAUNCH_CHECK();
     g_launches += 1;
   }
