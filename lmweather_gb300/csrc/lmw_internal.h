@@ -46,6 +46,10 @@ inline std::atomic<uint64_t> &alloc_counter() {
   return n;
 }
 
+// GB300: multiprocessors, and the shared memory of one in bytes
+constexpr int kSMs = 152;
+constexpr size_t kSmemPerSM = 233472;
+
 // Device buffer owned by an engine object.
 template <class T> struct DevBuf {
   T *p = nullptr;

@@ -33,8 +33,8 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // of one member, FP64: T85 44.4 -> 35.3 us, T170 105 -> 99; split form, T170: 49 -> 40). Past five
 // CTAs per SM the share no longer pays (T31 x 3 with tracer, 768 CTAs in clusters of eight: 3.64 ms a run held to six, 3.54 free).
 inline size_t even_share(size_t need, long ctas) {
-  const long share = (ctas + 151) / 152;
-  return share > 5 ? need : std::max(need, static_cast<size_t>(233472 / (share + 1) - 768));
+  const long share = (ctas + kSMs - 1) / kSMs;
+  return share > 5 ? need : std::max(need, kSmemPerSM / (share + 1) - 768);
 }
 
 // launch of a kernel that calls pdl_wait, in clusters of `cluster` CTAs along x

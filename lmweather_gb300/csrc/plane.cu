@@ -258,23 +258,23 @@ __global__ void plane_coef(double *c, double half, double full, double sixth) {
 // the least to do, counting the FP64 instructions per warp of a tile: 2 for each loaded point, 17 for each corner, 33
 // for each cell (sixteen rows lose 4 % to the halo, eight 7 %). Measured, us a stage: 200 x 100 in form 1 5.2, 2 7.0,
 // 3 8.5; 400 x 200 (too tall for form 1) in 2 13.8, 3 15.1.
-constexpr int PLANE_SMS = 152, PLANE_TY = 16;
+constexpr int PLANE_TY = 16;
 struct Tiling {
   int form, ctas, ty;  // ty: rows of the tallest tile
 };
 Tiling plane_tiling(int nx, int ny) {
   const int tx = (nx + TX - 1) / TX;
-  if (tx * ny <= PLANE_SMS) return {0, tx * ny, 1};
+  if (tx * ny <= kSMs) return {0, tx * ny, 1};
   for (int per_sm = 1; per_sm <= 2; per_sm++) {
-    const int least = per_sm * PLANE_SMS / tx;  // CTAs of the column with the fewest
-    if (least > 0 && (ny + least - 1) / least <= PLANE_TY && (per_sm * PLANE_SMS + tx - 1) / tx <= ny)
-      return {per_sm, per_sm * PLANE_SMS, (ny + least - 1) / least};
+    const int least = per_sm * kSMs / tx;  // CTAs of the column with the fewest
+    if (least > 0 && (ny + least - 1) / least <= PLANE_TY && (per_sm * kSMs + tx - 1) / tx <= ny)
+      return {per_sm, per_sm * kSMs, (ny + least - 1) / least};
   }
   Tiling best{3, 0, 0};
   double bc = 1e300;
   for (int rows = (ny + PLANE_TY - 1) / PLANE_TY; rows <= (ny + 7) / 8; rows++) {
     const int ty = (ny + rows - 1) / rows, load = ((ty + 2) * (TX + 2) + 31) / 32, corner = ((ty + 1) * (TX + 1) + 31) / 32;
-    const double cost = static_cast<double>((tx * rows + PLANE_SMS - 1) / PLANE_SMS) * (2 * load + 17 * corner + 33 * ty);
+    const double cost = static_cast<double>((tx * rows + kSMs - 1) / kSMs) * (2 * load + 17 * corner + 33 * ty);
     if (cost < bc) {
       bc = cost;
       best = {3, tx * rows, ty};
@@ -681,7 +681,7 @@ PlaneEngine::PlaneEngine(const PlaneConfig &c) : p(c) {
   coef.alloc(4);
   for (DevBuf<double> *b : {&h0, &u0, &ha, &ua, &hb, &ub, &ah, &au}) b->alloc(ncell());
   for (DevBuf<double> *b : {&v0, &va, &vb, &av}) b->alloc(nvpt());
-  nblk_red = 2 * 152;
+  nblk_red = 2 * kSMs;
   part.alloc(static_cast<size_t>(nblk_red) * (RED_SUMS + RED_MAXS));
   dred.alloc(1);
   hred.alloc(1);

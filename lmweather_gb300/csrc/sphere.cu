@@ -2145,7 +2145,7 @@ void SphereEngine::autotune_split() {
         // one CTA per work item (persistent CTAs, ana_grid > 0, measured no faster on GB300 and are not tried)
         cands.push_back({2, both, 0, ns, dir, ba, 1e30, 2});
         // the 80-register form only pays where three CTAs fit in shared memory
-        if (3 * (ba + 1024) <= 233472) cands.push_back({2, both, 0, ns, dir, ba, 1e30, 3});
+        if (3 * (ba + 1024) <= kSmemPerSM) cands.push_back({2, both, 0, ns, dir, ba, 1e30, 3});
         // the warp-specialised persistent form (direct operands), one or two CTAs per SM
         if (dir == 1 && ns >= 2)
           for (int ctas = 1; ctas <= 2; ctas++) {

@@ -71,7 +71,7 @@ struct SplitPlan {
   int ana_ws = 0;             // 0: split_ana; 1 or 2: the warp-specialised persistent form with that many CTAs per SM
   int grid_fixed = 1;         // 1: the grid kernel compiled for the transform length (lengths 2^6..2^10); 0: any length
   int syn_ws = 0;             // 0: split_syn; 1 or 2: the warp-specialised persistent synthesis with that many CTAs per SM
-  int nsm = 152;              // multiprocessors of the device (the persistent grid)
+  int nsm = kSMs;              // multiprocessors of the device (the persistent grid)
   int ra_pair = 32;           // largest ra16[2m] + ra16[2m + 1]
   // 1: the linear terms of the tendencies (gravity-wave terms of the mean height, the Laplacian of Phi, the
   // untilted Coriolis terms) added in spectral space, in FP32 from the FP32 stage input; only the nonlinear
@@ -1904,7 +1904,7 @@ inline void build_split_plan(SplitPlan &sp, const HostTables &h, int B, int term
   // latitude pairs per grid CTA: four when that still gives two CTAs per SM
   sp.jb = 1;
   for (int jb = SPLIT_JB_MAX; jb > 1; jb /= 2)
-    if (nh % jb == 0 && static_cast<long>(nh / jb) * B >= 2 * 152) {
+    if (nh % jb == 0 && static_cast<long>(nh / jb) * B >= 2 * kSMs) {
       sp.jb = jb;
       break;
     }
@@ -1971,7 +1971,7 @@ inline bool ws_layout(const SplitPlan &sp, int both, int ns, int ctas, size_t *s
   *slot = static_cast<int>(sl);
   if (2 * bc * ctas > 512) return false;
   if (total > sp.budget_bytes) return false;
-  if (ctas == 2 && 2 * (total + 1024 + 2048) > 233472) return false;
+  if (ctas == 2 && 2 * (total + 1024 + 2048) > kSmemPerSM) return false;
   return ctas == 1 || ctas == 2;
 }
 
@@ -1993,7 +1993,7 @@ inline bool syn_ws_layout(const SplitPlan &sp, int sl, int ns, int ctas, size_t 
   *slot = static_cast<int>(st);
   if (2 * bc * ctas > 512) return false;
   if (total > sp.budget_bytes) return false;
-  if (ctas == 2 && 2 * (total + 1024 + 2048) > 233472) return false;
+  if (ctas == 2 && 2 * (total + 1024 + 2048) > kSmemPerSM) return false;
   return ctas == 1 || ctas == 2;
 }
 

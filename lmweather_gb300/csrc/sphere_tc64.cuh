@@ -588,14 +588,14 @@ inline void build_tc64(Tc64Plan &p, const HostTables &h, const SphDev &d, double
   p.err.alloc(1);
   p.err.p[0] = 0;
   // members per synthesis tile: two share an MMA (its 128 rows) where one each would not fit the SMs at once
-  p.nbt = B > 1 && static_cast<long>(M) * p.nsl * B > 2 * 152 ? 2 : 1;
+  p.nbt = B > 1 && static_cast<long>(M) * p.nsl * B > 2 * kSMs ? 2 : 1;
   p.ntiles = (B + p.nbt - 1) / p.nbt;
   // Table chunks in flight: three where several CTAs share an SM and hide one another's waits, else as many as there are
   // and fit, so that all of them have arrived when the predecessor ends
   const auto stages = [](long ctas, size_t a, size_t stage, int chunks) {
-    const size_t room = 225 * 1024 / static_cast<size_t>(std::max(1l, std::min(2l, (ctas + 151) / 152))) - 1024;
+    const size_t room = 225 * 1024 / static_cast<size_t>(std::max(1l, std::min(2l, (ctas + kSMs - 1) / kSMs))) - 1024;
     const int fit = room > a ? static_cast<int>((room - a) / stage) : 0;
-    return ctas > 2 * 152 ? 3 : std::max(3, std::min({fit, chunks, T64_STAGES}));
+    return ctas > 2 * kSMs ? 3 : std::max(3, std::min({fit, chunks, T64_STAGES}));
   };
   const size_t a_syn = static_cast<size_t>(p.kc_max) * 30 * T64_SBO + 8 * T64_SBO + 256, a_ana = static_cast<size_t>(2) * (p.nhk / 16) * 30 * T64_SBO;
   p.ns = stages(static_cast<long>(M) * p.nsl * p.ntiles, a_syn, static_cast<size_t>(T64_DIG) * p.lrows * 32, p.kc_max);
@@ -605,7 +605,7 @@ inline void build_tc64(Tc64Plan &p, const HostTables &h, const SphDev &d, double
   p.nsa = stages(alone ? 1 : static_cast<long>(M) * B, a_ana, ana_stage, 2 * (p.nhk / 16));
   // 512 threads shorten the digits, the sums and the update of a CTA that shares its SM with at most one other; more CTAs of
   // 256 overlap their phases better (T170 x 4, one CTA per SM: 88.2 us with 256 threads, 82.1 with 512)
-  p.wide = alone || static_cast<long>(M) * B <= 2 * 152;
+  p.wide = alone || static_cast<long>(M) * B <= 2 * kSMs;
   const size_t red_ana = static_cast<size_t>(p.wide ? 4 : 2) * 128 * 33 * sizeof(int) + 16 + static_cast<size_t>(16) * (N + 3) * sizeof(double);
   p.smem_ana = std::max(static_cast<size_t>(p.nsa) * ana_stage + a_ana, red_ana);
   DevBuf<double> P1;

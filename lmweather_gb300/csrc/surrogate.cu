@@ -215,7 +215,7 @@ void gemm(const GemmArgs &g, cudaStream_t s) {
   // so that two tiles share an SM
   const int tiles = (g.M / 128) * (g.N / 128);
   if (wide) stage_launch(mlp_gemm<256, S256>, dim3(g.N / 256, g.M / 128), 128, smem_bytes(256, S256), s, 1, g);
-  else if (tiles <= 152) stage_launch(mlp_gemm<128, S128_ONE>, dim3(g.N / 128, g.M / 128), 128, smem_bytes(128, S128_ONE), s, 1, g);
+  else if (tiles <= kSMs) stage_launch(mlp_gemm<128, S128_ONE>, dim3(g.N / 128, g.M / 128), 128, smem_bytes(128, S128_ONE), s, 1, g);
   else stage_launch(mlp_gemm<128, S128>, dim3(g.N / 128, g.M / 128), 128, smem_bytes(128, S128), s, 1, g);
   g_launches += 1;
 }
