@@ -1388,13 +1388,14 @@ void SphereEngine::set_orography(const double *hs, size_t n, int member) {
 
 // Grids that are handed out, diagnosed or kept as a reference come from plain FP64 sums, which keep the relative accuracy of
 // each wavenumber at each latitude (the sliced sums keep it to the largest coefficient and table value of the row: a T170
-// flow of m = 80 alone had no digit right at the poles). T170, one member: 82 us against 18. The stability limit (`limit`,
-// which needs the maxima alone) takes the synthesis of the stages
+// flow of m = 80 alone had no digit right at the poles). T170, one member: 82 us against 18. The stability limit (`limit`),
+// which needs the maxima alone, takes the synthesis of the stages above 32 latitude pairs (stable_dt at T106: 189 us against
+// 214; at T42 86 against 83, at T21 76.5 against 71.5)
 void SphereEngine::synth_grids(int member_first, int count, bool limit) {
   SphDev d = make_sph(*this, *tab);
   const size_t st = static_cast<size_t>(member_first) * 3 * ntri;
   const size_t fo = static_cast<size_t>(member_first) * nlat * 4 * M;
-  if (limit && tc64) {
+  if (limit && tc64 && nh > 32) {
     syn64_launch(d, tc64_dev(*tc64, ntri + M), tc64->smem_syn(tc64->nbt), count, reinterpret_cast<const double2 *>(x0.p) + st, reinterpret_cast<double2 *>(four.p) + fo, stream);
     g_launches += 1;
     return;
