@@ -1,7 +1,9 @@
 // Programmatic dependent launch: a kernel launched with stage_launch may start while its predecessor drains. It waits in
 // pdl_wait (everything the predecessor wrote is then visible, and the predecessor had waited for its own) before it
-// touches anything an earlier kernel writes, and lets its successor start with pdl_trigger when only its outputs are
-// left. In a kernel launched without the attribute both do nothing.
+// touches anything an earlier kernel writes, and lets its successor start with pdl_trigger (the first thread of a CTA counts
+// for it) when only its outputs are left. The persistent split kernels, whose CTAs are as many on every SM, trigger
+// right after their wait: a successor then takes no SM from CTAs still to come, and it waits for all of them all the
+// same. In a kernel launched without the attribute both do nothing.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -408,7 +408,8 @@ __global__ void __launch_bounds__(GRID_THREADS) sph_grid(SphDev d, SphTab<R> t, 
 // FFT of one row of n = 2^logn complex values, decimation in time from bit-reversed to natural order, in place: one
 // thread per butterfly and component, so that n threads share the chain. x = u + w v takes two FMAs per component and
 // y = u - w v = 2 u - x one, six FP64 operations per butterfly instead of eight; the first two stages, whose twiddles
-// are 1 and +-i, take four. Both components of a butterfly sit in neighbouring lanes of one warp, which reads all
+// are 1 and +-i, take four. (The rounding of x enters y: an FFT's error is 2 to 4 % above that of separate sums, 3.06e-16
+// against 2.99e-16 of the norm at 512 points; a step's error against 64-bit values does not show it.) Both components of a butterfly sit in neighbouring lanes of one warp, which reads all
 // their inputs before it writes. Twiddles: those of stage st at tw[2^st + lo], lo < 2^st,
 // contiguous (from the table's stride they met on one bank).
 constexpr int G64_CTAS = 5;

@@ -10,7 +10,7 @@
 //              B w_d, V Phi w_d at parity 1 - s against H.
 // Three launches per stage:
 //   split_syn     per (m, member tile): H then P through a pipeline of bulk asynchronous copies (cp.async.bulk,
-//                 the TMA engine) into shared memory, MMAs by one thread, accumulators read back with tcgen05.ld
+//                 the TMA engine) into shared memory, MMAs by one converged warp, accumulators read back with tcgen05.ld
 //                 and combined into the Fourier coefficients of U, V, zeta and Phi at both mirror latitudes.
 //   split_grid    per (block of latitude pairs, member): FP32 FFTs and products (the same arithmetic as
 //                 sph_grid<float>), then the folded analysis inputs, stored m-major so that the analysis reads
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(SPLIT_SYN_WS_THREADS, CTAS) split_syn_ws(SphDe
       it++;
     }
   }
-  pdl_trigger();
+  pdl_trigger();  // in effect at once: lanes without a role come here after the wait (see pdl.cuh)
   __syncthreads();
   if (tid == 0) {
     if (!s_fail) {
@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(GRID_THREADS, FMAX < 4 ? 3 : 2) split_grid(Sph
 // as the scalar operation does, so the values are split_grid's bit for bit. The BF16 pieces of two latitudes are
 // rounded by one conversion, and the third pieces only where a plan keeps them. JB = 1 pairs the fields U and V, zeta and
 // Phi. Rows are padded by one element per 16 (sixteen-element groups) or 8 against bank conflicts.
-// T85 x 128: 90.1 -> 78.8 us; T42 x 384: 59.4 -> 56.7; T21 x 512: 26.6 -> 16.6; T106 x 18 (three pieces): 65.6 -> 53.6.
+// T85 x 128: 90.1 -> 80.7 us; T42 x 384: 59.4 -> 56.7; T21 x 512: 26.6 -> 16.6; T106 x 18 (three pieces): 65.6 -> 53.6.
 __device__ __forceinline__ uint64_t pk(float a, float b) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -1514,6 +1514,7 @@ __global__ void __launch_bounds__(SPLIT_ANA_THREADS, MINB) split_ana(SphDev d, S
   calls++;
   }
   const uint32_t tmem = tslot;
+  // one item per CTA: its update is left
   if (m_slowest) pdl_trigger();
   // accumulators -> shared memory [row][ld + 1] (the operand and pipeline buffers are free now); the odd row
   // stride puts the rows that one warp writes at once on different banks
@@ -1552,7 +1553,7 @@ __global__ void __launch_bounds__(SPLIT_ANA_THREADS, MINB) split_ana(SphDev d, S
 // epilogue runs while the next item's operands load and multiply: thread 0 streams the H and P chunks of the CTA's
 // items (m, parity or both, member tile) through a ring of ns fixed-size stages; warp 1 issues the MMAs of item i
 // into tensor-memory accumulator buffer i % 2 and commits it to accf[i % 2]; warps 2..9 (256 threads) wait for it,
-// copy it to shared memory, release the buffer (acce[i % 2]) and run the epilogue (ana_coef, the same arithmetic as
+// copy it to shared memory, release the buffer (acce[i % 2]) and run the epilogue (ana_load and ana_update, the same arithmetic as
 // split_ana). Items are dealt by snake_item. Every wait is bounded; after a failure each role stops,
 // the CTA drains its own copies and MMAs and frees its tensor memory.
 template <bool BOTH, int CTAS>
@@ -1755,7 +1756,7 @@ __global__ void __launch_bounds__(SPLIT_WS_THREADS, CTAS) split_ana_ws(SphDev d,
       it++;
     }
   }
-  pdl_trigger();
+  pdl_trigger();  // in effect at once: lanes without a role come here after the wait (see pdl.cuh)
   __syncthreads();
   if (tid == 0) {
     // every MMA issued has finished (and its arrivals landed) before the CTA releases its memory; after a failure the

@@ -7,9 +7,16 @@
 // eight digits of seven bits (d_0 up to 128, the others -64..63), which BF16 holds exactly. The products of two digits
 // summed over a row of at most 172 coefficients or 128 latitudes, for all digit pairs (i, j) of one order s = i + j, stay
 // below 2^23, so the FP32 accumulators of tcgen05 hold them exactly. The eight orders s = 0..7 are then added as 64-bit
-// integers and rounded once. What is left out, the digits below 2^-57 of a row's largest element and the orders from 8
-// on (2^-55 of the largest product), is below FP64's own rounding of such a sum, and the result depends neither on
-// the order of summation nor on how members are batched. A row with an infinity or NaN gives NaN.
+// integers and rounded once: a sum of K products of rows below 2^ea and 2^eb is within 1.4 K 2^-55 2^(ea + eb) and one rounding
+// of the exact one (each operand rounded by 2^-57 of its row, the orders from 8 on left out), and depends neither on the
+// order of summation nor on how members are batched. A row with an infinity or NaN gives NaN.
+// That is a bound by norm, by the largest coefficient and the largest table value of a row. Of a wavenumber's largest value the
+// error is 0.04e-15 to 0.9e-15 (T170, spectra from flat to n^-3; plain FP64 sums 0.06e-15 to 1.7e-15). A value far below it, as a
+// high wavenumber has towards the poles where its large coefficients meet table values far below the row's largest,
+// keeps fewer digits than a plain sum would give it, or none. A stage adds such values to those of all other
+// wavenumbers in an FFT, whose rounding is by norm as well, and its sums over latitudes are dominated by the others: the
+// error of a step against 64-bit values is that of plain sums (T21 to T170, eight states each, to three digits). What
+// is handed out as a grid takes plain sums (SphereEngine::synth_grids).
 //
 // All orders of one table digit j come from one MMA: A holds digit i of its rows in row block i, under seven blocks of
 // zeros, and for table digit j the MMA starts j blocks higher, which puts digit i into row block i + j of the accumulator.

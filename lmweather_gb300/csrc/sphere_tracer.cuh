@@ -1,6 +1,7 @@
 // Passive tracer q on the FP64 path (included by sphere.cu): the reference's tracer tendency
 // dq = A(q delta) - D(U q, V q) (cpp/sphere.cpp:250-263), i.e. -v . grad q, advanced by the same RK4 stages as the
-// flow and filtered with Phi's del^4 factor. Three kernels per stage beside the flow's three:
+// flow and filtered with Phi's del^4 factor. Up to T170 the flow's kernels carry it (sphere_tc64.cuh, sph_grid64); above, three
+// kernels per stage beside the flow's three. trc_synth also forms the tracer's grids, at every truncation:
 //   trc_synth     per (m, 32 latitudes): Fourier coefficients of q and delta at both mirror latitudes
 //   trc_grid      per latitude pair: U, V (from the flow's synthesis), q, delta -> inverse FFTs -> U q, V q, q delta
 //                 -> forward FFTs -> weighted, folded analysis inputs

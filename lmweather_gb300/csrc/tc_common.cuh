@@ -76,12 +76,6 @@ __device__ __forceinline__ uint32_t idesc_m128(int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma(uint32_t dtmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dtmem), "l"(ad),
-               "l"(bd), "r"(idesc), "r"(accumulate)
-               : "memory");
-}
-
 // The MMA role is a whole warp whose control flow is uniform, with the instruction predicated on one elected lane:
 // descriptors and addresses then stay in uniform registers, where the instruction takes them from. Issued by a lone
 // thread of a divergent branch, each MMA took about 115 cycles whatever its size.
@@ -101,9 +95,6 @@ __device__ __forceinline__ void commit(bool leader, uint32_t bar) {
   asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar),
                "r"(static_cast<uint32_t>(leader))
                : "memory");
-}
-__device__ __forceinline__ void commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
