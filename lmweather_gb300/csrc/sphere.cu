@@ -30,7 +30,7 @@ struct SphereTables {
   HostTables host;
   DevBuf<double> Ps, Hs, Pa, Ha;  // coefficient-major [tri][jh] (synthesis) and latitude-major [jh][tri] (analysis)
   DevBuf<double> mu, w, wd, cosl, r2om, kfac, lapl;
-  DevBuf<double2> tw;
+  DevBuf<double2> tw, ff;         // exp(-2 pi i k / nlon), k < nlon/2; factors of the FP64 grid stage's FFTs
   // FP32 copies for the reduced-precision stage kernels
   DevBuf<float> Ps32, Hs32, Pa32, Ha32, w32, wd32, r2om32, kfac32, lapl32;
   DevBuf<float2> tw32;  // exp(-2 pi i k / nlon), k < nlon/2
@@ -406,24 +406,15 @@ __global__ void __launch_bounds__(GRID_THREADS) sph_grid(SphDev d, SphTab<R> t, 
 // distributed shared memory, one of the five products and its forward transform.
 //
 // FFT of one row of n = 2^logn complex values, decimation in time from bit-reversed to natural order, in place: one
-// thread per butterfly and component, so that n threads share the chain. x = u + w v takes two FMAs per component and
-// y = u - w v = 2 u - x one, six FP64 operations per butterfly instead of eight; the first two stages, whose twiddles
-// are 1 and +-i, take four. (The rounding of x enters y: an FFT's error is 2 to 4 % above that of separate sums, 3.06e-16
-// against 2.99e-16 of the norm at 512 points; a step's error against 64-bit values does not show it.) Both components of a butterfly sit in neighbouring lanes of one warp, which reads all
-// their inputs before it writes. Twiddles: those of stage st at tw[2^st + lo], lo < 2^st,
-// contiguous (from the table's stride they met on one bank).
+// thread per butterfly and component (fft64.cuh: six FP64 operations per butterfly, four in the first two stages), so that n threads
+// share the chain. Both components of a butterfly sit in neighbouring lanes of one warp, which reads all their inputs
+// before it writes. Factors: those of stage st at tw[2^st + lo], lo < 2^st, contiguous (from a table's stride
+// they met on one bank).
 constexpr int G64_CTAS = 5;
 __host__ __device__ constexpr int g64_threads(int n) { return n < 32 ? 32 : n < 256 ? n : 256; }
 
-__device__ __forceinline__ void fft64_twiddles(double2 *tw, int logn, const double2 *__restrict__ table) {
-  for (int e = threadIdx.x; e < 1 << logn; e += blockDim.x) {
-    const int st = 31 - __clz(e | 1);
-    tw[e] = table[(e - (1 << st)) << (logn - 1 - st) & ((1 << (logn - 1)) - 1)];
-  }
-}
-// -x or x, on the integer pipe: the compiler's negation by a condition was an FP64 operation (T170 grid: 61.9 -> 48.3 us)
-__device__ __forceinline__ double flip(double x, bool neg) {
-  return __hiloint2double(__double2hiint(x) ^ (neg ? static_cast<int>(0x80000000u) : 0), __double2loint(x));
+__device__ __forceinline__ void fft64_load(double2 *tw, int n, const double2 *__restrict__ factors) {
+  for (int e = threadIdx.x; e < n; e += blockDim.x) tw[e] = factors[e];
 }
 template <bool INV> __device__ __forceinline__ void fft64(double2 *s, int logn, const double2 *tw) {
   const int n = 1 << logn;
@@ -435,18 +426,7 @@ template <bool INV> __device__ __forceinline__ void fft64(double2 *s, int logn, 
       const double u = *us;
       const double2 v = s[i0 + h];
       double x, y;
-      if (st < 2) {
-        // w = 1, or for the odd butterflies of stage 1 +i (inverse) or -i: i v = (-v.y, v.x)
-        const double ts = flip(lo == 0 ? (c ? v.y : v.x) : (c ? v.x : v.y), lo != 0 && (c == 0) == INV);
-        x = u + ts;
-        y = u - ts;
-      } else {
-        // component c of w v (w conjugated for the inverse): w.x v.x - w.y v.y or w.x v.y + w.y v.x
-        const double2 w = tw[h + lo];
-        const double a = c ? v.y : v.x, b = c ? v.x : v.y, wi = flip(w.y, (c != 0) == INV);
-        x = fma(w.x, a, fma(wi, b, u));
-        y = fma(2.0, u, -x);
-      }
+      fft64_butterfly<INV>(st, lo, c, u, v, tw, x, y);
       __syncwarp(n < 32 ? (1u << n) - 1u : 0xffffffffu);
       *us = x;
       *ys = y;
@@ -500,8 +480,8 @@ __device__ __forceinline__ void g64_fold(const double2 *s, const SphDev &d, doub
   }
 }
 
-// grid: (CTAS nh, B), clusters of CTAS along x. T42, one member: 22.5 -> 7.2 us; T170: 64.5 -> 48.3 us; T42 x 16:
-// 57.4 -> 41.5 us
+// grid: (CTAS nh, B), clusters of CTAS along x. T42, one member: 22.5 -> 7.3 us; T170: 64.5 -> 47.1 us; T42 x 16:
+// 57.4 -> 40.6 us
 // CTAS = 8: with the tracer, whose q and delta (fourq [B][nlat][2][M]) are two more inverse transforms and U q, V q and q delta
 // three more products (foldq [B][nh][3][2][M]).
 template <int CTAS>
@@ -514,7 +494,7 @@ __global__ void __launch_bounds__(256) sph_grid64(SphDev d, SphTab<double> t, co
   double2 *inv = g64_sm, *fwd = g64_sm + n, *tw = g64_sm + 2 * n;
   const int r = static_cast<int>(cluster_rank()), jh = blockIdx.x / CTAS, b = blockIdx.y;
   const int js = jh, jn = d.nlat - 1 - jh;
-  fft64_twiddles(tw, d.logn, t.tw);
+  fft64_load(tw, n, d.ff);
   if (r < FIELDS)
     for (int e = threadIdx.x; e < n; e += blockDim.x) inv[e] = make_double2(0.0, 0.0);
   const int gf = d.gflag[b];
@@ -1111,6 +1091,7 @@ static SphDev make_sph(const SphereEngine &e, const SphereTables &t) {
   d.kfac = t.kfac.p;
   d.lapl = t.lapl.p;
   d.tw = t.tw.p;
+  d.ff = t.ff.p;
   d.trim = t.trim.p;
   d.trin = t.trin.p;
   d.gflag = e.gflag.p;
@@ -1230,6 +1211,14 @@ SphereEngine::SphereEngine(const SphereConfig &c) : p(c) {
   }
   tab->tw.alloc(tw.size());
   copy_in(tab->tw.p, tw.data(), tw.size() * sizeof(double2), stream);
+  if (p.precision == kFP64) {
+    std::vector<double> ff(2 * static_cast<size_t>(nlon));
+    int logn = 0;
+    while ((1 << logn) < nlon) logn++;
+    fft64_factors(logn, ff.data());
+    tab->ff.alloc(nlon);
+    copy_in(tab->ff.p, ff.data(), ff.size() * sizeof(double), stream);
+  }
   if (p.precision != kFP64) {
     auto up32 = [&](DevBuf<float> &dst, const std::vector<double> &src) {
       std::vector<float> f(src.begin(), src.end());

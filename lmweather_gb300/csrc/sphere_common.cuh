@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fft64.cuh"
 #include "pdl.cuh"
 
 namespace lmw {
@@ -11,7 +12,7 @@ struct SphDev {
   int N, M, nlat, nlon, nh, ntri, logn;
   double a, g;
   const double *Ps, *Hs, *Pa, *Ha, *mu, *w, *wd, *cosl, *r2om, *kfac, *lapl;
-  const double2 *tw;
+  const double2 *tw, *ff;
   const int *trim, *trin, *tri;
   // per member: bit 0 = the Coriolis grid is tilted (read fgrid, else f = om2 mu), bit 1 = orography (read hsgrid)
   const int *gflag;

@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) trc_grid(SphDev d, SphTab<double> t, cons
   double2 *inv = g64_sm, *fwd = g64_sm + n, *tw = g64_sm + 2 * n;
   const int r = static_cast<int>(cluster_rank()), jh = blockIdx.x / TRC_CTAS, b = blockIdx.y;
   const int js = jh, jn = d.nlat - 1 - jh;
-  fft64_twiddles(tw, d.logn, t.tw);
+  fft64_load(tw, n, d.ff);
   for (int e = threadIdx.x; e < n; e += blockDim.x) inv[e] = make_double2(0.0, 0.0);
   const double wt = r < 2 ? t.wd[js] : t.w[js];
   __syncthreads();
