@@ -15,8 +15,8 @@
 // high wavenumber has towards the poles where its large coefficients meet table values far below the row's largest,
 // keeps fewer digits than a plain sum would give it, or none. A stage adds such values to those of all other
 // wavenumbers in an FFT, whose rounding is by norm as well, and its sums over latitudes are dominated by the others: against
-// extended precision the error of each wavenumber after two steps is 0.88 to 1.02 of that with plain sums and radix-2 FFTs for
-// delta and Phi, 0.56 to 1.02 for zeta (T21 to T106; a small perturbation of a zonal flow, steep and flat spectra). What is
+// extended precision the error of each wavenumber after two steps is 0.86 to 1.02 of that with plain sums and radix-2 FFTs for
+// delta and Phi, 0.56 to 1.02 for zeta (T21 to T170; a small perturbation of a zonal flow, steep and flat spectra). What is
 // handed out as a grid takes plain sums (SphereEngine::synth_grids).
 //
 // All orders of one table digit j come from one MMA: A holds digit i of its rows in row block i, under seven blocks of
